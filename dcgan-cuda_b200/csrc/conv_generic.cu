@@ -1,14 +1,18 @@
-// CUDA-core fp32 convolution kernels for arbitrary shapes (DCG_PREC_FP32).
+// CUDA-core fp32 convolution kernels (DCG_PREC_FP32, and every shape the tensor path cannot take).
 //
-// These play the role of the reference's naive kernels (src/gpu/conv2d_naive.hh:
-// one thread per output element) and are the path every shape the tensor-core
-// kernels cannot take falls back to.  They are written for exactness, not speed:
-// each output is accumulated in the order the reference's CPU code uses, with
-// unfused IEEE multiplies and adds, so the results are bit-comparable with
-// src/cpu/ops.hxx:
+// They are written for exactness first: each output is accumulated in the order the reference's CPU code
+// uses, with unfused IEEE multiplies and adds, so the results are bit-comparable with src/cpu/ops.hxx:
 //   forward      : one accumulator over (channel, kernel row, kernel column), ops.hxx:227-246
 //   input grad   : per output filter an inner sum over taps, filters added in order, ops.hxx:650-679
 //   kernel grad  : per image an inner sum over output pixels, images added in order, ops.hxx:754-772
+// Within that order there is no K split; what is free is how the outputs are spread over threads and how
+// the operands reach them.  conv_ordered_fwd_kernel, conv_ordered_dx_kernel (by parity class) and
+// conv_ordered_dk_kernel are register-tiled GEMMs on operand tiles that cp.async gathers straight from the
+// NHWC / HWIO tensors; the conv_*_generic kernels further down (one thread per output, as
+// src/gpu/conv2d_naive.hh) remain for kernels with more than kOrdMaxTaps taps, whose tiles would not fit.
+#include <mutex>
+#include <type_traits>
+
 #include "common.cuh"
 #include "conv.cuh"
 
@@ -17,6 +21,628 @@ namespace {
 
 constexpr int kThreads = 128;
 
+constexpr int kOrdSmem = 227 * 1024;
+constexpr int kOrdMaxTaps = 25;   // taps of one accumulation chain: bounds the operand tiles in shared memory
+
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// W consecutive floats of an operand tile
+template <int W>
+__device__ __forceinline__ void lds_vec(const float* s, float (&v)[W])
+{
+    if constexpr (W == 1) {
+        v[0] = *s;
+    } else if constexpr (W == 2) {
+        const float2 t = *reinterpret_cast<const float2*>(s);
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        static_assert(W == 4, "1, 2 or 4 floats");
+        const float4 t = *reinterpret_cast<const float4*>(s);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
+}
+
+// ---- forward and input gradient as ordered implicit GEMMs -----------------------------------------------
+// out[pixel, channel] over K = (contracted channel q outermost, tap innermost), the reference's loop nest.
+// An operand whose contracted channel is its contiguous axis (x, dy, and the weights of the input gradient) is
+// gathered sixteen bytes - four channels of one (row, tap) - at a time with cp.async and kept as it comes:
+// [row][channel quad][tap][4], row pitch 4 mod 8 words so that eight rows start in different bank quads.  The
+// weights of the forward are rows of output channels, [q][tap][channel].  Taps outside the image are zero-filled,
+// which adds +0 where the reference skips: the same bits.  Two stages of QC channels x all taps.
+// Bound by issue (the sum must stay unfused: two instructions per product; packed f32x2 arithmetic was measured
+// and is no faster, its operands have to be duplicated) and, where the outputs are few, by the latency of the
+// chain of dependent adds.  Measured, 5x5 / stride 2 layers: 18 TFLOP/s (a multiply and an add counted as two) of the
+// 37 that 148 x 128 lanes issue where a 4 x 4 thread tile is used, 7-11 at batch 8; the 256 -> 512 forward of 8
+// images takes 122 us, one thread per output took 2.5 ms; a training iteration at batch 8 6.2 ms against 89.7.
+struct OrdGeom {      // one class of output pixels and what its taps read
+    int mh, mw;       // pixels of the class
+    int SH, SW, SC;   // the source tensor
+    int Th, Tw;       // taps
+    int eh, ew, sh, sw;   // source row of (pixel row i, tap row a): i * sh + eh + a
+};
+
+constexpr int kOrdQuads = 25;   // 16-byte words of one operand row in a stage: taps x channel quads, at most
+
+// What one thread copies of a channel-contiguous operand tile in every stage: (row, quad, tap) items tid, tid + THREADS, ...
+// Their places do not change from stage to stage - a stage only moves the channel on - so they are worked out once.
+template <int ROWS, int THREADS>
+struct Gather {
+    static constexpr int ITEMS = (ROWS * kOrdQuads + THREADS - 1) / THREADS;
+    int off[ITEMS];   // element offset of channel 0 of the item's quad, -1: zero-fill, -2: no item
+    // src_off(row, tap): element offset of channel 0, or -1
+    template <typename F>
+    __device__ __forceinline__ void plan(int T, int quads, F src_off)
+    {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const int idx = threadIdx.x + i * THREADS, row = idx % ROWS, tq = idx / ROWS;
+            off[i] = -2;
+            if (tq < T * quads) {
+                const int g = tq / T, o = src_off(row, tq - g * T);
+                off[i] = o < 0 ? -1 : o + 4 * g;
+            }
+        }
+    }
+    __device__ __forceinline__ void load(uint32_t dst, int pitch, int T, const float* src, int q0, int qc, int SC, bool vec) const
+    {
+        const bool tail = q0 + qc > SC;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            if (off[i] == -2) continue;
+            const int idx = threadIdx.x + i * THREADS, row = idx % ROWS, tq = idx / ROWS;
+            const uint32_t d = dst + 4u * (uint32_t)(row * pitch + 4 * tq);
+            const int left = tail ? SC - q0 - 4 * (tq / T) : 4;   // channels of this quad that exist
+            const bool in = off[i] >= 0;
+            const float* s = src + (in ? off[i] + q0 : 0);
+            if (vec) {
+                cp_async16(d, s, in && left > 0);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) cp_async4(d + 4u * u, s + u, in && u < left);
+            }
+        }
+    }
+};
+
+// Pixel rows of the A operand.
+template <int ROWS, int THREADS>
+__device__ __forceinline__ void gather_pixels(Gather<ROWS, THREADS>& ga, const OrdGeom& g, int quads, long long m0, long long pixels)
+{
+    ga.plan(g.Th * g.Tw, quads, [&](int row, int tap) {
+        const long long p = m0 + row;
+        if (p >= pixels) return -1;
+        const int j = (int)(p % g.mw);
+        const long long t = p / g.mw;
+        const int a = tap / g.Tw, r = (int)(t % g.mh) * g.sh + g.eh + a, c = j * g.sw + g.ew + tap - a * g.Tw;
+        if (r < 0 || r >= g.SH || c < 0 || c >= g.SW) return -1;
+        return (int)((((t / g.mh) * g.SH + r) * g.SW + c) * g.SC);
+    });
+}
+
+__host__ __device__ constexpr int ord_pitch(int tile) { return tile + 4; }
+__host__ __device__ constexpr int ord_row_pitch(int taps, int qc) { return taps * qc % 8 == 0 ? taps * qc + 4 : taps * qc; }
+
+template <int TM, int TN, int TX, int TY, int U>   // U divides the number of taps
+__global__ void __launch_bounds__(TX * TY)
+conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k, float* __restrict__ y,
+                        const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec_a, const int vec_b)
+{
+    constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY, LDB = ord_pitch(BNT);
+    extern __shared__ __align__(16) float smem[];
+    pdl_enter();
+    const OrdGeom g{d.ho, d.wo, d.h, d.w, d.c, d.kh, d.kw, -d.pad_top, -d.pad_left, d.stride_h, d.stride_w};
+    const int T = d.kh * d.kw, tid = threadIdx.x;
+    const long long pixels = (long long)d.n * d.ho * d.wo, m0 = (long long)blockIdx.x * BMT;
+    const int n0 = blockIdx.y * BNT;
+    const int pitch = ord_row_pitch(T, QC), stage = BMT * pitch + QC * T * LDB;
+    const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(smem);
+    Gather<BMT, THREADS> ga;
+    gather_pixels(ga, g, QC >> 2, m0, pixels);
+    // weights: rows (q, tap) of output channels, sixteen bytes at a time where the channel count allows
+    constexpr int COLS = BNT / 4, BITEMS = (4 * kOrdQuads * COLS + THREADS - 1) / THREADS;
+    int boff[BITEMS];
+#pragma unroll
+    for (int i = 0; i < BITEMS; ++i) {
+        const int idx = tid + i * THREADS, nn = 4 * (idx % COLS), r = idx / COLS, q = r / T;
+        boff[i] = r < QC * T && n0 + nn < d.o ? ((r - q * T) * d.c + q) * d.o + n0 + nn : -1;
+    }
+    auto load_stage = [&](int q0, int buf) {
+        const uint32_t as = smem0 + 4u * (uint32_t)(buf * stage), bs = as + 4u * (uint32_t)(BMT * pitch);
+        ga.load(as, pitch, T, x, q0, QC, d.c, vec_a);
+        if (vec_b) {
+            const int rows = min(QC, d.c - q0) * T;
+#pragma unroll
+            for (int i = 0; i < BITEMS; ++i) {
+                const int idx = tid + i * THREADS, r = idx / COLS;
+                if (r < rows) cp_async16(bs + 4u * (uint32_t)(r * LDB + 4 * (idx % COLS)), k + (boff[i] < 0 ? 0 : boff[i] + q0 * d.o), boff[i] >= 0);
+            }
+        } else {
+            for (int idx = tid; idx < min(QC, d.c - q0) * T * BNT; idx += THREADS) {
+                const int nn = idx % BNT, r = idx / BNT, q = r / T;
+                const bool in = n0 + nn < d.o;
+                cp_async4(bs + 4u * (uint32_t)(r * LDB + nn), in ? k + ((long long)(r - q * T) * d.c + q0 + q) * d.o + n0 + nn : k, in);
+            }
+        }
+        cp_async_commit();
+    };
+
+    const int tx = tid % TX, ty = tid / TX;
+    float acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    load_stage(0, 0);
+    int buf = 0;
+    for (int q0 = 0; q0 < d.c; q0 += QC, buf ^= 1) {
+        if (q0 + QC < d.c) load_stage(q0 + QC, buf ^ 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* as = smem + buf * stage + ty * pitch;
+        const float* bs = smem + buf * stage + BMT * pitch + tx * TN;
+        const int qn = min(QC, d.c - q0);
+        for (int q = 0; q < qn; ++q) {
+            const float* ap[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) ap[i] = as + i * TY * pitch + 4 * T * (q >> 2) + (q & 3);
+            for (int t = 0; t < T; t += U, bs += U * LDB) {
+                // operands and products of U taps first: only the adds form a chain
+                float a[U][TM][1], b[U][TN];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+#pragma unroll
+                    for (int i = 0; i < TM; ++i) lds_vec<1>(ap[i] + 4 * u, a[u][i]);
+                    lds_vec<TN>(bs + u * LDB, b[u]);
+                }
+#pragma unroll
+                for (int i = 0; i < TM; ++i) ap[i] += 4 * U;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(a[u][i][0], b[u][j]));
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const long long p = m0 + ty + i * TY;
+        if (p >= pixels) continue;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int ch = n0 + tx * TN + j;
+            if (ch >= d.o) continue;
+            const size_t idx = (size_t)p * d.o + ch;
+            y[idx] = epilogue_apply(ep, acc[i][j], idx, ch);
+        }
+    }
+}
+
+// Input gradient: the taps of one filter are summed first, the filters' sums added in order - so four filters at a time
+// are four independent chains, read as 16-byte words of both operands.  Each parity class of output pixels
+// (blockIdx.z) runs by itself: only taps that meet a dy pixel exist.
+template <int TM, int TN, int TX, int TY>
+__global__ void __launch_bounds__(TX * TY)
+conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k, float* __restrict__ dx,
+                       const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec)
+{
+    constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY;
+    extern __shared__ __align__(16) float smem[];
+    pdl_enter();
+    const int ph = blockIdx.z / d.stride_w, pw = blockIdx.z % d.stride_w, tid = threadIdx.x;
+    const int P = d.kh - 1 - d.pad_top, Q = d.kw - 1 - d.pad_left;
+    int r0h = (P - ph) % d.stride_h, r0w = (Q - pw) % d.stride_w;   // first tap (in flipped order) of this class
+    if (r0h < 0) r0h += d.stride_h;
+    if (r0w < 0) r0w += d.stride_w;
+    OrdGeom g;
+    g.mh = (d.h - ph + d.stride_h - 1) / d.stride_h; g.mw = (d.w - pw + d.stride_w - 1) / d.stride_w;
+    g.SH = d.ho; g.SW = d.wo; g.SC = d.o;
+    g.Th = r0h < d.kh ? (d.kh - 1 - r0h) / d.stride_h + 1 : 0;
+    g.Tw = r0w < d.kw ? (d.kw - 1 - r0w) / d.stride_w + 1 : 0;
+    g.eh = (ph + r0h - P) / d.stride_h; g.ew = (pw + r0w - Q) / d.stride_w;   // exact divisions
+    g.sh = g.sw = 1;
+    const int T = g.Th * g.Tw;
+    const long long pixels = (long long)d.n * g.mh * g.mw, m0 = (long long)blockIdx.x * BMT;
+    if (m0 >= pixels) return;
+    const int n0 = blockIdx.y * BNT;
+    const int pitch = ord_row_pitch(T, QC), stage = (BMT + BNT) * pitch;
+    const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(smem);
+    Gather<BMT, THREADS> ga;
+    Gather<BNT, THREADS> gb;
+    if (T > 0) {
+        gather_pixels(ga, g, QC >> 2, m0, pixels);
+        gb.plan(T, QC >> 2, [&](int row, int tap) {
+            const int a = tap / g.Tw, c = n0 + row;
+            const int kt = (d.kh - 1 - r0h - d.stride_h * a) * d.kw + d.kw - 1 - r0w - d.stride_w * (tap - a * g.Tw);
+            return c < d.c ? (kt * d.c + c) * d.o : -1;
+        });
+    }
+    auto load_stage = [&](int q0, int buf) {
+        const uint32_t as = smem0 + 4u * (uint32_t)(buf * stage);
+        ga.load(as, pitch, T, dy, q0, QC, d.o, vec);
+        gb.load(as + 4u * (uint32_t)(BMT * pitch), pitch, T, k, q0, QC, d.o, vec);
+        cp_async_commit();
+    };
+    const int tx = tid % TX, ty = tid / TX;
+    float tot[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) tot[i][j] = 0.f;
+    if (T > 0) {
+        load_stage(0, 0);
+        int buf = 0;
+        for (int q0 = 0; q0 < d.o; q0 += QC, buf ^= 1) {
+            if (q0 + QC < d.o) load_stage(q0 + QC, buf ^ 1);
+            else cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+            const float *as[TM], *bs[TN];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) as[i] = smem + buf * stage + (ty + i * TY) * pitch;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) bs[j] = smem + buf * stage + (BMT + tx + j * TX) * pitch;
+            const int quads = min(QC, d.o - q0 + 3) >> 2;
+            auto chunk = [&](auto taps_c) {
+                constexpr int TC = decltype(taps_c)::value;   // taps at compile time, 0: run time
+                for (int q = 0; q < quads; ++q) {
+                    float val[TM][TN][4];
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) val[i][j][0] = val[i][j][1] = val[i][j][2] = val[i][j][3] = 0.f;
+                    // U taps: operands first, then their products and sums
+                    auto taps = [&](auto u_c) {
+                        constexpr int U = decltype(u_c)::value;
+                        float a[U][TM][4], b[U][TN][4];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+#pragma unroll
+                            for (int i = 0; i < TM; ++i) lds_vec<4>(as[i] + 4 * u, a[u][i]);
+#pragma unroll
+                            for (int j = 0; j < TN; ++j) lds_vec<4>(bs[j] + 4 * u, b[u][j]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < TM; ++i) as[i] += 4 * U;
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) bs[j] += 4 * U;
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+#pragma unroll
+                            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                                for (int j = 0; j < TN; ++j)
+#pragma unroll
+                                    for (int f = 0; f < 4; ++f)
+                                        val[i][j][f] = __fadd_rn(val[i][j][f], __fmul_rn(a[u][i][f], b[u][j][f]));
+                    };
+                    if constexpr (TC > 0) {
+#pragma unroll
+                        for (int t = 0; t + 1 < TC; t += 2) taps(std::integral_constant<int, 2>());
+                        if constexpr (TC % 2 != 0) taps(std::integral_constant<int, 1>());
+                    } else {
+                        for (int t = 0; t < T; ++t) taps(std::integral_constant<int, 1>());
+                    }
+                    // filters beyond the last are zero-filled: they add +0
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int i = 0; i < TM; ++i)
+#pragma unroll
+                            for (int j = 0; j < TN; ++j) tot[i][j] = __fadd_rn(tot[i][j], val[i][j][u]);
+                }
+            };
+            switch (T) {   // the classes of 5 x 5 / stride 2 (and 3 x 3): taps unrolled
+            case 4: chunk(std::integral_constant<int, 4>()); break;
+            case 6: chunk(std::integral_constant<int, 6>()); break;
+            case 9: chunk(std::integral_constant<int, 9>()); break;
+            default: chunk(std::integral_constant<int, 0>()); break;
+            }
+            __syncthreads();
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const long long p = m0 + ty + i * TY;
+        if (p >= pixels) continue;
+        const int jj = (int)(p % g.mw);
+        const long long t = p / g.mw;
+        const size_t pix = ((size_t)(t / g.mh) * d.h + (size_t)(t % g.mh) * d.stride_h + ph) * d.w + (size_t)jj * d.stride_w + pw;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int ch = n0 + tx + j * TX;
+            if (ch >= d.c) continue;
+            const size_t idx = pix * d.c + ch;
+            dx[idx] = epilogue_apply(ep, tot[i][j], idx, ch);
+        }
+    }
+}
+
+// ---- kernel gradient as an ordered GEMM -------------------------------------------------------------------
+// dk[(tap, c), o] over K = (image outermost, output pixel innermost): the pixels of an image are summed
+// first, the images' sums added in order.  Rows are (tap, channel) pairs, so a 3-channel layer fills its
+// tiles as well as a 256-channel one.  Both operands are contiguous along the tile axes: a stage is KP pixels,
+// A as [pixel][row] (16-byte copies where the channel count allows), B as [pixel][filter].  GROUPS thread groups
+// of a block take every GROUPS-th image each and hand their sums over in shared memory, where the first group adds
+// them in image order: more of the GPU for layers with few weights, same bits.
+template <int TM, int TN, int TX, int TY, int GROUPS>
+__global__ void __launch_bounds__(TX * TY * GROUPS)
+conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dk,
+                       const dcg_conv_desc d, const int vec_a, const int vec_b)
+{
+    constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY, KP = 32, LDA = ord_pitch(BMT), LDB = ord_pitch(BNT);
+    constexpr int STAGE = KP * (LDA + LDB);
+    extern __shared__ __align__(16) float smem[];
+    pdl_enter();
+    const int group = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
+    const int M = d.kh * d.kw * d.c, P = d.ho * d.wo;
+    const int m0 = blockIdx.x * BMT, n0 = blockIdx.y * BNT;
+    float* mine = smem + group * 2 * STAGE;
+    const uint32_t mine0 = (uint32_t)__cvta_generic_to_shared(mine);
+    // gather roles: one row quad (or row) of A and one filter quad (or filter) of B, every few pixels
+    const int aw = vec_a ? 4 : 1, bw = vec_b ? 4 : 1;
+    const int acols = BMT / aw, bcols = BNT / bw;
+    const int ac = (tid % acols) * aw, ar0 = tid / acols, arstep = THREADS / acols;
+    const int bc = (tid % bcols) * bw, br0 = tid / bcols, brstep = THREADS / bcols;
+    const int m = m0 + ac;
+    const bool m_in = m < M, o_in = n0 + bc < d.o;
+    const int c = m % d.c, tap = m / d.c, dh = (tap / d.kw) - d.pad_top, dw = (tap % d.kw) - d.pad_left;
+    auto load_stage = [&](int n, int p0, int buf) {
+        if (n < d.n) {
+            const uint32_t as = mine0 + 4u * (uint32_t)(buf * STAGE), bs = as + 4u * (uint32_t)(KP * LDA);
+            const int rows = min(KP, P - p0);
+            int r = ar0, a = (p0 + ar0) / d.wo, b = (p0 + ar0) % d.wo;
+            const float* xn = x + (long long)n * d.h * d.w * d.c + c;
+            for (; r < rows; r += arstep) {
+                const int h = d.stride_h * a + dh, w = d.stride_w * b + dw;
+                const bool in = m_in && h >= 0 && h < d.h && w >= 0 && w < d.w;
+                const float* s = in ? xn + ((long long)h * d.w + w) * d.c : x;
+                const uint32_t dst = as + 4u * (uint32_t)(r * LDA + ac);
+                if (vec_a) cp_async16(dst, s, in);
+                else cp_async4(dst, s, in);
+                b += arstep;
+                while (b >= d.wo) { b -= d.wo; ++a; }
+            }
+            const float* g = dy + ((long long)n * P + p0) * d.o + n0 + bc;
+            for (r = br0; r < rows; r += brstep) {
+                const float* s = o_in ? g + (long long)r * d.o : dy;
+                const uint32_t dst = bs + 4u * (uint32_t)(r * LDB + bc);
+                if (vec_b) cp_async16(dst, s, o_in);
+                else cp_async4(dst, s, o_in);
+            }
+        }
+        cp_async_commit();
+    };
+    const int tx = tid % TX, ty = tid / TX;
+    float val[TM][TN], tot[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) val[i][j] = tot[i][j] = 0.f;
+    const int rounds = (d.n + GROUPS - 1) / GROUPS, chunks = (P + KP - 1) / KP;
+    load_stage(group, 0, 0);
+    int buf = 0;
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int n = rd * GROUPS + group;
+        for (int ck = 0; ck < chunks; ++ck, buf ^= 1) {
+            if (ck + 1 < chunks) load_stage(n, (ck + 1) * KP, buf ^ 1);
+            else if (rd + 1 < rounds) load_stage(n + GROUPS, 0, buf ^ 1);
+            else cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+            if (n < d.n) {
+                const float* as = mine + buf * STAGE + ty * TM;
+                const float* bs = mine + buf * STAGE + KP * LDA + tx * TN;
+                const int rows = min(KP, P - ck * KP);
+                constexpr int U = TM * TN <= 4 ? 8 : 4;
+                int r = 0;
+                for (; r + U <= rows; r += U) {
+                    float a[U][TM], b[U][TN];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        lds_vec<TM>(as + u * LDA, a[u]);
+                        lds_vec<TN>(bs + u * LDB, b[u]);
+                    }
+                    as += U * LDA;
+                    bs += U * LDB;
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int i = 0; i < TM; ++i)
+#pragma unroll
+                            for (int j = 0; j < TN; ++j) val[i][j] = __fadd_rn(val[i][j], __fmul_rn(a[u][i], b[u][j]));
+                }
+                for (; r < rows; ++r) {
+                    float a[TM], b[TN];
+                    lds_vec<TM>(as, a);
+                    lds_vec<TN>(bs, b);
+                    as += LDA;
+                    bs += LDB;
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) val[i][j] = __fadd_rn(val[i][j], __fmul_rn(a[i], b[j]));
+                }
+            }
+            __syncthreads();
+        }
+        if (GROUPS == 1) {
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) { tot[i][j] = __fadd_rn(tot[i][j], val[i][j]); val[i][j] = 0.f; }
+        } else {
+            float* red = smem + GROUPS * 2 * STAGE;   // [group][item][thread]
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    red[(group * TM * TN + i * TN + j) * THREADS + tid] = val[i][j];
+                    val[i][j] = 0.f;
+                }
+            __syncthreads();
+            if (group == 0)
+                for (int g = 0; g < GROUPS && rd * GROUPS + g < d.n; ++g)
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j)
+                            tot[i][j] = __fadd_rn(tot[i][j], red[(g * TM * TN + i * TN + j) * THREADS + tid]);
+            // the barrier of the next stage comes before anybody overwrites `red`
+        }
+    }
+    if (group != 0) return;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int row = m0 + ty * TM + i;
+        if (row >= M) continue;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int o = n0 + tx * TN + j;
+            if (o < d.o) dk[(size_t)row * d.o + o] = tot[i][j];
+        }
+    }
+}
+
+bool ordered_ok(const dcg_conv_desc& d)
+{
+    // element offsets are 32-bit
+    const long long x = (long long)d.n * d.h * d.w * d.c, y = (long long)d.n * d.ho * d.wo * d.o, k = (long long)d.kh * d.kw * d.c * d.o;
+    return d.kh * d.kw <= kOrdMaxTaps && x < (1ll << 31) && y < (1ll << 31) && k < (1ll << 31);
+}
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// Channels per stage: kOrdQuads words of `taps` each, no more than there are.
+int ord_channels(int taps, int contracted)
+{
+    int qc = kOrdQuads / (taps > 0 ? taps : 1) * 4;
+    const int all = (contracted + 3) / 4 * 4;
+    if (qc > 32) qc = 32;
+    if (qc > all) qc = all;
+    return qc < 4 ? 4 : qc;
+}
+
+template <int TM, int TN, int TX, int TY, int U>
+int launch_ordered_fwd_taps(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
+{
+    constexpr int BMT = TM * TY, BNT = TN * TX;
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(conv_ordered_fwd_kernel<TM, TN, TX, TY, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
+    });
+    DCG_CUDA(attr_err);
+    const int taps = d.kh * d.kw, qc = ord_channels(taps, d.c);
+    const size_t smem = (size_t)2 * (BMT * ord_row_pitch(taps, qc) + qc * taps * ord_pitch(BNT)) * sizeof(float);
+    const long long pixels = (long long)d.n * d.ho * d.wo;
+    const dim3 grid((unsigned)((pixels + BMT - 1) / BMT), (unsigned)((d.o + BNT - 1) / BNT));
+    launch_pdl(conv_ordered_fwd_kernel<TM, TN, TX, TY, U>, grid, TX * TY, smem, stream, x, k, y, d, ep, qc,
+               d.c % 4 == 0 && aligned16(x) ? 1 : 0, d.o % 4 == 0 && aligned16(k) ? 1 : 0);
+    DCG_LAUNCH_CHECK("conv_ordered_fwd_kernel");
+    return DCG_OK;
+}
+
+template <int TM, int TN, int TX, int TY>
+int launch_ordered_fwd_tile(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
+{
+    const int taps = d.kh * d.kw;
+    if (TM * TN <= 4 && taps == 25) return launch_ordered_fwd_taps<TM, TN, TX, TY, TM * TN <= 4 ? 25 : 5>(d, x, k, y, ep, stream);
+    if (taps % 5 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, 5>(d, x, k, y, ep, stream);
+    if (taps % 4 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, 4>(d, x, k, y, ep, stream);
+    if (taps % 3 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, 3>(d, x, k, y, ep, stream);
+    return launch_ordered_fwd_taps<TM, TN, TX, TY, 1>(d, x, k, y, ep, stream);
+}
+
+template <int TM, int TN, int TX, int TY>
+int launch_ordered_dx_tile(const dcg_conv_desc& d, const float* dy, const float* k, float* dx, const EpilogueArgs& ep, cudaStream_t stream)
+{
+    constexpr int BMT = TM * TY, BNT = TN * TX;
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(conv_ordered_dx_kernel<TM, TN, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
+    });
+    DCG_CUDA(attr_err);
+    const int mh = (d.h + d.stride_h - 1) / d.stride_h, mw = (d.w + d.stride_w - 1) / d.stride_w;   // of the largest class
+    const int taps = ((d.kh + d.stride_h - 1) / d.stride_h) * ((d.kw + d.stride_w - 1) / d.stride_w);
+    const int qc = ord_channels(taps, d.o);
+    const size_t smem = (size_t)2 * (BMT + BNT) * ord_row_pitch(taps, qc) * sizeof(float);
+    const dim3 grid((unsigned)(((long long)d.n * mh * mw + BMT - 1) / BMT), (unsigned)((d.c + BNT - 1) / BNT),
+                    (unsigned)(d.stride_h * d.stride_w));
+    launch_pdl(conv_ordered_dx_kernel<TM, TN, TX, TY>, grid, TX * TY, smem, stream, dy, k, dx, d, ep, qc,
+               d.o % 4 == 0 && aligned16(dy) && aligned16(k) ? 1 : 0);
+    DCG_LAUNCH_CHECK("conv_ordered_dx_kernel");
+    return DCG_OK;
+}
+
+// Tile choice by outputs per lane of the GPU (SMs x 128): the wider the thread tile the fewer instructions an output
+// costs per K step, but a scheduler needs a few warps to hide the chain of dependent adds and the shared-memory
+// latency.
+constexpr double kOrdWide = 32, kOrdNormal = 5, kOrdDkGrouped = 2;
+
+double outputs_per_lane(double outputs) { return outputs / (128.0 * sm_count()); }
+
+int launch_ordered_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
+{
+    const double per_lane = outputs_per_lane((double)d.n * d.ho * d.wo * d.o);
+    if (per_lane >= kOrdWide) return launch_ordered_fwd_tile<4, 4, 16, 16>(d, x, k, y, ep, stream);
+    if (per_lane >= kOrdNormal) return launch_ordered_fwd_tile<2, 2, 16, 16>(d, x, k, y, ep, stream);
+    return launch_ordered_fwd_tile<1, 2, 8, 16>(d, x, k, y, ep, stream);
+}
+
+int launch_ordered_dx(const dcg_conv_desc& d, const float* dy, const float* k, float* dx, const EpilogueArgs& ep, cudaStream_t stream)
+{
+    const double per_lane = outputs_per_lane((double)d.n * d.h * d.w * d.c);
+    if (d.c <= 4) return launch_ordered_dx_tile<1, 4, 1, 128>(d, dy, k, dx, ep, stream);   // RGB images: a pixel per thread
+    if (per_lane >= kOrdWide) return launch_ordered_dx_tile<4, 2, 16, 16>(d, dy, k, dx, ep, stream);
+    if (per_lane >= kOrdNormal) return launch_ordered_dx_tile<2, 2, 16, 16>(d, dy, k, dx, ep, stream);
+    return launch_ordered_dx_tile<1, 2, 8, 16>(d, dy, k, dx, ep, stream);
+}
+
+template <int TM, int TN, int TX, int TY, int GROUPS>
+int launch_ordered_dk_tile(const dcg_conv_desc& d, const float* x, const float* dy, float* dk, cudaStream_t stream)
+{
+    constexpr int BMT = TM * TY, BNT = TN * TX;
+    const size_t smem = (size_t)GROUPS * 2 * 32 * (ord_pitch(BMT) + ord_pitch(BNT)) * 4 + (GROUPS > 1 ? (size_t)GROUPS * BMT * BNT * 4 : 0);
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(conv_ordered_dk_kernel<TM, TN, TX, TY, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
+    });
+    DCG_CUDA(attr_err);
+    const int M = d.kh * d.kw * d.c;
+    const dim3 grid((unsigned)((M + BMT - 1) / BMT), (unsigned)((d.o + BNT - 1) / BNT));
+    launch_pdl(conv_ordered_dk_kernel<TM, TN, TX, TY, GROUPS>, grid, TX * TY * GROUPS, smem, stream, x, dy, dk, d,
+               d.c % 4 == 0 && aligned16(x) ? 1 : 0, d.o % 4 == 0 && aligned16(dy) ? 1 : 0);
+    DCG_LAUNCH_CHECK("conv_ordered_dk_kernel");
+    return DCG_OK;
+}
+
+int launch_ordered_dk(const dcg_conv_desc& d, const float* x, const float* dy, float* dk, cudaStream_t stream)
+{
+    // the images of a batch are parallel work as well (GROUPS); outputs per lane as above
+    const double per_lane = (double)d.kh * d.kw * d.c * d.o / (128.0 * sm_count());
+    if (per_lane >= kOrdWide) return launch_ordered_dk_tile<4, 4, 16, 16, 1>(d, x, dy, dk, stream);
+    if (per_lane < kOrdDkGrouped && d.n > 1) return launch_ordered_dk_tile<1, 2, 4, 8, 16>(d, x, dy, dk, stream);
+    if (d.n > 2) return launch_ordered_dk_tile<4, 4, 8, 8, 4>(d, x, dy, dk, stream);
+    return launch_ordered_dk_tile<2, 2, 8, 8, 1>(d, x, dy, dk, stream);
+}
+
+
+// ---- one thread per output: kernels with many taps ----------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
 conv_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ k,
                         float* __restrict__ y, const dcg_conv_desc d, const EpilogueArgs ep,
@@ -126,6 +752,7 @@ int conv_fwd_generic(const dcg_conv_desc& d, const float* x, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.ho * d.wo * d.o;
     if (total == 0) return DCG_OK;
+    if (ordered_ok(d)) return launch_ordered_fwd(d, x, k, y, ep, stream);
     conv_fwd_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, k, y, d, ep, total);
     DCG_LAUNCH_CHECK("conv_fwd_generic_kernel");
@@ -137,6 +764,7 @@ int conv_dx_generic(const dcg_conv_desc& d, const float* dy, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.h * d.w * d.c;
     if (total == 0) return DCG_OK;
+    if (ordered_ok(d)) return launch_ordered_dx(d, dy, k, dx, ep, stream);
     conv_dx_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         dy, k, dx, d, ep, total);
     DCG_LAUNCH_CHECK("conv_dx_generic_kernel");
@@ -148,6 +776,7 @@ int conv_dk_generic(const dcg_conv_desc& d, const float* x, const float* dy, flo
 {
     const size_t total = (size_t)d.kh * d.kw * d.c * d.o;
     if (total == 0) return DCG_OK;
+    if (ordered_ok(d)) return launch_ordered_dk(d, x, dy, dk, stream);
     conv_dk_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, dy, dk, d, total);
     DCG_LAUNCH_CHECK("conv_dk_generic_kernel");

@@ -123,6 +123,33 @@ def test_dx_with_parity_classes_fused(pkg, dev, orc, shape):
     _check(dx0, dx_ref, pkg.PREC_TF32, pkg, "dx, one tile per class")
 
 
+# one shape or more for every thread tile of the ordered fp32 kernels (few / some / many outputs per lane, RGB input gradient,
+# kernel gradient with the images over 1, 4 and 16 thread groups), with and without 16-byte copies of either operand, tap
+# counts with and without an unrolled form, tiles and channel quads that are not full, and a kernel too large for them
+ORDERED_SHAPES = [
+    (2, 96, 101, 5, 3, 36, 1), (2, 64, 80, 68, 3, 6, 1), (3, 5, 6, 164, 5, 156, 1), (2, 9, 7, 36, 5, 44, 2), (5, 9, 7, 36, 5, 44, 2),
+    (17, 6, 5, 3, 4, 34, 2), (2, 33, 65, 12, 1, 20, 1), (4, 24, 40, 33, 5, 40, 2), (1, 11, 9, 2, 7, 3, 2), (1, 5, 4, 7, 2, 3, 3),
+]
+
+
+@pytest.mark.parametrize("shape", ORDERED_SHAPES)
+def test_fp32_ordered_kernels_match_oracle_bit_for_bit(pkg, dev, orc, shape):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    x, k = seeded((N, H, W, C), 234), seeded((K, K, C, O), 235)
+    pad = (oracle.same_pad(H, K, s), oracle.same_pad(W, K, s))
+    y_ref = orc.conv2d(x, k, (s, s))
+    dy, b = seeded(y_ref.shape, 236), seeded((O,), 237)
+    xd, kd, dyd, bd = (torch.from_numpy(a).to(dev) for a in (x, k, dy, b))
+    y = F.conv2d_fwd(xd, kd, (s, s), epilogue=F.make_epilogue(bias=bd, act=pkg.ACT_LEAKY), precision=pkg.PREC_FP32)
+    dx = F.conv2d_dx(dyd, kd, (H, W), (s, s), precision=pkg.PREC_FP32)
+    dk = F.conv2d_dk(xd, dyd, (K, K), (s, s), precision=pkg.PREC_FP32)
+    torch.cuda.synchronize()
+    _check(y, orc.vect_relu_leaky(orc.mvrow_add(y_ref.reshape(-1, O), b), 0.2).reshape(y_ref.shape), pkg.PREC_FP32, pkg, "fwd")
+    _check(dx, orc.conv2d_input_grad(dy, k, s, (H, W)), pkg.PREC_FP32, pkg, "dx")
+    _check(dk, orc.conv2d_kernel_grad(dy, x, s, pad), pkg.PREC_FP32, pkg, "dk")
+
+
 @pytest.mark.parametrize("shape", [(40, 64, 64, 3, 5, 64, 2), (40, 60, 52, 3, 5, 64, 2), (37, 64, 64, 4, 5, 32, 2)])
 def test_three_channel_layers_with_persistent_ctas(pkg, dev, orc, shape):
     """More tiles than SMs: the forward of a <= 4-channel layer and the GEMM of its input gradient run as
