@@ -590,6 +590,9 @@ extern "C" int dcg_run_node(dcg_context* ctx, const dcg_node* nd)
 
 namespace dcg {
 int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t n, cudaStream_t stream);
+int softmax_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t rows, size_t cols, cudaStream_t stream);
+int matmul_act(const float* a, const float* b, const float* bias, float* out, size_t m, size_t n, size_t p, int act, float alpha,
+               float* act_out, cudaStream_t stream);
 int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const float* gate,
                     float* gated_out, int gate_act, float gate_alpha, cudaStream_t stream);
 }  // namespace dcg
@@ -688,18 +691,32 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
         if (i + 1 < count && !(nodes[i + 1].flags & DCG_NODE_SIDE)) {
             const dcg_node& a = nodes[i];
             const dcg_node& b = nodes[i + 1];
-            // dense layer + activation (tensor path only)
+            // dense layer + activation
             const int act = act_of_node(b.type);
             if (a.type == DCG_OP_MAT_MUL_ADD && act >= 0 && b.in1 == a.out1 && b.len1 == a.len1 * a.len3 && b.out1 != a.out1) {
                 const int st = run_dense_on_tensor_path(ctx, &a, act, b.type == DCG_OP_RELU_LEAKY ? b.alpha_leaky : 0.f, b.out1);
                 if (st < 0) return st;
                 if (st == 0) { i += 2; continue; }
+                // a small one on the CUDA cores (the fp32 path keeps one launch per node)
+                ProfScope scope(ctx->precision == DCG_PREC_FP32 ? nullptr : ctx, "mat_mul_add", 0.0);
+                const int cs = ctx->precision == DCG_PREC_FP32 ? 1 : dcg::matmul_act(a.in1, a.in2, a.in3, a.out1, a.len1, a.len2, a.len3, act,
+                                                                                            b.type == DCG_OP_RELU_LEAKY ? b.alpha_leaky : 0.f, b.out1, ctx->stream);
+                if (cs < 0) return cs;
+                if (cs == 0) { i += 2; continue; }
             }
             // loss + its gradient on the same labels and logits
             if (a.type == DCG_OP_SIGMOID_CROSS_ENTROPY && b.type == DCG_OP_SIGMOID_CROSS_ENTROPY_GRAD && a.in1 == b.in1 &&
                 a.in2 == b.in2 && a.len1 == b.len1 && a.len1 <= 65536 && a.out1 != b.out1) {
                 ProfScope scope(ctx, "sigmoid_xent_with_grad", 0.0);
                 const int st = dcg::sigmoid_xent_with_grad(a.in1, a.in2, a.out1, b.out1, a.len1, ctx->stream);
+                if (st) return st;
+                i += 2;
+                continue;
+            }
+            if (a.type == DCG_OP_SOFTMAX_CROSS_ENTROPY && b.type == DCG_OP_SOFTMAX_CROSS_ENTROPY_GRAD && a.in1 == b.in1 &&
+                a.in2 == b.in2 && a.len1 == b.len1 && a.len2 == b.len2 && a.len1 <= 256 && a.out1 != b.out1) {
+                ProfScope scope(ctx, "softmax_xent_with_grad", 0.0);
+                const int st = dcg::softmax_xent_with_grad(a.in1, a.in2, a.out1, b.out1, a.len1, a.len2, ctx->stream);
                 if (st) return st;
                 i += 2;
                 continue;

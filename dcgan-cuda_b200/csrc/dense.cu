@@ -1,91 +1,189 @@
 // Dense-layer matrix products (src/gpu/matmul.cu:11-86): the generator's
 // 100 -> 8192 projection, the discriminator's 8192 -> 1 head, and the MNIST MLP.
 //
-// These are small and HBM/latency bound (the largest operand is 3.3 MB), so they
-// stay on CUDA cores: a shared-memory tiled kernel that accumulates each output
-// over k in ascending order with unfused multiply/add - bit-identical to the
-// reference CPU loops (src/cpu/ops.hxx:56-105,375-390) - plus three shape
-// specialists for the DCGAN layers: short reduction / wide output (100 -> 8192 and
-// its weight gradient), few outputs / long reduction (8192 -> 1), and tall output
-// from a transposed operand (the head's weight gradient).
+// These are small and HBM / latency bound (the largest operand is 3.3 MB), so they stay on CUDA cores.
+// gemm_ordered_kernel accumulates each output over k in ascending order with unfused multiply / add - bit-identical to
+// the reference CPU loops (src/cpu/ops.hxx:56-105,375-390); two shape specialists go with it: few outputs / long
+// reduction (8192 -> 1), and tall output from a transposed operand (the head's weight gradient).
+#include <cstdint>
+#include <mutex>
+
 #include "common.cuh"
 
 namespace dcg {
 namespace {
 
-constexpr int TILE = 64;  // output tile edge
-constexpr int KT = 16;    // k-tile depth
-constexpr int TPB = 256;  // 16 x 16 threads, 4 x 4 outputs each
+constexpr int TPB = 256;
 
-// Operand views: element (row, col) of the logical [rows x cols] matrix.
-// TRANS: the logical matrix is the transpose of the stored row-major one.
-template <bool TRANS>
-__device__ __forceinline__ float load_elem(const float* __restrict__ p, size_t r, size_t c,
-                                           size_t rows, size_t cols)
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, bool in, int bytes)
 {
-    return TRANS ? __ldg(p + c * rows + r) : __ldg(p + r * cols + c);
+    const int n = in ? bytes : 0;   // 0: zero-fill
+    if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
-// out[m,p] = A[m,n] * B[n,p] (+ bias[p]); A, B through the views above.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(TPB)
-gemm_tiled_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                  const float* __restrict__ bias, float* __restrict__ out,
-                  size_t m, size_t n, size_t p, const float* __restrict__ gate, float* __restrict__ gated_out,
-                  int gate_act, float gate_alpha)
+// W consecutive floats of an operand tile
+template <int W>
+__device__ __forceinline__ void tile_read(const float* s, float (&v)[W])
 {
-    pdl_enter();
-    __shared__ float As[KT][TILE + 1];  // [k][row]
-    __shared__ float Bs[KT][TILE + 1];  // [k][col]
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const size_t row0 = (size_t)blockIdx.y * TILE, col0 = (size_t)blockIdx.x * TILE;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    if constexpr (W == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(s);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (W == 2) {
+        const float2 t = *reinterpret_cast<const float2*>(s);
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        v[0] = *s;
+    }
+}
 
-    for (size_t k0 = 0; k0 < n; k0 += KT) {
-        for (int e = threadIdx.x; e < KT * TILE; e += TPB) {
-            // pick the fast-varying index along the contiguous memory direction
-            int kk, rr;
-            if (TA) { rr = e % TILE; kk = e / TILE; } else { kk = e % KT; rr = e / KT; }
-            const size_t r = row0 + rr, k = k0 + kk;
-            As[kk][rr] = (r < m && k < n) ? load_elem<TA>(a, r, k, m, n) : 0.f;
-            int cc;
-            if (TB) { kk = e % KT; cc = e / KT; } else { cc = e % TILE; kk = e / TILE; }
-            const size_t c = col0 + cc, k2 = k0 + kk;
-            Bs[kk][cc] = (c < p && k2 < n) ? load_elem<TB>(b, k2, c, n, p) : 0.f;
+// What follows the sum of an output: + bias[col], the value itself to `out`, an activation of it or its product with the
+// activation gradient at gate[] to `out2` (same expressions as bias_act_kernel and act_grad_kernel).
+struct DenseEpilogue {
+    const float* bias;
+    const float* gate;
+    float* out2;
+    int act;         // of out2: activation, or with `gate` the activation whose gradient gates
+    float alpha;
+};
+
+// out[m,p] = A[m,n] B[n,p]: TM x TN outputs per thread, TX x TY threads per block, STAGES stages of KC = 64 reduction steps
+// filled with cp.async.  TA / TB: the logical matrix is the transpose of the stored row-major one.  An operand whose
+// reduction axis is contiguous keeps it so in shared memory ([row][k], four steps per 16-byte read), the other is
+// [k][row].  What is beyond an edge is zero-filled; the zeros add +0 to the sums.
+// Latency-bound at the sizes of this library: many small tiles and all loads of several stages in flight matter more than
+// operand reuse (100 x 784 x 100: 160 us with one 64 x 64 tile per block and blocking loads, 8 us as 49 tiles of 16 x 16).
+template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES>
+__global__ void __launch_bounds__(TX * TY)
+gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const int m, const int n,
+                    const int p, const DenseEpilogue e, const int vec_a, const int vec_b)
+{
+    constexpr int BM = TM * TY, BN = TN * TX, THREADS = TX * TY, KC = 64;
+    constexpr int LDA = TA ? BM + 4 : KC + 4, LDB = TB ? KC + 4 : BN + 4;
+    constexpr int A_FLOATS = (TA ? KC : BM) * LDA, STAGE = A_FLOATS + (TB ? BN : KC) * LDB;
+    extern __shared__ __align__(16) float smem[];
+    pdl_enter();
+    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+    const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(smem);
+
+    // copies a tile of `inner` contiguous elements x `outer` lines, element (o, i) of the stored matrix at base[o * ld + i]
+    auto copy_tile = [&](uint32_t dst, int pitch, const float* base, int o0, int i0, int outer, int inner, int o_end, int i_end, int vec) {
+        const int w = vec ? 4 : 1, per_line = inner / w;
+        for (int idx = tid; idx < outer * per_line; idx += THREADS) {
+            const int o = idx / per_line, i = (idx - o * per_line) * w;
+            const bool in = o0 + o < o_end && i0 + i < i_end;
+            cp_async(dst + 4u * (uint32_t)(o * pitch + i), in ? base + (size_t)(o0 + o) * i_end + i0 + i : base, in, 4 * w);
+        }
+    };
+    auto load_stage = [&](int k0, int buf) {
+        if (k0 < n) {
+            const uint32_t as = smem0 + 4u * (uint32_t)(buf * STAGE), bs = as + 4u * (uint32_t)A_FLOATS;
+            const int kc = min(KC, (n - k0 + 3) & ~3);
+            if (TA) copy_tile(as, LDA, a, k0, row0, kc, BM, n, m, vec_a);
+            else copy_tile(as, LDA, a, row0, k0, BM, kc, m, n, vec_a);
+            if (TB) copy_tile(bs, LDB, b, col0, k0, BN, kc, p, n, vec_b);
+            else copy_tile(bs, LDB, b, k0, col0, kc, BN, n, p, vec_b);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) load_stage(s * KC, s);
+    int buf = 0;
+    for (int k0 = 0; k0 < n; k0 += KC) {
+        load_stage(k0 + (STAGES - 1) * KC, (buf + STAGES - 1) % STAGES);
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+        __syncthreads();
+        const float* as = smem + buf * STAGE + (TA ? ty * TM : ty * TM * LDA);
+        const float* bs = smem + buf * STAGE + A_FLOATS + (TB ? tx * LDB : tx * TN);   // TB: columns tx, tx + TX, ...
+        const int kc = min(KC, (n - k0 + 3) & ~3);
+#pragma unroll 4
+        for (int k = 0; k < kc; k += 4) {
+            float av[4][TM], bv[4][TN];
+            if (TA) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) tile_read<TM>(as + (k + u) * LDA, av[u]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    float v[4];
+                    tile_read<4>(as + i * LDA + k, v);
+                    av[0][i] = v[0]; av[1][i] = v[1]; av[2][i] = v[2]; av[3][i] = v[3];
+                }
+            }
+            if (TB) {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    float v[4];
+                    tile_read<4>(bs + j * TX * LDB + k, v);
+                    bv[0][j] = v[0]; bv[1][j] = v[1]; bv[2][j] = v[2]; bv[3][j] = v[3];
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) tile_read<TN>(bs + (k + u) * LDB, bv[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(av[u][i], bv[u][j]));
         }
         __syncthreads();
-        const int klim = (n - k0 < (size_t)KT) ? (int)(n - k0) : KT;
-        for (int kk = 0; kk < klim; ++kk) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(av[i], bv[j]));
-        }
-        __syncthreads();
+        buf = (buf + 1) % STAGES;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const size_t r = row0 + ty * 4 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int r = row0 + ty * TM + i;
         if (r >= m) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const size_t c = col0 + tx * 4 + j;
+        for (int j = 0; j < TN; ++j) {
+            const int c = col0 + (TB ? tx + j * TX : tx * TN + j);
             if (c >= p) continue;
+            const size_t idx = (size_t)r * p + c;
             float v = acc[i][j];
-            if (bias) v = __fadd_rn(v, __ldg(bias + c));
-            out[r * p + c] = v;
-            // the activation gradient that follows the product in a backward list, same expression as act_grad_kernel
-            if (gate) gated_out[r * p + c] = act_grad_apply(__ldg(gate + r * p + c), v, gate_act, gate_alpha);
+            if (e.bias) v = __fadd_rn(v, __ldg(e.bias + c));
+            out[idx] = v;
+            if (e.out2) e.out2[idx] = e.gate ? act_grad_apply(__ldg(e.gate + idx), v, e.act, e.alpha) : act_apply(v, e.act, e.alpha);
+        }
+    }
+}
+
+// Outer product of a column and a row (n == 1: the input gradient of the head, 64 x 1 times 1 x 8192): four columns per
+// thread, nothing to stage.  Memory-bound: the gate is read and both outputs written once.
+__global__ void __launch_bounds__(TPB)
+gemm_outer_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const size_t m, const size_t p4,
+                  const DenseEpilogue e)
+{
+    pdl_enter();
+    const size_t total = m * p4, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const size_t r = i / p4, c4 = i - r * p4;
+        const float av = __ldg(a + r);
+        const float4 bv = __ldg(reinterpret_cast<const float4*>(b) + c4);
+        float v[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __fadd_rn(0.f, __fmul_rn(av, v[u]));
+        if (e.bias) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(e.bias) + c4);
+            v[0] = __fadd_rn(v[0], w.x); v[1] = __fadd_rn(v[1], w.y); v[2] = __fadd_rn(v[2], w.z); v[3] = __fadd_rn(v[3], w.w);
+        }
+        reinterpret_cast<float4*>(out)[i] = make_float4(v[0], v[1], v[2], v[3]);
+        if (e.out2) {
+            if (e.gate) {
+                const float4 g = __ldg(reinterpret_cast<const float4*>(e.gate) + i);
+                v[0] = act_grad_apply(g.x, v[0], e.act, e.alpha); v[1] = act_grad_apply(g.y, v[1], e.act, e.alpha);
+                v[2] = act_grad_apply(g.z, v[2], e.act, e.alpha); v[3] = act_grad_apply(g.w, v[3], e.act, e.alpha);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = act_apply(v[u], e.act, e.alpha);
+            }
+            reinterpret_cast<float4*>(e.out2)[i] = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
 }
@@ -121,84 +219,6 @@ gemm_long_k_kernel(const float* __restrict__ a, const float* __restrict__ b,
     if (threadIdx.x == 0) out[o] = bias ? part[0] + __ldg(bias + c) : part[0];
 }
 
-// Short reduction, wide output (the generator's projection and its weight gradient):
-// out[m,p] = A[m,n] B[n,p] (+bias) with n <= 256 and B row-major.  A block owns 128 columns and
-// RB rows: the RB x n slab of A sits in shared memory, every thread walks one column of B
-// (coalesced across the block) and keeps RB accumulators.  k ascends, multiply and add stay
-// unfused: the same rounding sequence as the reference loops (src/cpu/ops.hxx:56-105).
-constexpr int RB = 8;
-template <bool TA>
-__global__ void __launch_bounds__(128)
-gemm_wide_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                 const float* __restrict__ bias, float* __restrict__ out,
-                 size_t m, size_t n, size_t p)
-{
-    pdl_enter();
-    __shared__ __align__(16) float As[256 * RB];   // [k][RB]
-    const size_t row0 = (size_t)blockIdx.y * RB;
-    for (int e = threadIdx.x; e < (int)n * RB; e += 128) {
-        int kk, rr;
-        if (TA) { rr = e % RB; kk = e / RB; } else { kk = e % (int)n; rr = e / (int)n; }
-        const size_t r = row0 + rr;
-        As[kk * RB + rr] = r < m ? load_elem<TA>(a, r, (size_t)kk, m, n) : 0.f;
-    }
-    __syncthreads();
-    const size_t c = (size_t)blockIdx.x * 128 + threadIdx.x;
-    if (c >= p) return;
-    float acc[RB];
-#pragma unroll
-    for (int i = 0; i < RB; ++i) acc[i] = 0.f;
-    const float* bc = b + c;
-    int k = 0;
-    // sixteen loads of B in flight per thread: the kernel is latency-bound otherwise (one warp walks
-    // a column of B with nothing else to overlap the memory round trips)
-    for (; k + 16 <= (int)n; k += 16) {
-        float bv[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) bv[u] = __ldg(bc + (size_t)(k + u) * p);
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const float4* ak = reinterpret_cast<const float4*>(As + (k + u) * RB);
-#pragma unroll
-            for (int q = 0; q < RB / 4; ++q) {
-                const float4 av = ak[q];
-                acc[4 * q + 0] = __fadd_rn(acc[4 * q + 0], __fmul_rn(av.x, bv[u]));
-                acc[4 * q + 1] = __fadd_rn(acc[4 * q + 1], __fmul_rn(av.y, bv[u]));
-                acc[4 * q + 2] = __fadd_rn(acc[4 * q + 2], __fmul_rn(av.z, bv[u]));
-                acc[4 * q + 3] = __fadd_rn(acc[4 * q + 3], __fmul_rn(av.w, bv[u]));
-            }
-        }
-    }
-    for (; k + 4 <= (int)n; k += 4) {
-        float bv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) bv[u] = __ldg(bc + (size_t)(k + u) * p);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float4* ak = reinterpret_cast<const float4*>(As + (k + u) * RB);
-#pragma unroll
-            for (int q = 0; q < RB / 4; ++q) {
-                const float4 av = ak[q];
-                acc[4 * q + 0] = __fadd_rn(acc[4 * q + 0], __fmul_rn(av.x, bv[u]));
-                acc[4 * q + 1] = __fadd_rn(acc[4 * q + 1], __fmul_rn(av.y, bv[u]));
-                acc[4 * q + 2] = __fadd_rn(acc[4 * q + 2], __fmul_rn(av.z, bv[u]));
-                acc[4 * q + 3] = __fadd_rn(acc[4 * q + 3], __fmul_rn(av.w, bv[u]));
-            }
-        }
-    }
-    for (; k < (int)n; ++k) {
-        const float bv = __ldg(bc + (size_t)k * p);
-#pragma unroll
-        for (int i = 0; i < RB; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(As[k * RB + i], bv));
-    }
-    const float bb = bias ? __ldg(bias + c) : 0.f;
-#pragma unroll
-    for (int i = 0; i < RB; ++i) {
-        const size_t r = row0 + i;
-        if (r < m) out[r * p + c] = bias ? __fadd_rn(acc[i], bb) : acc[i];
-    }
-}
-
 // Tall output with a handful of columns from a transposed left operand (the discriminator head's
 // weight gradient, x^T dy): out[r,c] = sum_k A^T[k,r] B[k,c]; one thread per output, loads
 // coalesced along r, k ascending, unfused.
@@ -212,41 +232,92 @@ gemm_tall_tn_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
     const size_t c = o / m, r = o % m;   // r fastest across threads: coalesced reads of A^T
     float s = 0.f;
     size_t k = 0;
-    for (; k + 16 <= n; k += 16) {
-        float av[16], bw[16];
+    for (; k + 32 <= n; k += 32) {
+        float av[32], bw[32];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) { av[u] = __ldg(a + (k + u) * m + r); bw[u] = __ldg(b + (k + u) * p + c); }
+        for (int u = 0; u < 32; ++u) { av[u] = __ldg(a + (k + u) * m + r); bw[u] = __ldg(b + (k + u) * p + c); }
 #pragma unroll
-        for (int u = 0; u < 16; ++u) s = __fadd_rn(s, __fmul_rn(av[u], bw[u]));
+        for (int u = 0; u < 32; ++u) s = __fadd_rn(s, __fmul_rn(av[u], bw[u]));
     }
     for (; k < n; ++k) s = __fadd_rn(s, __fmul_rn(__ldg(a + k * m + r), __ldg(b + k * p + c)));
     out[r * p + c] = s;
 }
 
-template <bool TA>
-int launch_wide(const float* a, const float* b, const float* bias, float* out, size_t m, size_t n,
-                size_t p, cudaStream_t stream)
+bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
+
+template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES>
+int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const DenseEpilogue& e, cudaStream_t stream)
 {
-    const dim3 grid((unsigned)((p + 127) / 128), (unsigned)((m + RB - 1) / RB));
-    launch_pdl(gemm_wide_kernel<TA>, grid, 128, 0, stream, a, b, bias, out, m, n, p);
-    DCG_LAUNCH_CHECK("gemm_wide_kernel");
+    constexpr int BM = TM * TY, BN = TN * TX, KC = 64;
+    constexpr size_t smem = (size_t)STAGES * ((TA ? KC * (BM + 4) : BM * (KC + 4)) + (TB ? BN * (KC + 4) : KC * (BN + 4))) * sizeof(float);
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    });
+    DCG_CUDA(attr_err);
+    const dim3 grid((unsigned)((p + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
+    const int vec_a = (TA ? m : n) % 4 == 0 && aligned16(a), vec_b = (TB ? n : p) % 4 == 0 && aligned16(b);
+    launch_pdl(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES>, grid, TX * TY, smem, stream, a, b, out, (int)m, (int)n, (int)p, e,
+               vec_a, vec_b);
+    DCG_LAUNCH_CHECK("gemm_ordered_kernel");
     return DCG_OK;
 }
 
-inline bool wide_shape(size_t m, size_t n, size_t p) { return n <= 256 && p >= 512 && m <= 65535u * RB; }
-
+// Tile choice by outputs per lane of the GPU, as for the ordered convolutions: few outputs go one to a thread over as many
+// blocks as there are, with four stages in flight.  A handful of rows (a small batch through the generator's
+// projection) gets flat tiles, so that few of its threads idle.
 template <bool TA, bool TB>
-int launch_tiled(const float* a, const float* b, const float* bias, float* out, size_t m, size_t n,
-                 size_t p, cudaStream_t stream, const char* name, const float* gate = nullptr, float* gated_out = nullptr,
-                 int gate_act = 0, float gate_alpha = 0.f)
+int launch_ordered(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const DenseEpilogue& e, cudaStream_t stream)
 {
-    const dim3 grid((unsigned)((p + TILE - 1) / TILE), (unsigned)((m + TILE - 1) / TILE));
-    launch_pdl(gemm_tiled_kernel<TA, TB>, grid, TPB, 0, stream, a, b, bias, out, m, n, p, gate, gated_out, gate_act, gate_alpha);
-    DCG_LAUNCH_CHECK(name);
-    return DCG_OK;
+    DCG_CHECK_ARG(m < (1u << 30) && n < (1u << 30) && p < (1u << 30), "dense: %zu x %zu x %zu is too large", m, n, p);
+    DCG_CHECK_ARG((m + 3) / 4 <= 65535u * 16, "dense: %zu rows are too many", m);
+    if (!TA && n == 1 && p % 4 == 0 && aligned16(b) && aligned16(out) && aligned16(e.bias) && aligned16(e.gate) && aligned16(e.out2)) {
+        size_t blocks = (m * (p / 4) + TPB - 1) / TPB;
+        const size_t cap = (size_t)sm_count() * 8;
+        if (blocks > cap) blocks = cap;
+        launch_pdl(gemm_outer_kernel, (unsigned)blocks, TPB, 0, stream, a, b, out, m, p / 4, e);
+        DCG_LAUNCH_CHECK("gemm_outer_kernel");
+        return DCG_OK;
+    }
+    const double per_lane = (double)m * (double)p / (128.0 * sm_count());
+    if (m <= 8 && p >= 512) return launch_tile<TA, TB, 1, 1, 32, 8, 3>(a, b, out, m, n, p, e, stream);
+    if (per_lane >= 20) return launch_tile<TA, TB, 4, 4, 16, 16, 2>(a, b, out, m, n, p, e, stream);
+    if (per_lane >= 5) return launch_tile<TA, TB, 2, 2, 16, 16, 3>(a, b, out, m, n, p, e, stream);
+    return launch_tile<TA, TB, 1, 1, 16, 16, 4>(a, b, out, m, n, p, e, stream);
+}
+
+int matmul_nn(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const DenseEpilogue& e, cudaStream_t stream)
+{
+    if (m * p <= 4096 && n >= 1024 && !e.out2) {
+        launch_pdl(gemm_long_k_kernel, (unsigned)(m * p), TPB, 0, stream, a, b, e.bias, out, m, n, p);
+        DCG_LAUNCH_CHECK("gemm_long_k_kernel");
+        return DCG_OK;
+    }
+    return launch_ordered<false, false>(a, b, out, m, n, p, e, stream);
 }
 
 }  // namespace
+
+// dcg_matmul followed by an activation of its result as one launch (node fusion of the backend).  Not for the shapes of
+// gemm_long_k_kernel: returns 1 there.
+int matmul_act(const float* a, const float* b, const float* bias, float* out, size_t m, size_t n, size_t p, int act, float alpha,
+               float* act_out, cudaStream_t stream)
+{
+    if (m * p <= 4096 && n >= 1024) return 1;
+    DCG_CHECK_ARG(a && b && out && act_out && m > 0 && n > 0 && p > 0, "matmul_act: bad arguments");
+    return matmul_nn(a, b, out, m, n, p, DenseEpilogue{bias, nullptr, act_out, act, alpha}, stream);
+}
+
+// dcg_matmul_nt followed by dcg_act_grad(gate, out) -> gated_out as one launch (node fusion of the backend).
+int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const float* gate,
+                    float* gated_out, int gate_act, float gate_alpha, cudaStream_t stream)
+{
+    DCG_CHECK_ARG(a && b && out && gate && gated_out && m > 0 && n > 0 && p > 0, "matmul_nt_gated: bad arguments");
+    return launch_ordered<false, true>(a, b, out, m, n, p, DenseEpilogue{nullptr, gate, gated_out, gate_act, gate_alpha}, stream);
+}
+
 }  // namespace dcg
 
 using namespace dcg;
@@ -255,42 +326,24 @@ extern "C" int dcg_matmul(const float* a, const float* b, const float* bias, flo
                           size_t n, size_t p, dcg_stream_t stream)
 {
     DCG_CHECK_ARG(a && b && out && m > 0 && n > 0 && p > 0, "dcg_matmul: bad arguments");
-    if (m * p <= 4096 && n >= 1024) {
-        launch_pdl(gemm_long_k_kernel, (unsigned)(m * p), TPB, 0, as_stream(stream), a, b, bias, out, m, n, p);
-        DCG_LAUNCH_CHECK("gemm_long_k_kernel");
-        return DCG_OK;
-    }
-    if (wide_shape(m, n, p)) return launch_wide<false>(a, b, bias, out, m, n, p, as_stream(stream));
-    return launch_tiled<false, false>(a, b, bias, out, m, n, p, as_stream(stream), "gemm_tiled_kernel<nn>");
+    return matmul_nn(a, b, out, m, n, p, DenseEpilogue{bias, nullptr, nullptr, DCG_ACT_NONE, 0.f}, as_stream(stream));
 }
 
 extern "C" int dcg_matmul_tn(const float* a, const float* b, float* out, size_t m, size_t n,
                              size_t p, dcg_stream_t stream)
 {
     DCG_CHECK_ARG(a && b && out && m > 0 && n > 0 && p > 0, "dcg_matmul_tn: bad arguments");
-    if (wide_shape(m, n, p)) return launch_wide<true>(a, b, nullptr, out, m, n, p, as_stream(stream));
     if (p <= 8 && m >= 1024) {
         launch_pdl(gemm_tall_tn_kernel, (unsigned)((m * p + 63) / 64), 64, 0, as_stream(stream), a, b, out, m, n, p);
         DCG_LAUNCH_CHECK("gemm_tall_tn_kernel");
         return DCG_OK;
     }
-    return launch_tiled<true, false>(a, b, nullptr, out, m, n, p, as_stream(stream), "gemm_tiled_kernel<tn>");
+    return launch_ordered<true, false>(a, b, out, m, n, p, DenseEpilogue{}, as_stream(stream));
 }
-
-namespace dcg {
-// dcg_matmul_nt followed by dcg_act_grad(gate, out) -> gated_out as one launch (node fusion of the backend).
-int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const float* gate,
-                    float* gated_out, int gate_act, float gate_alpha, cudaStream_t stream)
-{
-    DCG_CHECK_ARG(a && b && out && gate && gated_out && m > 0 && n > 0 && p > 0, "matmul_nt_gated: bad arguments");
-    return launch_tiled<false, true>(a, b, nullptr, out, m, n, p, stream, "gemm_tiled_kernel<nt>", gate, gated_out, gate_act,
-                                     gate_alpha);
-}
-}  // namespace dcg
 
 extern "C" int dcg_matmul_nt(const float* a, const float* b, float* out, size_t m, size_t n,
                              size_t p, dcg_stream_t stream)
 {
     DCG_CHECK_ARG(a && b && out && m > 0 && n > 0 && p > 0, "dcg_matmul_nt: bad arguments");
-    return launch_tiled<false, true>(a, b, nullptr, out, m, n, p, as_stream(stream), "gemm_tiled_kernel<nt>");
+    return launch_ordered<false, true>(a, b, out, m, n, p, DenseEpilogue{}, as_stream(stream));
 }

@@ -424,14 +424,9 @@ mse_grad_kernel(const float* __restrict__ y, const float* __restrict__ y_hat,
 
 // ---- softmax family: one warp per row (src/cpu/ops.hxx:129-186,418-430) ---------
 // mode 0: softmax, 1: log_softmax, 2: (softmax - y)/rows
-__global__ void __launch_bounds__(kThreads)
-softmax_rows_kernel(const float* __restrict__ a, const float* __restrict__ y,
-                    float* __restrict__ out, size_t rows, size_t cols, int mode)
+__device__ __forceinline__ void softmax_row(const float* __restrict__ a, const float* __restrict__ y, float* __restrict__ out,
+                                            size_t row, size_t rows, size_t cols, int mode, int lane)
 {
-    pdl_enter();
-    const size_t row = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (row >= rows) return;
     const float* ar = a + row * cols;
     float mx = -INFINITY;
     for (size_t c = lane; c < cols; c += 32) mx = fmaxf(mx, __ldg(ar + c));
@@ -452,13 +447,19 @@ softmax_rows_kernel(const float* __restrict__ a, const float* __restrict__ y,
     }
 }
 
-// -(1/rows) sum_ij y_ij (logit_ij - logsumexp_i)
-__global__ void __launch_bounds__(512)
-softmax_xent_kernel(const float* __restrict__ y, const float* __restrict__ logits,
-                    float* __restrict__ out, size_t rows, size_t cols)
+__global__ void __launch_bounds__(kThreads)
+softmax_rows_kernel(const float* __restrict__ a, const float* __restrict__ y,
+                    float* __restrict__ out, size_t rows, size_t cols, int mode)
 {
     pdl_enter();
-    __shared__ float red[32];
+    const size_t row = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row < rows) softmax_row(a, y, out, row, rows, cols, mode, threadIdx.x & 31);
+}
+
+// -(1/rows) sum_ij y_ij (logit_ij - logsumexp_i)
+__device__ __forceinline__ float softmax_xent_block(const float* __restrict__ y, const float* __restrict__ logits, size_t rows,
+                                                    size_t cols, float* red)
+{
     float acc = 0.f;
     for (size_t r = threadIdx.x; r < rows; r += blockDim.x) {
         const float* lr = logits + r * cols;
@@ -469,8 +470,31 @@ softmax_xent_kernel(const float* __restrict__ y, const float* __restrict__ logit
         const float logsum = mx + logf(e);
         for (size_t c = 0; c < cols; ++c) acc += y[r * cols + c] * (lr[c] - logsum);
     }
-    acc = block_sum(acc, red);
+    return block_sum(acc, red);
+}
+
+__global__ void __launch_bounds__(512)
+softmax_xent_kernel(const float* __restrict__ y, const float* __restrict__ logits,
+                    float* __restrict__ out, size_t rows, size_t cols)
+{
+    pdl_enter();
+    __shared__ float red[32];
+    const float acc = softmax_xent_block(y, logits, rows, cols, red);
     if (threadIdx.x == 0) out[0] = -acc / (float)rows;
+}
+
+// Loss and its gradient in one launch, for the few rows one block gets through in the time a second launch would take: the
+// expressions and the orders of the two kernels above, so the results are bit-identical.
+__global__ void __launch_bounds__(512)
+softmax_xent_both_kernel(const float* __restrict__ y, const float* __restrict__ logits, float* __restrict__ loss,
+                         float* __restrict__ grad, size_t rows, size_t cols)
+{
+    pdl_enter();
+    __shared__ float red[32];
+    for (size_t row = threadIdx.x >> 5; row < rows; row += blockDim.x >> 5)
+        softmax_row(logits, y, grad, row, rows, cols, 2, threadIdx.x & 31);
+    const float acc = softmax_xent_block(y, logits, rows, cols, red);
+    if (threadIdx.x == 0) loss[0] = -acc / (float)rows;
 }
 
 // Count of rows whose first maximum sits at the same column in both matrices.
@@ -748,6 +772,14 @@ int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, flo
     DCG_CHECK_ARG(y && logits && loss && grad && n > 0, "sigmoid_xent_with_grad: bad arguments");
     launch_pdl(sigmoid_xent_both_kernel, 1, 512, 0, stream, y, logits, loss, grad, n);
     DCG_LAUNCH_CHECK("sigmoid_xent_both_kernel");
+    return DCG_OK;
+}
+// dcg_softmax_xent and dcg_softmax_xent_grad as one launch; few rows.
+int softmax_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t rows, size_t cols, cudaStream_t stream)
+{
+    DCG_CHECK_ARG(y && logits && loss && grad && rows > 0 && cols > 0, "softmax_xent_with_grad: bad arguments");
+    launch_pdl(softmax_xent_both_kernel, 1, 512, 0, stream, y, logits, loss, grad, rows, cols);
+    DCG_LAUNCH_CHECK("softmax_xent_both_kernel");
     return DCG_OK;
 }
 }  // namespace dcg

@@ -235,6 +235,29 @@ def test_small_neighbours_fuse_into_one_launch(pkg, dev, prec_name):
     assert results[True][1] == (4 if prec_name == "fp32" else 3)
 
 
+@pytest.mark.parametrize("rows", [3, 100, 257])
+def test_classifier_pairs_fuse_into_one_launch(pkg, dev, rows):
+    """A small dense layer + activation, and softmax cross-entropy + its gradient (up to 256 rows), as one launch each:
+    every output of the unfused list, bit for bit."""
+    N = pkg.nodes
+    x, w, b = _t(seeded((rows, 36), 1), dev), _t(seeded((36, 10), 2), dev), _t(seeded((10,), 3), dev)
+    y = torch.eye(10, device=dev)[torch.arange(rows, device=dev) % 10].contiguous()
+    results = {}
+    for fuse in (False, True):
+        z, a, d = (torch.empty((rows, 10), device=dev) for _ in range(3))
+        loss = torch.empty((1,), device=dev)
+        nodes = [N.op_mat_mul_add(x, w, b, z, rows, 36, 10), N.op_tanh(z, a, z.numel()),
+                 N.op_softmax_cross_entropy(y, z, loss, rows, 10), N.op_softmax_cross_entropy_grad(y, z, d, rows, 10)]
+        ctx = pkg.Context(pkg.PREC_TF32)
+        ctx.run(nodes, fuse=fuse)
+        torch.cuda.synchronize()
+        results[fuse] = [t.cpu().numpy() for t in (z, a, loss, d)], ctx.launch_count()
+        ctx.close()
+    for p, q in zip(results[False][0], results[True][0]):
+        assert np.array_equal(p, q)
+    assert results[False][1] == 4 and results[True][1] == (2 if rows <= 256 else 3)
+
+
 def test_reshape_is_an_alias_and_unknown_nodes_fail(pkg, dev):
     """Reshape lowers to no instruction at all (src/ops/reshape.cu:20-44): the consumer reads the
     producer's buffer, so it is bit-exact by construction.  Unknown node types are errors."""

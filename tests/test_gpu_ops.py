@@ -136,6 +136,23 @@ def test_dense(pkg, dev, orc, m, n, p):
     assert np.array_equal(dx.cpu().numpy(), orc.mtm_mul(dy, b))
 
 
+# every tile of the ordered kernel (flat for a few rows, 1 x 1 / 2 x 2 / 4 x 4 outputs per thread), its edges and reduction
+# remainders, with and without 16-byte copies, and the outer product of n == 1
+@pytest.mark.parametrize("m,n,p", [(1, 100, 8192), (8, 37, 513), (17, 784, 100), (100, 10, 784), (130, 65, 800), (300, 33, 1281),
+                                   (640, 130, 602), (5, 1, 44), (3, 1, 7), (33, 3, 8193)])
+def test_dense_is_bit_exact(pkg, dev, orc, m, n, p):
+    L = pkg.lib
+    a, b, bias, dy = seeded((m, n), 530), seeded((n, p), 531), seeded((p,), 532), seeded((m, p), 533)
+    ad, bd, biasd, dyd = (_t(t, dev) for t in (a, b, bias, dy))
+    out, dw, dx = torch.empty((m, p), device=dev), torch.empty((n, p), device=dev), torch.empty((m, n), device=dev)
+    pkg._lib.check(L.dcg_matmul(ad.data_ptr(), bd.data_ptr(), biasd.data_ptr(), out.data_ptr(), m, n, p, _s()))
+    pkg._lib.check(L.dcg_matmul_tn(ad.data_ptr(), dyd.data_ptr(), dw.data_ptr(), n, m, p, _s()))
+    pkg._lib.check(L.dcg_matmul_nt(dyd.data_ptr(), bd.data_ptr(), dx.data_ptr(), m, p, n, _s()))
+    assert np.array_equal(out.cpu().numpy(), orc.mat_mul_add(a, b, bias))
+    assert np.array_equal(dw.cpu().numpy(), orc.tmm_mul(a, dy))
+    assert np.array_equal(dx.cpu().numpy(), orc.mtm_mul(dy, b))
+
+
 def test_losses(pkg, dev, orc):
     L = pkg.lib
     for n in (64, 1000):
