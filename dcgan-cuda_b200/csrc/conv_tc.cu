@@ -182,6 +182,35 @@ struct PlanX3 {
 // with: measured slower at batch 64, the 256 -> 512 forward layer 38 us against 23 us.)
 int tile_width(int n_ch) { return n_ch >= 128 ? 128 : n_ch; }
 
+// How many clusters of s CTAs with one CTA's full shared memory each are resident at a time.
+int cluster_fit(int s)
+{
+    constexpr int kDevices = 64;
+    static std::mutex mutex;
+    static int fit[kDevices][kMaxCluster + 1];   // 0: not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) { cudaGetLastError(); return sm_count() / s; }
+    std::lock_guard<std::mutex> lock(mutex);
+    int& f = fit[dev][s];
+    if (f == 0) {
+        auto kernel = conv_tc_kernel<MODE_FWD, false>;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(s * sm_count()));
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = kMaxSmem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = sm_count() / s; }
+        f = n > 0 ? n : -1;
+    }
+    return f;
+}
+
 // K partitions of a tile.  Measured on every DCGAN layer at batch 64 (per-CTA timelines, partition
 // counts 1..8 forced): the shortest launch is the one with about ONE CTA per SM - a deeper pipeline
 // per CTA and half the partial-tile traffic beat a second resident CTA (e.g. the 256 -> 512 forward
@@ -207,7 +236,11 @@ int choose_splits(int tiles, int min_stages_per_tile, int ctas_per_sm = 1)
     int s = (ctas_per_sm * sms) / tiles;
     const int cap = min_stages_per_tile / 4;         // keep at least 4 K stages per CTA
     if (s > cap) s = cap;
-    if (s > kMaxCluster) s = kMaxCluster;
+    if (s > kMaxCluster) s = kMaxCluster;   // (9 to 16, the non-portable sizes, were measured: no launch got shorter)
+    // A cluster lives inside one GPC, so fewer clusters are resident than the SM count suggests (15 of 8 CTAs on the
+    // 148-SM part, not 18), and one cluster too many is a second wave: the 64 -> 128 forward of 8 images took 16.7 us as
+    // 16 clusters of 8 and takes 10.4 us as 16 of 6.
+    while (s > 1 && tiles > cluster_fit(s)) --s;
     return s < 1 ? 1 : s;
 }
 
