@@ -225,13 +225,6 @@ int choose_splits(int tiles, int min_stages_per_tile, int ctas_per_sm = 1)
         return f > kMaxCluster ? kMaxCluster : f;
     }
     const int sms = sm_count();
-    if (t_plan_x3) {
-        // 3xTF32: as many partitions as the cluster allows - each accumulation chain in the tensor
-        // core gets shorter, and the partitions are added in fp32 round-to-nearest
-        int s = min_stages_per_tile / 4;
-        if (s > kMaxCluster) s = kMaxCluster;
-        return s < 1 ? 1 : s;
-    }
     if (tiles >= sms) return 1;
     int s = (ctas_per_sm * sms) / tiles;
     const int cap = min_stages_per_tile / 4;         // keep at least 4 K stages per CTA
@@ -248,10 +241,17 @@ void finish_plan(Plan& pl)
 {
     Params& p = pl.p;
     const int b_stage = p.bn * BK * 4;
-    const int per_stage = (A_STAGE_BYTES + b_stage) * (p.x3 ? 2 : 1);   // 3xTF32: operand + residual tiles
+    const int per_stage = A_STAGE_BYTES + b_stage;
+    if (p.x3) {
+        // A and its residual take 64 TMEM columns per stage, what the accumulators (two and the small terms', or one of each
+        // where two do not fit) leave; the residuals of B, which are made ahead of that, up to four tiles
+        p.x3_slots = (512 - (p.bn <= 128 ? 3 : 2) * p.bn) / 64;
+        p.x3_slots = p.x3_slots >= 4 ? 4 : 2;   // powers of two
+        p.x3_bslots = 4;
+    }
     // two CTAs per SM when the grid has more CTAs than SMs, else one deep pipeline
     const int budget = (pl.grid > sm_count() && p.bn <= 128 && !p.x3) ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
-    int stages = budget / per_stage;
+    int stages = (budget - (p.x3 ? p.x3_bslots * b_stage : 0)) / per_stage;
     if (stages > 8) stages = 8;
     static const int forced_stages = env_int("DCG_TC_STAGES");
     if (forced_stages > 0 && forced_stages < stages) stages = forced_stages;
@@ -259,11 +259,15 @@ void finish_plan(Plan& pl)
     // the epilogue parks the 128 x bn tile (padded rows) and 128 row offsets in the (by then idle) stage ring
     while ((size_t)stages * per_stage < (size_t)kRedFloats(p.bn) * 4 + BM * 8) ++stages;
     p.stages = stages;
+    if (p.x3 && stages < 4) {   // a stage is released before its slot is used again
+        p.x3_bslots = 2;
+        p.x3_slots = 2;
+    }
 #ifdef DCG_TC_TRACING
     static const int debug = env_int("DCG_TC_DEBUG");
     p.debug = debug;
 #endif
-    pl.smem = (size_t)stages * per_stage + 1024 /*alignment slack*/ + 24 * stages + 32;
+    pl.smem = (size_t)stages * per_stage + (p.x3 ? (size_t)p.x3_bslots * b_stage : 0) + 1024 /*alignment slack*/ + 24 * stages + 64;
     p.skip_stage = -1;
     p.wait_cycles = kWaitCycles;
     pl.partial_bytes = p.splits > 1 ? (size_t)pl.grid * BM * p.bn * sizeof(float) : 0;
@@ -589,7 +593,7 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3((unsigned)(64 + 128 * (p.x3 ? kGroups<true> : kGroups<false>)));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];

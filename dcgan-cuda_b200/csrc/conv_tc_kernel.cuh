@@ -5,12 +5,43 @@
 namespace dcg {
 namespace {
 
+// ---- 3xTF32: blocks of stages ---------------------------------------------------------------------
+// The short chains used to come from eight K partitions per tile, each a CTA with its set-up, its partial tile through L2
+// and its epilogue; now a CTA sums blocks of stages in registers and the partitions follow the SM count as for plain
+// TF32.  Measured, 128 -> 256 channels at batch 64: forward 91 -> 49 us, input gradient 124 -> 61, kernel gradient
+// 80 -> 57; relative error against float64 4e-7 at every layer (3.6e-7 to 4.7e-6 before).
+constexpr int kX3Block = 4;   // K stages per block: sixteen truncating steps in a row
+constexpr int kX3Slabs = 2;    // 32-column slabs per epilogue warp: bn <= 160, every third slab
+// Groups of four epilogue warps, one warp per TMEM lane quadrant each.  3xTF32 has three: taking a stage apart is bound by
+// latency, and with two groups it paced the loop.
+template <bool X3> constexpr int kGroups = X3 ? 3 : 2;
+
+// Adds the accumulator's slabs of this warp to `sum`.
+__device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs][32], uint32_t tmem_quad, int group, int bn)
+{
+#pragma unroll
+    for (int sl = 0; sl < kX3Slabs; ++sl) {
+        const int c0 = group * 32 + sl * 32 * kGroups<true>;
+        if (c0 < bn) {
+            uint32_t r[32];
+            const bool full = bn - c0 >= 32;
+            if (full) tmem_ld_32x32b_x32(tmem_quad + (uint32_t)c0, r);
+            else tmem_ld_32x32b_x16(tmem_quad + (uint32_t)c0, r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int q = 0; q < 32; ++q)
+                if (q < 16 || full) sum[sl][q] = __fadd_rn(sum[sl][q], __uint_as_float(r[q]));
+        }
+    }
+}
+
 // ---- the kernel ---------------------------------------------------------------------------------
 template <int MODE, bool X3>
-__global__ void __launch_bounds__(kThreads, X3 ? 1 : 2)
+__global__ void __launch_bounds__(64 + 128 * kGroups<X3>, X3 ? 1 : 2)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ Params p)
 {
+    constexpr int G = kGroups<X3>, EPI = 128 * G;   // epilogue threads
     extern __shared__ uint8_t smem_raw[];
     if (threadIdx.x == 64) TC_TRACE(3072);
     TC_CTA_TRACE(0);
@@ -19,16 +50,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const long long wait_limit = p.wait_cycles;
     const uint32_t a_base = smem_base;
     const uint32_t b_base = a_base + (uint32_t)p.stages * A_STAGE_BYTES;
-    // 3xTF32: residual tiles (operand minus its TF32 part) of every stage follow the operand tiles
-    const uint32_t as_base = b_base + (uint32_t)p.stages * b_stage_bytes;
-    const uint32_t bs_base = as_base + (uint32_t)p.stages * A_STAGE_BYTES;
-    const uint32_t bar_base = X3 ? bs_base + (uint32_t)p.stages * b_stage_bytes : as_base;
+    // 3xTF32: residual tiles of B (operand minus its TF32 part) follow the operand tiles; A and its residual go to TMEM
+    const uint32_t bs_base = b_base + (uint32_t)p.stages * b_stage_bytes;
+    const uint32_t bar_base = X3 ? bs_base + (uint32_t)p.x3_bslots * b_stage_bytes : bs_base;
     // barriers: full[stages], empty[stages], tmem_full; then the TMEM base address word
     const uint32_t full_bar = bar_base;
     const uint32_t empty_bar = bar_base + 8u * p.stages;
     const uint32_t resid_bar = bar_base + 16u * p.stages;     // 3xTF32: residual tiles of the stage are written
     const uint32_t tmem_full_bar = bar_base + 24u * p.stages;
     const uint32_t tmem_slot = tmem_full_bar + 8u;
+    const uint32_t promo_full_bar = tmem_full_bar + 16u;      // 3xTF32, [2]: a block of kX3Block stages is summed ...
+    const uint32_t promo_empty_bar = tmem_full_bar + 32u;     // ... [2] and taken over into registers
     uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -38,19 +70,31 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(full_bar + 8u * s, 1);
             mbar_init(empty_bar + 8u * s, 1);
-            mbar_init(resid_bar + 8u * s, kEpi);
+            mbar_init(resid_bar + 8u * s, 128);
         }
         mbar_init(tmem_full_bar, 1);
+        if (X3) {
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(promo_full_bar + 8u * i, 1);
+                mbar_init(promo_empty_bar + 8u * i, EPI);
+            }
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     }
-    // 3xTF32 keeps the two small cross terms in an accumulator of their own (columns bn .. 2*bn): the
-    // tensor core rounds its accumulator toward zero at every step, an error that grows with the
-    // number of steps and with the accumulator's size, so the long chain of large terms is kept as
-    // short as in the plain TF32 kernel and the small terms round among themselves
+    // 3xTF32 keeps the two small cross terms in an accumulator of their own: the tensor core rounds its
+    // accumulator toward zero at every step, an error that grows with the number of steps and with the
+    // accumulator's size, so the small terms round among themselves.  The accumulator of the large terms is added (round to
+    // nearest) to registers of the epilogue warps after every kX3Block stages; where TMEM has room there are two of
+    // it, and the tensor core goes on in the other one.  The A operand is read from TMEM (32 columns of values, 32 of
+    // residuals per slot): three MMAs per K step take 12 KB from shared memory instead of 24, which is what would pace
+    // the loop.  Columns: x3_mains accumulators, the small terms, x3_slots A slots.
+    const int x3_mains = X3 && p.bn <= 128 ? 2 : 1;
+    const int x3_a0 = (x3_mains + 1) * p.bn;
+    const int x3_slot_mask = p.x3_slots - 1, x3_bslot_mask = p.x3_bslots - 1;   // powers of two
     int tmem_cols = 32;
-    while (tmem_cols < (X3 ? 2 * p.bn : p.bn)) tmem_cols <<= 1;
+    while (tmem_cols < (X3 ? x3_a0 + 64 * p.x3_slots : p.bn)) tmem_cols <<= 1;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -130,6 +174,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     float* red = reinterpret_cast<float*>(smem_raw + (a_base - smem_u32(smem_raw)));
     long long* s_rowoff = reinterpret_cast<long long*>(red + kRedFloats(p.bn));
 
+    float x3_sum[X3 ? kX3Slabs : 1][32];   // 3xTF32: the blocks of stages taken over so far
+    if constexpr (X3) {
+#pragma unroll
+        for (int sl = 0; sl < kX3Slabs; ++sl)
+#pragma unroll
+            for (int q = 0; q < 32; ++q) x3_sum[sl][q] = 0.f;
+    }
+
     if (warp == 0) {
         // ===== TMA producer =====
         // One thread issues every load.  All position bookkeeping is incremental: an integer division
@@ -207,7 +259,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1) {
         // ===== MMA issuer =====
         {
-            const int a_mn = (MODE == MODE_DK) ? 1 : 0;
+            const int a_mn = (MODE == MODE_DK && !X3) ? 1 : 0;
             const int b_mn = (MODE == MODE_DX) ? 0 : 1;
             const uint32_t idesc = make_idesc(a_mn, b_mn, p.bn, BM);
             // K-major tile: rows of 128 B, 8-row groups 1024 B apart (stride offset); one MMA (K = 8)
@@ -229,7 +281,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             {
             for (int it = 0; it < nq; ++it) {
                 if (!mbar_wait_warp(full_bar + 8u * s, phase, 1, it, wait_limit)) break;
-                if (X3 && !mbar_wait_warp(resid_bar + 8u * s, phase, 3, it, wait_limit)) break;
+                if (X3 && !mbar_wait_warp(resid_bar + 8u * s, phase, 3, it, wait_limit)) break;   // (implies full_bar)
+                // a new block starts from zero once the epilogue warps have taken the last one over
+                const int block = it / kX3Block;
+                const bool block_start = X3 && it % kX3Block == 0;
+                const int buf = block & (x3_mains - 1);
+                if (block_start && block >= x3_mains &&
+                    !mbar_wait_warp(promo_empty_bar + 8u * buf, (uint32_t)((block >> (x3_mains - 1)) - 1) & 1u, 6, it, wait_limit))
+                    break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
                 TC_TRACE(1024 + it);
@@ -241,15 +300,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (X3) {
                         // a*b ~ a_hi*b_lo + a_lo*b_hi + a_hi*b_hi, the small terms first; the tensor core
                         // reads the TF32 part (top 19 bits) of whatever fp32 word it is given
-                        const uint64_t ares = adesc + (uint64_t)((as_base - a_base) >> 4);
-                        const uint64_t bres = bdesc + (uint64_t)((bs_base - b_base) >> 4);
+                        const uint32_t ahi = tmem_d + (uint32_t)(x3_a0 + 64 * (it & x3_slot_mask)), alo = ahi + 32u;
+                        const uint32_t d_main = tmem_d + (uint32_t)(buf * p.bn), d_small = tmem_d + (uint32_t)(x3_mains * p.bn);
+                        const uint64_t bres = bdesc0 + (uint64_t)((bs_base - b_base) >> 4) + (uint64_t)((uint32_t)(it & x3_bslot_mask) * b_stage16);
 #pragma unroll
                         for (int kk = 0; kk < BK / 8; ++kk) {
-                            const uint64_t ka = (uint64_t)(kk * (a_step >> 4)), kb = (uint64_t)(kk * (b_step >> 4));
-                            const uint32_t first = (it > 0 || kk > 0) ? 1u : 0u;
-                            tcgen05_mma_tf32(tmem_d + (uint32_t)p.bn, adesc + ka, bres + kb, idesc, first);
-                            tcgen05_mma_tf32(tmem_d + (uint32_t)p.bn, ares + ka, bdesc + kb, idesc, 1u);
-                            tcgen05_mma_tf32(tmem_d, adesc + ka, bdesc + kb, idesc, first);
+                            const uint64_t kb = (uint64_t)(kk * (b_step >> 4));
+                            tcgen05_mma_tf32_ts(d_small, ahi + 8u * kk, bres + kb, idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                            tcgen05_mma_tf32_ts(d_small, alo + 8u * kk, bdesc + kb, idesc, 1u);
+                            tcgen05_mma_tf32_ts(d_main, ahi + 8u * kk, bdesc + kb, idesc, (!block_start || kk > 0) ? 1u : 0u);
                         }
                     } else {
 #pragma unroll
@@ -258,6 +317,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                              idesc, (it > 0 || kk > 0) ? 1u : 0u);
                     }
                     tcgen05_commit(empty_bar + 8u * s);  // frees the stage once these MMAs have read it
+                    if (X3 && it % kX3Block == kX3Block - 1 && it + 1 < nq) tcgen05_commit(promo_full_bar + 8u * buf);
                 }
                 TC_TRACE(2048 + it);
                 }
@@ -300,27 +360,74 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 row_off = tap_off + (unsigned long long)ch0 * p.O + o;
             }
         }
-        if (X3) {
-            // ===== 3xTF32: these four warps turn every landed stage into its residual tiles =====
-            // residual = value - (value with the low 13 mantissa bits cleared); element-wise on the raw
-            // bytes of the stage, so the swizzled layout carries over unchanged
-            const int tid_r = threadIdx.x - 64;
+        if constexpr (X3) {
+            // ===== 3xTF32: these warps take the landed stages apart, the groups of four in turn =====
+            // residual = value - (value with the low 13 mantissa bits cleared).  A: thread = row, values and residuals to
+            // the stage's TMEM columns.  B: element-wise on the raw bytes of the stage, so the swizzled layout carries
+            // over unchanged.
+            // Everything but the stores to TMEM is done before the slot is free, so that little stands between the MMAs that
+            // free it and those that read it next.
+            const int group = (warp - 2) >> 2, tid_r = (threadIdx.x - 64) & 127;
+            int turn = 0;
+            const int b_q = b_stage_bytes / 16;   // 16-byte words of a B tile
+            const int blocks = (nq + kX3Block - 1) / kX3Block;
+            int taken = 0;                        // blocks taken over so far
             int s = 0;
             uint32_t phase = 0;
-            const int a_q = A_STAGE_BYTES / 16, b_q = b_stage_bytes / 16;   // 16-byte words per tile
+            // the MMAs of the stage n before this one have completed (it was released)
+            auto mma_done = [&](int n, int it) {
+                if (it < n) return true;
+                const bool wrap = s < n;
+                const int j = wrap ? s - n + p.stages : s - n;
+                return __all_sync(0xffffffffu, mbar_wait(empty_bar + 8u * j, wrap ? phase ^ 1u : phase, 8, it, wait_limit)) != 0;
+            };
             for (int it = 0; it < nq; ++it) {
-                if (!mbar_wait(full_bar + 8u * s, phase, 4, it, wait_limit)) break;
-                const float4* asrc = reinterpret_cast<const float4*>(smem_raw + (a_base + (uint32_t)s * A_STAGE_BYTES - smem_u32(smem_raw)));
-                float4* adst = reinterpret_cast<float4*>(smem_raw + (as_base + (uint32_t)s * A_STAGE_BYTES - smem_u32(smem_raw)));
-                const float4* bsrc = reinterpret_cast<const float4*>(smem_raw + (b_base + (uint32_t)s * b_stage_bytes - smem_u32(smem_raw)));
-                float4* bdst = reinterpret_cast<float4*>(smem_raw + (bs_base + (uint32_t)s * b_stage_bytes - smem_u32(smem_raw)));
+                if (turn == group) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(full_bar + 8u * s, phase, 4, it, wait_limit))) break;
+                    const uint8_t* asrc = smem_raw + (a_base + (uint32_t)s * A_STAGE_BYTES - smem_u32(smem_raw));
+                    float v[32];
+                    if (MODE != MODE_DK) {   // K-major: the row's 128 bytes, 16-byte chunk j at j ^ (row & 7)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float4 t = *reinterpret_cast<const float4*>(asrc + row * 128 + ((j ^ (row & 7)) << 4));
+                            v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
+                        }
+                    } else {                 // MN-major: [32-row chunk][k][128 bytes], 32-byte chunk j at j ^ (k & 3)
+#pragma unroll
+                        for (int k = 0; k < 32; ++k)
+                            v[k] = *reinterpret_cast<const float*>(asrc + quad * 4096 + k * 128 + (((lane >> 3) ^ (k & 3)) << 5) + (lane & 7) * 4);
+                    }
+                    if (!mma_done(p.x3_bslots, it)) break;
+                    const float4* bsrc = reinterpret_cast<const float4*>(smem_raw + (b_base + (uint32_t)s * b_stage_bytes - smem_u32(smem_raw)));
+                    float4* bdst = reinterpret_cast<float4*>(smem_raw + (bs_base + (uint32_t)(it & x3_bslot_mask) * b_stage_bytes - smem_u32(smem_raw)));
 #pragma unroll 4
-                for (int i = tid_r; i < a_q; i += kEpi) adst[i] = tf32_residual(asrc[i]);
-#pragma unroll 4
-                for (int i = tid_r; i < b_q; i += kEpi) bdst[i] = tf32_residual(bsrc[i]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> tensor core reads
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(resid_bar + 8u * s) : "memory");
+                    for (int i = tid_r; i < b_q; i += 128) bdst[i] = tf32_residual(bsrc[i]);
+                    if (!mma_done(p.x3_slots, it)) break;
+                    const uint32_t ahi = tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)(x3_a0 + 64 * (it & x3_slot_mask));
+                    tmem_st_32x32b_x32(ahi, v);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = tf32_residual_1(v[j]);
+                    tmem_st_32x32b_x32(ahi + 32u, v);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> tensor core reads
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(resid_bar + 8u * s) : "memory");
+                }
+                if (++turn == G) turn = 0;
                 if (++s == p.stages) { s = 0; phase ^= 1u; }
+                // a block is taken over once the first two stages of the next one are ready, so that the tensor core finds
+                // work right after it
+                if (taken + 1 < blocks && it == min((taken + 1) * kX3Block + 1, nq - 1)) {
+                    const int buf = taken & (x3_mains - 1);
+                    bool got = mbar_wait(promo_full_bar + 8u * buf, (uint32_t)(taken >> (x3_mains - 1)) & 1u, 7, it, wait_limit);
+                    got = __all_sync(0xffffffffu, got);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (!got) break;
+                    x3_take_over(x3_sum, tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.bn), group, p.bn);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(promo_empty_bar + 8u * buf) : "memory");
+                    ++taken;
+                }
             }
         }
         bool ok = mbar_wait(tmem_full_bar, 0, 2, 0, wait_limit);
@@ -357,22 +464,28 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp >= 2) {
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
-        // the two warps of a lane quadrant (2..5 and 6..9) take alternate 32-column slabs
-        for (int c0 = ((warp - 2) >> 2) * 32; c0 < p.bn; c0 += 64) {
+        // the warps of a lane quadrant (one per group) take the 32-column slabs in turn
+        for (int c0 = ((warp - 2) >> 2) * 32; c0 < p.bn; c0 += 32 * G) {
             uint32_t r[32];
-            const uint32_t taddr = tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+            const uint32_t tquad = tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+            const uint32_t taddr = tquad + (X3 ? (uint32_t)(((nq > 0 ? (nq - 1) / kX3Block : 0) & (x3_mains - 1)) * p.bn) : 0u);
             const bool full = p.bn - c0 >= 32;   // bn is a multiple of 16: the last slab has 32 or 16 columns
             if (full) tmem_ld_32x32b_x32(taddr, r);
             else tmem_ld_32x32b_x16(taddr, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (X3) {   // add the accumulator of the small terms
+            if constexpr (X3) {   // add the accumulator of the small terms, then the blocks taken over before
                 uint32_t r2[32];
-                if (full) tmem_ld_32x32b_x32(taddr + (uint32_t)p.bn, r2);
-                else tmem_ld_32x32b_x16(taddr + (uint32_t)p.bn, r2);
+                if (full) tmem_ld_32x32b_x32(tquad + (uint32_t)(x3_mains * p.bn), r2);
+                else tmem_ld_32x32b_x16(tquad + (uint32_t)(x3_mains * p.bn), r2);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int q = 0; q < 32; ++q)
-                    if (q < 16 || full) r[q] = __float_as_uint(__fadd_rn(__uint_as_float(r[q]), __uint_as_float(r2[q])));
+                for (int sl = 0; sl < kX3Slabs; ++sl)
+                    if (c0 / (32 * G) == sl) {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q)
+                            if (q < 16 || full)
+                                r[q] = __float_as_uint(__fadd_rn(__fadd_rn(x3_sum[sl][q], __uint_as_float(r[q])), __uint_as_float(r2[q])));
+                    }
             }
             if (vec) {
                 if (multi) {
@@ -405,7 +518,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     TC_CTA_TRACE(3);
     __syncwarp();
     if (multi && finish_here) cluster_sync_all();
-    else if (warp >= 2) asm volatile("bar.sync 1, %0;" ::"n"(kEpi) : "memory");
+    else if (warp >= 2) asm volatile("bar.sync 1, %0;" ::"n"(EPI) : "memory");
     if (threadIdx.x == 64) TC_TRACE(3002);
     TC_CTA_TRACE(4);
 
@@ -419,13 +532,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // consecutive lanes on consecutive quads, so a warp stores whole 128-byte row segments.
             const int Qm = min(QPO, qpr - part * QPO);
             const bool by_row = multi || p.planes;               // thread = row (else: lanes walk the quads of a row)
-            // by_row: the two threads of a row (tid_e and tid_e + 128) take alternate quads
+            // by_row: the G threads of a row (tid_e, tid_e + 128, ...) take the quads in turn
             const int my_row = tid_e & (BM - 1), my_half = tid_e >> 7;
             const int row_quads = multi ? Qm : qpr;              // by_row: quads of this row's share
-            const int per_thread = by_row ? (row_quads > my_half ? (row_quads - my_half + 1) / 2 : 0)
-                                          : qpr / 2;            // single: 128 * qpr items over 256 threads (qpr is even)
+            const int per_thread = by_row ? (row_quads > my_half ? (row_quads - my_half + G - 1) / G : 0)
+                                          : (BM * qpr + EPI - 1) / EPI;   // single: 128 * qpr items over all threads
             const int quad0 = ch0 >> 2;                          // planes: global index of this tile's first quad
-            const int step_r = kEpi / qpr, step_q = kEpi % qpr;  // single: how (row, quad) moves when the item index grows by kEpi
+            const int step_r = EPI / qpr, step_q = EPI % qpr;    // single: how (row, quad) moves when the item index grows by EPI
             int rr = tid_e / qpr, q = tid_e % qpr;
             const long long my_ro = s_rowoff[my_row];
             const float4* red4 = reinterpret_cast<const float4*>(red);
@@ -439,7 +552,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const bool in = base + u < per_thread;
-                        const int qd = part * QPO + (in ? my_half + 2 * (base + u) : 0);
+                        const int qd = part * QPO + (in ? my_half + G * (base + u) : 0);
                         cq[u] = qd << 2;
                         goff[u] = (!in || my_ro < 0 || cq[u] >= ncols_valid) ? -1
                                   : p.planes ? my_ro + (long long)((unsigned long long)(quad0 + qd) * p.plane_stride)
@@ -462,7 +575,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 } else {
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const bool in = base + u < per_thread;
+                        const bool in = base + u < per_thread && rr < BM;
                         cq[u] = q << 2;
                         const long long ro = in ? s_rowoff[rr] : -1;
                         goff[u] = (ro < 0 || cq[u] >= ncols_valid) ? -1 : ro + cq[u];
@@ -526,14 +639,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // thread = row; share = every S-th column.  Used where consecutive ROWS are adjacent in
             // memory (DK with the channel roles swapped, narrow-channel DK) and for channel counts
             // that rule out 16-byte stores.
-            const int my_row = tid_e & (BM - 1), my_half = tid_e >> 7;   // the two threads of a row take alternate columns
+            const int my_row = tid_e & (BM - 1), my_half = tid_e >> 7;   // the G threads of a row take the columns in turn
             const long long ro = s_rowoff[my_row];
-            for (int cl0 = 0; 2 * cl0 + my_half < CL; cl0 += 4) {   // four columns at a time: their loads are in flight together
+            for (int cl0 = 0; G * cl0 + my_half < CL; cl0 += 4) {   // four columns at a time: their loads are in flight together
                 float acc[4];
                 int cols[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const int cl = 2 * (cl0 + u) + my_half;
+                    const int cl = G * (cl0 + u) + my_half;
                     const int col = cl * S + part;
                     cols[u] = (cl < CL && col < ncols_valid) ? col : -1;
                     const int cc = cols[u] < 0 ? 0 : cols[u];
