@@ -48,9 +48,7 @@ extern "C" size_t dcg_conv_workspace_bytes(const dcg_conv_desc* desc, int kind, 
 {
     if (!desc || precision == DCG_PREC_FP32) return 0;
     if (kind < kConvFwd || kind > kConvDk) return 0;
-    const bool x3 = precision == DCG_PREC_3XTF32;
-    if (!conv_tc_supported(*desc, kind, x3)) return 0;
-    return conv_tc_workspace(*desc, kind, x3);
+    return conv_tc_workspace(*desc, kind, precision == DCG_PREC_3XTF32);   // 0 where the tensor path does not take the shape
 }
 
 extern "C" int dcg_conv2d_fwd(const dcg_conv_desc* desc, const float* x, const float* k, float* y,

@@ -48,6 +48,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -905,16 +906,29 @@ struct CacheEntry {
     Prepared prep;
 };
 
+// Keys are compared and hashed as bytes: they are zeroed before they are filled in.
+template <typename Key>
+struct BytesEqual {
+    bool operator()(const Key& u, const Key& v) const { return std::memcmp(&u, &v, sizeof(Key)) == 0; }
+};
+template <typename Key>
+struct BytesHash {
+    size_t operator()(const Key& k) const
+    {
+        static_assert(sizeof(Key) % 4 == 0, "hashed by 32-bit words");
+        uint32_t w[sizeof(Key) / 4];
+        std::memcpy(w, &k, sizeof(Key));
+        uint64_t h = 0xcbf29ce484222325ull;
+        for (uint32_t v : w) h = (h ^ v) * 0x100000001b3ull;
+        return (size_t)(h ^ (h >> 29));
+    }
+};
+
 constexpr size_t kCacheEntries = 512;
 std::mutex g_cache_mutex;
 std::vector<CacheEntry> g_cache;
+std::unordered_map<CacheKey, size_t, BytesHash<CacheKey>, BytesEqual<CacheKey>> g_cache_at;   // where in g_cache
 size_t g_cache_next = 0;
-
-bool same_key(const CacheKey& u, const CacheKey& v)
-{
-    return u.dev == v.dev && u.kind == v.kind && u.x3 == v.x3 && u.a == v.a && u.b == v.b &&
-           u.ws == v.ws && u.ws_bytes == v.ws_bytes && std::memcmp(&u.d, &v.d, sizeof(dcg_conv_desc)) == 0;
-}
 
 // FWD: plan and maps for y = conv(x, k).  xp / k4 of a narrow-channel layer live in the scratch.
 int build_fwd(const dcg_conv_desc& d, const float* x, const float* k, void* ws, size_t ws_bytes, Prepared& pr)
@@ -1035,8 +1049,8 @@ int prepared_call(int kind, const dcg_conv_desc& d, const void* a, const void* b
     key.d = d; key.a = a; key.b = b; key.ws = ws; key.ws_bytes = ws_bytes;
     {
         std::lock_guard<std::mutex> lock(g_cache_mutex);
-        for (const CacheEntry& e : g_cache)
-            if (same_key(e.key, key)) { out = e.prep; return DCG_OK; }
+        const auto it = g_cache_at.find(key);
+        if (it != g_cache_at.end()) { out = g_cache[it->second].prep; return DCG_OK; }
     }
     int st;
     switch (kind) {
@@ -1046,31 +1060,57 @@ int prepared_call(int kind, const dcg_conv_desc& d, const void* a, const void* b
     }
     if (st) return st;
     std::lock_guard<std::mutex> lock(g_cache_mutex);
+    if (g_cache_at.count(key)) return DCG_OK;   // another thread was faster
     if (g_cache.size() < kCacheEntries) {
+        g_cache_at[key] = g_cache.size();
         g_cache.push_back(CacheEntry{key, out});
     } else {
+        g_cache_at.erase(g_cache[g_cache_next].key);
+        g_cache_at[key] = g_cache_next;
         g_cache[g_cache_next] = CacheEntry{key, out};
         g_cache_next = (g_cache_next + 1) % kCacheEntries;
     }
     return DCG_OK;
 }
 
+// ---- what the entry points ask before a call: does the tensor path take the shape, and how much scratch does it need ----
+struct QueryKey {
+    int dev, kind, x3;
+    dcg_conv_desc d;
+};
+struct QueryAnswer {
+    bool supported;
+    size_t ws_bytes;
+};
+std::mutex g_query_mutex;
+std::unordered_map<QueryKey, QueryAnswer, BytesHash<QueryKey>, BytesEqual<QueryKey>> g_query;
+
+QueryAnswer query(const dcg_conv_desc& d, int kind, bool x3)
+{
+    QueryKey key;
+    std::memset(&key, 0, sizeof(key));
+    if (cudaGetDevice(&key.dev) != cudaSuccess) { cudaGetLastError(); key.dev = -1; }
+    key.kind = kind; key.x3 = x3; key.d = d;
+    {
+        std::lock_guard<std::mutex> lock(g_query_mutex);
+        const auto it = g_query.find(key);
+        if (it != g_query.end()) return it->second;
+    }
+    PlanX3 scope(x3);
+    Plan pl;
+    QueryAnswer a{make_plan(d, kind, pl), 0};
+    if (a.supported) a.ws_bytes = pl.ws_bytes;
+    std::lock_guard<std::mutex> lock(g_query_mutex);
+    if (g_query.size() >= 4096) g_query.clear();
+    g_query[key] = a;
+    return a;
+}
+
 }  // namespace
 
-bool conv_tc_supported(const dcg_conv_desc& d, int kind, bool x3)
-{
-    PlanX3 scope(x3);
-    Plan pl;
-    return make_plan(d, kind, pl);
-}
+bool conv_tc_supported(const dcg_conv_desc& d, int kind, bool x3) { return query(d, kind, x3).supported; }
 
-size_t conv_tc_workspace(const dcg_conv_desc& d, int kind, bool x3)
-{
-    PlanX3 scope(x3);
-    Plan pl;
-    if (!make_plan(d, kind, pl)) return 0;
-    return pl.ws_bytes;
-}
+size_t conv_tc_workspace(const dcg_conv_desc& d, int kind, bool x3) { return query(d, kind, x3).ws_bytes; }
 
 int conv_tc_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep,
                 void* ws, size_t ws_bytes, cudaStream_t stream, bool x3)

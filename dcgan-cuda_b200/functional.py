@@ -27,7 +27,8 @@ def _p(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device as a handle (torch.cuda.current_stream() builds an object around it)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def conv_desc(x_shape, k_shape, strides=(2, 2), pad=None, out_hw=None):
@@ -73,14 +74,30 @@ def _workspace(dev):
     return _ws[dev]
 
 
+# What a call with these shapes, strides, pads and precision needs besides its tensors: descriptor (by reference), scratch
+# bytes, output shape.  A layer is called with the same ones over and over, and working them out costs more than the launch.
+_calls = {}
+
+
+def _call(kind, x_shape, k_shape, strides, pad, out_hw, precision):
+    key = (kind, x_shape, k_shape, tuple(strides), pad, out_hw, precision)
+    call = _calls.get(key)
+    if call is None:
+        d = conv_desc(x_shape, k_shape, strides, pad, out_hw)
+        shape = ((d.n, d.ho, d.wo, d.o), (d.n, d.h, d.w, d.c), (d.kh, d.kw, d.c, d.o))[kind]
+        if len(_calls) >= 1024:
+            _calls.clear()
+        call = _calls[key] = ctypes.byref(d), int(lib.dcg_conv_workspace_bytes(ctypes.byref(d), kind, precision)), shape
+    return call
+
+
 def conv2d_fwd(x, k, strides=(2, 2), pad=None, out_hw=None, epilogue=None, precision=_lib.PREC_TF32,
                out=None):
-    d = conv_desc(x.shape, k.shape, strides, pad, out_hw)
+    d, need, shape = _call(_lib.KIND_FWD, x.shape, k.shape, strides, pad, out_hw, precision)
     if out is None:
-        out = torch.empty((d.n, d.ho, d.wo, d.o), dtype=torch.float32, device=x.device)
-    ws, nb = _workspace(x.device).get(lib.dcg_conv_workspace_bytes(ctypes.byref(d), _lib.KIND_FWD, precision))
-    check(lib.dcg_conv2d_fwd(ctypes.byref(d), _p(x), _p(k), _p(out),
-                             ctypes.byref(epilogue) if epilogue is not None else None, precision,
+        out = torch.empty(shape, dtype=torch.float32, device=x.device)
+    ws, nb = _workspace(x.device).get(need) if need else (None, 0)
+    check(lib.dcg_conv2d_fwd(d, _p(x), _p(k), _p(out), ctypes.byref(epilogue) if epilogue is not None else None, precision,
                              ws, nb, _stream()))
     return out
 
@@ -88,28 +105,26 @@ def conv2d_fwd(x, k, strides=(2, 2), pad=None, out_hw=None, epilogue=None, preci
 def conv2d_dx(dy, k, in_hw, strides=(2, 2), pad=None, epilogue=None, precision=_lib.PREC_TF32, out=None):
     """Input gradient of conv2d: dy [n, ho, wo, o], k [kh, kw, c, o] -> dx [n, h, w, c]."""
     n, ho, wo, o = dy.shape
-    kh, kw, c, o2 = k.shape
+    c, o2 = k.shape[2:]
     assert o == o2
-    d = conv_desc((n, in_hw[0], in_hw[1], c), k.shape, strides, pad, (ho, wo))
+    d, need, shape = _call(_lib.KIND_DX, (n, in_hw[0], in_hw[1], c), k.shape, strides, pad, (ho, wo), precision)
     if out is None:
-        out = torch.empty((n, in_hw[0], in_hw[1], c), dtype=torch.float32, device=dy.device)
-    ws, nb = _workspace(dy.device).get(lib.dcg_conv_workspace_bytes(ctypes.byref(d), _lib.KIND_DX, precision))
-    check(lib.dcg_conv2d_dx(ctypes.byref(d), _p(dy), _p(k), _p(out),
-                            ctypes.byref(epilogue) if epilogue is not None else None, precision,
+        out = torch.empty(shape, dtype=torch.float32, device=dy.device)
+    ws, nb = _workspace(dy.device).get(need) if need else (None, 0)
+    check(lib.dcg_conv2d_dx(d, _p(dy), _p(k), _p(out), ctypes.byref(epilogue) if epilogue is not None else None, precision,
                             ws, nb, _stream()))
     return out
 
 
 def conv2d_dk(x, dy, k_hw, strides=(2, 2), pad=None, precision=_lib.PREC_TF32, out=None):
     """Kernel gradient of conv2d: x [n, h, w, c], dy [n, ho, wo, o] -> dk [kh, kw, c, o]."""
-    n, h, w, c = x.shape
     n2, ho, wo, o = dy.shape
-    assert n == n2
-    d = conv_desc(x.shape, (k_hw[0], k_hw[1], c, o), strides, pad, (ho, wo))
+    assert x.shape[0] == n2
+    d, need, shape = _call(_lib.KIND_DK, x.shape, (k_hw[0], k_hw[1], x.shape[3], o), strides, pad, (ho, wo), precision)
     if out is None:
-        out = torch.empty((k_hw[0], k_hw[1], c, o), dtype=torch.float32, device=x.device)
-    ws, nb = _workspace(x.device).get(lib.dcg_conv_workspace_bytes(ctypes.byref(d), _lib.KIND_DK, precision))
-    check(lib.dcg_conv2d_dk(ctypes.byref(d), _p(x), _p(dy), _p(out), precision, ws, nb, _stream()))
+        out = torch.empty(shape, dtype=torch.float32, device=x.device)
+    ws, nb = _workspace(x.device).get(need) if need else (None, 0)
+    check(lib.dcg_conv2d_dk(d, _p(x), _p(dy), _p(out), precision, ws, nb, _stream()))
     return out
 
 
@@ -134,6 +149,7 @@ def colsum(a, out=None):
     rows = a.numel() // cols
     if out is None:
         out = torch.empty((cols,), dtype=torch.float32, device=a.device)
-    ws, nb = _workspace(a.device).get(lib.dcg_colsum_workspace_bytes(rows, cols))
+    need = lib.dcg_colsum_workspace_bytes(rows, cols)
+    ws, nb = _workspace(a.device).get(need) if need else (None, 0)
     check(lib.dcg_colsum(_p(a), _p(out), rows, cols, ws, nb, _stream()))
     return out
