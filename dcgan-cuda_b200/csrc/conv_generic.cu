@@ -58,7 +58,7 @@ __device__ __forceinline__ void lds_vec(const float* s, float (&v)[W])
 // gathered sixteen bytes - four channels of one (row, tap) - at a time with cp.async and kept as it comes:
 // [row][channel quad][tap][4], row pitch 4 mod 8 words so that eight rows start in different bank quads.  The
 // weights of the forward are rows of output channels, [q][tap][channel].  Taps outside the image are zero-filled,
-// which adds +0 where the reference skips: the same bits.  Two stages of QC channels x all taps.
+// which adds +0 where the reference skips: the same bits.  Two to four stages of QC channels x all taps.
 // Bound by issue (the sum must stay unfused: two instructions per product; packed f32x2 arithmetic was measured
 // and is no faster, its operands have to be duplicated) and, where the outputs are few, by the latency of the
 // chain of dependent adds.  Measured, 5x5 / stride 2 layers: 18 TFLOP/s (a multiply and an add counted as two) of the
@@ -132,7 +132,7 @@ __device__ __forceinline__ void gather_pixels(Gather<ROWS, THREADS>& ga, const O
 __host__ __device__ constexpr int ord_pitch(int tile) { return tile + 4; }
 __host__ __device__ constexpr int ord_row_pitch(int taps, int qc) { return taps * qc % 8 == 0 ? taps * qc + 4 : taps * qc; }
 
-template <int TM, int TN, int TX, int TY, int U>   // U divides the number of taps
+template <int TM, int TN, int TX, int TY, int STAGES, int U>   // U divides the number of taps
 __global__ void __launch_bounds__(TX * TY)
 conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k, float* __restrict__ y,
                         const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec_a, const int vec_b)
@@ -182,12 +182,17 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-    load_stage(0, 0);
-    int buf = 0;
-    for (int q0 = 0; q0 < d.c; q0 += QC, buf ^= 1) {
-        if (q0 + QC < d.c) load_stage(q0 + QC, buf ^ 1);
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s * QC < d.c) load_stage(s * QC, s);
         else cp_async_commit();
-        cp_async_wait<1>();
+    }
+    int buf = 0, next = STAGES - 1;
+    for (int q0 = 0; q0 < d.c; q0 += QC) {
+        if (q0 + (STAGES - 1) * QC < d.c) load_stage(q0 + (STAGES - 1) * QC, next);
+        else cp_async_commit();
+        next = next + 1 == STAGES ? 0 : next + 1;
+        cp_async_wait<STAGES - 1>();
         __syncthreads();
         const float* as = smem + buf * stage + ty * pitch;
         const float* bs = smem + buf * stage + BMT * pitch + tx * TN;
@@ -216,6 +221,7 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
             }
         }
         __syncthreads();
+        buf = buf + 1 == STAGES ? 0 : buf + 1;
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -234,7 +240,7 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
 // Input gradient: the taps of one filter are summed first, the filters' sums added in order - so four filters at a time
 // are four independent chains, read as 16-byte words of both operands.  Each parity class of output pixels
 // (blockIdx.z) runs by itself: only taps that meet a dy pixel exist.
-template <int TM, int TN, int TX, int TY>
+template <int TM, int TN, int TX, int TY, int STAGES>
 __global__ void __launch_bounds__(TX * TY)
 conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k, float* __restrict__ dx,
                        const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec)
@@ -283,12 +289,17 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
 #pragma unroll
         for (int j = 0; j < TN; ++j) tot[i][j] = 0.f;
     if (T > 0) {
-        load_stage(0, 0);
-        int buf = 0;
-        for (int q0 = 0; q0 < d.o; q0 += QC, buf ^= 1) {
-            if (q0 + QC < d.o) load_stage(q0 + QC, buf ^ 1);
+#pragma unroll
+        for (int s = 0; s < STAGES - 1; ++s) {
+            if (s * QC < d.o) load_stage(s * QC, s);
             else cp_async_commit();
-            cp_async_wait<1>();
+        }
+        int buf = 0, next = STAGES - 1;
+        for (int q0 = 0; q0 < d.o; q0 += QC) {
+            if (q0 + (STAGES - 1) * QC < d.o) load_stage(q0 + (STAGES - 1) * QC, next);
+            else cp_async_commit();
+            next = next + 1 == STAGES ? 0 : next + 1;
+            cp_async_wait<STAGES - 1>();
             __syncthreads();
             const float *as[TM], *bs[TN];
 #pragma unroll
@@ -352,6 +363,7 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
             default: chunk(std::integral_constant<int, 0>()); break;
             }
             __syncthreads();
+            buf = buf + 1 == STAGES ? 0 : buf + 1;
         }
     }
 #pragma unroll
@@ -378,7 +390,7 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
 // A as [pixel][row] (16-byte copies where the channel count allows), B as [pixel][filter].  GROUPS thread groups
 // of a block take every GROUPS-th image each and hand their sums over in shared memory, where the first group adds
 // them in image order: more of the GPU for layers with few weights, same bits.
-template <int TM, int TN, int TX, int TY, int GROUPS>
+template <int TM, int TN, int TX, int TY, int STAGES, int GROUPS>
 __global__ void __launch_bounds__(TX * TY * GROUPS)
 conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dk,
                        const dcg_conv_desc d, const int vec_a, const int vec_b)
@@ -390,7 +402,7 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
     const int group = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
     const int M = d.kh * d.kw * d.c, P = d.ho * d.wo;
     const int m0 = blockIdx.x * BMT, n0 = blockIdx.y * BNT;
-    float* mine = smem + group * 2 * STAGE;
+    float* mine = smem + group * STAGES * STAGE;
     const uint32_t mine0 = (uint32_t)__cvta_generic_to_shared(mine);
     // gather roles: one row quad (or row) of A and one filter quad (or filter) of B, every few pixels
     const int aw = vec_a ? 4 : 1, bw = vec_b ? 4 : 1;
@@ -433,15 +445,21 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
 #pragma unroll
         for (int j = 0; j < TN; ++j) val[i][j] = tot[i][j] = 0.f;
     const int rounds = (d.n + GROUPS - 1) / GROUPS, chunks = (P + KP - 1) / KP;
-    load_stage(group, 0, 0);
-    int buf = 0;
+    // stages run through the images of this group one after the other
+    int ln = group, lck = 0;
+    auto load_next = [&](int b) {
+        load_stage(ln, lck * KP, b);
+        if (++lck == chunks) { lck = 0; ln += GROUPS; }
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) load_next(s);
+    int buf = 0, next = STAGES - 1;
     for (int rd = 0; rd < rounds; ++rd) {
         const int n = rd * GROUPS + group;
-        for (int ck = 0; ck < chunks; ++ck, buf ^= 1) {
-            if (ck + 1 < chunks) load_stage(n, (ck + 1) * KP, buf ^ 1);
-            else if (rd + 1 < rounds) load_stage(n + GROUPS, 0, buf ^ 1);
-            else cp_async_commit();
-            cp_async_wait<1>();
+        for (int ck = 0; ck < chunks; ++ck) {
+            load_next(next);
+            next = next + 1 == STAGES ? 0 : next + 1;
+            cp_async_wait<STAGES - 1>();
             __syncthreads();
             if (n < d.n) {
                 const float* as = mine + buf * STAGE + ty * TM;
@@ -478,6 +496,7 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
                 }
             }
             __syncthreads();
+            buf = buf + 1 == STAGES ? 0 : buf + 1;
         }
         if (GROUPS == 1) {
 #pragma unroll
@@ -485,7 +504,7 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
 #pragma unroll
                 for (int j = 0; j < TN; ++j) { tot[i][j] = __fadd_rn(tot[i][j], val[i][j]); val[i][j] = 0.f; }
         } else {
-            float* red = smem + GROUPS * 2 * STAGE;   // [group][item][thread]
+            float* red = smem + GROUPS * STAGES * STAGE;   // [group][item][thread]
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -535,54 +554,54 @@ int ord_channels(int taps, int contracted)
     return qc < 4 ? 4 : qc;
 }
 
-template <int TM, int TN, int TX, int TY, int U>
+template <int TM, int TN, int TX, int TY, int STAGES, int U>
 int launch_ordered_fwd_taps(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_ordered_fwd_kernel<TM, TN, TX, TY, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
+        attr_err = cudaFuncSetAttribute(conv_ordered_fwd_kernel<TM, TN, TX, TY, STAGES, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
     });
     DCG_CUDA(attr_err);
     const int taps = d.kh * d.kw, qc = ord_channels(taps, d.c);
-    const size_t smem = (size_t)2 * (BMT * ord_row_pitch(taps, qc) + qc * taps * ord_pitch(BNT)) * sizeof(float);
+    const size_t smem = (size_t)STAGES * (BMT * ord_row_pitch(taps, qc) + qc * taps * ord_pitch(BNT)) * sizeof(float);
     const long long pixels = (long long)d.n * d.ho * d.wo;
     const dim3 grid((unsigned)((pixels + BMT - 1) / BMT), (unsigned)((d.o + BNT - 1) / BNT));
-    launch_pdl(conv_ordered_fwd_kernel<TM, TN, TX, TY, U>, grid, TX * TY, smem, stream, x, k, y, d, ep, qc,
+    launch_pdl(conv_ordered_fwd_kernel<TM, TN, TX, TY, STAGES, U>, grid, TX * TY, smem, stream, x, k, y, d, ep, qc,
                d.c % 4 == 0 && aligned16(x) ? 1 : 0, d.o % 4 == 0 && aligned16(k) ? 1 : 0);
     DCG_LAUNCH_CHECK("conv_ordered_fwd_kernel");
     return DCG_OK;
 }
 
-template <int TM, int TN, int TX, int TY>
+template <int TM, int TN, int TX, int TY, int STAGES>
 int launch_ordered_fwd_tile(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
 {
     const int taps = d.kh * d.kw;
-    if (TM * TN <= 4 && taps == 25) return launch_ordered_fwd_taps<TM, TN, TX, TY, TM * TN <= 4 ? 25 : 5>(d, x, k, y, ep, stream);
-    if (taps % 5 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, 5>(d, x, k, y, ep, stream);
-    if (taps % 4 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, 4>(d, x, k, y, ep, stream);
-    if (taps % 3 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, 3>(d, x, k, y, ep, stream);
-    return launch_ordered_fwd_taps<TM, TN, TX, TY, 1>(d, x, k, y, ep, stream);
+    if (TM * TN <= 4 && taps == 25) return launch_ordered_fwd_taps<TM, TN, TX, TY, STAGES, TM * TN <= 4 ? 25 : 5>(d, x, k, y, ep, stream);
+    if (taps % 5 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, STAGES, 5>(d, x, k, y, ep, stream);
+    if (taps % 4 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, STAGES, 4>(d, x, k, y, ep, stream);
+    if (taps % 3 == 0) return launch_ordered_fwd_taps<TM, TN, TX, TY, STAGES, 3>(d, x, k, y, ep, stream);
+    return launch_ordered_fwd_taps<TM, TN, TX, TY, STAGES, 1>(d, x, k, y, ep, stream);
 }
 
-template <int TM, int TN, int TX, int TY>
+template <int TM, int TN, int TX, int TY, int STAGES>
 int launch_ordered_dx_tile(const dcg_conv_desc& d, const float* dy, const float* k, float* dx, const EpilogueArgs& ep, cudaStream_t stream)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_ordered_dx_kernel<TM, TN, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
+        attr_err = cudaFuncSetAttribute(conv_ordered_dx_kernel<TM, TN, TX, TY, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
     });
     DCG_CUDA(attr_err);
     const int mh = (d.h + d.stride_h - 1) / d.stride_h, mw = (d.w + d.stride_w - 1) / d.stride_w;   // of the largest class
     const int taps = ((d.kh + d.stride_h - 1) / d.stride_h) * ((d.kw + d.stride_w - 1) / d.stride_w);
     const int qc = ord_channels(taps, d.o);
-    const size_t smem = (size_t)2 * (BMT + BNT) * ord_row_pitch(taps, qc) * sizeof(float);
+    const size_t smem = (size_t)STAGES * (BMT + BNT) * ord_row_pitch(taps, qc) * sizeof(float);
     const dim3 grid((unsigned)(((long long)d.n * mh * mw + BMT - 1) / BMT), (unsigned)((d.c + BNT - 1) / BNT),
                     (unsigned)(d.stride_h * d.stride_w));
-    launch_pdl(conv_ordered_dx_kernel<TM, TN, TX, TY>, grid, TX * TY, smem, stream, dy, k, dx, d, ep, qc,
+    launch_pdl(conv_ordered_dx_kernel<TM, TN, TX, TY, STAGES>, grid, TX * TY, smem, stream, dy, k, dx, d, ep, qc,
                d.o % 4 == 0 && aligned16(dy) && aligned16(k) ? 1 : 0);
     DCG_LAUNCH_CHECK("conv_ordered_dx_kernel");
     return DCG_OK;
@@ -598,34 +617,34 @@ double outputs_per_lane(double outputs) { return outputs / (128.0 * sm_count());
 int launch_ordered_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
 {
     const double per_lane = outputs_per_lane((double)d.n * d.ho * d.wo * d.o);
-    if (per_lane >= kOrdWide) return launch_ordered_fwd_tile<4, 4, 16, 16>(d, x, k, y, ep, stream);
-    if (per_lane >= kOrdNormal) return launch_ordered_fwd_tile<2, 2, 16, 16>(d, x, k, y, ep, stream);
-    return launch_ordered_fwd_tile<1, 2, 8, 16>(d, x, k, y, ep, stream);
+    if (per_lane >= kOrdWide) return launch_ordered_fwd_tile<4, 4, 16, 16, 2>(d, x, k, y, ep, stream);
+    if (per_lane >= kOrdNormal) return launch_ordered_fwd_tile<2, 2, 16, 16, 2>(d, x, k, y, ep, stream);
+    return launch_ordered_fwd_tile<1, 2, 8, 16, 4>(d, x, k, y, ep, stream);
 }
 
 int launch_ordered_dx(const dcg_conv_desc& d, const float* dy, const float* k, float* dx, const EpilogueArgs& ep, cudaStream_t stream)
 {
     const double per_lane = outputs_per_lane((double)d.n * d.h * d.w * d.c);
-    if (d.c <= 4) return launch_ordered_dx_tile<1, 4, 1, 128>(d, dy, k, dx, ep, stream);   // RGB images: a pixel per thread
-    if (per_lane >= kOrdWide) return launch_ordered_dx_tile<4, 2, 16, 16>(d, dy, k, dx, ep, stream);
-    if (per_lane >= kOrdNormal) return launch_ordered_dx_tile<2, 2, 16, 16>(d, dy, k, dx, ep, stream);
-    return launch_ordered_dx_tile<1, 2, 8, 16>(d, dy, k, dx, ep, stream);
+    if (d.c <= 4) return launch_ordered_dx_tile<1, 4, 1, 128, 2>(d, dy, k, dx, ep, stream);   // RGB images: a pixel per thread
+    if (per_lane >= kOrdWide) return launch_ordered_dx_tile<4, 2, 16, 16, 2>(d, dy, k, dx, ep, stream);
+    if (per_lane >= kOrdNormal) return launch_ordered_dx_tile<2, 2, 16, 16, 2>(d, dy, k, dx, ep, stream);
+    return launch_ordered_dx_tile<1, 2, 8, 16, 4>(d, dy, k, dx, ep, stream);
 }
 
-template <int TM, int TN, int TX, int TY, int GROUPS>
+template <int TM, int TN, int TX, int TY, int STAGES, int GROUPS>
 int launch_ordered_dk_tile(const dcg_conv_desc& d, const float* x, const float* dy, float* dk, cudaStream_t stream)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX;
-    const size_t smem = (size_t)GROUPS * 2 * 32 * (ord_pitch(BMT) + ord_pitch(BNT)) * 4 + (GROUPS > 1 ? (size_t)GROUPS * BMT * BNT * 4 : 0);
+    const size_t smem = (size_t)GROUPS * STAGES * 32 * (ord_pitch(BMT) + ord_pitch(BNT)) * 4 + (GROUPS > 1 ? (size_t)GROUPS * BMT * BNT * 4 : 0);
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_ordered_dk_kernel<TM, TN, TX, TY, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
+        attr_err = cudaFuncSetAttribute(conv_ordered_dk_kernel<TM, TN, TX, TY, STAGES, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
     });
     DCG_CUDA(attr_err);
     const int M = d.kh * d.kw * d.c;
     const dim3 grid((unsigned)((M + BMT - 1) / BMT), (unsigned)((d.o + BNT - 1) / BNT));
-    launch_pdl(conv_ordered_dk_kernel<TM, TN, TX, TY, GROUPS>, grid, TX * TY * GROUPS, smem, stream, x, dy, dk, d,
+    launch_pdl(conv_ordered_dk_kernel<TM, TN, TX, TY, STAGES, GROUPS>, grid, TX * TY * GROUPS, smem, stream, x, dy, dk, d,
                d.c % 4 == 0 && aligned16(x) ? 1 : 0, d.o % 4 == 0 && aligned16(dy) ? 1 : 0);
     DCG_LAUNCH_CHECK("conv_ordered_dk_kernel");
     return DCG_OK;
@@ -635,10 +654,10 @@ int launch_ordered_dk(const dcg_conv_desc& d, const float* x, const float* dy, f
 {
     // the images of a batch are parallel work as well (GROUPS); outputs per lane as above
     const double per_lane = (double)d.kh * d.kw * d.c * d.o / (128.0 * sm_count());
-    if (per_lane >= kOrdWide) return launch_ordered_dk_tile<4, 4, 16, 16, 1>(d, x, dy, dk, stream);
-    if (per_lane < kOrdDkGrouped && d.n > 1) return launch_ordered_dk_tile<1, 2, 4, 8, 16>(d, x, dy, dk, stream);
-    if (d.n > 2) return launch_ordered_dk_tile<4, 4, 8, 8, 4>(d, x, dy, dk, stream);
-    return launch_ordered_dk_tile<2, 2, 8, 8, 1>(d, x, dy, dk, stream);
+    if (per_lane >= kOrdWide) return launch_ordered_dk_tile<4, 4, 16, 16, 2, 1>(d, x, dy, dk, stream);
+    if (per_lane < kOrdDkGrouped && d.n >= 8) return launch_ordered_dk_tile<1, 2, 4, 8, 4, 16>(d, x, dy, dk, stream);
+    if (per_lane >= kOrdDkGrouped && d.n > 2) return launch_ordered_dk_tile<4, 4, 8, 8, 2, 4>(d, x, dy, dk, stream);
+    return launch_ordered_dk_tile<2, 2, 8, 8, 4, 1>(d, x, dy, dk, stream);
 }
 
 

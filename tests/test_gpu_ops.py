@@ -72,6 +72,14 @@ def test_activations_and_grads(pkg, dev, orc, n):
     assert np.array_equal(var.cpu().numpy(), orc.vect_update(d, a, -0.37))
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 7), (3, 4), (100, 10), (100, 100), (128, 512), (256, 36), (257, 128), (513, 10), (120, 40), (31, 8200)])
+def test_colsum_of_a_few_hundred_rows(pkg, dev, rows, cols):
+    """One block per column tile up to 32 rows per thread row, partial sums beyond: both sides of that line."""
+    a = seeded((rows, cols), 515)
+    got = pkg.functional.colsum(_t(a, dev)).cpu().numpy()
+    np.testing.assert_allclose(got, a.astype(np.float64).sum(axis=0), rtol=0, atol=2e-6 * rows ** 0.5)
+
+
 def test_golden_small_ops(pkg, dev, golden):
     """The reference's unit-test tensors for bias add, activation gradients, losses, argmax."""
     L, g = pkg.lib, golden
