@@ -35,7 +35,7 @@
 // This file is the host side (tensor maps, planning, the plan cache, launches, entry points); the
 // device code of this translation unit sits in the headers it includes:
 //   conv_tc_common.cuh   constants, kernel parameters, PTX wrappers, descriptors
-//   conv_tc_kernel.cuh   conv_tc_kernel<MODE, X3>, the general kernel described above
+//   conv_tc_kernel.cuh   conv_tc_kernel<MODE, KIND>, the general kernel described above
 //   conv_tc_dxf.cuh      conv_dxf_kernel: input gradient with all parity classes of a pixel tile in one
 //                        CTA, their accumulators merged into wide MMAs
 //   conv_tc_short.cuh    conv_fwd_short_kernel: the short-K forward GEMMs of the 3-channel layers as
@@ -178,11 +178,6 @@ struct PlanX3 {
     ~PlanX3() { t_plan_x3 = saved; }
 };
 
-// Accumulator width for a layer with n_ch output columns.  (256-column tiles halve how often an A
-// tile is fetched from L2 but leave one CTA per SM with nothing to overlap its set-up and epilogue
-// with: measured slower at batch 64, the 256 -> 512 forward layer 38 us against 23 us.)
-int tile_width(int n_ch) { return n_ch >= 128 ? 128 : n_ch; }
-
 // How many clusters of s CTAs with one CTA's full shared memory each are resident at a time.
 int cluster_fit(int s)
 {
@@ -194,7 +189,7 @@ int cluster_fit(int s)
     std::lock_guard<std::mutex> lock(mutex);
     int& f = fit[dev][s];
     if (f == 0) {
-        auto kernel = conv_tc_kernel<MODE_FWD, false>;
+        auto kernel = conv_tc_kernel<MODE_FWD, kShared>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(s * sm_count()));
@@ -238,6 +233,49 @@ int choose_splits(int tiles, int min_stages_per_tile, int ctas_per_sm = 1)
     return s < 1 ? 1 : s;
 }
 
+// Shared memory of one of two CTAs per SM holds three stages up to this accumulator width.
+constexpr int kMaxSharedWidth = 160;
+
+// Accumulator width (columns of one tile) and K partitions for n_ch output columns: the quickest of the widths that split
+// n_ch evenly, by a model of the launch in SM clocks.  Its terms were read off per-CTA timelines:
+//   * a stage (K = 32) takes 300 clocks up to 128 columns - four MMAs of 69, the rest the hand-over, which kDual hides - and
+//     up to 512 at 256, where the MMAs alone set the pace (the full rate of the tensor core); the first is 1200 clocks away;
+//   * 3xTF32 takes 1150 clocks at 64 columns and 1550 at 128, the larger part of them to take the A operand apart;
+//   * the epilogue takes time per column, and two to three times that where partial tiles go through L2;
+//   * up to kMaxSharedWidth columns two CTAs share an SM, so that one's epilogue hides behind the other's stages.
+// 256 columns win where the tiles still fill the chip: the 128 -> 256 forward of 256 images takes 40.4 us for 46.7 with 128,
+// the 256 -> 512 kernel gradient 46 for 53.  They lose where they need more partitions (256 -> 512 forward of 64 images: 22
+// for 17), and where partitions would be many, narrow tiles win (128 -> 256 forward of 8 images, 64 columns: 8.8 for 10.1).
+// Channel counts between the powers of two get one tile instead of two (96 -> 160 forward of 13 images of 51 x 75: 35 for 59).
+// `m_count`: tiles along the other axis, times classes or taps; `store_cost`: clocks per column of an unpartitioned epilogue.
+struct Tiling {
+    int bn, n_tiles, splits, grid;
+    double cost;
+};
+Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost)
+{
+    static const int forced = env_int("DCG_TC_BN");
+    const int sms = sm_count();
+    const int widest = t_plan_x3 ? 128 : 256;   // 3xTF32: accumulators, residuals and A operands share TMEM
+    Tiling best{};
+    for (int n_tiles = (n_ch + widest - 1) / widest; n_tiles <= (n_ch + 63) / 64; ++n_tiles) {
+        Tiling t;
+        t.bn = ((n_ch + n_tiles - 1) / n_tiles + granule - 1) / granule * granule;
+        if (forced >= granule && forced <= widest && n_ch >= forced) t.bn = forced / granule * granule;
+        t.n_tiles = (n_ch + t.bn - 1) / t.bn;
+        t.splits = choose_splits(m_count * t.n_tiles, min_stages);
+        t.grid = m_count * t.n_tiles * t.splits;
+        const int waves = (t.grid + sms - 1) / sms;
+        const double stage = t_plan_x3 ? 750.0 + 6.25 * t.bn
+                             : t.bn > 128 ? 300.0 + (t.bn - 128) * (212.0 / 128) : t.bn <= 64 && waves == 1 ? 250.0 : 300.0;
+        const double loop = 1200.0 + (max_stages + t.splits - 1) / t.splits * stage;
+        const double epilogue = t.bn * (t.splits > 1 ? 55.0 : (double)store_cost);
+        t.cost = t.bn <= kMaxSharedWidth && !t_plan_x3 ? waves * loop + epilogue : waves * (loop + epilogue);
+        if (best.grid == 0 || t.cost < best.cost) best = t;
+    }
+    return best;
+}
+
 void finish_plan(Plan& pl)
 {
     Params& p = pl.p;
@@ -251,14 +289,17 @@ void finish_plan(Plan& pl)
         p.x3_bslots = 4;
     }
     // two CTAs per SM when the grid has more CTAs than SMs, else one deep pipeline
-    const int budget = (pl.grid > sm_count() && p.bn <= 128 && !p.x3) ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
+    const bool half = pl.grid > sm_count() && p.bn <= kMaxSharedWidth && !p.x3;
+    p.kind = p.x3 ? kX3 : half ? kShared : p.bn <= 64 ? kDual : p.splits == 1 ? kAlone : kShared;
+    const int budget = half ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
     int stages = (budget - (p.x3 ? p.x3_bslots * b_stage : 0)) / per_stage;
     if (stages > 8) stages = 8;
     static const int forced_stages = env_int("DCG_TC_STAGES");
     if (forced_stages > 0 && forced_stages < stages) stages = forced_stages;
     if (stages < 2) stages = 2;
+    if (p.kind == kDual) stages &= ~1;
     // the epilogue parks the 128 x bn tile (padded rows) and 128 row offsets in the (by then idle) stage ring
-    while ((size_t)stages * per_stage < (size_t)kRedFloats(p.bn) * 4 + BM * 8) ++stages;
+    while ((size_t)stages * per_stage < (size_t)kRedFloats(p.bn) * 4 + BM * 8) stages += p.kind == kDual ? 2 : 1;
     p.stages = stages;
     if (p.x3 && stages < 4) {   // a stage is released before its slot is used again
         p.x3_bslots = 2;
@@ -302,7 +343,15 @@ void base_params(Params& p, const dcg_conv_desc& d)
     p.m_tiles = 1; p.n_tiles = 1; p.splits = 1; p.kchunks = 1;
 }
 
-bool plan_fwd(const dcg_conv_desc& d, Plan& pl)
+void use_tiling(Plan& pl, const Tiling& t)
+{
+    pl.p.bn = t.bn; pl.p.n_tiles = t.n_tiles; pl.p.splits = t.splits;
+    pl.grid = t.grid;
+}
+
+// `fit`: the tile follows the layer; the GEMM of a narrow-channel input gradient keeps 128 columns and power-of-two boxes, as
+// the kernel with a resident B operand wants them.
+bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
 {
     const bool narrow = narrow_ok(d);
     if (!narrow && (d.c % 4 != 0 || d.o % 32 != 0 || d.stride_h > 8 || d.stride_w > 8)) return false;
@@ -311,18 +360,23 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl)
     pixel_tile(BM, d.wo, d.ho, p.TW, p.TH, p.TN);
     if (p.TW * d.stride_w > 256 || p.TH * d.stride_h > 256) return false;
     p.tiles_w = (d.wo + p.TW - 1) / p.TW; p.tiles_h = (d.ho + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
-    p.bn = narrow ? (d.o >= 128 ? 128 : d.o) : tile_width(d.o);
-    p.n_tiles = (d.o + p.bn - 1) / p.bn;
     p.kchunks = (d.c + BK - 1) / BK;
-    const int tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.n_tiles;
+    const int m_count = p.tiles_w * p.tiles_h * p.tiles_n;
     if (narrow) {
         p.narrow = 1;
         p.kchunks = 1;
         narrow_geometry(d, pl);
         pl.k4_bytes = (size_t)d.kh * 32 * d.o * sizeof(float);
     }
-    p.splits = choose_splits(tiles, narrow ? d.kh : d.kh * d.kw * p.kchunks);
-    pl.grid = tiles * p.splits;
+    const int stages = narrow ? d.kh : d.kh * d.kw * p.kchunks;
+    if (narrow || !fit) {
+        p.bn = d.o >= 128 ? 128 : d.o;
+        p.n_tiles = (d.o + p.bn - 1) / p.bn;
+        p.splits = choose_splits(m_count * p.n_tiles, stages);
+        pl.grid = m_count * p.n_tiles * p.splits;
+    } else {
+        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35));
+    }
     finish_plan(pl);
     return true;
 }
@@ -336,8 +390,6 @@ dcg_conv_desc dx_gemm_desc(const dcg_conv_desc& d, int Jp)
     return g;
 }
 
-bool plan_fwd(const dcg_conv_desc& d, Plan& pl);
-
 bool plan_dx(const dcg_conv_desc& d, Plan& pl)
 {
     if (d.c <= 4 && d.o % 32 == 0 && d.stride_h <= d.kh && d.stride_w <= d.kw) {
@@ -345,7 +397,7 @@ bool plan_dx(const dcg_conv_desc& d, Plan& pl)
         pl.Jp = Jp;
         pl.k2_bytes = (size_t)d.o * Jp * sizeof(float);
         pl.ycol_bytes = (size_t)d.n * d.ho * d.wo * Jp * sizeof(float);
-        if (plan_fwd(dx_gemm_desc(d, Jp), pl)) {
+        if (plan_fwd(dx_gemm_desc(d, Jp), pl, false)) {
             pl.p.planes = 1;
             pl.p.plane_stride = (unsigned long long)d.n * d.ho * d.wo * 4ull;
             pl.p.o_store = d.kh * d.kw * 4;   // the planes beyond the last tap are padding
@@ -360,16 +412,12 @@ bool plan_dx(const dcg_conv_desc& d, Plan& pl)
     const int ha = (d.h + d.stride_h - 1) / d.stride_h, wa = (d.w + d.stride_w - 1) / d.stride_w;
     pixel_tile(BM, wa, ha, p.TW, p.TH, p.TN);
     p.tiles_w = (wa + p.TW - 1) / p.TW; p.tiles_h = (ha + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
-    int bn = (d.c + 15) / 16 * 16;
-    if (bn > 128) bn = tile_width(bn);
-    p.bn = bn;
-    p.n_tiles = (d.c + p.bn - 1) / p.bn;
     p.kchunks = (d.o + BK - 1) / BK;
     const int classes = d.stride_h * d.stride_w;
-    const int tiles = classes * p.tiles_w * p.tiles_h * p.tiles_n * p.n_tiles;
     const int min_taps = (d.kh / d.stride_h) * (d.kw / d.stride_w);
-    p.splits = choose_splits(tiles, (min_taps < 1 ? 1 : min_taps) * p.kchunks);
-    pl.grid = tiles * p.splits;
+    const int max_taps = ((d.kh + d.stride_h - 1) / d.stride_h) * ((d.kw + d.stride_w - 1) / d.stride_w);
+    use_tiling(pl, choose_tiling(classes * p.tiles_w * p.tiles_h * p.tiles_n, d.c, 16, (min_taps < 1 ? 1 : min_taps) * p.kchunks,
+                                 max_taps * p.kchunks, 20));
     finish_plan(pl);
     return true;
 }
@@ -559,11 +607,8 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     p.swap = (d.c < BM && d.o > d.c) ? 1 : 0;
     const int m_ch = p.swap ? d.o : d.c, n_ch = p.swap ? d.c : d.o;
     p.m_tiles = (m_ch + BM - 1) / BM;
-    p.bn = tile_width(n_ch);
-    p.n_tiles = (n_ch + p.bn - 1) / p.bn;
-    const int tiles = d.kh * d.kw * p.m_tiles * p.n_tiles;
-    p.splits = choose_splits(tiles, p.tiles_w * p.tiles_h * p.tiles_n);
-    pl.grid = tiles * p.splits;
+    const int stages = p.tiles_w * p.tiles_h * p.tiles_n;
+    use_tiling(pl, choose_tiling(d.kh * d.kw * p.m_tiles, n_ch, 32, stages, stages, 20));
     finish_plan(pl);
     return true;
 }
@@ -594,7 +639,8 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)(64 + 128 * (p.x3 ? kGroups<true> : kGroups<false>)));
+    static const int groups[] = {kGroups<kShared>, kGroups<kX3>, kGroups<kAlone>, kGroups<kDual>};
+    cfg.blockDim = dim3((unsigned)(64 + 128 * groups[p.kind]));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -614,8 +660,10 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    const cudaError_t err = p.x3 ? cudaLaunchKernelEx(&cfg, conv_tc_kernel<MODE, true>, ma, mb, p)
-                                 : cudaLaunchKernelEx(&cfg, conv_tc_kernel<MODE, false>, ma, mb, p);
+    using Kernel = void (*)(CUtensorMap, CUtensorMap, Params);
+    static const Kernel kernels[] = {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>,
+                                     conv_tc_kernel<MODE, kDual>};
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernels[p.kind], ma, mb, p);
     if (err != cudaSuccess) return fail(DCG_ERR_CUDA, "conv_tc_kernel launch: %s", cudaGetErrorString(err));
     count_launch();
     return DCG_OK;
@@ -628,9 +676,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, c
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_tc_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-        if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(conv_tc_kernel<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        for (auto kernel : {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>, conv_tc_kernel<MODE, kDual>})
+            if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     });
     if (attr_err != cudaSuccess)
         return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_tc_kernel): %s", cudaGetErrorString(attr_err));

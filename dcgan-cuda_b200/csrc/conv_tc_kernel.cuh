@@ -1,4 +1,4 @@
-// conv_tc_kernel<MODE, X3>: the general tcgen05 implicit-GEMM convolution kernel (forward, input gradient by parity
+// conv_tc_kernel<MODE, KIND>: the general tcgen05 implicit-GEMM convolution kernel (forward, input gradient by parity
 // class, kernel gradient; TF32 and 3xTF32).  Included by conv_tc.cu only.
 #pragma once
 
@@ -12,16 +12,26 @@ namespace {
 // 80 -> 57; relative error against float64 4e-7 at every layer (3.6e-7 to 4.7e-6 before).
 constexpr int kX3Block = 4;   // K stages per block: sixteen truncating steps in a row
 constexpr int kX3Slabs = 2;    // 32-column slabs per epilogue warp: bn <= 160, every third slab
+
+// Kinds of launch.
+//   kShared   the plain one; two CTAs per SM where the grid is large enough
+//   kX3       3xTF32
+//   kAlone    one CTA per SM and no K partitions: more threads for the epilogue (64 -> 128 forward of 64 images 16.6 -> 15.5
+//             us; with partitions the cluster barrier of the larger CTA costs more, +0.6 to 1 us)
+//   kDual     one CTA per SM and at most 64 columns: the MMAs of a stage are too short to cover the hand-over to the next, so
+//             two warps issue them in turn, each into an accumulator of its own, and two warps load (64 -> 128 kernel
+//             gradient of 64 images 22.9 -> 20.4 us; from 128 columns on there was nothing to gain)
+enum Kind { kShared, kX3, kAlone, kDual };
 // Groups of four epilogue warps, one warp per TMEM lane quadrant each.  3xTF32 has three: taking a stage apart is bound by
 // latency, and with two groups it paced the loop.
-template <bool X3> constexpr int kGroups = X3 ? 3 : 2;
+template <int KIND> constexpr int kGroups = KIND == kX3 ? 3 : KIND == kAlone ? 4 : 2;
 
 // Adds the accumulator's slabs of this warp to `sum`.
 __device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs][32], uint32_t tmem_quad, int group, int bn)
 {
 #pragma unroll
     for (int sl = 0; sl < kX3Slabs; ++sl) {
-        const int c0 = group * 32 + sl * 32 * kGroups<true>;
+        const int c0 = group * 32 + sl * 32 * kGroups<kX3>;
         if (c0 < bn) {
             uint32_t r[32];
             const bool full = bn - c0 >= 32;
@@ -36,12 +46,16 @@ __device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs][32], uint32_
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
-template <int MODE, bool X3>
-__global__ void __launch_bounds__(64 + 128 * kGroups<X3>, X3 ? 1 : 2)
+template <int MODE, int KIND>
+__global__ void __launch_bounds__(64 + 128 * kGroups<KIND>, KIND == kShared ? 2 : 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ Params p)
 {
-    constexpr int G = kGroups<X3>, EPI = 128 * G;   // epilogue threads
+    constexpr bool X3 = KIND == kX3;
+    // Warps that take the stages in turn, as producers and as MMA issuers.  With two of them the ring has an even number of
+    // stages: a stage is then always the same warp's, which makes the parity of its barriers unambiguous.
+    constexpr int W = KIND == kDual ? 2 : 1;
+    constexpr int G = kGroups<KIND>, EPI = 128 * G;   // epilogue threads
     extern __shared__ uint8_t smem_raw[];
     if (threadIdx.x == 64) TC_TRACE(3072);
     TC_CTA_TRACE(0);
@@ -72,7 +86,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             mbar_init(empty_bar + 8u * s, 1);
             mbar_init(resid_bar + 8u * s, 128);
         }
-        mbar_init(tmem_full_bar, 1);
+        mbar_init(tmem_full_bar, W);
         if (X3) {
             for (int i = 0; i < 2; ++i) {
                 mbar_init(promo_full_bar + 8u * i, 1);
@@ -94,7 +108,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int x3_a0 = (x3_mains + 1) * p.bn;
     const int x3_slot_mask = p.x3_slots - 1, x3_bslot_mask = p.x3_bslots - 1;   // powers of two
     int tmem_cols = 32;
-    while (tmem_cols < (X3 ? x3_a0 + 64 * p.x3_slots : p.bn)) tmem_cols <<= 1;
+    while (tmem_cols < (X3 ? x3_a0 + 64 * p.x3_slots : W * p.bn)) tmem_cols <<= 1;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -182,14 +196,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int q = 0; q < 32; ++q) x3_sum[sl][q] = 0.f;
     }
 
-    if (warp == 0) {
+    const int walker = warp >> 1;   // kDual: warps 0 and 1 take the even stages; 2 and 3, until their epilogue, the odd ones
+    if (warp == 0 || (W == 2 && warp == 2)) {
         // ===== TMA producer =====
         // One thread issues every load.  All position bookkeeping is incremental: an integer division
         // costs this lone thread ~100 cycles, and the loop has to turn around in well under the 256
         // cycles the tensor core needs per stage.
         {
             const uint32_t tx_bytes = (uint32_t)(A_STAGE_BYTES + b_stage_bytes);
-            int s = 0;
+            int s = walker;
             uint32_t phase = 0;
             // counters of stage q0: FWD (chunk, tap, di, dj); DX (chunk, -, th, tw); DK (-, tile_n, tile_h, tile_w)
             int chunk = 0, tap = 0, di = 0, dj = 0;
@@ -202,7 +217,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 dj = q0 % p.tiles_w; di = (q0 / p.tiles_w) % p.tiles_h; tap = q0 / (p.tiles_w * p.tiles_h);
             }
             const int wrap_dj = (MODE == MODE_FWD) ? p.KW : taps_w;
-            for (int it = 0; it < nq; ++it) {
+            auto advance = [&] {
+                if (MODE == MODE_DK) {
+                    if (++dj == p.tiles_w) { dj = 0; if (++di == p.tiles_h) { di = 0; ++tap; } }
+                } else if (++chunk == p.kchunks) {
+                    chunk = 0; ++tap;
+                    if (++dj == wrap_dj) { dj = 0; ++di; }
+                }
+            };
+            if (walker == 1) advance();
+            for (int it = walker; it < nq; it += W) {
                 if (!mbar_wait_warp(empty_bar + 8u * s, phase ^ 1u, 0, it, wait_limit)) break;
                 const uint32_t fb = full_bar + 8u * s;
                 if (it != p.skip_stage && elect_one()) {
@@ -246,17 +270,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
                 }
-                // advance to the next stage
-                if (MODE == MODE_DK) {
-                    if (++dj == p.tiles_w) { dj = 0; if (++di == p.tiles_h) { di = 0; ++tap; } }
-                } else if (++chunk == p.kchunks) {
-                    chunk = 0; ++tap;
-                    if (++dj == wrap_dj) { dj = 0; ++di; }
-                }
-                if (++s == p.stages) { s = 0; phase ^= 1u; }
+                // on to this warp's next stage
+#pragma unroll
+                for (int i = 0; i < W; ++i) advance();
+                if ((s += W) >= p.stages) { s -= p.stages; phase ^= 1u; }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 || (W == 2 && warp == 3)) {
         // ===== MMA issuer =====
         {
             const int a_mn = (MODE == MODE_DK && !X3) ? 1 : 0;
@@ -276,10 +296,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const uint64_t adesc0 = make_smem_desc(a_base, a_lbo, a_sbo, a_lay);
             const uint64_t bdesc0 = make_smem_desc(b_base, b_lbo, b_sbo, b_lay);
             const uint32_t a_stage16 = A_STAGE_BYTES >> 4, b_stage16 = (uint32_t)b_stage_bytes >> 4;
-            int s = 0;
+            const uint32_t tmem_w = tmem_d + (uint32_t)(walker * p.bn);   // kDual: the accumulator of this warp's stages
+            int s = walker;
             uint32_t phase = 0;
             {
-            for (int it = 0; it < nq; ++it) {
+            for (int it = walker; it < nq; it += W) {
                 if (!mbar_wait_warp(full_bar + 8u * s, phase, 1, it, wait_limit)) break;
                 if (X3 && !mbar_wait_warp(resid_bar + 8u * s, phase, 3, it, wait_limit)) break;   // (implies full_bar)
                 // a new block starts from zero once the epilogue warps have taken the last one over
@@ -313,20 +334,22 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     } else {
 #pragma unroll
                         for (int kk = 0; kk < BK / 8; ++kk)
-                            tcgen05_mma_tf32(tmem_d, adesc + (uint64_t)(kk * (a_step >> 4)), bdesc + (uint64_t)(kk * (b_step >> 4)),
-                                             idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                            tcgen05_mma_tf32(tmem_w, adesc + (uint64_t)(kk * (a_step >> 4)), bdesc + (uint64_t)(kk * (b_step >> 4)),
+                                             idesc, (it >= W || kk > 0) ? 1u : 0u);
                     }
                     tcgen05_commit(empty_bar + 8u * s);  // frees the stage once these MMAs have read it
                     if (X3 && it % kX3Block == kX3Block - 1 && it + 1 < nq) tcgen05_commit(promo_full_bar + 8u * buf);
                 }
                 TC_TRACE(2048 + it);
                 }
-                if (++s == p.stages) { s = 0; phase ^= 1u; }
+                if ((s += W) >= p.stages) { s -= p.stages; phase ^= 1u; }
             }
             if (elect_one()) tcgen05_commit(tmem_full_bar);   // accumulator complete (or abandoned)
             }
         }
-    } else {
+    }
+    __syncwarp();
+    if (warp >= 2) {
         // ===== epilogue, part 1 (warps 2..5; TMEM lane quadrant = warp % 4; thread = accumulator row) =====
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
@@ -473,6 +496,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (full) tmem_ld_32x32b_x32(taddr, r);
             else tmem_ld_32x32b_x16(taddr, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (W == 2 && nq > 1) {   // the odd stages' accumulator
+                uint32_t r2[32];
+                if (full) tmem_ld_32x32b_x32(tquad + (uint32_t)p.bn, r2);
+                else tmem_ld_32x32b_x16(tquad + (uint32_t)p.bn, r2);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int q = 0; q < 32; ++q)
+                    if (q < 16 || full) r[q] = __float_as_uint(__fadd_rn(__uint_as_float(r[q]), __uint_as_float(r2[q])));
+            }
             if constexpr (X3) {   // add the accumulator of the small terms, then the blocks taken over before
                 uint32_t r2[32];
                 if (full) tmem_ld_32x32b_x32(tquad + (uint32_t)(x3_mains * p.bn), r2);

@@ -318,6 +318,30 @@ def test_full_batch_layers_tf32_vs_fp32_path(pkg, dev, layer):
     assert abs(lhs - (dk * k.double()).sum().item()) <= tol
 
 
+# accumulators 64, 96, 160 and 256 columns wide, one CTA per SM with and without K partitions, and two MMA warps on one, two
+# and an odd number of stages
+TILING_SHAPES = [
+    (13, 75, 51, 96, 3, 160, 1), (160, 16, 16, 128, 5, 256, 2), (4, 16, 16, 192, 3, 320, 1), (3, 22, 18, 64, 3, 96, 1),
+    (5, 13, 11, 32, 3, 224, 2), (1, 7, 5, 32, 1, 32, 1), (1, 7, 9, 64, 1, 64, 1), (2, 17, 9, 32, 5, 64, 1), (70, 9, 9, 64, 2, 128, 2),
+]
+
+
+@pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", TILING_SHAPES)
+def test_tile_widths(pkg, dev, shape, prec_name):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    x, k, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
+                ((51, (N, H, W, C)), (52, (K, K, C, O)), (53, (N, -(-H // s), -(-W // s), O))))
+    got, ref = ([F.conv2d_fwd(x, k, (s, s), precision=p), F.conv2d_dx(dy, k, (H, W), (s, s), precision=p),
+                 F.conv2d_dk(x, dy, (K, K), (s, s), precision=p)] for p in (getattr(pkg, PRECS[prec_name]), pkg.PREC_FP32))
+    torch.cuda.synchronize()
+    assert pkg.lib.dcg_device_status() == 0
+    tol = TF32_TOL if prec_name == "tf32" else 1e-4   # the fp32 path sums tens of thousands of pixels one by one
+    for name, a, b in zip(("fwd", "dx", "dk"), got, ref):
+        assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
+
+
 @pytest.mark.parametrize("batch", [20, 28, 40, 56, 100])
 def test_k_partition_counts(pkg, dev, batch):
     """The number of K partitions of a tile (= thread-block cluster size) follows the tile count:
