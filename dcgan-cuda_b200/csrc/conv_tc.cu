@@ -144,6 +144,20 @@ void pixel_tile(int total, int Wd, int Hd, int& tw, int& th, int& tn)
     tn = total / (tw * th);
 }
 
+// The same, or the box that covers the image with the fewest copies where that is fewer: 17 x 7 of the 128 rows for images
+// of 51 x 75 (429 boxes of 13 images; 64 x 2 takes 494).  `whole`: every row of the tile has to hold a pixel.
+void pixel_tile_fit(int total, int Wd, int Hd, int Nd, int sw, int sh, bool whole, int& tw, int& th, int& tn)
+{
+    pixel_tile(total, Wd, Hd, tw, th, tn);
+    auto boxes = [&](int a, int b, int c) { return (long long)((Wd + a - 1) / a) * ((Hd + b - 1) / b) * ((Nd + c - 1) / c); };
+    long long best = boxes(tw, th, tn);
+    for (int a = 1; a <= total && a * sw <= 256; whole ? a *= 2 : ++a)
+        for (int b = 1; a * b <= total && b * sh <= 256; whole ? b *= 2 : ++b) {
+            const int c = total / (a * b);
+            if (boxes(a, b, c) < best) { best = boxes(a, b, c); tw = a; th = b; tn = c; }
+        }
+}
+
 struct Plan {
     Params p;
     int grid;
@@ -247,12 +261,13 @@ constexpr int kMaxSharedWidth = 160;
 // the 256 -> 512 kernel gradient 46 for 53.  They lose where they need more partitions (256 -> 512 forward of 64 images: 22
 // for 17), and where partitions would be many, narrow tiles win (128 -> 256 forward of 8 images, 64 columns: 8.8 for 10.1).
 // Channel counts between the powers of two get one tile instead of two (96 -> 160 forward of 13 images of 51 x 75: 35 for 59).
-// `m_count`: tiles along the other axis, times classes or taps; `store_cost`: clocks per column of an unpartitioned epilogue.
+// `m_count`: tiles along the other axis, times classes or taps; `store_cost`: clocks per column of an unpartitioned epilogue;
+// `loads`: TMA loads per stage, of which two are in the figures above.
 struct Tiling {
     int bn, n_tiles, splits, grid;
     double cost;
 };
-Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost)
+Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost, int loads = 2)
 {
     static const int forced = env_int("DCG_TC_BN");
     const int sms = sm_count();
@@ -268,7 +283,7 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
         const int waves = (t.grid + sms - 1) / sms;
         const double stage = t_plan_x3 ? 750.0 + 6.25 * t.bn
                              : t.bn > 128 ? 300.0 + (t.bn - 128) * (212.0 / 128) : t.bn <= 64 && waves == 1 ? 250.0 : 300.0;
-        const double loop = 1200.0 + (max_stages + t.splits - 1) / t.splits * stage;
+        const double loop = 1200.0 + (max_stages + t.splits - 1) / t.splits * (stage + 20.0 * (loads - 2));
         const double epilogue = t.bn * (t.splits > 1 ? 55.0 : (double)store_cost);
         t.cost = t.bn <= kMaxSharedWidth && !t_plan_x3 ? waves * loop + epilogue : waves * (loop + epilogue);
         if (best.grid == 0 || t.cost < best.cost) best = t;
@@ -290,7 +305,7 @@ void finish_plan(Plan& pl)
     }
     // two CTAs per SM when the grid has more CTAs than SMs, else one deep pipeline
     const bool half = pl.grid > sm_count() && p.bn <= kMaxSharedWidth && !p.x3;
-    p.kind = p.x3 ? kX3 : half ? kShared : p.bn <= 64 ? kDual : p.splits == 1 ? kAlone : kShared;
+    p.kind = p.x3 ? kX3 : half ? kShared : p.bn <= 64 || p.mt > 1 ? kDual : p.splits == 1 ? kAlone : kShared;
     const int budget = half ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
     int stages = (budget - (p.x3 ? p.x3_bslots * b_stage : 0)) / per_stage;
     if (stages > 8) stages = 8;
@@ -340,7 +355,7 @@ void base_params(Params& p, const dcg_conv_desc& d)
     p.x3 = t_plan_x3;
     p.N = d.n; p.H = d.h; p.W = d.w; p.C = d.c; p.KH = d.kh; p.KW = d.kw; p.O = d.o;
     p.Ho = d.ho; p.Wo = d.wo; p.sh = d.stride_h; p.sw = d.stride_w; p.pt = d.pad_top; p.pl = d.pad_left;
-    p.m_tiles = 1; p.n_tiles = 1; p.splits = 1; p.kchunks = 1;
+    p.m_tiles = 1; p.n_tiles = 1; p.splits = 1; p.kchunks = 1; p.mt = 1;
 }
 
 void use_tiling(Plan& pl, const Tiling& t)
@@ -357,7 +372,8 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
     if (!narrow && (d.c % 4 != 0 || d.o % 32 != 0 || d.stride_h > 8 || d.stride_w > 8)) return false;
     Params& p = pl.p;
     base_params(p, d);
-    pixel_tile(BM, d.wo, d.ho, p.TW, p.TH, p.TN);
+    if (narrow || !fit) pixel_tile(BM, d.wo, d.ho, p.TW, p.TH, p.TN);
+    else pixel_tile_fit(BM, d.wo, d.ho, d.n, d.stride_w, d.stride_h, false, p.TW, p.TH, p.TN);
     if (p.TW * d.stride_w > 256 || p.TH * d.stride_h > 256) return false;
     p.tiles_w = (d.wo + p.TW - 1) / p.TW; p.tiles_h = (d.ho + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
     p.kchunks = (d.c + BK - 1) / BK;
@@ -410,7 +426,7 @@ bool plan_dx(const dcg_conv_desc& d, Plan& pl)
     Params& p = pl.p;
     base_params(p, d);
     const int ha = (d.h + d.stride_h - 1) / d.stride_h, wa = (d.w + d.stride_w - 1) / d.stride_w;
-    pixel_tile(BM, wa, ha, p.TW, p.TH, p.TN);
+    pixel_tile_fit(BM, wa, ha, d.n, 1, 1, false, p.TW, p.TH, p.TN);
     p.tiles_w = (wa + p.TW - 1) / p.TW; p.tiles_h = (ha + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
     p.kchunks = (d.o + BK - 1) / BK;
     const int classes = d.stride_h * d.stride_w;
@@ -578,7 +594,7 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     if (!narrow && (d.c % 32 != 0 || d.o % 32 != 0 || d.stride_h > 8 || d.stride_w > 8)) return false;
     Params& p = pl.p;
     base_params(p, d);
-    pixel_tile(BK, d.wo, d.ho, p.TW, p.TH, p.TN);   // 32 output pixels per K stage
+    pixel_tile_fit(BK, d.wo, d.ho, d.n, d.stride_w, d.stride_h, true, p.TW, p.TH, p.TN);   // 32 output pixels per K stage
     if (p.TW * d.stride_w > 256 || p.TH * d.stride_h > 256) return false;
     p.tiles_w = (d.wo + p.TW - 1) / p.TW; p.tiles_h = (d.ho + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
     if (narrow) {
@@ -602,13 +618,19 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
         finish_plan(pl);
         return true;
     }
-    // M (128 accumulator rows) is the input-channel axis - dk rows are then contiguous along the
-    // accumulator columns - unless that would leave the M tile part empty and o can fill it
-    p.swap = (d.c < BM && d.o > d.c) ? 1 : 0;
-    const int m_ch = p.swap ? d.o : d.c, n_ch = p.swap ? d.c : d.o;
-    p.m_tiles = (m_ch + BM - 1) / BM;
-    const int stages = p.tiles_w * p.tiles_h * p.tiles_n;
-    use_tiling(pl, choose_tiling(d.kh * d.kw * p.m_tiles, n_ch, 32, stages, stages, 20));
+    // M (128 accumulator rows) is the input-channel axis, so that dk rows are contiguous along the accumulator columns,
+    // with the channels of four or two taps on top of one another where there are only 32 or 64 of them; or M is the
+    // output-channel axis, where that is quicker.
+    const int stages = p.tiles_w * p.tiles_h * p.tiles_n, taps = d.kh * d.kw;
+    const int mt = d.c == 64 && taps >= 2 ? 2 : d.c == 32 && taps >= 4 ? 4 : 1;
+    const int rows_c = (d.c + BM - 1) / BM, rows_o = (d.o + BM - 1) / BM;
+    static const int roles = env_int("DCG_TC_ROLES");
+    const Tiling plain = choose_tiling((taps + mt - 1) / mt * rows_c, d.o, 32, stages, stages, 20, 1 + mt);
+    const Tiling swapped = choose_tiling(taps * rows_o, d.c, 32, stages, stages, 30);
+    p.swap = roles ? roles == 2 : swapped.cost < plain.cost;
+    p.m_tiles = p.swap ? rows_o : rows_c;
+    p.mt = p.swap ? 1 : mt;
+    use_tiling(pl, p.swap ? swapped : plain);
     finish_plan(pl);
     return true;
 }
@@ -663,7 +685,14 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
     using Kernel = void (*)(CUtensorMap, CUtensorMap, Params);
     static const Kernel kernels[] = {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>,
                                      conv_tc_kernel<MODE, kDual>};
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernels[p.kind], ma, mb, p);
+    Kernel kernel = kernels[p.kind];
+    if constexpr (MODE == MODE_DK) {
+        static const Kernel more_taps[2][4] = {
+            {conv_tc_kernel<MODE_DK, kShared, 2>, conv_tc_kernel<MODE_DK, kX3, 2>, nullptr, conv_tc_kernel<MODE_DK, kDual, 2>},
+            {conv_tc_kernel<MODE_DK, kShared, 4>, conv_tc_kernel<MODE_DK, kX3, 4>, nullptr, conv_tc_kernel<MODE_DK, kDual, 4>}};
+        if (p.mt > 1) kernel = more_taps[p.mt / 4][p.kind];
+    }
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
     if (err != cudaSuccess) return fail(DCG_ERR_CUDA, "conv_tc_kernel launch: %s", cudaGetErrorString(err));
     count_launch();
     return DCG_OK;
@@ -678,6 +707,10 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, c
     std::call_once(once, [] {
         for (auto kernel : {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>, conv_tc_kernel<MODE, kDual>})
             if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        if constexpr (MODE == MODE_DK)
+            for (auto kernel : {conv_tc_kernel<MODE_DK, kShared, 2>, conv_tc_kernel<MODE_DK, kShared, 4>, conv_tc_kernel<MODE_DK, kX3, 2>, conv_tc_kernel<MODE_DK, kX3, 4>,
+                                conv_tc_kernel<MODE_DK, kDual, 2>, conv_tc_kernel<MODE_DK, kDual, 4>})
+                if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     });
     if (attr_err != cudaSuccess)
         return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_tc_kernel): %s", cudaGetErrorString(attr_err));
@@ -808,7 +841,7 @@ bool short_ok(const Plan& pl)
 {
     static const int off = [] { const char* v = getenv("DCG_TC_SHORT"); return v && atoi(v) == 0 ? 1 : 0; }();
     const Params& p = pl.p;
-    if (off || p.x3 || p.splits != 1 || p.n_tiles != 1 || p.bn > 128 || p.bn % 32 != 0) return false;
+    if (off || p.x3 || p.splits != 1 || p.n_tiles != 1 || p.bn > 128 || p.bn % 32 != 0 || p.TW * p.TH * p.TN != BM) return false;
     const int ksteps = p.narrow ? p.KH : p.KH * p.KW * p.kchunks;
     if (!p.narrow && (p.KH != 1 || p.KW != 1 || !p.planes)) return false;   // the GEMM of the 3-channel input gradient
     if (p.narrow && p.planes) return false;
@@ -1078,7 +1111,7 @@ int build_dk(const dcg_conv_desc& d, const float* x, const float* dy, void* ws, 
         pr.ma = mdy; pr.mb = mx;
         return DCG_OK;
     }
-    const int x_chunks = p.swap ? p.bn / 32 : BM / 32, dy_chunks = p.swap ? BM / 32 : p.bn / 32;
+    const int x_chunks = p.swap ? p.bn / 32 : BM / 32 / p.mt, dy_chunks = p.swap ? BM / 32 : p.bn / 32;
     if ((st = map_act_5d(&mx, x, d.n, d.h, d.w, d.c, p.TW, p.TH, p.TN, d.stride_w, d.stride_h, x_chunks))) return st;
     if ((st = map_act_5d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, dy_chunks))) return st;
     if (p.swap) { pr.ma = mdy; pr.mb = mx; }

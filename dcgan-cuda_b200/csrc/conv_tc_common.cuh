@@ -66,6 +66,7 @@ struct Params {
     long long wait_cycles;        // SM clocks after which a barrier wait gives up
     int kchunks;                  // 32-wide chunks along the contracted channel axis (FWD: C, DX: O)
     int kind;                     // which conv_tc_kernel (enum Kind)
+    int mt;                       // DK: kernel taps whose input channels share the 128 rows of an M tile (1, 2, 4)
     int swap;                     // DK: M axis is o (A from dy, B from x)
     int narrow;                   // FWD/DK with <= 4 input channels: x is read through the window map
     int ext_finish;               // the K partitions only write partials; a second kernel adds them (narrow DK)

@@ -318,8 +318,9 @@ def test_full_batch_layers_tf32_vs_fp32_path(pkg, dev, layer):
     assert abs(lhs - (dk * k.double()).sum().item()) <= tol
 
 
-# accumulators 64, 96, 160 and 256 columns wide, one CTA per SM with and without K partitions, and two MMA warps on one, two
-# and an odd number of stages
+# accumulators 64, 96, 160 and 256 columns wide, one CTA per SM with and without K partitions, two MMA warps on one, two and
+# an odd number of stages, pixel boxes that do not fill their tile, and kernel gradients with the channels of two or four
+# taps in one tile, the last one part empty
 TILING_SHAPES = [
     (13, 75, 51, 96, 3, 160, 1), (160, 16, 16, 128, 5, 256, 2), (4, 16, 16, 192, 3, 320, 1), (3, 22, 18, 64, 3, 96, 1),
     (5, 13, 11, 32, 3, 224, 2), (1, 7, 5, 32, 1, 32, 1), (1, 7, 9, 64, 1, 64, 1), (2, 17, 9, 32, 5, 64, 1), (70, 9, 9, 64, 2, 128, 2),
@@ -328,7 +329,7 @@ TILING_SHAPES = [
 
 @pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
 @pytest.mark.parametrize("shape", TILING_SHAPES)
-def test_tile_widths(pkg, dev, shape, prec_name):
+def test_tile_widths_and_pixel_boxes(pkg, dev, shape, prec_name):
     F = pkg.functional
     N, H, W, C, K, O, s = shape
     x, k, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
