@@ -520,7 +520,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
         finished[best] = true;
         t.order[ci] = best;
     }
-    // stages: a window with its pairs, at most pb per stage (the stage ring holds about 48 KB per stage)
+    // stages: a window with its pairs, at most pb per stage (about 48 KB)
     const int b_tile = bn * BK * 4;
     int pb = (48 * 1024 - A_STAGE_BYTES) / b_tile;
     if (pb > 4) pb = 4;
@@ -529,9 +529,9 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     // of one row / one column parity are neighbours, so that the pairs of a window merge into wide MMAs
     for (int c = 0; c < ncls; ++c) t.slot_of_class[c] = c;
     if (d.stride_h == 2 && d.stride_w == 2) { t.slot_of_class[2] = 3; t.slot_of_class[3] = 2; }
-    int last_stage[4] = {-1, -1, -1, -1}, last_pair[4] = {0, 0, 0, 0};
+    int last_stage[4] = {-1, -1, -1, -1};
     bool started[4] = {false, false, false, false};
-    int ns = 0;
+    int ns = 0, max_units = 0;
     for (size_t w = 0; w < wins.size(); ++w) {
         if (wins[w].first < -128 || wins[w].first > 127 || wins[w].second < -128 || wins[w].second > 127) return false;
         // the pairs of this window in TMEM order
@@ -546,41 +546,37 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
             CfWin& cw = t.win[ns];
             cw.sy = (signed char)wins[w].first; cw.sx = (signed char)wins[w].second;
             const size_t end = std::min(mine.size(), first + (size_t)pb);
-            int group_start = -1;
             for (size_t a = first; a < end; ++a) {
                 const Pair& q = mine[a];
-                const int j = cw.n;
                 const int slot = t.slot_of_class[q.cls];
-                const bool fresh = !started[q.cls];
-                cw.cls[j] = (unsigned char)q.cls; cw.kh[j] = (unsigned char)q.kh; cw.kw[j] = (unsigned char)q.kw;
-                cw.slot[j] = (unsigned char)slot;
-                if (fresh) cw.fresh |= (unsigned char)(1u << j);
+                const int fresh = started[q.cls] ? 0 : 1;
+                cw.kh[cw.n] = (unsigned char)q.kh; cw.kw[cw.n] = (unsigned char)q.kw;
                 // joins the running MMA if its accumulator follows directly, starts the same way and N stays <= 256
-                const bool join = group_start >= 0 && cw.slot[j - 1] + 1 == slot &&
-                                  (((cw.fresh >> group_start) & 1u) != 0) == fresh &&
-                                  (cw.glen[group_start] + 1) * bn <= 256;
-                if (join) ++cw.glen[group_start];
-                else { group_start = j; cw.glen[j] = 1; }
-                last_stage[q.cls] = ns; last_pair[q.cls] = j;
+                CfRun* run = cw.runs > 0 ? &cw.run[cw.runs - 1] : nullptr;
+                if (run && run->slot + run->count == slot && run->fresh == fresh && (run->count + 1) * bn <= 256) ++run->count;
+                else cw.run[cw.runs++] = {1, (unsigned char)slot, cw.n, (unsigned char)fresh};
+                last_stage[q.cls] = ns;
                 ++cw.n;
             }
-            for (int j = 0; j < cw.n; ++j) started[cw.cls[j]] = true;
+            for (size_t a = first; a < end; ++a) started[mine[a].cls] = true;
+            cw.units = (unsigned char)((A_STAGE_BYTES + cw.n * b_tile + kCfUnit - 1) / kCfUnit);
+            if (cw.units > max_units) max_units = cw.units;
             ++ns;
         }
     }
     t.nwin = ns;
     for (int c = 0; c < ncls; ++c) {
         if (last_stage[c] < 0) return false;
-        t.win[last_stage[c]].last |= (unsigned char)(1u << last_pair[c]);
+        t.win[last_stage[c]].last |= (unsigned char)(1u << c);
     }
-    t.slot_bytes = A_STAGE_BYTES + pb * b_tile;
     p.splits = 1;
     pl.grid = tiles;
-    int stages = (kMaxSmem - 1024 - kCfRedBytes() - 256) / t.slot_bytes;
-    if (stages > 8) stages = 8;
-    if (stages < 3) return false;
-    p.stages = stages;
-    pl.smem = (size_t)stages * t.slot_bytes + 1024 + kCfRedBytes() + 16 * stages + 64;
+    const int fixed = 1024 + kCfEpi / 32 * kCfPatch + 16 * kCfMaxUnits + 64;
+    int units = (kMaxSmem - fixed) / kCfUnit;
+    if (units > kCfMaxUnits) units = kCfMaxUnits;
+    if (units < 3 * max_units) return false;   // three stages in flight
+    p.stages = units;
+    pl.smem = (size_t)units * kCfUnit + fixed;
     p.skip_stage = -1;
     p.wait_cycles = kWaitCycles;
     pl.partial_bytes = 0;
@@ -815,7 +811,7 @@ int launch_dxf(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t st
     p.wait_cycles = g_wait_cycles.load();
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)pr.pl.grid);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kCfThreads);
     cfg.dynamicSmemBytes = pr.pl.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
