@@ -571,7 +571,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     }
     p.splits = 1;
     pl.grid = tiles;
-    const int fixed = 1024 + kCfEpi / 32 * kCfPatch + 16 * kCfMaxUnits + 64;
+    const int fixed = 1024 + kCfEpi / 32 * kCfPatch + 16 * kCfBars + 64;
     int units = (kMaxSmem - fixed) / kCfUnit;
     if (units > kCfMaxUnits) units = kCfMaxUnits;
     if (units < 3 * max_units) return false;   // three stages in flight

@@ -23,8 +23,9 @@ namespace {
 //
 // A load takes about 1750 clocks to land while the chip is busy, so what is in flight paces the short stages: with slots
 // sized for the longest one (48 KB) a stage of two pairs took 650 clocks for 277 of MMAs.  The ring is therefore cut into
-// units of 16 KB, of which a stage takes the two or three that it needs, with a barrier per unit.  The epilogue has 16
-// warps, each of which transposes 32 rows x 16 columns in a patch of its own - no block-wide barrier - and asks for the
+// units of 16 KB, of which a stage takes the two or three that it needs, and its barriers go by the stage's number.  Issuing
+// five loads takes a warp as long as their MMAs take, so two warps load the stages in turn.  The epilogue has 16 warps,
+// each of which transposes 32 rows x 16 columns in a patch of its own - no block-wide barrier - and asks for the
 // gate before the class is complete.
 //
 // The accumulators of the classes sit side by side in TMEM, and the weight tiles of a stage are stacked
@@ -54,7 +55,8 @@ struct CfTable {
 };
 constexpr int kCfUnit = A_STAGE_BYTES;     // ring unit
 constexpr int kCfMaxUnits = 16;
-constexpr int kCfEpi = 512, kCfThreads = 64 + kCfEpi;
+constexpr int kCfBars = 16;                // barrier pairs: stage q uses pair q % 16 (every stage takes two units or more: at most 8 in flight)
+constexpr int kCfEpi = 512, kCfThreads = 64 + kCfEpi + 32;   // producer, MMA, 16 epilogue warps, second producer
 constexpr int kCfPatch = 32 * 16 * 4;      // bytes of an epilogue warp's patch
 
 // The fused chain over four 16-byte items at once: every optional step is tested once.  goff < 0 marks an item that is not
@@ -132,9 +134,9 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int units = p.stages;                             // ring units
     const uint32_t patch_base = ring + (uint32_t)(units * kCfUnit);
     const uint32_t bar_base = patch_base + (uint32_t)(kCfEpi / 32 * kCfPatch);
-    const uint32_t full_bar = bar_base;                     // [unit]: the stage that starts there has landed
-    const uint32_t empty_bar = bar_base + 8u * units;       // [unit]: the MMAs that read it have completed
-    const uint32_t cls_bar = bar_base + 16u * units;        // accumulator of class c complete
+    const uint32_t full_bar = bar_base;                     // the stage has landed
+    const uint32_t empty_bar = bar_base + 8u * kCfBars;     // the MMAs that read it have completed
+    const uint32_t cls_bar = bar_base + 16u * kCfBars;      // accumulator of class c complete
     const uint32_t tmem_slot = cls_bar + 32u;
     uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem0));
 
@@ -143,7 +145,7 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const uint32_t b_bytes = (uint32_t)p.bn * BK * 4;
 
     if (threadIdx.x == 0) {
-        for (int u = 0; u < units; ++u) {
+        for (int u = 0; u < kCfBars; ++u) {
             mbar_init(full_bar + 8u * u, 1);
             mbar_init(empty_bar + 8u * u, 1);
         }
@@ -173,10 +175,18 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    if (warp == 0) {
-        // ===== TMA producer: for every table entry, for every channel chunk: the window, then its weight tiles =====
-        int u = 0, it = 0;
-        uint32_t phase = 0;   // bit u: parity of unit u's next use
+    if (warp == 0 || warp == 2 + kCfEpi / 32) {
+        // ===== TMA producers: for every table entry, for every channel chunk: the window, then its weight tiles =====
+        // Both walk all stages, to know where each one lies, and load the even ones or the odd ones.
+        const int mine = warp == 0 ? 0 : 1;
+        int u = 0, q = 0;
+        uint32_t used = 0;                // bit u: unit u has been part of a stage ...
+        unsigned long long owner = 0;     // ... four bits per unit: the last such stage's number modulo 16
+        auto own = [&](int first, int end, int stage) {
+            const unsigned long long mask = (~0ull >> (64 - 4 * (end - first))) << (4 * first);
+            owner = (owner & ~mask) | ((0x1111111111111111ull * (unsigned long long)(stage & 15)) & mask);
+            used |= ((1u << (end - first)) - 1u) << first;
+        };
         bool alive = true;
         for (int w = 0; w < nwin && alive; ++w) {
             const CfWin& wn = t.win[w];
@@ -185,21 +195,29 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
             for (int j = 0; j < 4; ++j) { kh[j] = wn.kh[j]; kw[j] = wn.kw[j]; }
             const uint32_t tx_bytes = (uint32_t)A_STAGE_BYTES + (uint32_t)np * b_bytes;
-            for (int chunk = 0; chunk < p.kchunks; ++chunk, ++it) {
-                if (u + nu > units) u = 0;   // a stage is contiguous
-                for (int i = 0; i < nu && alive; ++i)
-                    alive = mbar_wait_warp(empty_bar + 8u * (u + i), ((phase >> (u + i)) & 1u) ^ 1u, 0, it, wait_limit);
-                if (!alive) break;
-                phase ^= ((1u << nu) - 1u) << u;
-                if (elect_one()) {
-                    const uint32_t fb = full_bar + 8u * u;
-                    const uint32_t dst = ring + (uint32_t)(u * kCfUnit);
-                    mbar_expect_tx(fb, tx_bytes);
-                    tma_load_4d(dst, &map_a, fb, chunk * BK, aj, ai, n0);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (j < np) tma_load_4d(dst + (uint32_t)A_STAGE_BYTES + (uint32_t)j * b_bytes, &map_b, fb, chunk * BK, ch0, kw[j], kh[j]);
+            for (int chunk = 0; chunk < p.kchunks; ++chunk, ++q) {
+                if (u + nu > units) {   // a stage is contiguous; what is left over counts as the last stage's
+                    own(u, units, q - 1);
+                    u = 0;
                 }
+                if ((q & 1) == mine) {
+                    // stages complete in order: the last unit's owner is the youngest that has to be out of the way
+                    const int last = u + nu - 1;
+                    if ((used >> last) & 1u) {
+                        const int slot = (int)(owner >> (4 * last)) & 15, prev = q - 1 - ((q - 1 - slot) & 15);
+                        if (!mbar_wait_warp(empty_bar + 8u * slot, (uint32_t)(prev >> 4) & 1u, 0, q, wait_limit)) { alive = false; break; }
+                    }
+                    if (elect_one()) {
+                        const uint32_t fb = full_bar + 8u * (q & 15);
+                        const uint32_t dst = ring + (uint32_t)(u * kCfUnit);
+                        mbar_expect_tx(fb, tx_bytes);
+                        tma_load_4d(dst, &map_a, fb, chunk * BK, aj, ai, n0);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (j < np) tma_load_4d(dst + (uint32_t)A_STAGE_BYTES + (uint32_t)j * b_bytes, &map_b, fb, chunk * BK, ch0, kw[j], kh[j]);
+                    }
+                }
+                own(u, u + nu, q);
                 u += nu;
                 if (u == units) u = 0;
             }
@@ -230,14 +248,13 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             return r;
         };
         int u = 0, it = 0;
-        uint32_t phase = 0, done = 0;   // bit u of `phase`: parity of the next stage that starts at unit u
+        uint32_t done = 0;
         bool alive = true;
         Runs cur = fetch(0), next = cur;
         for (int w = 0; w < nwin && alive; ++w) {
             for (int chunk = 0; chunk < p.kchunks; ++chunk, ++it) {
                 if (u + cur.units > units) u = 0;
-                if (!mbar_wait_warp(full_bar + 8u * u, (phase >> u) & 1u, 1, it, wait_limit)) { alive = false; break; }
-                phase ^= 1u << u;
+                if (!mbar_wait_warp(full_bar + 8u * (it & 15), (uint32_t)(it >> 4) & 1u, 1, it, wait_limit)) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const bool final_chunk = chunk == p.kchunks - 1;
                 if (elect_one()) {
@@ -252,7 +269,7 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                 tcgen05_mma_tf32(cur.acc[r], adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), cur.idesc[r],
                                                  (overwrite && kk == 0) ? 0u : 1u);
                         }
-                    for (int i = 0; i < cur.units; ++i) tcgen05_commit(empty_bar + 8u * (u + i));
+                    tcgen05_commit(empty_bar + 8u * (it & 15));
                     if (final_chunk) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
