@@ -1,8 +1,9 @@
-"""Builds libdcgan_b200.so from csrc/*.cu with nvcc for sm_100a, in-tree.
+"""Builds libdcgan_b200.so from csrc/*.cu with nvcc for sm_100a, in-tree, and _binding.so next to it.
 
 One nvcc invocation per translation unit (run in parallel), objects cached by
 modification time under csrc/build/, then one link step.  No GPU is needed:
-nvcc cross-compiles.
+nvcc cross-compiles.  _binding.so (csrc/torch_binding.cpp, g++) is the Python
+module through which functional.py calls the library on torch tensors.
 
 Run: ``python dcgan-cuda_b200/build.py [--force] [--verbose]``
 
@@ -14,12 +15,15 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libdcgan_b200.so")
+BINDING_SRC = os.path.join(CSRC, "torch_binding.cpp")
+BINDING = os.path.join(HERE, "_binding.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -56,7 +60,24 @@ def build(force=False, verbose=False):
         # library loads on a machine without a driver (symbol checks on CPU boxes).
         cmd = [NVCC] + ARCH + ["-shared", "-o", LIB] + objs
         subprocess.check_call(cmd)
+    _build_binding(force)
     return LIB
+
+
+def _build_binding(force):
+    newest = max(os.path.getmtime(p) for p in [BINDING_SRC] + _deps())
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= newest:
+        return
+    import torch
+    root = os.path.join(os.path.dirname(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"],
+           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-isystem", os.path.join(cuda, "include"), BINDING_SRC, "-o", BINDING,
+           "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+           "-L", HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    subprocess.check_call(cmd)
 
 
 if __name__ == "__main__":
