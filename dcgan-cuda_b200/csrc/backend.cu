@@ -593,6 +593,7 @@ int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, flo
 int softmax_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t rows, size_t cols, cudaStream_t stream);
 int matmul_act(const float* a, const float* b, const float* bias, float* out, size_t m, size_t n, size_t p, int act, float alpha,
                float* act_out, cudaStream_t stream);
+int matmul_tn_sums(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, float* sums, cudaStream_t stream);
 int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const float* gate,
                     float* gated_out, int gate_act, float gate_alpha, cudaStream_t stream);
 }  // namespace dcg
@@ -731,6 +732,18 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
                 if (st) return st;
                 i += 2;
                 continue;
+            }
+        }
+        if (i + 1 < count && !(nodes[i + 1].flags & DCG_NODE_SIDE)) {
+            // weight and bias gradient of a dense layer: both read the output gradient
+            const dcg_node& a = nodes[i];
+            const dcg_node& b = nodes[i + 1];
+            if (a.type == DCG_OP_TMAT_MAT_MUL && b.type == DCG_OP_MAT_SUM_COLS && b.in1 == a.in2 && b.len1 == a.len2 &&
+                b.len2 == a.len3 && a.out1 != b.out1 && a.out1 != b.in1 && ctx->precision != DCG_PREC_FP32) {
+                ProfScope scope(ctx, "tmat_mat_mul", 0.0);
+                const int st = dcg::matmul_tn_sums(a.in1, a.in2, a.out1, a.len1, a.len2, a.len3, b.out1, ctx->stream);
+                if (st < 0) return st;
+                if (st == 0) { i += 2; continue; }
             }
         }
         AdamTriple first;

@@ -7,6 +7,7 @@
 // reduction (8192 -> 1), and tall output from a transposed operand (the head's weight gradient).
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -45,20 +46,21 @@ struct DenseEpilogue {
     float* out2;
     int act;         // of out2: activation, or with `gate` the activation whose gradient gates
     float alpha;
+    float* sums;     // TA only: column sums of B, k ascending
 };
 
-// out[m,p] = A[m,n] B[n,p]: TM x TN outputs per thread, TX x TY threads per block, STAGES stages of KC = 64 reduction steps
+// out[m,p] = A[m,n] B[n,p]: TM x TN outputs per thread, TX x TY threads per block, STAGES stages of KC reduction steps
 // filled with cp.async.  TA / TB: the logical matrix is the transpose of the stored row-major one.  An operand whose
 // reduction axis is contiguous keeps it so in shared memory ([row][k], four steps per 16-byte read), the other is
 // [k][row].  What is beyond an edge is zero-filled; the zeros add +0 to the sums.
 // Latency-bound at the sizes of this library: many small tiles and all loads of several stages in flight matter more than
-// operand reuse (100 x 784 x 100: 160 us with one 64 x 64 tile per block and blocking loads, 8 us as 49 tiles of 16 x 16).
-template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES>
+// operand reuse (100 x 784 x 100: 160 us with one 64 x 64 tile per block and blocking loads).
+template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES, int KC>
 __global__ void __launch_bounds__(TX * TY)
 gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const int m, const int n,
                     const int p, const DenseEpilogue e, const int vec_a, const int vec_b)
 {
-    constexpr int BM = TM * TY, BN = TN * TX, THREADS = TX * TY, KC = 64;
+    constexpr int BM = TM * TY, BN = TN * TX, THREADS = TX * TY;
     constexpr int LDA = TA ? BM + 4 : KC + 4, LDB = TB ? KC + 4 : BN + 4;
     constexpr int A_FLOATS = (TA ? KC : BM) * LDA, STAGE = A_FLOATS + (TB ? BN : KC) * LDB;
     extern __shared__ __align__(16) float smem[];
@@ -67,23 +69,30 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
     const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
     const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(smem);
 
-    // copies a tile of `inner` contiguous elements x `outer` lines, element (o, i) of the stored matrix at base[o * ld + i]
-    auto copy_tile = [&](uint32_t dst, int pitch, const float* base, int o0, int i0, int outer, int inner, int o_end, int i_end, int vec) {
-        const int w = vec ? 4 : 1, per_line = inner / w;
+    // copies a tile of `inner` contiguous elements x `outer` lines, element (o, i) of the stored matrix at base[o * ld + i];
+    // `inner` and the width of a copy are constants, so that a thread's places take shifts, not divisions
+    auto copy_words = [&](auto inner_c, auto w_c, uint32_t dst, int pitch, const float* base, int o0, int i0, int outer, int limit, int o_end, int i_end) {
+        constexpr int w = decltype(w_c)::value, per_line = decltype(inner_c)::value / w;
         for (int idx = tid; idx < outer * per_line; idx += THREADS) {
             const int o = idx / per_line, i = (idx - o * per_line) * w;
+            if (i >= limit) continue;
             const bool in = o0 + o < o_end && i0 + i < i_end;
             cp_async(dst + 4u * (uint32_t)(o * pitch + i), in ? base + (size_t)(o0 + o) * i_end + i0 + i : base, in, 4 * w);
         }
     };
+    auto copy_tile = [&](auto inner_c, uint32_t dst, int pitch, const float* base, int o0, int i0, int outer, int limit, int o_end, int i_end, int vec) {
+        if (vec) copy_words(inner_c, std::integral_constant<int, 4>(), dst, pitch, base, o0, i0, outer, limit, o_end, i_end);
+        else copy_words(inner_c, std::integral_constant<int, 1>(), dst, pitch, base, o0, i0, outer, limit, o_end, i_end);
+    };
+    using std::integral_constant;
     auto load_stage = [&](int k0, int buf) {
         if (k0 < n) {
             const uint32_t as = smem0 + 4u * (uint32_t)(buf * STAGE), bs = as + 4u * (uint32_t)A_FLOATS;
             const int kc = min(KC, (n - k0 + 3) & ~3);
-            if (TA) copy_tile(as, LDA, a, k0, row0, kc, BM, n, m, vec_a);
-            else copy_tile(as, LDA, a, row0, k0, BM, kc, m, n, vec_a);
-            if (TB) copy_tile(bs, LDB, b, col0, k0, BN, kc, p, n, vec_b);
-            else copy_tile(bs, LDB, b, k0, col0, kc, BN, n, p, vec_b);
+            if (TA) copy_tile(integral_constant<int, BM>(), as, LDA, a, k0, row0, kc, BM, n, m, vec_a);
+            else copy_tile(integral_constant<int, KC>(), as, LDA, a, row0, k0, BM, kc, m, n, vec_a);
+            if (TB) copy_tile(integral_constant<int, KC>(), bs, LDB, b, col0, k0, BN, kc, p, n, vec_b);
+            else copy_tile(integral_constant<int, BN>(), bs, LDB, b, k0, col0, kc, BN, n, p, vec_b);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -94,6 +103,11 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) load_stage(s * KC, s);
+    // the blocks and threads of the first row add up B as well
+    const bool sum_b = TA && !TB && e.sums && blockIdx.y == 0 && ty == 0;
+    float bsum[TN];
+#pragma unroll
+    for (int j = 0; j < TN; ++j) bsum[j] = 0.f;
     int buf = 0;
     for (int k0 = 0; k0 < n; k0 += KC) {
         load_stage(k0 + (STAGES - 1) * KC, (buf + STAGES - 1) % STAGES);
@@ -102,7 +116,7 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
         const float* as = smem + buf * STAGE + (TA ? ty * TM : ty * TM * LDA);
         const float* bs = smem + buf * STAGE + A_FLOATS + (TB ? tx * LDB : tx * TN);   // TB: columns tx, tx + TX, ...
         const int kc = min(KC, (n - k0 + 3) & ~3);
-#pragma unroll 4
+#pragma unroll KC / 16
         for (int k = 0; k < kc; k += 4) {
             float av[4][TM], bv[4][TN];
             if (TA) {
@@ -127,6 +141,12 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
 #pragma unroll
                 for (int u = 0; u < 4; ++u) tile_read<TN>(bs + (k + u) * LDB, bv[u]);
             }
+            if (sum_b) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) bsum[j] = __fadd_rn(bsum[j], bv[u][j]);
+            }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -136,6 +156,11 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
         }
         __syncthreads();
         buf = (buf + 1) % STAGES;
+    }
+    if (sum_b) {
+#pragma unroll
+        for (int j = 0; j < TN; ++j)
+            if (col0 + tx * TN + j < p) e.sums[col0 + tx * TN + j] = bsum[j];
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -245,21 +270,21 @@ gemm_tall_tn_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
 
 bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
-template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES>
+template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES, int KC = 64>
 int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const DenseEpilogue& e, cudaStream_t stream)
 {
-    constexpr int BM = TM * TY, BN = TN * TX, KC = 64;
+    constexpr int BM = TM * TY, BN = TN * TX;
     constexpr size_t smem = (size_t)STAGES * ((TA ? KC * (BM + 4) : BM * (KC + 4)) + (TB ? BN * (KC + 4) : KC * (BN + 4))) * sizeof(float);
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES>,
+        attr_err = cudaFuncSetAttribute(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
     DCG_CUDA(attr_err);
     const dim3 grid((unsigned)((p + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
     const int vec_a = (TA ? m : n) % 4 == 0 && aligned16(a), vec_b = (TB ? n : p) % 4 == 0 && aligned16(b);
-    launch_pdl(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES>, grid, TX * TY, smem, stream, a, b, out, (int)m, (int)n, (int)p, e,
+    launch_pdl(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>, grid, TX * TY, smem, stream, a, b, out, (int)m, (int)n, (int)p, e,
                vec_a, vec_b);
     DCG_LAUNCH_CHECK("gemm_ordered_kernel");
     return DCG_OK;
@@ -285,6 +310,13 @@ int launch_ordered(const float* a, const float* b, float* out, size_t m, size_t 
     if (m <= 8 && p >= 512) return launch_tile<TA, TB, 1, 1, 32, 8, 3>(a, b, out, m, n, p, e, stream);
     if (per_lane >= 20) return launch_tile<TA, TB, 4, 4, 16, 16, 2>(a, b, out, m, n, p, e, stream);
     if (per_lane >= 5) return launch_tile<TA, TB, 2, 2, 16, 16, 3>(a, b, out, m, n, p, e, stream);
+    // Where 16 x 16 tiles would leave half of the SMs without a block, smaller ones; each sum is one chain of K steps, so what
+    // counts is how few warps share an SM and, for long ones, how many steps there are between two barriers (100 x 784 x 100:
+    // 11.8 us as 16 x 16 tiles, 9.7 as 8 x 16 of 128 steps; 100 x 100 x 10 2.9 as 8 x 8)
+    if (per_lane < 1 && n >= 512) return launch_tile<TA, TB, 1, 1, 8, 16, 4, 128>(a, b, out, m, n, p, e, stream);
+    if (per_lane < 1) return launch_tile<TA, TB, 1, 1, 8, 8, 4>(a, b, out, m, n, p, e, stream);
+    // (rows of A^T are contiguous: two to a thread are one read; 784 x 100 x 100 5.3 -> 4.4 us)
+    if (TA && per_lane >= 2) return launch_tile<TA, TB, 2, 1, 16, 8, 3>(a, b, out, m, n, p, e, stream);
     return launch_tile<TA, TB, 1, 1, 16, 16, 4>(a, b, out, m, n, p, e, stream);
 }
 
@@ -316,6 +348,17 @@ int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t
 {
     DCG_CHECK_ARG(a && b && out && gate && gated_out && m > 0 && n > 0 && p > 0, "matmul_nt_gated: bad arguments");
     return launch_ordered<false, true>(a, b, out, m, n, p, DenseEpilogue{nullptr, gate, gated_out, gate_act, gate_alpha}, stream);
+}
+
+// dcg_matmul_tn and the column sums of its right operand as one launch (node fusion of the backend): the weight and the bias
+// gradient of a dense layer.  Not for the shapes of gemm_tall_tn_kernel: returns 1 there.
+int matmul_tn_sums(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, float* sums, cudaStream_t stream)
+{
+    if (p <= 8 && m >= 1024) return 1;
+    DCG_CHECK_ARG(a && b && out && sums && m > 0 && n > 0 && p > 0, "matmul_tn_sums: bad arguments");
+    DenseEpilogue e{};
+    e.sums = sums;
+    return launch_ordered<true, false>(a, b, out, m, n, p, e, stream);
 }
 
 }  // namespace dcg
