@@ -108,13 +108,13 @@ int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* d
 // Activation [N, Hh, Ww, Cc] as a 4-D map (c, w, h, n) with a (32, tw, th, tn)-element box and
 // traversal strides (1, sw, sh, 1).
 int map_act_4d(CUtensorMap* map, const float* base, int N, int Hh, int Ww, int Cc, int tw, int th, int tn,
-               int sw, int sh)
+               int sw, int sh, bool mn_major = false)
 {
     const cuuint64_t dims[4] = {(cuuint64_t)Cc, (cuuint64_t)Ww, (cuuint64_t)Hh, (cuuint64_t)N};
     const cuuint64_t strides[3] = {(cuuint64_t)Cc * 4, (cuuint64_t)Ww * Cc * 4, (cuuint64_t)Hh * Ww * Cc * 4};
     const cuuint32_t box[4] = {32, (cuuint32_t)(tw * sw), (cuuint32_t)(th * sh), (cuuint32_t)tn};
     const cuuint32_t es[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
-    return encode_map(map, base, 4, dims, false, strides, box, es);
+    return encode_map(map, base, 4, dims, mn_major, strides, box, es);
 }
 
 // Activation [N, Hh, Ww, Cc] as a 5-D map (c%32, w, h, n, c/32): box (32, tw, th, tn, chunks) lands in
@@ -262,12 +262,12 @@ constexpr int kMaxSharedWidth = 160;
 // for 17), and where partitions would be many, narrow tiles win (128 -> 256 forward of 8 images, 64 columns: 8.8 for 10.1).
 // Channel counts between the powers of two get one tile instead of two (96 -> 160 forward of 13 images of 51 x 75: 35 for 59).
 // `m_count`: tiles along the other axis, times classes or taps; `store_cost`: clocks per column of an unpartitioned epilogue;
-// `loads`: TMA loads per stage, of which two are in the figures above.
+// `loads`: TMA loads per stage, of which two are in the figures above; `b_pieces`: B comes in loads of 32 columns.
 struct Tiling {
     int bn, n_tiles, splits, grid;
     double cost;
 };
-Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost, int loads = 2)
+Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost, int loads = 2, bool b_pieces = false)
 {
     static const int forced = env_int("DCG_TC_BN");
     const int sms = sm_count();
@@ -283,7 +283,7 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
         const int waves = (t.grid + sms - 1) / sms;
         const double stage = t_plan_x3 ? 750.0 + 6.25 * t.bn
                              : t.bn > 128 ? 300.0 + (t.bn - 128) * (212.0 / 128) : t.bn <= 64 && waves == 1 ? 250.0 : 300.0;
-        const double loop = 1200.0 + (max_stages + t.splits - 1) / t.splits * (stage + 20.0 * (loads - 2));
+        const double loop = 1200.0 + (max_stages + t.splits - 1) / t.splits * (stage + 20.0 * (loads - 2 + (b_pieces ? (t.bn + 31) / 32 - 1 : 0)));
         const double epilogue = t.bn * (t.splits > 1 ? 55.0 : (double)store_cost);
         t.cost = t.bn <= kMaxSharedWidth && !t_plan_x3 ? waves * loop + epilogue : waves * (loop + epilogue);
         if (best.grid == 0 || t.cost < best.cost) best = t;
@@ -344,6 +344,19 @@ void narrow_geometry(const dcg_conv_desc& d, Plan& pl)
     pl.xp_bytes = (size_t)d.n * pl.Hp * pl.Wp * 16;
 }
 
+// The channels of an MN-major operand lie in rows of 32 (one swizzle span).  A tensor map with the rows as a dimension of
+// their own - one box per stage - exists for multiples of 32 only; other multiples of four are loaded row by row, the last
+// one filled up with zeros.  The loads cost the producer more, but the CUDA cores, the other choice, take 5 to 15 times as
+// long: 100 -> 132 forward, 3x3, of 8 images of 64 x 64 46 us for 645, 36 -> 100 kernel gradient, 5x5 / stride 2, of 16
+// images of 40 x 40 21.5 for 130.  Below eight channels a tile holds too little, and 3xTF32 takes 10 us however small the
+// layer is, which a few million products do not (12 -> 20, 3x3 / stride 2, of 4 images of 16 x 16: 10.4 and 6.4).
+bool pieces_ok(const dcg_conv_desc& d, int channels)
+{
+    if (channels % 32 == 0) return true;
+    const double products = (double)d.n * d.ho * d.wo * d.kh * d.kw * d.c * d.o;
+    return channels % 4 == 0 && channels >= 8 && !(t_plan_x3 && products < 2e6);
+}
+
 bool narrow_ok(const dcg_conv_desc& d)
 {
     return d.c <= 4 && d.kw <= 8 && d.o % 32 == 0 && d.stride_h <= 8 && d.stride_w <= 8;
@@ -369,9 +382,11 @@ void use_tiling(Plan& pl, const Tiling& t)
 bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
 {
     const bool narrow = narrow_ok(d);
-    if (!narrow && (d.c % 4 != 0 || d.o % 32 != 0 || d.stride_h > 8 || d.stride_w > 8)) return false;
+    if (!narrow && (d.c % 4 != 0 || !pieces_ok(d, d.o) || d.stride_h > 8 || d.stride_w > 8)) return false;
     Params& p = pl.p;
     base_params(p, d);
+    const bool pieces = !narrow && d.o % 32 != 0;
+    if (pieces) { p.mt = 0; p.b_ch = d.o; }
     if (narrow || !fit) pixel_tile(BM, d.wo, d.ho, p.TW, p.TH, p.TN);
     else pixel_tile_fit(BM, d.wo, d.ho, d.n, d.stride_w, d.stride_h, false, p.TW, p.TH, p.TN);
     if (p.TW * d.stride_w > 256 || p.TH * d.stride_h > 256) return false;
@@ -391,7 +406,7 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
         p.splits = choose_splits(m_count * p.n_tiles, stages);
         pl.grid = m_count * p.n_tiles * p.splits;
     } else {
-        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35));
+        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35, 2, pieces));
     }
     finish_plan(pl);
     return true;
@@ -587,9 +602,10 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
 bool plan_dk(const dcg_conv_desc& d, Plan& pl)
 {
     const bool narrow = narrow_ok(d);
-    if (!narrow && (d.c % 32 != 0 || d.o % 32 != 0 || d.stride_h > 8 || d.stride_w > 8)) return false;
+    if (!narrow && (!pieces_ok(d, d.c) || !pieces_ok(d, d.o) || d.stride_h > 8 || d.stride_w > 8)) return false;
     Params& p = pl.p;
     base_params(p, d);
+    const bool pieces = !narrow && (d.c % 32 != 0 || d.o % 32 != 0);
     pixel_tile_fit(BK, d.wo, d.ho, d.n, d.stride_w, d.stride_h, true, p.TW, p.TH, p.TN);   // 32 output pixels per K stage
     if (p.TW * d.stride_w > 256 || p.TH * d.stride_h > 256) return false;
     p.tiles_w = (d.wo + p.TW - 1) / p.TW; p.tiles_h = (d.ho + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
@@ -618,14 +634,16 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     // with the channels of four or two taps on top of one another where there are only 32 or 64 of them; or M is the
     // output-channel axis, where that is quicker.
     const int stages = p.tiles_w * p.tiles_h * p.tiles_n, taps = d.kh * d.kw;
-    const int mt = d.c == 64 && taps >= 2 ? 2 : d.c == 32 && taps >= 4 ? 4 : 1;
+    const int mt = pieces ? 1 : d.c == 64 && taps >= 2 ? 2 : d.c == 32 && taps >= 4 ? 4 : 1;
     const int rows_c = (d.c + BM - 1) / BM, rows_o = (d.o + BM - 1) / BM;
     static const int roles = env_int("DCG_TC_ROLES");
-    const Tiling plain = choose_tiling((taps + mt - 1) / mt * rows_c, d.o, 32, stages, stages, 20, 1 + mt);
-    const Tiling swapped = choose_tiling(taps * rows_o, d.c, 32, stages, stages, 30);
+    auto row_pieces = [&](int ch) { return pieces ? (ch < BM ? (ch + 31) / 32 : BM / 32) - 1 : 0; };
+    const Tiling plain = choose_tiling((taps + mt - 1) / mt * rows_c, d.o, 32, stages, stages, 20, 1 + mt + row_pieces(d.c), pieces);
+    const Tiling swapped = choose_tiling(taps * rows_o, d.c, 32, stages, stages, 30, 2 + row_pieces(d.o), pieces);
     p.swap = roles ? roles == 2 : swapped.cost < plain.cost;
     p.m_tiles = p.swap ? rows_o : rows_c;
     p.mt = p.swap ? 1 : mt;
+    if (pieces) { p.mt = 0; p.a_ch = p.swap ? d.o : d.c; p.b_ch = p.swap ? d.c : d.o; }
     use_tiling(pl, p.swap ? swapped : plain);
     finish_plan(pl);
     return true;
@@ -681,13 +699,27 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
     using Kernel = void (*)(CUtensorMap, CUtensorMap, Params);
     static const Kernel kernels[] = {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>,
                                      conv_tc_kernel<MODE, kDual>};
+    int form = 0;
     Kernel kernel = kernels[p.kind];
+    if constexpr (MODE != MODE_DX) {
+        static const Kernel pieces[] = {conv_tc_kernel<MODE, kShared, 0>, conv_tc_kernel<MODE, kX3, 0>, conv_tc_kernel<MODE, kAlone, 0>,
+                                        conv_tc_kernel<MODE, kDual, 0>};
+        if (p.mt == 0) { form = 1; kernel = pieces[p.kind]; }
+    }
     if constexpr (MODE == MODE_DK) {
         static const Kernel more_taps[2][4] = {
             {conv_tc_kernel<MODE_DK, kShared, 2>, conv_tc_kernel<MODE_DK, kX3, 2>, nullptr, conv_tc_kernel<MODE_DK, kDual, 2>},
             {conv_tc_kernel<MODE_DK, kShared, 4>, conv_tc_kernel<MODE_DK, kX3, 4>, nullptr, conv_tc_kernel<MODE_DK, kDual, 4>}};
-        if (p.mt > 1) kernel = more_taps[p.mt / 4][p.kind];
+        if (p.mt > 1) { form = 2 + p.mt / 4; kernel = more_taps[p.mt / 4][p.kind]; }
     }
+    // each form is loaded when it is first needed, not all of them with the first convolution
+    static std::once_flag once[4][4];
+    static cudaError_t attr_err[4][4];
+    std::call_once(once[form][p.kind], [&] {
+        attr_err[form][p.kind] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    });
+    if (attr_err[form][p.kind] != cudaSuccess)
+        return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_tc_kernel): %s", cudaGetErrorString(attr_err[form][p.kind]));
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
     if (err != cudaSuccess) return fail(DCG_ERR_CUDA, "conv_tc_kernel launch: %s", cudaGetErrorString(err));
     count_launch();
@@ -698,18 +730,6 @@ template <int MODE>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, const EpilogueArgs& ep,
            int channels, void* ws, size_t ws_bytes, cudaStream_t stream)
 {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        for (auto kernel : {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>, conv_tc_kernel<MODE, kDual>})
-            if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-        if constexpr (MODE == MODE_DK)
-            for (auto kernel : {conv_tc_kernel<MODE_DK, kShared, 2>, conv_tc_kernel<MODE_DK, kShared, 4>, conv_tc_kernel<MODE_DK, kX3, 2>, conv_tc_kernel<MODE_DK, kX3, 4>,
-                                conv_tc_kernel<MODE_DK, kDual, 2>, conv_tc_kernel<MODE_DK, kDual, 4>})
-                if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    });
-    if (attr_err != cudaSuccess)
-        return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_tc_kernel): %s", cudaGetErrorString(attr_err));
     Params& p = pl.p;
     p.out = out;
     p.ep = ep;
@@ -1028,6 +1048,13 @@ int build_fwd(const dcg_conv_desc& d, const float* x, const float* k, void* ws, 
         return encode_map(&pr.mb, k4, 4, dims, true, strides, box, es);
     }
     if ((st = map_act_4d(&pr.ma, x, d.n, d.h, d.w, d.c, p.TW, p.TH, p.TN, d.stride_w, d.stride_h))) return st;
+    if (p.mt == 0) {   // k [tap][c][o] as (o, c, tap, 1), box (32, 32, 1, 1)
+        const cuuint64_t dims[4] = {(cuuint64_t)d.o, (cuuint64_t)d.c, (cuuint64_t)(d.kh * d.kw), 1};
+        const cuuint64_t strides[3] = {(cuuint64_t)d.o * 4, (cuuint64_t)d.c * d.o * 4, (cuuint64_t)d.kh * d.kw * d.c * d.o * 4};
+        const cuuint32_t box[4] = {32, 32, 1, 1};
+        const cuuint32_t es[4] = {1, 1, 1, 1};
+        return encode_map(&pr.mb, k, 4, dims, true, strides, box, es);
+    }
     // k [tap][c][o] as (o%32, c, tap, o/32), box (32, 32, 1, bn/32)
     const cuuint64_t dims[4] = {32, (cuuint64_t)d.c, (cuuint64_t)(d.kh * d.kw), (cuuint64_t)(d.o / 32)};
     const cuuint64_t strides[3] = {(cuuint64_t)d.o * 4, (cuuint64_t)d.c * d.o * 4, 128};
@@ -1105,6 +1132,13 @@ int build_dk(const dcg_conv_desc& d, const float* x, const float* dy, void* ws, 
         if ((st = map_window(&mx, xp, d, pl, p.TW, p.TH, p.TN, true, d.kh))) return st;
         if ((st = map_act_5d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, BM / 32))) return st;
         pr.ma = mdy; pr.mb = mx;
+        return DCG_OK;
+    }
+    if (p.mt == 0) {
+        if ((st = map_act_4d(&mx, x, d.n, d.h, d.w, d.c, p.TW, p.TH, p.TN, d.stride_w, d.stride_h, true))) return st;
+        if ((st = map_act_4d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, true))) return st;
+        pr.ma = p.swap ? mdy : mx;
+        pr.mb = p.swap ? mx : mdy;
         return DCG_OK;
     }
     const int x_chunks = p.swap ? p.bn / 32 : BM / 32 / p.mt, dy_chunks = p.swap ? BM / 32 : p.bn / 32;

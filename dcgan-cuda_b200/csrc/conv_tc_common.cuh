@@ -9,6 +9,7 @@ namespace {
 constexpr int BM = 128;                 // accumulator rows (TMEM lanes)
 constexpr int BK = 32;                  // K elements per pipeline stage (one 128-byte swizzle row)
 constexpr int A_STAGE_BYTES = BM * BK * 4;
+constexpr int kPieceBytes = 32 * BK * 4;   // 32 channels of a stage of an MN-major operand
 constexpr int kEpi = 256;               // epilogue threads: warps 2..9, two per TMEM lane quadrant
 constexpr int kThreads = 64 + kEpi;
 constexpr int kMaxSmem = 227 * 1024;
@@ -66,7 +67,8 @@ struct Params {
     long long wait_cycles;        // SM clocks after which a barrier wait gives up
     int kchunks;                  // 32-wide chunks along the contracted channel axis (FWD: C, DX: O)
     int kind;                     // which conv_tc_kernel (enum Kind)
-    int mt;                       // DK: kernel taps whose input channels share the 128 rows of an M tile (1, 2, 4)
+    int mt;                       // DK: kernel taps whose input channels share the 128 rows of an M tile (1, 2, 4); 0: one, and operands in pieces
+    int a_ch, b_ch;               // mt == 0: channels along M (DK) and N of the MN-major operands
     int swap;                     // DK: M axis is o (A from dy, B from x)
     int narrow;                   // FWD/DK with <= 4 input channels: x is read through the window map
     int ext_finish;               // the K partitions only write partials; a second kernel adds them (narrow DK)

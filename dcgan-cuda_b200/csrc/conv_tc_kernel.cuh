@@ -46,14 +46,16 @@ __device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs][32], uint32_
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
-// MT (kernel gradient only): kernel taps whose input channels share the 128 rows of an M tile.  A template argument, for a
+// TAPS (kernel gradient only): kernel taps whose input channels share the 128 rows of an M tile.  A template argument, for a
 // run-time choice takes the coordinates of the loads out of uniform registers (128 -> 256 gradient of 64 images 18.7 -> 21.6 us).
-template <int MODE, int KIND, int MT = 1>
+// 0: one tap, with the MN-major operands of ragged channel counts loaded in pieces of 32 channels.
+template <int MODE, int KIND, int TAPS = 1>
 __global__ void __launch_bounds__(64 + 128 * kGroups<KIND>, KIND == kShared ? 2 : 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ Params p)
 {
-    constexpr bool X3 = KIND == kX3;
+    constexpr bool X3 = KIND == kX3, PIECES = TAPS == 0;
+    constexpr int MT = PIECES ? 1 : TAPS;
     // Warps that take the stages in turn, as producers and as MMA issuers.  With two of them the ring has an even number of
     // stages: a stage is then always the same warp's, which makes the parity of its barriers unambiguous.
     constexpr int W = KIND == kDual ? 2 : 1;
@@ -138,8 +140,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // DX: parity class and its taps; DK: the kernel tap
     int ph = 0, pw = 0, rh = 0, rw = 0, eh = 0, ew = 0, taps_h = 1, taps_w = 1, tap_di = 0, tap_dj = 0;
     if (MODE == MODE_DX) {
-        ph = group / p.sw; pw = group % p.sw;
-        rh = (ph + p.pt) % p.sh; rw = (pw + p.pl) % p.sw;
+        // classes in the order of their first taps, so those with the most taps (9, 6, 6, 4 of 5 x 5 / stride 2) start first and
+        // a short one is what fills the last wave
+        rh = group / p.sw; rw = group % p.sw;
+        ph = (rh - p.pt % p.sh + p.sh) % p.sh; pw = (rw - p.pl % p.sw + p.sw) % p.sw;
         eh = (ph + p.pt) / p.sh; ew = (pw + p.pl) / p.sw;
         taps_h = rh < p.KH ? (p.KH - rh + p.sh - 1) / p.sh : 0;
         taps_w = rw < p.KW ? (p.KW - rw + p.sw - 1) / p.sw : 0;
@@ -205,7 +209,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // costs this lone thread ~100 cycles, and the loop has to turn around in well under the 256
         // cycles the tensor core needs per stage.
         {
-            const uint32_t tx_bytes = (uint32_t)((MODE == MODE_DK ? A_STAGE_BYTES : p.TW * p.TH * p.TN * BK * 4) + b_stage_bytes);
+            // MN-major operands of ragged channel counts come in pieces of 32 channels: only those that exist are loaded, what the
+            // others leave in their rows and columns is never stored
+            const int a_pieces = PIECES && MODE == MODE_DK ? min(BM / 32, (p.a_ch - m_tile * BM + 31) >> 5) : 0;
+            const int b_pieces = PIECES ? min(p.bn >> 5, (p.b_ch - n_tile * p.bn + 31) >> 5) : 0;
+            const uint32_t tx_bytes = (uint32_t)((MODE != MODE_DK ? p.TW * p.TH * p.TN * BK * 4 : PIECES ? a_pieces * kPieceBytes : A_STAGE_BYTES) +
+                                                 (PIECES ? b_pieces * kPieceBytes : b_stage_bytes));
             int s = walker;
             uint32_t phase = 0;
             // counters of stage q0: FWD (chunk, tap, di, dj); DX (chunk, -, th, tw); DK (-, tile_n, tile_h, tile_w)
@@ -257,7 +266,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         if (it < 128) TC_TRACE(256 + it);
                         tma_load_4d(a_dst, &map_a, fb, chunk * BK, p.sw * j0 + dj - p.pl, p.sh * i0 + di - p.pt, n0);
                         if (it < 128) TC_TRACE(512 + it);
-                        tma_load_4d(b_dst, &map_b, fb, 0, chunk * BK, tap, n_tile * (p.bn / 32));
+                        if constexpr (PIECES) {
+                            for (int i = 0; i < b_pieces; ++i)
+                                tma_load_4d(b_dst + i * kPieceBytes, &map_b, fb, n_tile * p.bn + 32 * i, chunk * BK, tap, 0);
+                        } else {
+                            tma_load_4d(b_dst, &map_b, fb, 0, chunk * BK, tap, n_tile * (p.bn / 32));
+                        }
                         if (it < 128) TC_TRACE(768 + it);
                     } else if (MODE == MODE_DX) {
                         // (di, dj) count the taps of this parity class: kernel tap (rh + sh*di, rw + sw*dj)
@@ -270,6 +284,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         if (p.narrow) {  // A: dy (rows o), B: the KH 32-float windows of 32 output pixels
                             tma_load_5d(a_dst, &map_a, fb, 0, pj, pi, pn, m_tile * (BM / 32));
                             tma_load_5d(b_dst, &map_b, fb, 0, pj, pi, pn, 0);   // box covers all KH kernel rows
+                        } else if (PIECES) {   // both operands
+                            const int aw = p.swap ? pj : xw, ah = p.swap ? pi : xh, bw = p.swap ? xw : pj, bh = p.swap ? xh : pi;
+                            for (int i = 0; i < a_pieces; ++i)
+                                tma_load_4d(a_dst + i * kPieceBytes, &map_a, fb, m_tile * BM + 32 * i, aw, ah, pn);
+                            for (int i = 0; i < b_pieces; ++i)
+                                tma_load_4d(b_dst + i * kPieceBytes, &map_b, fb, n_tile * p.bn + 32 * i, bw, bh, pn);
                         } else if (!p.swap) {   // A: x (rows c), B: dy (cols o)
                             tma_load_5d(a_dst, &map_a, fb, 0, xw, xh, pn, m_tile * (BM / 32));
                             if constexpr (MT > 1) tma_load_5d(a_dst + A_STAGE_BYTES / MT, &map_a, fb, 0, xw + ow1, xh + oh1, pn, 0);

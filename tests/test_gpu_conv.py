@@ -343,6 +343,30 @@ def test_tile_widths_and_pixel_boxes(pkg, dev, shape, prec_name):
         assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
 
 
+# channel counts that are no multiple of 32 on either side or both: one piece of 32 channels and several, the last of them
+# nearly empty and nearly full, more than one tile along each axis, K partitions and none
+RAGGED_SHAPES = [
+    (2, 12, 20, 36, 5, 40, 2), (3, 9, 11, 16, 3, 20, 1), (2, 16, 16, 132, 5, 100, 2), (5, 13, 11, 68, 3, 260, 2),
+    (1, 7, 9, 188, 1, 28, 1), (4, 20, 14, 32, 3, 36, 1), (4, 20, 14, 36, 3, 32, 1), (16, 24, 24, 60, 3, 156, 1),
+]
+
+
+@pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", RAGGED_SHAPES)
+def test_ragged_channel_counts(pkg, dev, shape, prec_name):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    x, k, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
+                ((54, (N, H, W, C)), (55, (K, K, C, O)), (56, (N, -(-H // s), -(-W // s), O))))
+    got, ref = ([F.conv2d_fwd(x, k, (s, s), precision=p), F.conv2d_dx(dy, k, (H, W), (s, s), precision=p),
+                 F.conv2d_dk(x, dy, (K, K), (s, s), precision=p)] for p in (getattr(pkg, PRECS[prec_name]), pkg.PREC_FP32))
+    torch.cuda.synchronize()
+    assert pkg.lib.dcg_device_status() == 0
+    tol = TF32_TOL if prec_name == "tf32" else 3e-5
+    for name, a, b in zip(("fwd", "dx", "dk"), got, ref):
+        assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
+
+
 @pytest.mark.parametrize("batch", [20, 28, 40, 56, 100])
 def test_k_partition_counts(pkg, dev, batch):
     """The number of K partitions of a tile (= thread-block cluster size) follows the tile count:
