@@ -248,11 +248,13 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY;
     extern __shared__ __align__(16) float smem[];
     pdl_enter();
-    const int ph = blockIdx.z / d.stride_w, pw = blockIdx.z % d.stride_w, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     const int P = d.kh - 1 - d.pad_top, Q = d.kw - 1 - d.pad_left;
-    int r0h = (P - ph) % d.stride_h, r0w = (Q - pw) % d.stride_w;   // first tap (in flipped order) of this class
-    if (r0h < 0) r0h += d.stride_h;
-    if (r0w < 0) r0w += d.stride_w;
+    // first tap (in flipped order) of this class: in this order the classes with the most taps start first
+    const int r0h = blockIdx.z / d.stride_w, r0w = blockIdx.z % d.stride_w;
+    int ph = (P - r0h) % d.stride_h, pw = (Q - r0w) % d.stride_w;
+    if (ph < 0) ph += d.stride_h;
+    if (pw < 0) pw += d.stride_w;
     OrdGeom g;
     g.mh = (d.h - ph + d.stride_h - 1) / d.stride_h; g.mw = (d.w - pw + d.stride_w - 1) / d.stride_w;
     g.SH = d.ho; g.SW = d.wo; g.SC = d.o;
@@ -609,8 +611,9 @@ int launch_ordered_dx_tile(const dcg_conv_desc& d, const float* dy, const float*
 
 // Tile choice by outputs per lane of the GPU (SMs x 128): the wider the thread tile the fewer instructions an output
 // costs per K step, but a scheduler needs a few warps to hide the chain of dependent adds and the shared-memory
-// latency.
-constexpr double kOrdWide = 32, kOrdNormal = 5, kOrdDkGrouped = 2;
+// latency: with one it issues an instruction every three clocks.  Forward of 8 images: 64 -> 128 75 -> 68 us with 2 x 4
+// outputs per thread (4 x 4: 92 and more), 256 -> 512 127 -> 121 with 2 x 2; 12 -> 32 of 4 images of 33 x 47 35 -> 18.
+constexpr double kOrdWide = 32, kOrdNormal = 5, kOrdFew = 3, kOrdDkGrouped = 2;
 
 double outputs_per_lane(double outputs) { return outputs / (128.0 * sm_count()); }
 
@@ -618,7 +621,9 @@ int launch_ordered_fwd(const dcg_conv_desc& d, const float* x, const float* k, f
 {
     const double per_lane = outputs_per_lane((double)d.n * d.ho * d.wo * d.o);
     if (per_lane >= kOrdWide) return launch_ordered_fwd_tile<4, 4, 16, 16, 2>(d, x, k, y, ep, stream);
+    if (per_lane >= 2 * kOrdNormal) return launch_ordered_fwd_tile<2, 4, 16, 16, 2>(d, x, k, y, ep, stream);
     if (per_lane >= kOrdNormal) return launch_ordered_fwd_tile<2, 2, 16, 16, 2>(d, x, k, y, ep, stream);
+    if (per_lane >= kOrdFew) return launch_ordered_fwd_tile<2, 2, 16, 8, 4>(d, x, k, y, ep, stream);
     return launch_ordered_fwd_tile<1, 2, 8, 16, 4>(d, x, k, y, ep, stream);
 }
 
