@@ -33,6 +33,8 @@ PREC_TF32, PREC_3XTF32, PREC_FP32 = 0, 1, 2
 KIND_FWD, KIND_DX, KIND_DK = 0, 1, 2
 
 NODE_OUT_DEAD = 1
+# what dcg_trainer_replay enqueues
+REPLAY_GENERATE, REPLAY_D_FWD_BWD, REPLAY_STEP = 0, 1, 2
 
 
 class ConvDesc(ctypes.Structure):
@@ -123,6 +125,7 @@ SIGNATURES = {
     "dcg_trainer_destroy": (None, [_P]),
     "dcg_trainer_tensor": (c_int, [_P, ctypes.c_char_p, ctypes.POINTER(_P), ctypes.POINTER(c_size_t)]),
     "dcg_trainer_generate": (c_int, [_P]),
+    "dcg_trainer_replay": (c_int, [_P, c_int, _P]),
     "dcg_trainer_d_fwd_bwd": (c_int, [_P]),
     "dcg_trainer_d_backward": (c_int, [_P]),
     "dcg_trainer_d_apply": (c_int, [_P, c_float]),

@@ -508,11 +508,11 @@ int run_list(dcg_trainer* t, const std::vector<dcg_node>& all, dcg_trainer::List
              size_t end = (size_t)-1)
 {
     if (end > all.size()) end = all.size();
-    const std::vector<dcg_node> L(all.begin() + begin, all.begin() + end);   // ~100 small records
+    auto run_nodes = [&] { return dcg_run_nodes(t->ctx, all.data() + begin, (int)(end - begin), t->cfg.fuse); };
     const bool eager = !t->use_graphs || g.failed || dcg::context_is_profiling(t->ctx);
     if (eager || g.eager_runs < 2) {
         if (!eager) ++g.eager_runs;
-        return dcg_run_nodes(t->ctx, L.data(), (int)L.size(), t->cfg.fuse);
+        return run_nodes();
     }
     if (g.exec && g.generation != dcg::context_generation(t->ctx)) {   // scratch moved or precision switched: stale
         cudaGraphExecDestroy(g.exec);
@@ -526,9 +526,9 @@ int run_list(dcg_trainer* t, const std::vector<dcg_node>& all, dcg_trainer::List
                 fprintf(stderr, "dcg_trainer: cudaStreamBeginCapture failed: %s\n", cudaGetErrorString(cudaGetLastError()));
             cudaGetLastError();
             g.failed = true;
-            return dcg_run_nodes(t->ctx, L.data(), (int)L.size(), t->cfg.fuse);
+            return run_nodes();
         }
-        const int st = dcg_run_nodes(t->ctx, L.data(), (int)L.size(), t->cfg.fuse);
+        const int st = run_nodes();
         const cudaError_t ce = cudaStreamEndCapture(t->stream, &graph);
         cudaError_t ie = cudaSuccess;
         if (st != DCG_OK || ce != cudaSuccess || !graph ||
@@ -540,7 +540,7 @@ int run_list(dcg_trainer* t, const std::vector<dcg_node>& all, dcg_trainer::List
             if (graph) cudaGraphDestroy(graph);
             g.exec = nullptr;
             g.failed = true;   // stay eager from here on
-            return dcg_run_nodes(t->ctx, L.data(), (int)L.size(), t->cfg.fuse);
+            return run_nodes();
         }
         cudaGraphDestroy(graph);
         g.launches = dcg_launches_total() - before;
@@ -914,6 +914,21 @@ extern "C" int dcg_trainer_step(dcg_trainer* t)
     }
     t->last_step_launches = dcg_launches_total() - before;
     return DCG_OK;
+}
+
+extern "C" int dcg_trainer_replay(dcg_trainer* t, int what, dcg_stream_t stream)
+{
+    DCG_CHECK_ARG(t && what >= 0 && what <= DCG_REPLAY_STEP, "dcg_trainer_replay: bad arguments");
+    dcg_trainer::ListGraph& g = what == DCG_REPLAY_GENERATE ? t->gen_graph : what == DCG_REPLAY_D_FWD_BWD ? t->dfb_graph : t->step_graph;
+    if (!t->use_graphs || g.failed || !g.exec || g.generation != dcg::context_generation(t->ctx) || t->cfg.world > 1 ||
+        dcg::context_is_profiling(t->ctx))
+        return 0;
+    // a captured graph runs on any stream
+    const cudaStream_t own = t->stream;
+    t->stream = dcg::as_stream(stream);
+    const int st = what == DCG_REPLAY_GENERATE ? dcg_trainer_generate(t) : what == DCG_REPLAY_D_FWD_BWD ? dcg_trainer_d_fwd_bwd(t) : dcg_trainer_step(t);
+    t->stream = own;
+    return st ? st : 1;
 }
 
 // ---- checkpoints -----------------------------------------------------------------------------------

@@ -59,6 +59,8 @@ class Trainer:
             self._dp = self._make_communicator(world, process_group)
         check(lib.dcg_trainer_create_dp(ctypes.byref(self._h), ctypes.byref(self.cfg), self.stream.cuda_stream, self._dp))
         self._views = {}
+        self._device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+        self._joined = None   # the caller's stream that is in order after all work of the trainer
         self.x = self.tensor("x").view(batch, 64, 64, 3)
         self.z = self.tensor("z").view(batch, 100)
         self.g_out = self.tensor("g_out").view(batch, 64, 64, 3)
@@ -122,18 +124,40 @@ class Trainer:
             yield
             return
         caller = torch.cuda.current_stream(self.device)
+        if self._joined is not None and self._joined != caller:
+            self.stream.wait_stream(self._joined)   # what _replay put there
+        self._joined = None
         self.stream.wait_stream(caller)
         with torch.cuda.stream(self.stream):
             yield
         caller.wait_stream(self.stream)
+        self._joined = caller
+
+    def _replay(self, what):
+        """Enqueues a captured graph on the caller's stream itself, if that is the one the trainer was last called from:
+        everything the trainer has enqueued is then in order before it, and the two waits between the streams (5 us of a
+        pass that takes 40) are not needed.  False: not possible, take the usual way."""
+        if self._joined is None or torch._C._cuda_getDevice() != self._device_index:
+            return False
+        stream = torch._C._cuda_getCurrentRawStream(self._device_index)
+        if stream != self._joined.cuda_stream:
+            return False
+        status = lib.dcg_trainer_replay(self._h, what, stream)
+        if status < 0:
+            check(status)
+        return status == 1
 
     def generate(self):
+        if self._replay(_lib.REPLAY_GENERATE):
+            return self.g_out
         with self._on_stream():
             check(lib.dcg_trainer_generate(self._h))
         return self.g_out
 
     def d_fwd_bwd(self):
         """Discriminator forward + backward on self.x against labels of ones (all layer gradients)."""
+        if self._replay(_lib.REPLAY_D_FWD_BWD):
+            return
         with self._on_stream():
             check(lib.dcg_trainer_d_fwd_bwd(self._h))
 
@@ -179,6 +203,8 @@ class Trainer:
 
     def step(self):
         """One training iteration on inputs already resident in self.x / self.z."""
+        if self._replay(_lib.REPLAY_STEP):
+            return
         with self._on_stream():
             self._step()
 

@@ -401,6 +401,11 @@ void dcg_trainer_destroy(dcg_trainer* t);
 int dcg_trainer_tensor(dcg_trainer* t, const char* name, float** ptr, size_t* count);
 /* Generator forward only (z -> g_out): dcgan/main.cu:252-269. */
 int dcg_trainer_generate(dcg_trainer* t);
+/* dcg_trainer_generate / _d_fwd_bwd / _step on `stream` instead of the trainer's own, as soon as their graph has been
+ * captured (single GPU only): 1 if it was enqueued, 0 if the caller has to take the usual call, negative on error.  The
+ * caller orders `stream` against the trainer's stream. */
+enum dcg_replay { DCG_REPLAY_GENERATE = 0, DCG_REPLAY_D_FWD_BWD = 1, DCG_REPLAY_STEP = 2 };
+int dcg_trainer_replay(dcg_trainer* t, int what, dcg_stream_t stream);
 /* Discriminator forward + backward on the real images "x" alone against labels of all ones: sigmoid
  * cross-entropy, then the kernel, bias and input gradient of every layer (the image gradient lands
  * in the generator-output gradient buffer).  Weight gradients go to "d_gradb0..9".  A measurement and

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import oracle
+from conftest import seeded
 from oracle import dcgan_model as M
 
 pytestmark = pytest.mark.gpu
@@ -160,6 +161,31 @@ def test_graph_replay_equals_eager(pkg, dev, monkeypatch):
     (l0, d0, g0), (l1, d1, g1) = results
     assert l0 == l1
     assert torch.equal(d0, d1) and torch.equal(g0, g1)
+
+
+@pytest.mark.parametrize("streams", [1, 2])
+def test_replay_on_the_callers_stream_equals_eager(pkg, dev, monkeypatch, streams):
+    """Captured graphs run on the stream the trainer was last called from, and in order when the calls change streams."""
+    runs = {}
+    for replay in (True, False):
+        if not replay:
+            monkeypatch.setattr(pkg.Trainer, "_replay", lambda self, what: False)
+        tr = pkg.Trainer(batch=4, seed=7, precision=pkg.PREC_FP32)
+        tr.x.copy_(torch.from_numpy(seeded((4, 64, 64, 3), 1)))
+        callers = [torch.cuda.current_stream(), torch.cuda.Stream()][:streams]
+        images, losses = [], []
+        for i in range(12):
+            stream = callers[i // 2 % streams]
+            stream.wait_stream(callers[(i // 2 - 1) % streams])   # the inputs and outputs below are the caller's to order
+            with torch.cuda.stream(stream):
+                tr.z.copy_(torch.from_numpy(seeded((4, 100), i)), non_blocking=True)
+                images.append(tr.generate().clone())
+                tr.step()
+                losses.append(tr.d_loss.clone())
+        torch.cuda.synchronize()
+        runs[replay] = [t.cpu() for t in images + losses + [tr.tensor("d_params"), tr.tensor("g_params")]]
+        tr.close()
+    assert all(torch.equal(a, b) for a, b in zip(runs[True], runs[False]))
 
 
 def test_g_backward_in_two_parts(pkg, dev):
