@@ -151,9 +151,12 @@ void pixel_tile_fit(int total, int Wd, int Hd, int Nd, int sw, int sh, bool whol
     pixel_tile(total, Wd, Hd, tw, th, tn);
     auto boxes = [&](int a, int b, int c) { return (long long)((Wd + a - 1) / a) * ((Hd + b - 1) / b) * ((Nd + c - 1) / c); };
     long long best = boxes(tw, th, tn);
+    // fewer images than fit: nothing is loaded for the others (one sampled image 41.3 -> 36.2 us)
+    if (!whole && tn > Nd) tn = Nd;
     for (int a = 1; a <= total && a * sw <= 256; whole ? a *= 2 : ++a)
         for (int b = 1; a * b <= total && b * sh <= 256; whole ? b *= 2 : ++b) {
-            const int c = total / (a * b);
+            int c = total / (a * b);
+            if (!whole && c > Nd) c = Nd;
             if (boxes(a, b, c) < best) { best = boxes(a, b, c); tw = a; th = b; tn = c; }
         }
 }
@@ -357,9 +360,17 @@ bool pieces_ok(const dcg_conv_desc& d, int channels)
     return channels % 4 == 0 && channels >= 8 && !(t_plan_x3 && products < 2e6);
 }
 
-bool narrow_ok(const dcg_conv_desc& d)
+int pad32(int channels) { return (channels + 31) / 32 * 32; }
+
+bool narrow_ok(const dcg_conv_desc& d, double min_products)
 {
-    return d.c <= 4 && d.kw <= 8 && d.o % 32 == 0 && d.stride_h <= 8 && d.stride_w <= 8;
+    // Other output channels than multiples of 32: dy in pieces, the weights padded.  The repacks are a launch more, by the end
+    // of which the CUDA cores are done with a small layer (3 -> 20 forward of 8 images of 32 x 32 6.7 us, 3 -> 180 of 4 of
+    // 64 x 64 14 against 8); their kernel gradients take longest, for few outputs sum many pixels in order (3 -> 100, 5x5 /
+    // stride 2, of 32 images of 96 x 96 402 us against 20, forward 142 against 26).
+    const double products = (double)d.n * d.ho * d.wo * d.kh * d.kw * d.c * d.o;
+    const bool o_ok = d.o % 32 == 0 || (d.o % 4 == 0 && d.o >= 8 && products >= min_products);
+    return d.c <= 4 && d.kw <= 8 && o_ok && d.stride_h <= 8 && d.stride_w <= 8;
 }
 
 void base_params(Params& p, const dcg_conv_desc& d)
@@ -381,7 +392,7 @@ void use_tiling(Plan& pl, const Tiling& t)
 // the kernel with a resident B operand wants them.
 bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
 {
-    const bool narrow = narrow_ok(d);
+    const bool narrow = narrow_ok(d, 4e6);
     if (!narrow && (d.c % 4 != 0 || !pieces_ok(d, d.o) || d.stride_h > 8 || d.stride_w > 8)) return false;
     Params& p = pl.p;
     base_params(p, d);
@@ -397,11 +408,11 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
         p.narrow = 1;
         p.kchunks = 1;
         narrow_geometry(d, pl);
-        pl.k4_bytes = (size_t)d.kh * 32 * d.o * sizeof(float);
+        pl.k4_bytes = (size_t)d.kh * 32 * pad32(d.o) * sizeof(float);
     }
     const int stages = narrow ? d.kh : d.kh * d.kw * p.kchunks;
     if (narrow || !fit) {
-        p.bn = d.o >= 128 ? 128 : d.o;
+        p.bn = d.o >= 128 ? 128 : pad32(d.o);
         p.n_tiles = (d.o + p.bn - 1) / p.bn;
         p.splits = choose_splits(m_count * p.n_tiles, stages);
         pl.grid = m_count * p.n_tiles * p.splits;
@@ -601,7 +612,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
 
 bool plan_dk(const dcg_conv_desc& d, Plan& pl)
 {
-    const bool narrow = narrow_ok(d);
+    const bool narrow = narrow_ok(d, 4e5);
     if (!narrow && (!pieces_ok(d, d.c) || !pieces_ok(d, d.o) || d.stride_h > 8 || d.stride_w > 8)) return false;
     Params& p = pl.p;
     base_params(p, d);
@@ -616,6 +627,7 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
         if (d.kh * 32 > 256) return false;
         p.narrow = 1;
         p.swap = 1;
+        if (d.o % 32 != 0) { p.mt = 0; p.a_ch = d.o; }
         p.m_tiles = (d.o + BM - 1) / BM;
         p.bn = 32 * d.kh;
         p.n_tiles = 1;
@@ -774,10 +786,10 @@ int narrow_prepare(const dcg_conv_desc& d, const Plan& pl, const float* x, const
     *xp_out = xp;
     if (k4_out) {   // forward: image and weights in one launch
         float* k4 = reinterpret_cast<float*>(base + pl.k4_off());
-        const int total = d.kh * 32 * d.o;
+        const int total = d.kh * 32 * pad32(d.o);
         const int k4_blocks = (total + 255) / 256;
         launch_pdl(repack_narrow_k4_kernel, (unsigned)(blocks + k4_blocks), 256, 0, stream, x, reinterpret_cast<float4*>(xp),
-                   d.n, d.h, d.w, d.c, pl.Hp, pl.Wp, d.pad_top, d.pad_left, k, k4, d.kh, d.kw, d.o, k4_blocks);
+                   d.n, d.h, d.w, d.c, pl.Hp, pl.Wp, d.pad_top, d.pad_left, k, k4, d.kh, d.kw, d.o, pad32(d.o), k4_blocks);
         DCG_LAUNCH_CHECK("repack_narrow_k4_kernel");
         *k4_out = k4;
     } else {
@@ -860,7 +872,7 @@ bool short_ok(const Plan& pl)
     if (off || p.x3 || p.splits != 1 || p.n_tiles != 1 || p.bn > 128 || p.bn % 32 != 0 || p.TW * p.TH * p.TN != BM) return false;
     const int ksteps = p.narrow ? p.KH : p.KH * p.KW * p.kchunks;
     if (!p.narrow && (p.KH != 1 || p.KW != 1 || !p.planes)) return false;   // the GEMM of the 3-channel input gradient
-    if (p.narrow && p.planes) return false;
+    if (p.narrow && (p.planes || p.O % 32 != 0)) return false;
     if (ksteps < 1 || ksteps * p.bn * BK * 4 > kShortMaxB) return false;
     return pl.grid > sm_count();
 }
@@ -1041,8 +1053,8 @@ int build_fwd(const dcg_conv_desc& d, const float* x, const float* k, void* ws, 
         const float* k4 = reinterpret_cast<const float*>(base + pl.k4_off());
         if ((st = map_window(&pr.ma, xp, d, pl, p.TW, p.TH, p.TN, false, 1))) return st;
         // k4 [kh][slot][o] as (o%32, slot, kh, o/32), box (32, 32, 1, bn/32)
-        const cuuint64_t dims[4] = {32, 32, (cuuint64_t)d.kh, (cuuint64_t)(d.o / 32)};
-        const cuuint64_t strides[3] = {(cuuint64_t)d.o * 4, (cuuint64_t)32 * d.o * 4, 128};
+        const cuuint64_t dims[4] = {32, 32, (cuuint64_t)d.kh, (cuuint64_t)(pad32(d.o) / 32)};
+        const cuuint64_t strides[3] = {(cuuint64_t)pad32(d.o) * 4, (cuuint64_t)32 * pad32(d.o) * 4, 128};
         const cuuint32_t box[4] = {32, 32, 1, (cuuint32_t)(p.bn / 32)};
         const cuuint32_t es[4] = {1, 1, 1, 1};
         return encode_map(&pr.mb, k4, 4, dims, true, strides, box, es);
@@ -1130,7 +1142,9 @@ int build_dk(const dcg_conv_desc& d, const float* x, const float* dy, void* ws, 
             return fail(DCG_ERR_WORKSPACE, "conv (tensor path, narrow input): workspace %zu < %zu bytes", ws_bytes, pl.ws_bytes);
         const float* xp = reinterpret_cast<const float*>(static_cast<uint8_t*>(ws) + pl.xp_off());
         if ((st = map_window(&mx, xp, d, pl, p.TW, p.TH, p.TN, true, d.kh))) return st;
-        if ((st = map_act_5d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, BM / 32))) return st;
+        st = p.mt == 0 ? map_act_4d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, true)
+                       : map_act_5d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, BM / 32);
+        if (st) return st;
         pr.ma = mdy; pr.mb = mx;
         return DCG_OK;
     }

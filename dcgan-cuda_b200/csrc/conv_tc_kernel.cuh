@@ -214,7 +214,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int a_pieces = PIECES && MODE == MODE_DK ? min(BM / 32, (p.a_ch - m_tile * BM + 31) >> 5) : 0;
             const int b_pieces = PIECES ? min(p.bn >> 5, (p.b_ch - n_tile * p.bn + 31) >> 5) : 0;
             const uint32_t tx_bytes = (uint32_t)((MODE != MODE_DK ? p.TW * p.TH * p.TN * BK * 4 : PIECES ? a_pieces * kPieceBytes : A_STAGE_BYTES) +
-                                                 (PIECES ? b_pieces * kPieceBytes : b_stage_bytes));
+                                                 (PIECES && !p.narrow ? b_pieces * kPieceBytes : b_stage_bytes));
             int s = walker;
             uint32_t phase = 0;
             // counters of stage q0: FWD (chunk, tap, di, dj); DX (chunk, -, th, tw); DK (-, tile_n, tile_h, tile_w)
@@ -282,7 +282,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         const int pj = dj * p.TW, pi = di * p.TH, pn = tap * p.TN;
                         const int xw = p.sw * pj + tap_dj - p.pl, xh = p.sh * pi + tap_di - p.pt;
                         if (p.narrow) {  // A: dy (rows o), B: the KH 32-float windows of 32 output pixels
-                            tma_load_5d(a_dst, &map_a, fb, 0, pj, pi, pn, m_tile * (BM / 32));
+                            if constexpr (PIECES) {
+                                for (int i = 0; i < a_pieces; ++i)
+                                    tma_load_4d(a_dst + i * kPieceBytes, &map_a, fb, m_tile * BM + 32 * i, pj, pi, pn);
+                            } else {
+                                tma_load_5d(a_dst, &map_a, fb, 0, pj, pi, pn, m_tile * (BM / 32));
+                            }
                             tma_load_5d(b_dst, &map_b, fb, 0, pj, pi, pn, 0);   // box covers all KH kernel rows
                         } else if (PIECES) {   // both operands
                             const int aw = p.swap ? pj : xw, ah = p.swap ? pi : xh, bw = p.swap ? xw : pj, bh = p.swap ? xh : pi;

@@ -69,20 +69,20 @@ repack_narrow_kernel(const float* __restrict__ x, float4* __restrict__ xp, int N
 }
 
 // Both repacks of a narrow-channel forward in one launch: blocks [0, gridDim.x - k4_blocks) build
-// the padded 4-channel image, the last k4_blocks blocks the weights k4 [KH][32][O] (row 4*dj + c).
+// the padded 4-channel image, the last k4_blocks blocks the weights k4 [KH][32][OP] (row 4*dj + c; zeros beyond O).
 __global__ void __launch_bounds__(256)
 repack_narrow_k4_kernel(const float* __restrict__ x, float4* __restrict__ xp, int N, int H, int W, int C,
                         int Hp, int Wp, int pt, int pl, const float* __restrict__ k, float* __restrict__ k4,
-                        int KH, int KW, int O, int k4_blocks)
+                        int KH, int KW, int O, int OP, int k4_blocks)
 {
     pdl_enter();
     const int x_blocks = (int)gridDim.x - k4_blocks;
     if ((int)blockIdx.x >= x_blocks) {
-        const int total = KH * 32 * O;
+        const int total = KH * 32 * OP;
         for (int i = ((int)blockIdx.x - x_blocks) * blockDim.x + threadIdx.x; i < total; i += k4_blocks * blockDim.x) {
-            const int o = i % O, slot = (i / O) % 32, di = i / (O * 32);
+            const int o = i % OP, slot = (i / OP) % 32, di = i / (OP * 32);
             const int dj = slot >> 2, c = slot & 3;
-            k4[i] = (dj < KW && c < C) ? __ldg(k + (((size_t)di * KW + dj) * C + c) * O + o) : 0.f;
+            k4[i] = (dj < KW && c < C && o < O) ? __ldg(k + (((size_t)di * KW + dj) * C + c) * O + o) : 0.f;
         }
         return;
     }

@@ -348,6 +348,8 @@ def test_tile_widths_and_pixel_boxes(pkg, dev, shape, prec_name):
 RAGGED_SHAPES = [
     (2, 12, 20, 36, 5, 40, 2), (3, 9, 11, 16, 3, 20, 1), (2, 16, 16, 132, 5, 100, 2), (5, 13, 11, 68, 3, 260, 2),
     (1, 7, 9, 188, 1, 28, 1), (4, 20, 14, 32, 3, 36, 1), (4, 20, 14, 36, 3, 32, 1), (16, 24, 24, 60, 3, 156, 1),
+    # <= 4 input channels: dy in pieces, weights padded to 32; fewer images than a pixel box holds
+    (20, 33, 30, 3, 5, 36, 2), (9, 40, 40, 4, 3, 140, 1), (1, 200, 180, 1, 5, 12, 1), (3, 4, 4, 64, 5, 96, 2),
 ]
 
 
