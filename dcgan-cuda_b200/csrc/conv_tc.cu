@@ -931,9 +931,13 @@ bool plan_dx3(const dcg_conv_desc& d, Plan& pl, Dx3Args& g)
     if (off || t_plan_x3) return false;
     if (d.c > 4 || d.stride_h != 2 || d.stride_w != 2 || d.kh * d.kw > 32 || d.kh < 2 || d.kw < 2) return false;
     if (d.o % 32 != 0 || d.o > 64 || d.wo > 32 || d.pad_top >= d.kh || d.pad_left >= d.kw) return false;
-    // the most output rows (2R) whose contributing dy rows fit the 8 rows of a tile
+    // the most output rows (2R) whose contributing dy rows fit the 8 rows of a tile, but no more than it takes to give every SM
+    // a tile: the gather of a tile is what a small batch waits for (one image 6.7 us as 32 tiles of two rows, 9.0 as 6 of 12)
     int R = 0, lo = 0;
-    for (int r = kDx3Rows; r >= 1 && R == 0; --r) {
+    const int tiles_each = sm_count() / d.n > 1 ? sm_count() / d.n : 1, rows = (d.h + 1) / 2;
+    int widest = (rows + tiles_each - 1) / tiles_each;
+    if (widest > kDx3Rows) widest = kDx3Rows;
+    for (int r = widest; r >= 1 && R == 0; --r) {
         int mn = 1 << 30, mx = -(1 << 30);
         for (int hl = 0; hl < 2 * r; ++hl)
             for (int di = (hl + d.pad_top) & 1; di < d.kh; di += 2) {
@@ -942,7 +946,7 @@ bool plan_dx3(const dcg_conv_desc& d, Plan& pl, Dx3Args& g)
                 if (i < mn) mn = i;
                 if (i > mx) mx = i;
             }
-        if (mx - mn + 1 <= kDx3Rows) { R = r; lo = mn; }
+        if (mx - mn + 1 <= kDx3Rows) { R = r; lo = mn; g.mts = (mx - mn + 4) / 4; }
     }
     if (R == 0) return false;
     Params& p = pl.p;

@@ -18,6 +18,7 @@ namespace {
 // tile is being gathered (one TMEM accumulator per M tile, handed back as soon as it is in shared memory).
 struct Dx3Args {
     int R;            // dy rows owned per tile (2R output rows)
+    int mts;          // M tiles (four dy rows) that hold the rows contributing to them: 1 or 2
     int lo;           // first dy row a tile needs, relative to its first owned row (<= 0)
     int tiles_per_img, tiles;
 };
@@ -90,7 +91,7 @@ conv_dx3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int tile = blockIdx.x; tile < g.tiles && alive; tile += gridDim.x) {
             const int n = tile / g.tiles_per_img, t = tile - n * g.tiles_per_img;
             const int i_base = g.R * t + g.lo;
-            for (int mt = 0; mt < 2 && alive; ++mt)
+            for (int mt = 0; mt < g.mts && alive; ++mt)
                 for (int q = 0; q < ksteps; ++q, ++it) {
                     if (!mbar_wait_warp(empty_bar + 8u * s, phase ^ 1u, 0, it, wait_limit)) { alive = false; break; }
                     if (elect_one()) {
@@ -110,7 +111,7 @@ conv_dx3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         uint32_t phase = 0;
         bool alive = mbar_wait_warp(b_bar, 0, 1, -1, wait_limit);
         for (int tile = blockIdx.x; tile < g.tiles && alive; tile += gridDim.x, ++n) {
-            for (int mt = 0; mt < 2 && alive; ++mt) {
+            for (int mt = 0; mt < g.mts && alive; ++mt) {
                 // the epilogue has copied this accumulator's previous tile to shared memory (first tile: passes at once)
                 if (!mbar_wait_warp(acc_empty + 8u * mt, ((uint32_t)n & 1u) ^ 1u, 1, it, wait_limit)) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -144,7 +145,7 @@ conv_dx3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const int n = tile / g.tiles_per_img, t = tile - n * g.tiles_per_img;
             const int i_base = g.R * t + g.lo;
             bool ok = true;
-            for (int mt = 0; mt < 2; ++mt) {
+            for (int mt = 0; mt < g.mts; ++mt) {
                 bool got = mbar_wait(acc_full + 8u * mt, (uint32_t)n_it & 1u, 2, n_it, wait_limit);
                 got = __all_sync(0xffffffffu, got);
                 ok = ok && got;
