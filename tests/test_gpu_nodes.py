@@ -258,6 +258,26 @@ def test_classifier_pairs_fuse_into_one_launch(pkg, dev, rows):
     assert results[False][1] == 4 and results[True][1] == (2 if rows <= 256 else 3)
 
 
+@pytest.mark.parametrize("rows,ins,outs", [(1, 5, 3), (3, 36, 10), (100, 784, 100), (100, 100, 10), (257, 67, 33), (65, 1030, 9)])
+def test_weight_and_bias_gradient_of_a_dense_layer_share_a_launch(pkg, dev, rows, ins, outs):
+    """Few and many outputs per thread block, edges of its tiles, one row: the weight gradient bit for bit, the column sums up
+    to the order of their rows."""
+    N = pkg.nodes
+    a, d = _t(seeded((rows, ins), 1), dev), _t(seeded((rows, outs), 2), dev)
+    results = {}
+    for fuse in (False, True):
+        gw, gb = torch.empty((ins, outs), device=dev), torch.empty((outs,), device=dev)
+        ctx = pkg.Context(pkg.PREC_TF32)
+        ctx.run([N.op_tmat_mat_mul(a, d, gw, ins, rows, outs), N.op_mat_sum_cols(d, gb, rows, outs)], fuse=fuse)
+        torch.cuda.synchronize()
+        results[fuse] = gw.cpu().numpy(), gb.cpu().numpy(), ctx.launch_count()
+        ctx.close()
+    assert np.array_equal(results[True][0], results[False][0])
+    exact = d.double().sum(0).cpu().numpy()
+    assert np.abs(results[True][1] - exact).max() <= 1e-6 * np.abs(d.cpu().numpy()).sum(0).max()
+    assert results[False][2] == 2 and results[True][2] == 1
+
+
 def test_reshape_is_an_alias_and_unknown_nodes_fail(pkg, dev):
     """Reshape lowers to no instruction at all (src/ops/reshape.cu:20-44): the consumer reads the
     producer's buffer, so it is bit-exact by construction.  Unknown node types are errors."""
