@@ -8,6 +8,7 @@
 
 #include <atomic>
 
+#include "colsum.cuh"
 #include "common.cuh"
 
 namespace dcg {
@@ -281,63 +282,18 @@ colsum_partial_kernel(const float* __restrict__ a, float* __restrict__ partial,
     colsum_add_rows<VEC>(level2, n_groups, out, cols, tx_count, groups, smem);
 }
 
-// The same sums for a few hundred rows, a column tile per block: at most kSmallSlabs slabs of at most four rows per thread,
-// whose loads are all in flight at once.  Slabs, their trees and the order in which they are added are those of
-// colsum_partial_kernel, so the result is the same bit for bit; what is saved is the hand-over of partial sums between
-// blocks (100 x 100: 7.2 us with it, 3 us without) and the memset of the ticket words.
-constexpr int kSmallSlabs = 8;
+// The same sums for a few hundred rows, a column tile per block: at most kSmallSlabs slabs of at most four rows per lane, side
+// by side with all loads in flight at once.  The plan of colsum_partial_kernel sets the order of the additions and this kernel only
+// spreads them over threads, so the result is the same bit for bit; what is saved is the hand-over of partial sums between blocks
+// and the memset of the ticket words.
+constexpr unsigned kSmallSlabs = 8;
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
-colsum_small_kernel(const float* __restrict__ a, float* __restrict__ out, unsigned rows, unsigned cols, unsigned rows_per_slab,
-                    unsigned slabs, int tx_count)
+colsum_small_kernel(const float* __restrict__ a, float* __restrict__ out, unsigned rows, unsigned cols, const dcg::ColsumOrder order, int tile)
 {
     pdl_enter();
-    constexpr int W = VEC ? 4 : 1;
-    extern __shared__ float smem[];  // [slab][ty][tx][W]
-    const unsigned ty_count = blockDim.x / tx_count, tx = threadIdx.x % tx_count, ty = threadIdx.x / tx_count;
-    const unsigned groups = cols / W, group = blockIdx.x * tx_count + tx;
-    float acc[kSmallSlabs][W];
-#pragma unroll
-    for (int s = 0; s < kSmallSlabs; ++s) {
-#pragma unroll
-        for (int q = 0; q < W; ++q) acc[s][q] = 0.f;
-        if (s < (int)slabs && group < groups) {
-            const unsigned r1 = min((s + 1) * rows_per_slab, rows);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const unsigned r = s * rows_per_slab + ty + i * ty_count;
-                if (r < r1) {
-                    if constexpr (VEC) {
-                        const float4 v = __ldg(reinterpret_cast<const float4*>(a + (size_t)r * cols) + group);
-                        acc[s][0] += v.x; acc[s][1] += v.y; acc[s][2] += v.z; acc[s][3] += v.w;
-                    } else {
-                        acc[s][0] += __ldg(a + (size_t)r * cols + group);
-                    }
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int s = 0; s < kSmallSlabs; ++s)
-        if (s < (int)slabs)
-#pragma unroll
-            for (int q = 0; q < W; ++q) smem[((s * ty_count + ty) * tx_count + tx) * W + q] = acc[s][q];
-    __syncthreads();
-    for (unsigned h = ty_count >> 1; h > 0; h >>= 1) {
-        if (ty < h)
-            for (unsigned s = 0; s < slabs; ++s)
-#pragma unroll
-                for (int q = 0; q < W; ++q)
-                    smem[((s * ty_count + ty) * tx_count + tx) * W + q] += smem[((s * ty_count + ty + h) * tx_count + tx) * W + q];
-        __syncthreads();
-    }
-    if (ty == 0 && group < groups)
-#pragma unroll
-        for (int q = 0; q < W; ++q) {
-            float r = smem[tx * W + q];
-            for (unsigned s = 1; s < slabs; ++s) r += smem[(s * ty_count * tx_count + tx) * W + q];
-            out[(size_t)group * W + q] = r;
-        }
+    extern __shared__ float smem[];
+    dcg::colsum_tile_block<VEC>(a, out, rows, cols, order, tile, blockIdx.x, kThreads, smem);
 }
 
 // Stage 2: block = 32 columns x 8 slab lanes.  Lane ty adds slabs ty, ty+8, ... (four loads in
@@ -732,7 +688,7 @@ struct ColsumPlan {
     unsigned grid_x;    // column-group tiles
     unsigned slabs;     // row slabs = grid_y
     unsigned rows_per_slab;
-    bool small;         // all slabs of a column tile in one block
+    bool small;         // colsum_small_kernel takes it
 };
 
 ColsumPlan colsum_plan(size_t rows, size_t cols, bool ptr_aligned)
@@ -742,11 +698,6 @@ ColsumPlan colsum_plan(size_t rows, size_t cols, bool ptr_aligned)
     p.groups = (unsigned)(p.vec ? cols / 4 : cols);
     int tx = 1;
     while (tx < 32 && (unsigned)tx < p.groups) tx <<= 1;
-    // A few hundred rows are a matter of latency: columns are spread over more blocks (down to 64-byte pieces of a row) until
-    // a block has all rows in flight at once (100 x 100: 4.7 us as four blocks, 8.2 as one)
-    const int min_tx = p.vec ? 4 : 16;
-    if (rows <= (size_t)4 * (kThreads / min_tx))
-        while (tx > min_tx && rows > (size_t)4 * (kThreads / tx)) tx >>= 1;
     p.tx_count = tx;
     p.grid_x = (p.groups + tx - 1) / tx;
     const int ty = kThreads / tx;
@@ -761,7 +712,7 @@ ColsumPlan colsum_plan(size_t rows, size_t cols, bool ptr_aligned)
     if (p.rows_per_slab < 1) p.rows_per_slab = 1;
     p.slabs = (unsigned)((rows + p.rows_per_slab - 1) / p.rows_per_slab);
     if (p.slabs < 1) p.slabs = 1;
-    p.small = p.slabs <= (unsigned)kSmallSlabs && p.rows_per_slab <= 4u * (unsigned)ty;
+    p.small = p.slabs <= kSmallSlabs && p.rows_per_slab <= 4u * (unsigned)ty;
     return p;
 }
 
@@ -775,6 +726,24 @@ size_t colsum_partial_bytes(const ColsumPlan& p, size_t cols)
 }  // namespace
 
 namespace dcg {
+bool colsum_tile(size_t rows, size_t cols, bool aligned, int threads, unsigned max_slabs, ColsumTile& t)
+{
+    const ColsumPlan p = colsum_plan(rows, cols, aligned);
+    const int lanes = kThreads / p.tx_count;
+    if (p.slabs > max_slabs || p.rows_per_slab > 4u * (unsigned)lanes) return false;
+    const int places = (int)p.slabs * lanes;
+    // the widest tile whose rows are all in flight at once, and thereby the most blocks (100 x 100: 4.7 us as four blocks of
+    // eight column quads, 8.2 as one of 32 that takes the slabs one after the other)
+    int tile = 1;
+    while (tile < p.tx_count && 2 * tile * places <= threads) tile <<= 1;
+    t.order = ColsumOrder{p.rows_per_slab, p.slabs, lanes};
+    t.vec = p.vec;
+    t.tile = tile;
+    t.tiles = (p.groups + tile - 1) / tile;
+    t.smem = (size_t)places * tile * (p.vec ? 4 : 1) * sizeof(float);
+    return true;
+}
+
 // The launch behind dcg_colsum.  `tickets`: kColsumTicketBytes of zeroed device memory owned by the
 // caller of this launch (see above), or nullptr to finish with a second kernel instead.
 int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* workspace, size_t workspace_bytes,
@@ -782,14 +751,10 @@ int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* wo
 {
     const ColsumPlan p = colsum_plan(rows, cols, aligned16(a) && aligned16(workspace));
     const size_t need = colsum_partial_bytes(p, cols);
-    if (p.small) {
-        const size_t smem = (size_t)p.slabs * kThreads * (p.vec ? 4 : 1) * sizeof(float);
-        if (p.vec)
-            launch_pdl(colsum_small_kernel<true>, p.grid_x, kThreads, smem, stream, a, out, (unsigned)rows, (unsigned)cols,
-                       p.rows_per_slab, p.slabs, p.tx_count);
-        else
-            launch_pdl(colsum_small_kernel<false>, p.grid_x, kThreads, smem, stream, a, out, (unsigned)rows, (unsigned)cols,
-                       p.rows_per_slab, p.slabs, p.tx_count);
+    ColsumTile t;
+    if (p.small && colsum_tile(rows, cols, p.vec, kThreads, kSmallSlabs, t)) {
+        launch_pdl(t.vec ? colsum_small_kernel<true> : colsum_small_kernel<false>, t.tiles, kThreads, t.smem, stream, a, out,
+                   (unsigned)rows, (unsigned)cols, t.order, t.tile);
         DCG_LAUNCH_CHECK("colsum_small_kernel");
         return DCG_OK;
     }

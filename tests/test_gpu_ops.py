@@ -80,6 +80,57 @@ def test_colsum_of_a_few_hundred_rows(pkg, dev, rows, cols):
     np.testing.assert_allclose(got, a.astype(np.float64).sum(axis=0), rtol=0, atol=2e-6 * rows ** 0.5)
 
 
+def _column_sums_in_order(a, sms):
+    """The column sums with every fp32 addition where dcg_colsum has it: slabs of rows, in each a halving tree over lanes that
+    take every lanes-th row, then the slabs (sixteen at a time, where the column tiles are few) over lanes again."""
+    rows, cols = a.shape
+    groups = cols // 4 if cols % 4 == 0 else cols
+    tx = 1
+    while tx < 32 and tx < groups:
+        tx *= 2
+    lanes, tiles = 256 // tx, -(-groups // tx)
+    want = max(1, min(-(-4 * sms // tiles), 1008, -(-rows // (4 * lanes))))
+    per_slab = -(-rows // want)
+
+    def lane_sums(r, n):
+        acc = np.zeros((n, cols), np.float32)
+        for i in range(0, len(r), n):
+            acc[:len(r[i:i + n])] += r[i:i + n]
+        return acc
+
+    def add_slabs(r, n):
+        acc = lane_sums(r, n)
+        total = acc[0].copy()
+        for lane in acc[1:]:
+            total += lane
+        return total
+
+    slabs = []
+    for r0 in range(0, rows, per_slab):
+        acc, h = lane_sums(a[r0:min(r0 + per_slab, rows)], lanes), lanes // 2
+        while h:
+            acc[:h] += acc[h:2 * h]
+            h //= 2
+        slabs.append(acc[0].copy())
+    if len(slabs) == 1:
+        return slabs[0]
+    if tiles > 16:
+        return add_slabs(np.stack(slabs), 8)
+    while len(slabs) > 1:
+        slabs = [add_slabs(np.stack(slabs[g:g + 16]), lanes) for g in range(0, len(slabs), 16)]
+    return slabs[0]
+
+
+# one lane to 256 of them, slabs that one block adds up and slabs that meet through memory, more column tiles than have a ticket
+@pytest.mark.parametrize("cols", [1, 3, 4, 10, 33, 36, 64, 100, 128, 512, 2052, 8200])
+def test_colsum_order_of_additions(pkg, dev, cols):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for rows in (1, 2, 7, 31, 32, 33, 63, 64, 65, 100, 127, 128, 129, 200, 255, 256, 257, 300, 400, 511, 512, 513):
+        a = seeded((rows, cols), 516)
+        got = pkg.functional.colsum(_t(a, dev)).cpu().numpy()
+        assert np.array_equal(got, _column_sums_in_order(a, sms)), (rows, cols)
+
+
 def test_golden_small_ops(pkg, dev, golden):
     """The reference's unit-test tensors for bias add, activation gradients, losses, argmax."""
     L, g = pkg.lib, golden
