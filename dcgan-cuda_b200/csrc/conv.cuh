@@ -35,6 +35,8 @@ void conv_tc_set_hooks(long long wait_cycles, int skip_stage);
 // Input gradient with the parity classes of a tile in one CTA: 0 never, 1 where it pays (default), 2 wherever
 // the shape allows, anything else: back to the default.
 void conv_tc_set_dx_mode(int mode);
+// dcg_debug_conv_plan.  False: the tensor path does not take the shape.
+bool conv_tc_plan(const dcg_conv_desc& d, int kind, bool x3, int plan[6]);
 unsigned long long conv_tc_fused_dx_launches();   // launches of the class-fused kernel so far
 
 // Shape validation shared by the entry points: 0 or a negative dcg_status.

@@ -294,7 +294,8 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
     return best;
 }
 
-void finish_plan(Plan& pl)
+// False: the accumulators do not fit TMEM or the registers that take them over.
+bool finish_plan(Plan& pl)
 {
     Params& p = pl.p;
     const int b_stage = p.bn * BK * 4;
@@ -302,13 +303,15 @@ void finish_plan(Plan& pl)
     if (p.x3) {
         // A and its residual take 64 TMEM columns per stage, what the accumulators (two and the small terms', or one of each
         // where two do not fit) leave; the residuals of B, which are made ahead of that, up to four tiles
-        p.x3_slots = (512 - (p.bn <= 128 ? 3 : 2) * p.bn) / 64;
+        p.x3_slots = (512 - tmem_columns(kX3, p.bn, 0)) / 64;
         p.x3_slots = p.x3_slots >= 4 ? 4 : 2;   // powers of two
         p.x3_bslots = 4;
     }
     // two CTAs per SM when the grid has more CTAs than SMs, else one deep pipeline
     const bool half = pl.grid > sm_count() && p.bn <= kMaxSharedWidth && !p.x3;
     p.kind = p.x3 ? kX3 : half ? kShared : p.bn <= 64 || p.mt > 1 ? kDual : p.splits == 1 ? kAlone : kShared;
+    if (p.x3 && p.bn > kX3MaxWidth) return false;
+    if (tmem_columns(p.kind, p.bn, p.x3_slots) > (half ? 256 : 512)) return false;
     const int budget = half ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
     int stages = (budget - (p.x3 ? p.x3_bslots * b_stage : 0)) / per_stage;
     if (stages > 8) stages = 8;
@@ -334,6 +337,7 @@ void finish_plan(Plan& pl)
     pl.ws_bytes = pl.partial_bytes;
     if (pl.xp_bytes || pl.k4_bytes) pl.ws_bytes = pl.k4_off() + align_up(pl.k4_bytes, 256);
     if (pl.ycol_bytes) pl.ws_bytes = pl.ycol_off() + align_up(pl.ycol_bytes, 256);
+    return true;
 }
 
 // Padded-image geometry of a narrow-channel layer: rows s*i + di and columns s*j .. s*j + 7 of xp
@@ -419,8 +423,7 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
     } else {
         use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35, 2, pieces));
     }
-    finish_plan(pl);
-    return true;
+    return finish_plan(pl);
 }
 
 // The 1x1 FWD problem behind the DX of a narrow-channel layer: dy [n, ho, wo, o] times k2 [o][Jp].
@@ -460,8 +463,7 @@ bool plan_dx(const dcg_conv_desc& d, Plan& pl)
     const int max_taps = ((d.kh + d.stride_h - 1) / d.stride_h) * ((d.kw + d.stride_w - 1) / d.stride_w);
     use_tiling(pl, choose_tiling(classes * p.tiles_w * p.tiles_h * p.tiles_n, d.c, 16, (min_taps < 1 ? 1 : min_taps) * p.kchunks,
                                  max_taps * p.kchunks, 20));
-    finish_plan(pl);
-    return true;
+    return finish_plan(pl);
 }
 
 // When the input gradient fuses its parity classes (conv_dxf_kernel): 0 never, 1 where one CTA per tile fills the
@@ -623,24 +625,25 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     if (narrow) {
         // rows = output channels (from dy), columns = 32 window slots per kernel row: one tile holds
         // all of dk, so dy is read exactly once; the parallelism comes from partitioning the pixels
-        // over about as many CTAs as there are SMs, whose partial tiles a second kernel adds up
+        // over about as many CTAs as there are SMs, whose partial tiles a second kernel adds up.
+        // 3xTF32 of seven or eight kernel rows, which are wider than it can sum, takes two tiles of four
         if (d.kh * 32 > 256) return false;
         p.narrow = 1;
         p.swap = 1;
         if (d.o % 32 != 0) { p.mt = 0; p.a_ch = d.o; }
         p.m_tiles = (d.o + BM - 1) / BM;
-        p.bn = 32 * d.kh;
-        p.n_tiles = 1;
+        const int rows = p.x3 && 32 * d.kh > kX3MaxWidth ? (d.kh + 1) / 2 : d.kh;
+        p.bn = 32 * rows;
+        p.n_tiles = (d.kh + rows - 1) / rows;
         narrow_geometry(d, pl);
         const int k_stages = p.tiles_w * p.tiles_h * p.tiles_n;
-        int parts = sm_count() / p.m_tiles;
+        int parts = sm_count() / (p.m_tiles * p.n_tiles);
         if (parts > k_stages / 4) parts = k_stages / 4;   // at least 4 K stages per CTA
         if (parts < 1) parts = 1;
         p.splits = parts;
         p.ext_finish = parts > 1 ? 1 : 0;
-        pl.grid = p.m_tiles * p.splits;
-        finish_plan(pl);
-        return true;
+        pl.grid = p.m_tiles * p.n_tiles * p.splits;
+        return finish_plan(pl);
     }
     // M (128 accumulator rows) is the input-channel axis, so that dk rows are contiguous along the accumulator columns,
     // with the channels of four or two taps on top of one another where there are only 32 or 64 of them; or M is the
@@ -657,8 +660,7 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     p.mt = p.swap ? 1 : mt;
     if (pieces) { p.mt = 0; p.a_ch = p.swap ? d.o : d.c; p.b_ch = p.swap ? d.c : d.o; }
     use_tiling(pl, p.swap ? swapped : plain);
-    finish_plan(pl);
-    return true;
+    return finish_plan(pl);
 }
 
 bool make_plan(const dcg_conv_desc& d, int kind, Plan& pl)
@@ -757,8 +759,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, c
     const int st = launch_grid<MODE>(ma, mb, p, pl.grid, pl.smem, stream);
     if (st) return st;
     if (p.ext_finish) {
-        const dim3 fgrid((unsigned)p.bn, (unsigned)((p.O + 31) / 32));
-        launch_pdl(dk_narrow_finish_kernel, fgrid, 256, 0, stream, p.scratch, out, p.splits, p.bn, p.KH, p.KW, p.C, p.O);
+        const dim3 fgrid((unsigned)(p.bn * p.n_tiles), (unsigned)((p.O + 31) / 32));
+        launch_pdl(dk_narrow_finish_kernel, fgrid, 256, 0, stream, p.scratch, out, p.splits, p.bn, p.n_tiles, p.KH, p.KW, p.C, p.O);
         DCG_LAUNCH_CHECK("dk_narrow_finish_kernel");
     }
     return DCG_OK;
@@ -1145,7 +1147,7 @@ int build_dk(const dcg_conv_desc& d, const float* x, const float* dy, void* ws, 
         if (!ws || ws_bytes < pl.ws_bytes)
             return fail(DCG_ERR_WORKSPACE, "conv (tensor path, narrow input): workspace %zu < %zu bytes", ws_bytes, pl.ws_bytes);
         const float* xp = reinterpret_cast<const float*>(static_cast<uint8_t*>(ws) + pl.xp_off());
-        if ((st = map_window(&mx, xp, d, pl, p.TW, p.TH, p.TN, true, d.kh))) return st;
+        if ((st = map_window(&mx, xp, d, pl, p.TW, p.TH, p.TN, true, p.bn / 32))) return st;
         st = p.mt == 0 ? map_act_4d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, true)
                        : map_act_5d(&mdy, dy, d.n, d.ho, d.wo, d.o, p.TW, p.TH, p.TN, 1, 1, BM / 32);
         if (st) return st;
@@ -1309,6 +1311,17 @@ int conv_tc_dk(const dcg_conv_desc& d, const float* x, const float* dy, float* d
     return launch<MODE_DK>(pr.ma, pr.mb, pr.pl, dk, none, d.o, ws, ws_bytes, stream);
 }
 
+bool conv_tc_plan(const dcg_conv_desc& d, int kind, bool x3, int plan[6])
+{
+    PlanX3 scope(x3);
+    Plan pl;
+    if (!make_plan(d, kind, pl)) return false;
+    const Params& p = pl.p;
+    const int values[6] = {p.bn, p.n_tiles, p.splits, p.stages, tmem_columns(p.kind, p.bn, p.x3_slots), (int)pl.smem};
+    for (int i = 0; i < 6; ++i) plan[i] = values[i];
+    return true;
+}
+
 void conv_tc_set_dx_mode(int mode) { g_dxf_mode.store(mode < 0 || mode > 2 ? -1 : mode); }
 unsigned long long conv_tc_fused_dx_launches() { return g_dxf_launches.load(); }
 
@@ -1349,6 +1362,14 @@ extern "C" void dcg_debug_set_wait_limit(long long sm_clocks)
 extern "C" void dcg_debug_skip_stage(int stage) { dcg::conv_tc_set_hooks(0, stage < 0 ? -1 : stage); }
 
 extern "C" void dcg_debug_set_dx_mode(int mode) { dcg::conv_tc_set_dx_mode(mode); }
+extern "C" int dcg_debug_conv_plan(const dcg_conv_desc* desc, int kind, int precision, int plan[6])
+{
+    const int st = dcg::conv_check_desc(desc, "dcg_debug_conv_plan");
+    if (st) return st;
+    if (precision == DCG_PREC_FP32 || !plan || !dcg::conv_tc_plan(*desc, kind, precision == DCG_PREC_3XTF32, plan)) return DCG_ERR_UNSUPPORTED;
+    return DCG_OK;
+}
+
 extern "C" uint64_t dcg_debug_fused_dx_launches(void) { return dcg::conv_tc_fused_dx_launches(); }
 
 #ifdef DCG_TC_TRACING

@@ -11,7 +11,7 @@ namespace {
 // TF32.  Measured, 128 -> 256 channels at batch 64: forward 91 -> 49 us, input gradient 124 -> 61, kernel gradient
 // 80 -> 57; relative error against float64 4e-7 at every layer (3.6e-7 to 4.7e-6 before).
 constexpr int kX3Block = 4;   // K stages per block: sixteen truncating steps in a row
-constexpr int kX3Slabs = 2;    // 32-column slabs per epilogue warp: bn <= 160, every third slab
+constexpr int kX3Slabs = 2;    // 32-column slabs per epilogue warp, every third slab: at most 192 columns (kX3MaxWidth)
 
 // Kinds of launch.
 //   kShared   the plain one; two CTAs per SM where the grid is large enough
@@ -25,6 +25,15 @@ enum Kind { kShared, kX3, kAlone, kDual };
 // Groups of four epilogue warps, one warp per TMEM lane quadrant each.  3xTF32 has three: taking a stage apart is bound by
 // latency, and with two groups it paced the loop.
 template <int KIND> constexpr int kGroups = KIND == kX3 ? 3 : KIND == kAlone ? 4 : 2;
+
+constexpr int kX3MaxWidth = 32 * kGroups<kX3> * kX3Slabs;
+// 3xTF32: accumulators of the large terms.
+__host__ __device__ constexpr int x3_accumulators(int bn) { return bn <= 128 ? 2 : 1; }
+// TMEM columns of a CTA: at most 512, or 256 where two share an SM.
+__host__ __device__ constexpr int tmem_columns(int kind, int bn, int x3_slots)
+{
+    return kind == kX3 ? (x3_accumulators(bn) + 1) * bn + 64 * x3_slots : kind == kDual ? 2 * bn : bn;
+}
 
 // Adds the accumulator's slabs of this warp to `sum`.
 __device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs][32], uint32_t tmem_quad, int group, int bn)
@@ -108,11 +117,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // it, and the tensor core goes on in the other one.  The A operand is read from TMEM (32 columns of values, 32 of
     // residuals per slot): three MMAs per K step take 12 KB from shared memory instead of 24, which is what would pace
     // the loop.  Columns: x3_mains accumulators, the small terms, x3_slots A slots.
-    const int x3_mains = X3 && p.bn <= 128 ? 2 : 1;
+    const int x3_mains = X3 ? x3_accumulators(p.bn) : 1;
     const int x3_a0 = (x3_mains + 1) * p.bn;
     const int x3_slot_mask = p.x3_slots - 1, x3_bslot_mask = p.x3_bslots - 1;   // powers of two
     int tmem_cols = 32;
-    while (tmem_cols < (X3 ? x3_a0 + 64 * p.x3_slots : W * p.bn)) tmem_cols <<= 1;
+    while (tmem_cols < tmem_columns(KIND, p.bn, p.x3_slots)) tmem_cols <<= 1;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -148,7 +157,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         taps_h = rh < p.KH ? (p.KH - rh + p.sh - 1) / p.sh : 0;
         taps_w = rw < p.KW ? (p.KW - rw + p.sw - 1) / p.sw : 0;
     } else if (MODE == MODE_DK) {
-        if (p.narrow) { tap_di = 0; tap_dj = 0; }   // one tile holds every tap: 32 window slots per kernel row
+        if (p.narrow) { tap_di = 0; tap_dj = 0; }   // columns: 32 window slots per kernel row, all taps in one tile or two
         else { tap_di = group * MT / p.KW; tap_dj = group * MT % p.KW; }   // (the first one)
     }
     // K-stage range of this split
@@ -185,7 +194,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     long long col_stride = 1;         // element stride between accumulator columns in the output
     if (MODE == MODE_FWD) ncols_valid = min(p.bn, (p.o_store ? p.o_store : p.O) - ch0);
     else if (MODE == MODE_DX) ncols_valid = min(p.bn, p.C - ch0);
-    else if (p.narrow) { ncols_valid = 32 * p.KH; col_stride = p.O; }
+    else if (p.narrow) { ncols_valid = min(p.bn, 32 * p.KH - ch0); col_stride = p.O; }
     else if (!p.swap) ncols_valid = min(p.bn, p.O - ch0);
     else { ncols_valid = min(p.bn, p.C - ch0); col_stride = p.O; }
     // Row-contiguous outputs whose channel count allows 16-byte stores take the vector path.
@@ -281,14 +290,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         // (tap, di, dj) count the 32-pixel tiles along (n, h, w)
                         const int pj = dj * p.TW, pi = di * p.TH, pn = tap * p.TN;
                         const int xw = p.sw * pj + tap_dj - p.pl, xh = p.sh * pi + tap_di - p.pt;
-                        if (p.narrow) {  // A: dy (rows o), B: the KH 32-float windows of 32 output pixels
+                        if (p.narrow) {  // A: dy (rows o), B: the 32-float windows of 32 output pixels, one per kernel row
                             if constexpr (PIECES) {
                                 for (int i = 0; i < a_pieces; ++i)
                                     tma_load_4d(a_dst + i * kPieceBytes, &map_a, fb, m_tile * BM + 32 * i, pj, pi, pn);
                             } else {
                                 tma_load_5d(a_dst, &map_a, fb, 0, pj, pi, pn, m_tile * (BM / 32));
                             }
-                            tma_load_5d(b_dst, &map_b, fb, 0, pj, pi, pn, 0);   // box covers all KH kernel rows
+                            tma_load_5d(b_dst, &map_b, fb, 0, pj, pi, pn, n_tile * (p.bn / 32));   // the tile's kernel rows
                         } else if (PIECES) {   // both operands
                             const int aw = p.swap ? pj : xw, ah = p.swap ? pi : xh, bw = p.swap ? xw : pj, bh = p.swap ? xh : pi;
                             for (int i = 0; i < a_pieces; ++i)
@@ -741,7 +750,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (col < 0) continue;
                     unsigned long long id = (unsigned long long)ro + (unsigned long long)col * col_stride;
                     if (MODE == MODE_DK && p.narrow) {
-                        const int di = col >> 5, dj = (col & 31) >> 2, c = col & 3;   // slot = 4*dj + channel
+                        const int di = (ch0 + col) >> 5, dj = (col & 31) >> 2, c = col & 3;   // slot = 4*dj + channel
                         if (dj >= p.KW || c >= p.C) continue;                          // padding slots
                         id = (unsigned long long)ro + (unsigned long long)((di * p.KW + dj) * p.C + c) * p.O;
                     }

@@ -6,13 +6,13 @@ namespace dcg {
 namespace {
 
 // ---- narrow-channel DK: add the partitions' partial tiles -----------------------------------------
-// partial[m tile][partition][col][row] (col = 32 * kernel row + window slot, row = output channel).
+// partial[m tile][column tile][partition][col][row] (columns: 32 * kernel row + window slot, row = output channel).
 // Block = 32 rows x 8 lanes of one column: lane l adds partitions l, l+8, ... (all loads in
 // flight), the eight lane sums are then added in lane order - a fixed order for a given partition
 // count, so the result does not depend on timing.  blockIdx.x = column, blockIdx.y = 32-row group.
 __global__ void __launch_bounds__(256)
 dk_narrow_finish_kernel(const float* __restrict__ partial, float* __restrict__ dk, int parts, int bn,
-                        int KH, int KW, int C, int O)
+                        int n_tiles, int KH, int KW, int C, int O)
 {
     pdl_enter();
     __shared__ float lane_sum[8][32];
@@ -24,7 +24,7 @@ dk_narrow_finish_kernel(const float* __restrict__ partial, float* __restrict__ d
     const int mt = o / BM, row = o % BM;
     float acc = 0.f;
     if (o < O) {
-        const float* src = partial + ((size_t)mt * parts * bn + col) * BM + row;
+        const float* src = partial + ((size_t)(mt * n_tiles + col / bn) * parts * bn + col % bn) * BM + row;
         for (int sidx = l; sidx < parts; sidx += 8) acc = __fadd_rn(acc, __ldcg(src + (size_t)sidx * bn * BM));
     }
     lane_sum[l][r] = acc;

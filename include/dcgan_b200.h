@@ -468,10 +468,14 @@ const char* dcg_last_error(void);
  *  dcg_debug_set_dx_mode     which input-gradient kernel the tensor path plans: 0 = one tile per parity class,
  *                            1 = the parity classes of a tile fused in one CTA where one CTA per tile fills the
  *                            GPU (default), 2 = fused wherever the shape allows, < 0 = back to the default;
- *  dcg_debug_fused_dx_launches  how often the fused kernel has been launched (tests check which kernel ran). */
+ *  dcg_debug_fused_dx_launches  how often the fused kernel has been launched (tests check which kernel ran);
+ *  dcg_debug_conv_plan       how the general tensor-path kernel would run `desc` (kind and precision as for
+ *                            dcg_conv_workspace_bytes): tile width, column tiles, K partitions, stages, TMEM columns, bytes
+ *                            of shared memory; DCG_ERR_UNSUPPORTED where it does not take the shape.  Needs no GPU. */
 void dcg_debug_set_wait_limit(long long sm_clocks);
 void dcg_debug_skip_stage(int stage);
 void dcg_debug_set_dx_mode(int mode);
+int dcg_debug_conv_plan(const dcg_conv_desc* desc, int kind, int precision, int plan[6]);
 uint64_t dcg_debug_fused_dx_launches(void);   /* launches of the class-fused input-gradient kernel so far */
 /* Library version and the architecture the kernels were built for ("sm_100a"). */
 const char* dcg_build_info(void);

@@ -318,6 +318,30 @@ def test_full_batch_layers_tf32_vs_fp32_path(pkg, dev, layer):
     assert abs(lhs - (dk * k.double()).sum().item()) <= tol
 
 
+# six kernel rows fill one column tile of the kernel gradient in 3xTF32, seven and eight take two; also with K partitions and
+# without, more than 128 output channels, and a count that comes in pieces of 32
+@pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", [(2, 20, 18, 3, 6, 32, 2), (3, 21, 17, 3, 7, 64, 2), (2, 16, 19, 4, 8, 36, 1), (9, 33, 30, 1, 7, 160, 2),
+                                   (1, 9, 7, 3, 8, 32, 1)])
+def test_tall_kernels_of_rgb_layers(pkg, dev, orc, shape, prec_name):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    prec = getattr(pkg, PRECS[prec_name])
+    x, k = seeded((N, H, W, C), 234), seeded((K, K, C, O), 235) * np.float32(0.1)
+    pad = (oracle.same_pad(H, K, s), oracle.same_pad(W, K, s))
+    y_ref = orc.conv2d(x, k, (s, s))
+    dy = seeded(y_ref.shape, 236)
+    xd, kd, dyd = (torch.from_numpy(a).to(dev) for a in (x, k, dy))
+    y = F.conv2d_fwd(xd, kd, (s, s), precision=prec)
+    dx = F.conv2d_dx(dyd, kd, (H, W), (s, s), precision=prec)
+    dk = F.conv2d_dk(xd, dyd, (K, K), (s, s), precision=prec)
+    torch.cuda.synchronize()
+    assert pkg.lib.dcg_device_status() == 0
+    _check(y, y_ref, prec, pkg, "fwd")
+    _check(dx, orc.conv2d_input_grad(dy, k, s, (H, W)), prec, pkg, "dx")
+    _check(dk, orc.conv2d_kernel_grad(dy, x, s, pad), prec, pkg, "dk")
+
+
 # accumulators 64, 96, 160 and 256 columns wide, one CTA per SM with and without K partitions, two MMA warps on one, two and
 # an odd number of stages, pixel boxes that do not fill their tile, and kernel gradients with the channels of two or four
 # taps in one tile, the last one part empty
