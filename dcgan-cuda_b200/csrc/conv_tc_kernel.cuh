@@ -676,7 +676,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (e.bias) {
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
-                            const float4 bv = __ldg(reinterpret_cast<const float4*>(e.bias + ch0 + cq[u]));
+                            // (a tile may have more columns than there are channels left)
+                            const float4 bv = __ldg(reinterpret_cast<const float4*>(e.bias + ch0 + (cq[u] < ncols_valid ? cq[u] : 0)));
                             acc[u].x = __fadd_rn(acc[u].x, bv.x); acc[u].y = __fadd_rn(acc[u].y, bv.y);
                             acc[u].z = __fadd_rn(acc[u].z, bv.z); acc[u].w = __fadd_rn(acc[u].w, bv.w);
                         }

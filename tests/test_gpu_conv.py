@@ -393,6 +393,31 @@ def test_ragged_channel_counts(pkg, dev, shape, prec_name):
         assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
 
 
+# the last column tile has fewer channels than columns; the bias ends where the channels do, not where the tile does
+@pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", [(2, 12, 20, 36, 5, 40, 2), (1, 7, 9, 36, 1, 36, 1), (40, 24, 24, 60, 3, 260, 1), (5, 13, 11, 68, 3, 260, 2)])
+def test_ragged_channel_counts_with_epilogue(pkg, dev, shape, prec_name):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    ho, wo = -(-H // s), -(-W // s)
+    x, k, dy, gate = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
+                      ((57, (N, H, W, C)), (58, (K, K, C, O)), (59, (N, ho, wo, O)), (60, (N, H, W, C))))
+    bias_o, bias_c = (torch.full((n + 512,), float("nan"), device=dev) for n in (O, C))
+    bias_o[:O], bias_c[:C] = torch.from_numpy(seeded((O,), 61)), torch.from_numpy(seeded((C,), 62))
+    got = {}
+    for prec in (getattr(pkg, PRECS[prec_name]), pkg.PREC_FP32):
+        z, raw = torch.empty((N, ho, wo, O), device=dev), torch.empty((N, H, W, C), device=dev)
+        y = F.conv2d_fwd(x, k, (s, s), epilogue=F.make_epilogue(bias=bias_o[:O], act=pkg.ACT_TANH, pre_act=z), precision=prec)
+        dx = F.conv2d_dx(dy, k, (H, W), (s, s), precision=prec,
+                         epilogue=F.make_epilogue(bias=bias_c[:C], raw_out=raw, gate=gate, gate_act=pkg.ACT_TANH))
+        got[prec] = (y, z, dx, raw)
+    torch.cuda.synchronize()
+    assert pkg.lib.dcg_device_status() == 0
+    tol = TF32_TOL if prec_name == "tf32" else 3e-5
+    for name, a, b in zip(("y", "z", "dx", "raw"), *got.values()):
+        assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
+
+
 @pytest.mark.parametrize("batch", [20, 28, 40, 56, 100])
 def test_k_partition_counts(pkg, dev, batch):
     """The number of K partitions of a tile (= thread-block cluster size) follows the tile count:
