@@ -140,20 +140,18 @@ at::Tensor new_tensor(at::IntArrayRef shape, at::ScalarType type, c10::Device de
 {
     return at::detail::empty_cuda(shape, type, device, std::nullopt);
 }
-// The grow-only scratch buffer of a device.
-void* scratch(size_t need, c10::Device device, size_t& bytes)
-{
-    static std::unordered_map<int, at::Tensor>* buffers = new std::unordered_map<int, at::Tensor>;   // outlives the interpreter
-    bytes = 0;
-    if (need == 0) return nullptr;
-    at::Tensor& b = (*buffers)[device.index()];
-    if (!b.defined() || (size_t)b.numel() < need) {
-        b = at::Tensor();
-        b = new_tensor({(int64_t)(need * 1.25) + 256}, at::kByte, device);
+// The scratch of one call, from torch's caching allocator: held until the launches have been enqueued, and then only the same
+// stream gets the memory again.  A buffer kept for the next call would be shared by all streams and threads (kernels of two
+// streams would write the same partial tiles), and growing it would take it from under kernels and captured graphs that use it.
+struct Scratch {
+    at::Tensor memory;
+    size_t bytes;
+    Scratch(size_t need, c10::Device device) : bytes(need)
+    {
+        if (need) memory = new_tensor({(int64_t)need}, at::kByte, device);
     }
-    bytes = (size_t)b.numel();
-    return b.data_ptr();
-}
+    void* data() const { return bytes ? memory.data_ptr() : nullptr; }
+};
 
 void check(int status)
 {
@@ -192,16 +190,15 @@ PyObject* run_conv(int kind, const dcg_conv_desc& d, const at::Tensor& a, const 
     } else {
         dst = static_cast<float*>(tensor(out).data_ptr());
     }
-    size_t bytes;
-    void* ws = scratch(need, device, bytes);
+    const Scratch ws(need, device);
     const EpilogueView ep(epilogue);
     const float *pa = static_cast<const float*>(a.data_ptr()), *pb = static_cast<const float*>(b.data_ptr());
     void* stream = c10::cuda::getCurrentCUDAStream().stream();
     int status;
     Py_BEGIN_ALLOW_THREADS
-    if (kind == 0) status = dcg_conv2d_fwd(&d, pa, pb, dst, ep.ep, precision, ws, bytes, stream);
-    else if (kind == 1) status = dcg_conv2d_dx(&d, pa, pb, dst, ep.ep, precision, ws, bytes, stream);
-    else status = dcg_conv2d_dk(&d, pa, pb, dst, precision, ws, bytes, stream);
+    if (kind == 0) status = dcg_conv2d_fwd(&d, pa, pb, dst, ep.ep, precision, ws.data(), ws.bytes, stream);
+    else if (kind == 1) status = dcg_conv2d_dx(&d, pa, pb, dst, ep.ep, precision, ws.data(), ws.bytes, stream);
+    else status = dcg_conv2d_dk(&d, pa, pb, dst, precision, ws.data(), ws.bytes, stream);
     Py_END_ALLOW_THREADS
     check(status);
     if (out == Py_None) return THPVariable_Wrap(std::move(result));
@@ -286,13 +283,12 @@ PyObject* colsum(PyObject*, PyObject* const* a, Py_ssize_t n)
         } else {
             dst = static_cast<float*>(tensor(a[1]).data_ptr());
         }
-        size_t bytes;
-        void* ws = scratch(dcg_colsum_workspace_bytes((size_t)rows, (size_t)cols), t.device(), bytes);
+        const Scratch ws(dcg_colsum_workspace_bytes((size_t)rows, (size_t)cols), t.device());
         const float* src = static_cast<const float*>(t.data_ptr());
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
         int status;
         Py_BEGIN_ALLOW_THREADS
-        status = dcg_colsum(src, dst, (size_t)rows, (size_t)cols, ws, bytes, stream);
+        status = dcg_colsum(src, dst, (size_t)rows, (size_t)cols, ws.data(), ws.bytes, stream);
         Py_END_ALLOW_THREADS
         check(status);
         if (a[1] == Py_None) return THPVariable_Wrap(std::move(result));

@@ -4,6 +4,8 @@ DCG_PREC_FP32 keeps the reference CPU's summation order with unfused multiply/ad
 reproduce the oracle bit for bit.  DCG_PREC_TF32 (tcgen05, fp32 accumulate) must stay within
 1e-2 * max|ref| per output tensor - the tolerance stated for the TF32 tensor-core path.
 """
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -416,6 +418,43 @@ def test_ragged_channel_counts_with_epilogue(pkg, dev, shape, prec_name):
     tol = TF32_TOL if prec_name == "tf32" else 3e-5
     for name, a, b in zip(("y", "z", "dx", "raw"), *got.values()):
         assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
+
+
+@pytest.mark.parametrize("threads", [1, 2])
+def test_calls_on_two_streams_do_not_share_scratch(pkg, dev, threads):
+    """K partitions, padded images and column sums of two streams in flight together, from one thread and from two."""
+    F = pkg.functional
+
+    def work(i):
+        x, k, dy = (torch.from_numpy(seeded(t, 70 + i)).to(dev) for t in ((4 + i, 16, 16, 192), (3, 3, 192, 320), (4 + i, 8, 8, 320)))
+        rgb, k3, dy3 = (torch.from_numpy(seeded(t, 80 + i)).to(dev) for t in ((9 + i, 32, 32, 3), (5, 5, 3, 64), (9 + i, 16, 16, 64)))
+        rows = torch.from_numpy(seeded((5000 + i, 37), 90 + i)).to(dev)
+        return lambda: [F.conv2d_fwd(x, k), F.conv2d_dk(x, dy, (3, 3)), F.conv2d_fwd(rgb, k3), F.conv2d_dk(rgb, dy3, (5, 5)), F.colsum(rows)]
+
+    calls = [work(0), work(1)]
+    alone = [call() for call in calls]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], [[], []]
+
+    def run(indexes):
+        for _ in range(20):
+            for i in indexes:
+                with torch.cuda.stream(streams[i]):
+                    got[i].append(calls[i]())
+
+    if threads == 1:
+        run([0, 1])
+    else:
+        workers = [threading.Thread(target=run, args=([i],)) for i in (0, 1)]
+        for w in workers:
+            w.start()
+        for w in workers:
+            w.join()
+    torch.cuda.synchronize()
+    assert [len(g) for g in got] == [20, 20]
+    for i in (0, 1):
+        for again in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(alone[i], again))
 
 
 @pytest.mark.parametrize("batch", [20, 28, 40, 56, 100])
