@@ -8,6 +8,7 @@
 // handlers field for field, including which size array each handler reads.
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <set>
 #include <string>
@@ -306,6 +307,27 @@ inline int grad_act_of_node(int type)
     }
 }
 
+// ---- what a fused launch may write ----------------------------------------------------------------
+// Its blocks store outputs while others still read operands, so an output that lies over anything the launch reads (a gradient
+// written over its logits, an activation over the layer's input) is left to launches of its own, as in the unfused list.
+struct Operand {
+    const float* p;
+    size_t n;
+};
+bool disjoint(Operand a, Operand b)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a.p), y = reinterpret_cast<uintptr_t>(b.p);
+    return !a.p || !b.p || x + a.n * sizeof(float) <= y || y + b.n * sizeof(float) <= x;
+}
+bool disjoint(Operand a, std::initializer_list<Operand> others)
+{
+    for (const Operand& o : others)
+        if (!disjoint(a, o)) return false;
+    return true;
+}
+// Read element by element by the thread that writes the same element.
+bool same_or_disjoint(Operand a, Operand b) { return (a.p == b.p && a.n == b.n) || disjoint(a, b); }
+
 // Tries to run nodes[i..] as one fused convolution; returns the number of nodes
 // consumed (>= 1) or a negative status.
 int run_fused_conv(dcg_context* ctx, const dcg_node* nodes, int i, int count)
@@ -319,13 +341,17 @@ int run_fused_conv(dcg_context* ctx, const dcg_node* nodes, int i, int count)
     float* final_out = cc.out;
     bool raw_dead = (nodes[i].flags & DCG_NODE_OUT_DEAD) != 0;
     bool need_raw = false;
+    const size_t x_elems = (size_t)cc.d.n * cc.d.h * cc.d.w * cc.d.c, y_elems = (size_t)cc.d.n * cc.d.ho * cc.d.wo * cc.d.o;
+    const Operand in_a{cc.a, cc.kind == kConvFwd ? x_elems : y_elems}, in_b{cc.b, (size_t)cc.d.kh * cc.d.kw * cc.d.c * cc.d.o};
+    Operand bias{nullptr, 0};
 
     // bias add directly after
     if (i + used < count) {
         const dcg_node& b = nodes[i + used];
         if (b.type == DCG_OP_MAT_RVECT_ADD && b.in1 == cur && b.len2 == (size_t)cc.out_channels &&
-            b.len1 * b.len2 == cc.out_elems && b.out1 != cur) {
+            b.len1 * b.len2 == cc.out_elems && disjoint({b.out1, cc.out_elems}, {in_a, in_b, {b.in2, b.len2}, {cur, cc.out_elems}})) {
             ep.bias = b.in2;
+            bias = {b.in2, b.len2};
             need_raw = !raw_dead;
             cur = b.out1;
             final_out = b.out1;
@@ -336,7 +362,9 @@ int run_fused_conv(dcg_context* ctx, const dcg_node* nodes, int i, int count)
     if (i + used < count) {
         const dcg_node& a = nodes[i + used];
         const int act = act_of_node(a.type), gact = grad_act_of_node(a.type);
-        if (act >= 0 && a.in1 == cur && a.len1 == cc.out_elems && a.out1 != cur) {
+        const Operand out{a.out1, a.len1};
+        const bool apart = disjoint(out, {in_a, in_b, bias, {cur, cc.out_elems}, {cc.out, cc.out_elems}});
+        if (act >= 0 && a.in1 == cur && a.len1 == cc.out_elems && apart) {
             const bool prev_dead = (nodes[i + used - 1].flags & DCG_NODE_OUT_DEAD) != 0;
             if (ep.bias) {
                 if (!prev_dead) ep.pre_act = const_cast<float*>(cur);
@@ -347,8 +375,8 @@ int run_fused_conv(dcg_context* ctx, const dcg_node* nodes, int i, int count)
             ep.alpha = a.type == DCG_OP_RELU_LEAKY ? a.alpha_leaky : 0.f;
             final_out = a.out1;
             ++used;
-        } else if (gact >= 0 && !ep.bias && a.in2 == cur && a.len1 == cc.out_elems &&
-                   a.out1 != cur && a.in1 != cur) {
+        } else if (gact >= 0 && !ep.bias && a.in2 == cur && a.len1 == cc.out_elems && apart &&
+                   disjoint({a.in1, a.len1}, {cur, cc.out_elems}) && same_or_disjoint(out, {a.in1, a.len1})) {
             need_raw = !raw_dead;
             ep.gate = a.in1;
             ep.gate_act = gact;
@@ -694,7 +722,8 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
             const dcg_node& b = nodes[i + 1];
             // dense layer + activation
             const int act = act_of_node(b.type);
-            if (a.type == DCG_OP_MAT_MUL_ADD && act >= 0 && b.in1 == a.out1 && b.len1 == a.len1 * a.len3 && b.out1 != a.out1) {
+            if (a.type == DCG_OP_MAT_MUL_ADD && act >= 0 && b.in1 == a.out1 && b.len1 == a.len1 * a.len3 &&
+                disjoint({b.out1, b.len1}, {{a.in1, a.len1 * a.len2}, {a.in2, a.len2 * a.len3}, {a.in3, a.len3}, {a.out1, b.len1}})) {
                 const int st = run_dense_on_tensor_path(ctx, &a, act, b.type == DCG_OP_RELU_LEAKY ? b.alpha_leaky : 0.f, b.out1);
                 if (st < 0) return st;
                 if (st == 0) { i += 2; continue; }
@@ -707,7 +736,9 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
             }
             // loss + its gradient on the same labels and logits
             if (a.type == DCG_OP_SIGMOID_CROSS_ENTROPY && b.type == DCG_OP_SIGMOID_CROSS_ENTROPY_GRAD && a.in1 == b.in1 &&
-                a.in2 == b.in2 && a.len1 == b.len1 && a.len1 <= 65536 && a.out1 != b.out1) {
+                a.in2 == b.in2 && a.len1 == b.len1 && a.len1 <= 65536 &&
+                disjoint({a.out1, 1}, {{a.in1, a.len1}, {a.in2, a.len1}, {b.out1, b.len1}}) &&
+                same_or_disjoint({b.out1, b.len1}, {a.in1, a.len1}) && same_or_disjoint({b.out1, b.len1}, {a.in2, a.len1})) {
                 ProfScope scope(ctx, "sigmoid_xent_with_grad", 0.0);
                 const int st = dcg::sigmoid_xent_with_grad(a.in1, a.in2, a.out1, b.out1, a.len1, ctx->stream);
                 if (st) return st;
@@ -715,7 +746,9 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
                 continue;
             }
             if (a.type == DCG_OP_SOFTMAX_CROSS_ENTROPY && b.type == DCG_OP_SOFTMAX_CROSS_ENTROPY_GRAD && a.in1 == b.in1 &&
-                a.in2 == b.in2 && a.len1 == b.len1 && a.len2 == b.len2 && a.len1 <= 256 && a.out1 != b.out1) {
+                a.in2 == b.in2 && a.len1 == b.len1 && a.len2 == b.len2 && a.len1 <= 256 &&
+                disjoint({a.out1, 1}, {{a.in1, a.len1 * a.len2}, {a.in2, a.len1 * a.len2}}) &&
+                disjoint({b.out1, a.len1 * a.len2}, {{a.in1, a.len1 * a.len2}, {a.in2, a.len1 * a.len2}, {a.out1, 1}})) {
                 ProfScope scope(ctx, "softmax_xent_with_grad", 0.0);
                 const int st = dcg::softmax_xent_with_grad(a.in1, a.in2, a.out1, b.out1, a.len1, a.len2, ctx->stream);
                 if (st) return st;
@@ -724,8 +757,9 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
             }
             // x W^T + the activation gradient that gates it (the discriminator head's input gradient)
             const int gact = grad_act_of_node(b.type);
-            if (a.type == DCG_OP_MAT_TMAT_MUL && gact >= 0 && b.in2 == a.out1 && b.in1 != a.out1 && b.out1 != a.out1 &&
-                b.len1 == a.len1 * a.len3) {
+            if (a.type == DCG_OP_MAT_TMAT_MUL && gact >= 0 && b.in2 == a.out1 && b.len1 == a.len1 * a.len3 &&
+                disjoint({a.out1, b.len1}, {b.in1, b.len1}) && same_or_disjoint({b.out1, b.len1}, {b.in1, b.len1}) &&
+                disjoint({b.out1, b.len1}, {{a.in1, a.len1 * a.len2}, {a.in2, a.len2 * a.len3}, {a.out1, b.len1}})) {
                 ProfScope scope(ctx, "mat_tmat_mul_gated", 0.0);
                 const int st = dcg::matmul_nt_gated(a.in1, a.in2, a.out1, a.len1, a.len2, a.len3, b.in1, b.out1, gact,
                                                     b.type == DCG_OP_LEAKY_RELU_GRAD ? b.cons1 : 0.f, ctx->stream);
@@ -739,7 +773,8 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
             const dcg_node& a = nodes[i];
             const dcg_node& b = nodes[i + 1];
             if (a.type == DCG_OP_TMAT_MAT_MUL && b.type == DCG_OP_MAT_SUM_COLS && b.in1 == a.in2 && b.len1 == a.len2 &&
-                b.len2 == a.len3 && a.out1 != b.out1 && a.out1 != b.in1 && ctx->precision != DCG_PREC_FP32) {
+                b.len2 == a.len3 && ctx->precision != DCG_PREC_FP32 && disjoint({a.out1, a.len1 * a.len3}, {b.in1, b.len1 * b.len2}) &&
+                disjoint({b.out1, b.len2}, {{a.in1, a.len2 * a.len1}, {a.in2, a.len2 * a.len3}, {a.out1, a.len1 * a.len3}})) {
                 ProfScope scope(ctx, "tmat_mat_mul", 0.0);
                 const int st = dcg::matmul_tn_sums(a.in1, a.in2, a.out1, a.len1, a.len2, a.len3, b.out1, ctx->stream);
                 if (st < 0) return st;

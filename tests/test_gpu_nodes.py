@@ -258,6 +258,51 @@ def test_classifier_pairs_fuse_into_one_launch(pkg, dev, rows):
     assert results[False][1] == 4 and results[True][1] == (2 if rows <= 256 else 3)
 
 
+def _overwriting_lists(N, dev):
+    """(name, list of nodes, tensors to compare) where an output lies over something that the launch before it reads."""
+    def t(shape, seed):
+        return _t(seeded(shape, seed), dev)
+
+    y = torch.eye(10, device=dev)[torch.arange(100, device=dev) % 10].contiguous()
+    logits, loss = t((100, 10), 1), torch.zeros((1,), device=dev)
+    yield "softmax gradient over its logits", [N.op_softmax_cross_entropy(y, logits, loss, 100, 10),
+                                               N.op_softmax_cross_entropy_grad(y, logits, logits, 100, 10)], [logits, loss]
+    y2, x2, loss2 = t((999,), 2).abs(), t((999,), 3), torch.zeros((1,), device=dev)
+    yield "sigmoid gradient over its logits", [N.op_sigmoid_cross_entropy(y2, x2, loss2, 999),
+                                               N.op_sigmoid_cross_entropy_grad(y2, x2, x2, 999)], [x2, loss2]
+    x, w, b, z = t((96, 96), 4), t((96, 96), 5), t((96,), 6), torch.empty((96, 96), device=dev)
+    yield "activation over the layer's input", [N.op_mat_mul_add(x, w, b, z, 96, 96, 96), N.op_tanh(z, x, 96 * 96)], [x, z]
+    x3, w3, b3 = t((64, 64), 7), t((64, 64), 8), t((64,), 9)
+    both = torch.empty((65, 64), device=dev)
+    yield "activation one row on", [N.op_mat_mul_add(x3, w3, b3, both[:64], 64, 64, 64), N.op_relu(both[:64], both[1:], 64 * 64)], [both]
+    dz, w4, gate, da = t((96, 96), 10), t((96, 96), 11), t((96, 96), 12), torch.empty((96, 96), device=dev)
+    yield "gated gradient over the gradient", [N.op_mat_tmat_mul(dz, w4, da, 96, 96, 96), N.op_relu_grad(gate, da, dz, 96 * 96)], [dz, da]
+    a5, d5, gw = t((100, 100), 13), t((100, 100), 14), torch.empty((100, 100), device=dev)
+    yield "bias gradient over the layer's input", [N.op_tmat_mat_mul(a5, d5, gw, 100, 100, 100),
+                                                   N.op_mat_sum_cols(d5, a5[0], 100, 100)], [a5, gw]
+    x6, k6, z6 = t((2, 16, 16, 32), 15), t((3, 3, 32, 32), 16), torch.empty((2, 16, 16, 32), device=dev)
+    yield "activation over a convolution's input", [N.op_conv2d(x6, k6, (1, 1), 2, 2, z6, x6.shape, k6.shape),
+                                                    N.op_relu(z6, x6, x6.numel())], [x6, z6]
+
+
+def test_outputs_over_operands_are_not_fused(pkg, dev):
+    N = pkg.nodes
+    names = [name for name, _, _ in _overwriting_lists(N, dev)]
+    for at, name in enumerate(names):
+        results = {}
+        for fuse in (False, True):
+            _, nodes, tensors = list(_overwriting_lists(N, dev))[at]
+            ctx = pkg.Context(pkg.PREC_TF32)
+            ctx.run(nodes, fuse=fuse)
+            torch.cuda.synchronize()
+            results[fuse] = [t.cpu().numpy() for t in tensors], ctx.launch_count()
+            ctx.close()
+        for p, q in zip(results[False][0], results[True][0]):
+            assert np.array_equal(p, q), name
+        # one block takes the sigmoid pair, each element read and written by one thread: in place is as good as apart
+        assert results[True][1] == (1 if name.startswith("sigmoid") else results[False][1]), name
+
+
 @pytest.mark.parametrize("rows,ins,outs", [(1, 5, 3), (3, 36, 10), (100, 784, 100), (100, 100, 10), (257, 67, 33), (65, 1030, 9)])
 def test_weight_and_bias_gradient_of_a_dense_layer_share_a_launch(pkg, dev, rows, ins, outs):
     """Few and many outputs per thread block, edges of its tiles, one row: the weight gradient bit for bit, the column sums up
