@@ -9,6 +9,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "colsum.cuh"
 #include "common.cuh"
 
 namespace dcg {
@@ -46,7 +47,9 @@ struct DenseEpilogue {
     float* out2;
     int act;         // of out2: activation, or with `gate` the activation whose gradient gates
     float alpha;
-    float* sums;     // TA only: column sums of B, k ascending
+    float* sums;     // TA only: column sums of B, as dcg_colsum adds them, by the first `sum_rows` rows of blocks
+    ColsumTile sum;
+    int sum_rows;
 };
 
 // out[m,p] = A[m,n] B[n,p]: TM x TN outputs per thread, TX x TY threads per block, STAGES stages of KC reduction steps
@@ -66,7 +69,19 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
     extern __shared__ __align__(16) float smem[];
     pdl_enter();
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+    int block_row = blockIdx.y;
+    if constexpr (TA && !TB) {
+        if (block_row < e.sum_rows) {
+            for (unsigned tile = block_row * gridDim.x + blockIdx.x; tile < e.sum.tiles; tile += e.sum_rows * gridDim.x) {
+                if (e.sum.vec) colsum_tile_block<true>(b, e.sums, n, p, e.sum.order, e.sum.tile_shift, tile, THREADS, smem);
+                else colsum_tile_block<false>(b, e.sums, n, p, e.sum.order, e.sum.tile_shift, tile, THREADS, smem);
+                __syncthreads();
+            }
+            return;
+        }
+        block_row -= e.sum_rows;
+    }
+    const int row0 = block_row * BM, col0 = blockIdx.x * BN;
     const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(smem);
 
     // copies a tile of `inner` contiguous elements x `outer` lines, element (o, i) of the stored matrix at base[o * ld + i];
@@ -103,11 +118,6 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) load_stage(s * KC, s);
-    // the blocks and threads of the first row add up B as well
-    const bool sum_b = TA && !TB && e.sums && blockIdx.y == 0 && ty == 0;
-    float bsum[TN];
-#pragma unroll
-    for (int j = 0; j < TN; ++j) bsum[j] = 0.f;
     int buf = 0;
     for (int k0 = 0; k0 < n; k0 += KC) {
         load_stage(k0 + (STAGES - 1) * KC, (buf + STAGES - 1) % STAGES);
@@ -116,7 +126,8 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
         const float* as = smem + buf * STAGE + (TA ? ty * TM : ty * TM * LDA);
         const float* bs = smem + buf * STAGE + A_FLOATS + (TB ? tx * LDB : tx * TN);   // TB: columns tx, tx + TX, ...
         const int kc = min(KC, (n - k0 + 3) & ~3);
-#pragma unroll KC / 16
+        // (one output to a thread: 32 steps of A^T B at a time, whose reads are single words; 100 x 2000 x 100 29 -> 26 us)
+#pragma unroll (TA && !TB && TM * TN == 1 ? KC / 8 : KC / 16)
         for (int k = 0; k < kc; k += 4) {
             float av[4][TM], bv[4][TN];
             if (TA) {
@@ -141,12 +152,6 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
 #pragma unroll
                 for (int u = 0; u < 4; ++u) tile_read<TN>(bs + (k + u) * LDB, bv[u]);
             }
-            if (sum_b) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) bsum[j] = __fadd_rn(bsum[j], bv[u][j]);
-            }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -156,11 +161,6 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
         }
         __syncthreads();
         buf = (buf + 1) % STAGES;
-    }
-    if (sum_b) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j)
-            if (col0 + tx * TN + j < p) e.sums[col0 + tx * TN + j] = bsum[j];
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -270,8 +270,12 @@ gemm_tall_tn_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
 
 bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
+// Column sums that fit a block of any tile.
+constexpr unsigned kSumSlabs = 32;
+constexpr size_t kSumSmem = 8192;   // 512 lanes of 16 bytes
+
 template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES, int KC = 64>
-int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const DenseEpilogue& e, cudaStream_t stream)
+int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, DenseEpilogue e, cudaStream_t stream)
 {
     constexpr int BM = TM * TY, BN = TN * TX;
     constexpr size_t smem = (size_t)STAGES * ((TA ? KC * (BM + 4) : BM * (KC + 4)) + (TB ? BN * (KC + 4) : KC * (BN + 4))) * sizeof(float);
@@ -282,7 +286,14 @@ int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, 
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
     DCG_CUDA(attr_err);
-    const dim3 grid((unsigned)((p + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
+    dim3 grid((unsigned)((p + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
+    static_assert(smem >= kSumSmem && TX * TY <= 256, "the column sums run in the same blocks");
+    if (e.sums) {   // a block each for the column tiles, up to 32: they are not to crowd the others on some of the SMs
+        colsum_fit(e.sum, TX * TY);
+        const int rows = (int)((e.sum.tiles + grid.x - 1) / grid.x), most = grid.x >= 32 ? 1 : (int)(32 / grid.x);
+        e.sum_rows = rows < most ? rows : most;
+        grid.y += e.sum_rows;
+    }
     const int vec_a = (TA ? m : n) % 4 == 0 && aligned16(a), vec_b = (TB ? n : p) % 4 == 0 && aligned16(b);
     launch_pdl(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>, grid, TX * TY, smem, stream, a, b, out, (int)m, (int)n, (int)p, e,
                vec_a, vec_b);
@@ -351,12 +362,15 @@ int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t
 }
 
 // dcg_matmul_tn and the column sums of its right operand as one launch (node fusion of the backend): the weight and the bias
-// gradient of a dense layer.  Not for the shapes of gemm_tall_tn_kernel: returns 1 there.
+// gradient of a dense layer, both bit for bit.  Blocks of their own add the columns beside those of the product, which take as
+// long or longer: 100 x 784 x 100 4.1 us with and without them, 2.3 for the sums by themselves.  Not for the shapes of
+// gemm_tall_tn_kernel, nor for more rows than a block adds up (1024 where a column tile is 32 wide): returns 1 there.
 int matmul_tn_sums(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, float* sums, cudaStream_t stream)
 {
-    if (p <= 8 && m >= 1024) return 1;
+    if ((p <= 8 && m >= 1024) || m > (1u << 20)) return 1;
     DCG_CHECK_ARG(a && b && out && sums && m > 0 && n > 0 && p > 0, "matmul_tn_sums: bad arguments");
     DenseEpilogue e{};
+    if (!colsum_order(n, p, aligned16(b), kSumSlabs, e.sum) || (e.sum.order.slabs << e.sum.order.lane_shift) * 16 > kSumSmem) return 1;
     e.sums = sums;
     return launch_ordered<true, false>(a, b, out, m, n, p, e, stream);
 }

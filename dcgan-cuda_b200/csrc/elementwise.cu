@@ -289,11 +289,11 @@ colsum_partial_kernel(const float* __restrict__ a, float* __restrict__ partial,
 constexpr unsigned kSmallSlabs = 8;
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
-colsum_small_kernel(const float* __restrict__ a, float* __restrict__ out, unsigned rows, unsigned cols, const dcg::ColsumOrder order, int tile)
+colsum_small_kernel(const float* __restrict__ a, float* __restrict__ out, unsigned rows, unsigned cols, const dcg::ColsumOrder order, int tile_shift)
 {
     pdl_enter();
     extern __shared__ float smem[];
-    dcg::colsum_tile_block<VEC>(a, out, rows, cols, order, tile, blockIdx.x, kThreads, smem);
+    dcg::colsum_tile_block<VEC>(a, out, rows, cols, order, tile_shift, blockIdx.x, kThreads, smem);
 }
 
 // Stage 2: block = 32 columns x 8 slab lanes.  Lane ty adds slabs ty, ty+8, ... (four loads in
@@ -726,21 +726,19 @@ size_t colsum_partial_bytes(const ColsumPlan& p, size_t cols)
 }  // namespace
 
 namespace dcg {
-bool colsum_tile(size_t rows, size_t cols, bool aligned, int threads, unsigned max_slabs, ColsumTile& t)
+bool colsum_order(size_t rows, size_t cols, bool aligned, unsigned max_slabs, ColsumTile& t)
 {
     const ColsumPlan p = colsum_plan(rows, cols, aligned);
     const int lanes = kThreads / p.tx_count;
     if (p.slabs > max_slabs || p.rows_per_slab > 4u * (unsigned)lanes) return false;
-    const int places = (int)p.slabs * lanes;
-    // the widest tile whose rows are all in flight at once, and thereby the most blocks (100 x 100: 4.7 us as four blocks of
-    // eight column quads, 8.2 as one of 32 that takes the slabs one after the other)
-    int tile = 1;
-    while (tile < p.tx_count && 2 * tile * places <= threads) tile <<= 1;
-    t.order = ColsumOrder{p.rows_per_slab, p.slabs, lanes};
+    if (p.slabs > kSlabGroup * kSlabGroup) return false;   // (colsum_add_rows keeps four sums per lane from here on)
+    const bool tickets = p.grid_x <= (unsigned)kTicketTiles;   // otherwise colsum_final_kernel adds all slabs, over eight lanes
+    int lane_shift = 0;
+    while (1 << lane_shift < lanes) ++lane_shift;
+    t.order = ColsumOrder{p.rows_per_slab, p.slabs, tickets ? (unsigned)kSlabGroup : p.slabs, lane_shift, tickets ? lanes : 8};
     t.vec = p.vec;
-    t.tile = tile;
-    t.tiles = (p.groups + tile - 1) / tile;
-    t.smem = (size_t)places * tile * (p.vec ? 4 : 1) * sizeof(float);
+    t.groups = p.groups;
+    t.widest = 8 - lane_shift;   // the plan's own tile
     return true;
 }
 
@@ -752,9 +750,10 @@ int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* wo
     const ColsumPlan p = colsum_plan(rows, cols, aligned16(a) && aligned16(workspace));
     const size_t need = colsum_partial_bytes(p, cols);
     ColsumTile t;
-    if (p.small && colsum_tile(rows, cols, p.vec, kThreads, kSmallSlabs, t)) {
+    if (p.small && colsum_order(rows, cols, p.vec, kSmallSlabs, t)) {
+        colsum_fit(t, kThreads);
         launch_pdl(t.vec ? colsum_small_kernel<true> : colsum_small_kernel<false>, t.tiles, kThreads, t.smem, stream, a, out,
-                   (unsigned)rows, (unsigned)cols, t.order, t.tile);
+                   (unsigned)rows, (unsigned)cols, t.order, t.tile_shift);
         DCG_LAUNCH_CHECK("colsum_small_kernel");
         return DCG_OK;
     }

@@ -334,9 +334,7 @@ int dcg_run_node(dcg_context* ctx, const dcg_node* node);
  * input-gradient -> activation-gradient likewise, and every
  * moment_update / moment_update2 / adam_update triple of the list into one
  * multi-tensor launch.  Results are identical to unfused execution except for
- * buffers flagged DCG_NODE_OUT_DEAD and for the rounding of a mat_sum_cols that
- * follows the tmat_mat_mul of the same gradient (not in DCG_PREC_FP32): it then
- * adds its rows in ascending order, in the same launch. */
+ * buffers flagged DCG_NODE_OUT_DEAD. */
 int dcg_run_nodes(dcg_context* ctx, const dcg_node* nodes, int count, int fuse);
 
 /* ---- data parallelism ------------------------------------------------------

@@ -323,6 +323,29 @@ def test_weight_and_bias_gradient_of_a_dense_layer_share_a_launch(pkg, dev, rows
     assert results[False][2] == 2 and results[True][2] == 1
 
 
+@pytest.mark.parametrize("outs", [1, 4, 10, 33, 100, 512, 2052])
+def test_bias_gradient_beside_the_weight_gradient_is_the_column_sum(pkg, dev, outs):
+    """Bit for bit, whatever the rows; beyond what a block adds up the two run one after the other."""
+    N = pkg.nodes
+    counts = set()
+    for rows in (1, 9, 64, 65, 255, 257, 513, 700, 1000, 1024, 1025, 3000, 20000):
+        a, d = _t(seeded((rows, 40), 1), dev), _t(seeded((rows, outs), 2), dev)
+        results = {}
+        for fuse in (False, True):
+            gw, gb = torch.empty((40, outs), device=dev), torch.empty((outs,), device=dev)
+            ctx = pkg.Context(pkg.PREC_TF32)
+            ctx.run([N.op_tmat_mat_mul(a, d, gw, 40, rows, outs), N.op_mat_sum_cols(d, gb, rows, outs)], fuse=fuse)
+            torch.cuda.synchronize()
+            results[fuse] = gw.cpu().numpy(), gb.cpu().numpy()
+            if fuse:
+                counts.add((rows <= 1024, ctx.launch_count()))
+            ctx.close()
+        assert np.array_equal(results[True][0], results[False][0]) and np.array_equal(results[True][1], results[False][1]), rows
+        exact = d.double().sum(0).cpu().numpy()
+        assert np.abs(results[True][1] - exact).max() <= 1e-6 * np.abs(d.cpu().numpy()).sum(0).max()
+    assert (True, 1) in counts and (True, 2) not in counts and max(n for _, n in counts) >= 2
+
+
 def test_reshape_is_an_alias_and_unknown_nodes_fail(pkg, dev):
     """Reshape lowers to no instruction at all (src/ops/reshape.cu:20-44): the consumer reads the
     producer's buffer, so it is bit-exact by construction.  Unknown node types are errors."""
