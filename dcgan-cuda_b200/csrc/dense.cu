@@ -61,7 +61,7 @@ struct DenseEpilogue {
 template <bool TA, bool TB, int TM, int TN, int TX, int TY, int STAGES, int KC>
 __global__ void __launch_bounds__(TX * TY)
 gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const int m, const int n,
-                    const int p, const DenseEpilogue e, const int vec_a, const int vec_b)
+                    const int p, const DenseEpilogue e, const int vec_a, const int vec_b, const int vec_out)
 {
     constexpr int BM = TM * TY, BN = TN * TX, THREADS = TX * TY;
     constexpr int LDA = TA ? BM + 4 : KC + 4, LDB = TB ? KC + 4 : BN + 4;
@@ -166,6 +166,19 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
     for (int i = 0; i < TM; ++i) {
         const int r = row0 + ty * TM + i;
         if (r >= m) continue;
+        if constexpr (!TB && TN == 4) {
+            const int c = col0 + tx * TN;
+            if (vec_out && !e.out2) {   // whole rows of 16-byte words
+                if (c >= p) continue;
+                float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+                if (e.bias) {
+                    const float4 w = __ldg(reinterpret_cast<const float4*>(e.bias + c));
+                    v.x = __fadd_rn(v.x, w.x); v.y = __fadd_rn(v.y, w.y); v.z = __fadd_rn(v.z, w.z); v.w = __fadd_rn(v.w, w.w);
+                }
+                *reinterpret_cast<float4*>(out + (size_t)r * p + c) = v;
+                continue;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int c = col0 + (TB ? tx + j * TX : tx * TN + j);
@@ -179,8 +192,8 @@ gemm_ordered_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
     }
 }
 
-// Outer product of a column and a row (n == 1: the input gradient of the head, 64 x 1 times 1 x 8192): four columns per
-// thread, nothing to stage.  Memory-bound: the gate is read and both outputs written once.
+// Outer product of a column and a row (n == 1, whichever way the operands are stored: the input gradient of the head, 64 x 1
+// times 1 x 8192, weight gradients of one row): four columns per thread, nothing to stage.  Memory-bound: the gate is read and both outputs written once.
 __global__ void __launch_bounds__(TPB)
 gemm_outer_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const size_t m, const size_t p4,
                   const DenseEpilogue e)
@@ -295,8 +308,16 @@ int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, 
         grid.y += e.sum_rows;
     }
     const int vec_a = (TA ? m : n) % 4 == 0 && aligned16(a), vec_b = (TB ? n : p) % 4 == 0 && aligned16(b);
-    launch_pdl(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>, grid, TX * TY, smem, stream, a, b, out, (int)m, (int)n, (int)p, e,
-               vec_a, vec_b);
+    const int vec_out = p % 4 == 0 && aligned16(out) && aligned16(e.bias);
+    const auto kernel = gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>;
+    if (TM * TN < 16 || KC < 64) {
+        launch_pdl(kernel, grid, TX * TY, smem, stream, a, b, out, (int)m, (int)n, (int)p, e, vec_a, vec_b, vec_out);
+    } else {
+        // Long blocks, often fewer than SMs: launched while the previous kernel runs, they pile up on the SMs that it leaves free
+        // and stay there (100 x 256 x 8192 38 us so, 27.7 after it; the gradients of a 784-512-10 classifier's step at 1000 rows
+        // 271 and 164).  A launch that waits costs 0.3 us.
+        kernel<<<grid, TX * TY, smem, stream>>>(a, b, out, (int)m, (int)n, (int)p, e, vec_a, vec_b, vec_out);
+    }
     DCG_LAUNCH_CHECK("gemm_ordered_kernel");
     return DCG_OK;
 }
@@ -309,7 +330,7 @@ int launch_ordered(const float* a, const float* b, float* out, size_t m, size_t 
 {
     DCG_CHECK_ARG(m < (1u << 30) && n < (1u << 30) && p < (1u << 30), "dense: %zu x %zu x %zu is too large", m, n, p);
     DCG_CHECK_ARG((m + 3) / 4 <= 65535u * 16, "dense: %zu rows are too many", m);
-    if (!TA && n == 1 && p % 4 == 0 && aligned16(b) && aligned16(out) && aligned16(e.bias) && aligned16(e.gate) && aligned16(e.out2)) {
+    if (!e.sums && n == 1 && p % 4 == 0 && aligned16(b) && aligned16(out) && aligned16(e.bias) && aligned16(e.gate) && aligned16(e.out2)) {
         size_t blocks = (m * (p / 4) + TPB - 1) / TPB;
         const size_t cap = (size_t)sm_count() * 8;
         if (blocks > cap) blocks = cap;
@@ -319,6 +340,9 @@ int launch_ordered(const float* a, const float* b, float* out, size_t m, size_t 
     }
     const double per_lane = (double)m * (double)p / (128.0 * sm_count());
     if (m <= 8 && p >= 512) return launch_tile<TA, TB, 1, 1, 32, 8, 3>(a, b, out, m, n, p, e, stream);
+    // a few reduction steps: shorter lines to walk through, the rest is stores (784 x 2 x 512 2.8 us, 4.8 with 64 steps a stage;
+    // 4096 x 10 x 4096 29 and 58)
+    if (per_lane >= 20 && n <= 16) return launch_tile<TA, TB, 4, 4, 16, 16, 2, 16>(a, b, out, m, n, p, e, stream);
     if (per_lane >= 20) return launch_tile<TA, TB, 4, 4, 16, 16, 2>(a, b, out, m, n, p, e, stream);
     if (per_lane >= 5) return launch_tile<TA, TB, 2, 2, 16, 16, 3>(a, b, out, m, n, p, e, stream);
     // Where 16 x 16 tiles would leave half of the SMs without a block, smaller ones; each sum is one chain of K steps, so what

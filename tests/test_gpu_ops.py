@@ -212,6 +212,29 @@ def test_dense_is_bit_exact(pkg, dev, orc, m, n, p):
     assert np.array_equal(dx.cpu().numpy(), orc.mtm_mul(dy, b))
 
 
+# the form for a few reduction steps and its limits, the outer product from either storage, stores of whole words and of single
+# ones, unaligned operands and results
+@pytest.mark.parametrize("m,n,p,off", [(700, 1, 640, 0), (700, 2, 641, 0), (650, 15, 642, 0), (650, 16, 644, 0), (650, 17, 644, 0),
+                                       (700, 7, 644, 1), (130, 1, 600, 1), (1300, 16, 301, 0)])
+def test_dense_with_a_short_reduction(pkg, dev, orc, m, n, p, off):
+    L = pkg.lib
+
+    def put(t):
+        buf = torch.empty((t.size + off,), device=dev)
+        buf[off:] = torch.from_numpy(t.reshape(-1)).to(dev)
+        return buf[off:]
+
+    a, b, bias, at, bt = (seeded(s, 534 + i) for i, s in enumerate([(m, n), (n, p), (p,), (n, m), (p, n)]))
+    ad, bd, biasd, atd, btd = (put(t) for t in (a, b, bias, at, bt))
+    out, tn, nt = (put(np.zeros((m, p), np.float32)) for _ in range(3))
+    pkg._lib.check(L.dcg_matmul(ad.data_ptr(), bd.data_ptr(), biasd.data_ptr(), out.data_ptr(), m, n, p, _s()))
+    pkg._lib.check(L.dcg_matmul_tn(atd.data_ptr(), bd.data_ptr(), tn.data_ptr(), m, n, p, _s()))
+    pkg._lib.check(L.dcg_matmul_nt(ad.data_ptr(), btd.data_ptr(), nt.data_ptr(), m, n, p, _s()))
+    assert np.array_equal(out.cpu().numpy().reshape(m, p), orc.mat_mul_add(a, b, bias))
+    assert np.array_equal(tn.cpu().numpy().reshape(m, p), orc.tmm_mul(at, b))
+    assert np.array_equal(nt.cpu().numpy().reshape(m, p), orc.mtm_mul(a, bt))
+
+
 def test_losses(pkg, dev, orc):
     L = pkg.lib
     for n in (64, 1000):
