@@ -52,13 +52,147 @@ __device__ __forceinline__ void lds_vec(const float* s, float (&v)[W])
     }
 }
 
+// ---- one output as the reference's loops have it ------------------------------------------------------------
+// y[pixel, o] of pixel number `pixel`
+__device__ __forceinline__ float fwd_sum(const float* __restrict__ x, const float* __restrict__ k, const dcg_conv_desc& d, size_t pixel, int o)
+{
+    const int j = (int)(pixel % d.wo);
+    size_t t = pixel / d.wo;
+    const int i = (int)(t % d.ho);
+    const int n = (int)(t / d.ho);
+    const int h0 = i * d.stride_h - d.pad_top, w0 = j * d.stride_w - d.pad_left;
+    const float* xn = x + (size_t)n * d.h * d.w * d.c;
+    float val = 0.f;
+    for (int q = 0; q < d.c; ++q)
+        for (int di = 0; di < d.kh; ++di) {
+            const int h = h0 + di;
+            if (h < 0 || h >= d.h) continue;
+            for (int dj = 0; dj < d.kw; ++dj) {
+                const int w = w0 + dj;
+                if (w < 0 || w >= d.w) continue;
+                const float xv = __ldg(xn + ((size_t)h * d.w + w) * d.c + q);
+                const float kv = __ldg(k + (((size_t)di * d.kw + dj) * d.c + q) * d.o + o);
+                val = __fadd_rn(val, __fmul_rn(xv, kv));
+            }
+        }
+    return val;
+}
+
+// dx[n,i,j,c] = sum_o ( sum_{di,dj} dyz[n,i+di-P,j+dj-Q,o] * k[KH-1-di,KW-1-dj,c,o] ), dyz the
+// zero-inserted dy, P = KH-1-pad_top, Q = KW-1-pad_left (src/cpu/ops.hxx:618-629).
+__device__ __forceinline__ float dx_sum(const float* __restrict__ dy, const float* __restrict__ k, const dcg_conv_desc& d, size_t pixel, int c)
+{
+    const int j = (int)(pixel % d.w);
+    size_t t = pixel / d.w;
+    const int i = (int)(t % d.h);
+    const int n = (int)(t / d.h);
+    const int P = d.kh - 1 - d.pad_top, Q = d.kw - 1 - d.pad_left;
+    const float* dyn = dy + (size_t)n * d.ho * d.wo * d.o;
+    float total_v = 0.f;
+    for (int o = 0; o < d.o; ++o) {
+        float val = 0.f;
+        for (int di = 0; di < d.kh; ++di) {
+            const int ph = i + di - P;
+            if (ph < 0 || ph % d.stride_h != 0) continue;
+            const int a = ph / d.stride_h;
+            if (a >= d.ho) continue;
+            for (int dj = 0; dj < d.kw; ++dj) {
+                const int pw = j + dj - Q;
+                if (pw < 0 || pw % d.stride_w != 0) continue;
+                const int b = pw / d.stride_w;
+                if (b >= d.wo) continue;
+                const float g = __ldg(dyn + ((size_t)a * d.wo + b) * d.o + o);
+                const float kv = __ldg(k + (((size_t)(d.kh - 1 - di) * d.kw + (d.kw - 1 - dj)) * d.c + c) * d.o + o);
+                val = __fadd_rn(val, __fmul_rn(g, kv));
+            }
+        }
+        total_v = (o == 0) ? val : __fadd_rn(total_v, val);
+    }
+    return total_v;
+}
+
+// dk[row, o] = sum_n ( sum_{a,b} x[n,kh+s*a-pt,kw+s*b-pl,c] * dy[n,a,b,o] ), row = (kh * KW + kw) * C + c
+__device__ __forceinline__ float dk_sum(const float* __restrict__ x, const float* __restrict__ dy, const dcg_conv_desc& d, size_t row, int o)
+{
+    const int c = (int)(row % d.c);
+    size_t t = row / d.c;
+    const int kw = (int)(t % d.kw);
+    const int kh = (int)(t / d.kw);
+    float total_v = 0.f;
+    for (int n = 0; n < d.n; ++n) {
+        const float* xn = x + (size_t)n * d.h * d.w * d.c;
+        const float* dyn = dy + (size_t)n * d.ho * d.wo * d.o;
+        float val = 0.f;
+        for (int a = 0; a < d.ho; ++a) {
+            const int h = kh + d.stride_h * a - d.pad_top;
+            if (h < 0 || h >= d.h) continue;
+            for (int b = 0; b < d.wo; ++b) {
+                const int w = kw + d.stride_w * b - d.pad_left;
+                if (w < 0 || w >= d.w) continue;
+                const float xv = __ldg(xn + ((size_t)h * d.w + w) * d.c + c);
+                const float g = __ldg(dyn + ((size_t)a * d.wo + b) * d.o + o);
+                val = __fadd_rn(val, __fmul_rn(xv, g));
+            }
+        }
+        total_v = (n == 0) ? val : __fadd_rn(total_v, val);
+    }
+    return total_v;
+}
+
+// The ordered kernels multiply taps outside the image as zeros where the reference skips them.  That adds +0 and leaves the same
+// bits unless the other factor is infinite or NaN, and then the result is not finite either: a thread with such a result computes
+// its outputs again with the sums above.
+template <int TM, int TN>
+__device__ __forceinline__ bool all_finite(const float (&v)[TM][TN])
+{
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) ok = ok && isfinite(v[i][j]);
+    return ok;
+}
+// rows x cols outputs from (row0, col0) on, row_step and col_step apart.  Not inlined: nothing of it is live in the kernels' loops.
+__device__ __noinline__ void fwd_outputs_again(const float* x, const float* k, float* y, const dcg_conv_desc& d, const EpilogueArgs& ep,
+                                               long long row0, int row_step, int rows, int col0, int cols)
+{
+    const long long pixels = (long long)d.n * d.ho * d.wo;
+    for (int i = 0; i < rows * cols; ++i) {
+        const long long p = row0 + (long long)(i / cols) * row_step;
+        const int ch = col0 + i % cols;
+        if (p >= pixels || ch >= d.o) continue;
+        const size_t idx = (size_t)p * d.o + ch;
+        y[idx] = epilogue_apply(ep, fwd_sum(x, k, d, p, ch), idx, ch);
+    }
+}
+// (rows are the pixels (ph + stride * i, pw + stride * j), mh x mw of them)
+__device__ __noinline__ void dx_outputs_again(const float* dy, const float* k, float* dx, const dcg_conv_desc& d, const EpilogueArgs& ep, int ph,
+                                              int pw, int mh, int mw, long long row0, int row_step, int rows, int col0, int col_step, int cols)
+{
+    const long long pixels = (long long)d.n * mh * mw;
+    for (int i = 0; i < rows * cols; ++i) {
+        const long long p = row0 + (long long)(i / cols) * row_step, t = p / mw;
+        const int ch = col0 + i % cols * col_step;
+        if (p >= pixels || ch >= d.c) continue;
+        const size_t pix = ((size_t)(t / mh) * d.h + (size_t)(t % mh) * d.stride_h + ph) * d.w + (size_t)(p % mw) * d.stride_w + pw;
+        dx[pix * d.c + ch] = epilogue_apply(ep, dx_sum(dy, k, d, pix, ch), pix * d.c + ch, ch);
+    }
+}
+__device__ __noinline__ void dk_outputs_again(const float* x, const float* dy, float* dk, const dcg_conv_desc& d, int row0, int rows, int col0, int cols)
+{
+    for (int i = 0; i < rows * cols; ++i) {
+        const int row = row0 + i / cols, o = col0 + i % cols;
+        if (row < d.kh * d.kw * d.c && o < d.o) dk[(size_t)row * d.o + o] = dk_sum(x, dy, d, row, o);
+    }
+}
+
 // ---- forward and input gradient as ordered implicit GEMMs -----------------------------------------------
 // out[pixel, channel] over K = (contracted channel q outermost, tap innermost), the reference's loop nest.
 // An operand whose contracted channel is its contiguous axis (x, dy, and the weights of the input gradient) is
 // gathered sixteen bytes - four channels of one (row, tap) - at a time with cp.async and kept as it comes:
 // [row][channel quad][tap][4], row pitch 4 mod 8 words so that eight rows start in different bank quads.  The
-// weights of the forward are rows of output channels, [q][tap][channel].  Taps outside the image are zero-filled,
-// which adds +0 where the reference skips: the same bits.  Two to four stages of QC channels x all taps.
+// weights of the forward are rows of output channels, [q][tap][channel].  Taps outside the image are zero-filled
+// (see all_finite).  Two to four stages of QC channels x all taps.
 // Bound by issue (the sum must stay unfused: two instructions per product; packed f32x2 arithmetic was measured
 // and is no faster, its operands have to be duplicated) and, where the outputs are few, by the latency of the
 // chain of dependent adds.  Measured, 5x5 / stride 2 layers: 18 TFLOP/s (a multiply and an add counted as two) of the
@@ -135,7 +269,8 @@ __host__ __device__ constexpr int ord_row_pitch(int taps, int qc) { return taps 
 template <int TM, int TN, int TX, int TY, int STAGES, int U>   // U divides the number of taps
 __global__ void __launch_bounds__(TX * TY)
 conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k, float* __restrict__ y,
-                        const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec_a, const int vec_b)
+                        const __grid_constant__ dcg_conv_desc d, const __grid_constant__ EpilogueArgs ep, const int QC, const int vec_a,
+                        const int vec_b)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY, LDB = ord_pitch(BNT);
     extern __shared__ __align__(16) float smem[];
@@ -223,6 +358,7 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
         __syncthreads();
         buf = buf + 1 == STAGES ? 0 : buf + 1;
     }
+    if (!all_finite(acc)) return fwd_outputs_again(x, k, y, d, ep, m0 + ty, TY, TM, n0 + tx * TN, TN);
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const long long p = m0 + ty + i * TY;
@@ -243,7 +379,7 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
 template <int TM, int TN, int TX, int TY, int STAGES>
 __global__ void __launch_bounds__(TX * TY)
 conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k, float* __restrict__ dx,
-                       const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec)
+                       const __grid_constant__ dcg_conv_desc d, const __grid_constant__ EpilogueArgs ep, const int QC, const int vec)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY;
     extern __shared__ __align__(16) float smem[];
@@ -368,6 +504,7 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
             buf = buf + 1 == STAGES ? 0 : buf + 1;
         }
     }
+    if (!all_finite(tot)) return dx_outputs_again(dy, k, dx, d, ep, ph, pw, g.mh, g.mw, m0 + ty, TY, TM, n0 + tx, TX, TN);
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const long long p = m0 + ty + i * TY;
@@ -395,7 +532,7 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
 template <int TM, int TN, int TX, int TY, int STAGES, int GROUPS>
 __global__ void __launch_bounds__(TX * TY * GROUPS)
 conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dk,
-                       const dcg_conv_desc d, const int vec_a, const int vec_b)
+                       const __grid_constant__ dcg_conv_desc d, const int vec_a, const int vec_b)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY, KP = 32, LDA = ord_pitch(BMT), LDB = ord_pitch(BNT);
     constexpr int STAGE = KP * (LDA + LDB);
@@ -526,6 +663,7 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
         }
     }
     if (group != 0) return;
+    if (!all_finite(tot)) return dk_outputs_again(x, dy, dk, d, m0 + ty * TM, TM, n0 + tx * TN, TN);
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int row = m0 + ty * TM + i;
@@ -668,105 +806,31 @@ int launch_ordered_dk(const dcg_conv_desc& d, const float* x, const float* dy, f
 
 // ---- one thread per output: kernels with many taps ----------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
-conv_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ k,
-                        float* __restrict__ y, const dcg_conv_desc d, const EpilogueArgs ep,
-                        size_t total)
+conv_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ k, float* __restrict__ y,
+                        const __grid_constant__ dcg_conv_desc d, const EpilogueArgs ep, size_t total)
 {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int o = (int)(idx % d.o);
-    size_t t = idx / d.o;
-    const int j = (int)(t % d.wo); t /= d.wo;
-    const int i = (int)(t % d.ho);
-    const int n = (int)(t / d.ho);
-    const int h0 = i * d.stride_h - d.pad_top, w0 = j * d.stride_w - d.pad_left;
-    const float* xn = x + (size_t)n * d.h * d.w * d.c;
-    float val = 0.f;
-    for (int q = 0; q < d.c; ++q)
-        for (int di = 0; di < d.kh; ++di) {
-            const int h = h0 + di;
-            if (h < 0 || h >= d.h) continue;
-            for (int dj = 0; dj < d.kw; ++dj) {
-                const int w = w0 + dj;
-                if (w < 0 || w >= d.w) continue;
-                const float xv = __ldg(xn + ((size_t)h * d.w + w) * d.c + q);
-                const float kv = __ldg(k + (((size_t)di * d.kw + dj) * d.c + q) * d.o + o);
-                val = __fadd_rn(val, __fmul_rn(xv, kv));
-            }
-        }
-    y[idx] = epilogue_apply(ep, val, idx, o);
+    y[idx] = epilogue_apply(ep, fwd_sum(x, k, d, idx / d.o, o), idx, o);
 }
 
-// dx[n,i,j,c] = sum_o ( sum_{di,dj} dyz[n,i+di-P,j+dj-Q,o] * k[KH-1-di,KW-1-dj,c,o] ), dyz the
-// zero-inserted dy, P = KH-1-pad_top, Q = KW-1-pad_left (src/cpu/ops.hxx:618-629).
 __global__ void __launch_bounds__(kThreads)
-conv_dx_generic_kernel(const float* __restrict__ dy, const float* __restrict__ k,
-                       float* __restrict__ dx, const dcg_conv_desc d, const EpilogueArgs ep,
-                       size_t total)
+conv_dx_generic_kernel(const float* __restrict__ dy, const float* __restrict__ k, float* __restrict__ dx,
+                       const __grid_constant__ dcg_conv_desc d, const EpilogueArgs ep, size_t total)
 {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int c = (int)(idx % d.c);
-    size_t t = idx / d.c;
-    const int j = (int)(t % d.w); t /= d.w;
-    const int i = (int)(t % d.h);
-    const int n = (int)(t / d.h);
-    const int P = d.kh - 1 - d.pad_top, Q = d.kw - 1 - d.pad_left;
-    const float* dyn = dy + (size_t)n * d.ho * d.wo * d.o;
-    float total_v = 0.f;
-    for (int o = 0; o < d.o; ++o) {
-        float val = 0.f;
-        for (int di = 0; di < d.kh; ++di) {
-            const int ph = i + di - P;
-            if (ph < 0 || ph % d.stride_h != 0) continue;
-            const int a = ph / d.stride_h;
-            if (a >= d.ho) continue;
-            for (int dj = 0; dj < d.kw; ++dj) {
-                const int pw = j + dj - Q;
-                if (pw < 0 || pw % d.stride_w != 0) continue;
-                const int b = pw / d.stride_w;
-                if (b >= d.wo) continue;
-                const float g = __ldg(dyn + ((size_t)a * d.wo + b) * d.o + o);
-                const float kv = __ldg(k + (((size_t)(d.kh - 1 - di) * d.kw + (d.kw - 1 - dj)) * d.c + c) * d.o + o);
-                val = __fadd_rn(val, __fmul_rn(g, kv));
-            }
-        }
-        total_v = (o == 0) ? val : __fadd_rn(total_v, val);
-    }
-    dx[idx] = epilogue_apply(ep, total_v, idx, c);
+    dx[idx] = epilogue_apply(ep, dx_sum(dy, k, d, idx / d.c, c), idx, c);
 }
 
-// dk[kh,kw,c,o] = sum_n ( sum_{a,b} x[n,kh+s*a-pt,kw+s*b-pl,c] * dy[n,a,b,o] )
 __global__ void __launch_bounds__(kThreads)
-conv_dk_generic_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                       float* __restrict__ dk, const dcg_conv_desc d, size_t total)
+conv_dk_generic_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dk,
+                       const __grid_constant__ dcg_conv_desc d, size_t total)
 {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total) return;
-    const int o = (int)(idx % d.o);
-    size_t t = idx / d.o;
-    const int c = (int)(t % d.c); t /= d.c;
-    const int kw = (int)(t % d.kw);
-    const int kh = (int)(t / d.kw);
-    float total_v = 0.f;
-    for (int n = 0; n < d.n; ++n) {
-        const float* xn = x + (size_t)n * d.h * d.w * d.c;
-        const float* dyn = dy + (size_t)n * d.ho * d.wo * d.o;
-        float val = 0.f;
-        for (int a = 0; a < d.ho; ++a) {
-            const int h = kh + d.stride_h * a - d.pad_top;
-            if (h < 0 || h >= d.h) continue;
-            for (int b = 0; b < d.wo; ++b) {
-                const int w = kw + d.stride_w * b - d.pad_left;
-                if (w < 0 || w >= d.w) continue;
-                const float xv = __ldg(xn + ((size_t)h * d.w + w) * d.c + c);
-                const float g = __ldg(dyn + ((size_t)a * d.wo + b) * d.o + o);
-                val = __fadd_rn(val, __fmul_rn(xv, g));
-            }
-        }
-        total_v = (n == 0) ? val : __fadd_rn(total_v, val);
-    }
-    dk[idx] = total_v;
+    if (idx < total) dk[idx] = dk_sum(x, dy, d, idx / d.o, (int)(idx % d.o));
 }
 
 }  // namespace

@@ -152,6 +152,27 @@ def test_fp32_ordered_kernels_match_oracle_bit_for_bit(pkg, dev, orc, shape):
     _check(dk, orc.conv2d_kernel_grad(dy, x, s, pad), pkg.PREC_FP32, pkg, "dk")
 
 
+@pytest.mark.parametrize("shape", ORDERED_SHAPES + [(2, 20, 20, 6, 7, 10, 1)])
+def test_fp32_taps_outside_the_image_are_skipped(pkg, dev, orc, shape):
+    """Infinite and NaN factors of taps (pixels) that some outputs do not have: those outputs stay finite, as in the oracle."""
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    pad = (oracle.same_pad(H, K, s), oracle.same_pad(W, K, s))
+    ho, wo = -(-H // s), -(-W // s)
+    x, k, dy = seeded((N, H, W, C), 240), seeded((K, K, C, O), 241), seeded((N, ho, wo, O), 242)
+    k_bad, dy_bad = k.copy(), dy.copy()
+    k_bad[0, :, 0, 0], k_bad[K - 1, K - 1, C - 1, O - 1] = np.inf, np.nan
+    dy_bad[0, 0, :, 0], dy_bad[N - 1, ho - 1, wo - 1, O - 1] = -np.inf, np.nan
+    xd, kd, dyd, dy_badd = (torch.from_numpy(a).to(dev) for a in (x, k_bad, dy, dy_bad))
+    y = F.conv2d_fwd(xd, kd, (s, s), precision=pkg.PREC_FP32)
+    dx = F.conv2d_dx(dyd, kd, (H, W), (s, s), precision=pkg.PREC_FP32)
+    dk = F.conv2d_dk(xd, dy_badd, (K, K), (s, s), precision=pkg.PREC_FP32)
+    with np.errstate(invalid="ignore"):
+        refs = orc.conv2d(x, k_bad, (s, s)), orc.conv2d_input_grad(dy, k_bad, s, (H, W)), orc.conv2d_kernel_grad(dy_bad, x, s, pad)
+    for name, got, ref in zip(("fwd", "dx", "dk"), (y, dx, dk), refs):
+        assert np.array_equal(got.cpu().numpy(), ref, equal_nan=True), name
+
+
 @pytest.mark.parametrize("shape", [(40, 64, 64, 3, 5, 64, 2), (40, 60, 52, 3, 5, 64, 2), (37, 64, 64, 4, 5, 32, 2)])
 def test_three_channel_layers_with_persistent_ctas(pkg, dev, orc, shape):
     """More tiles than SMs: the forward of a <= 4-channel layer and the GEMM of its input gradient run as
