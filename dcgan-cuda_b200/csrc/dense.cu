@@ -226,6 +226,26 @@ gemm_outer_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
     }
 }
 
+// One thread per output, 64-bit indexes: axes of 2^30 and more, which the tiles' 32-bit ones do not hold.  Same sums.
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(TPB)
+gemm_long_axis_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const size_t m, const size_t n,
+                      const size_t p, const DenseEpilogue e)
+{
+    pdl_enter();
+    const size_t total = m * p, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
+        const size_t r = idx / p, c = idx - r * p;
+        float v = 0.f;
+#pragma unroll 8
+        for (size_t k = 0; k < n; ++k)
+            v = __fadd_rn(v, __fmul_rn(__ldg(TA ? a + k * m + r : a + r * n + k), __ldg(TB ? b + c * n + k : b + k * p + c)));
+        if (e.bias) v = __fadd_rn(v, __ldg(e.bias + c));
+        out[idx] = v;
+        if (e.out2) e.out2[idx] = e.gate ? act_grad_apply(__ldg(e.gate + idx), v, e.act, e.alpha) : act_apply(v, e.act, e.alpha);
+    }
+}
+
 // One block per output element, for m*p small and n long: out = A[m,n] B[n,p] (+bias).
 // Thread t adds elements t, t+256, ... in ascending order; the 256 thread sums are then added
 // in a fixed tree, so the result is independent of scheduling.
@@ -328,7 +348,6 @@ int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, 
 template <bool TA, bool TB>
 int launch_ordered(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const DenseEpilogue& e, cudaStream_t stream)
 {
-    DCG_CHECK_ARG(m < (1u << 30) && n < (1u << 30) && p < (1u << 30), "dense: %zu x %zu x %zu is too large", m, n, p);
     DCG_CHECK_ARG((m + 3) / 4 <= 65535u * 16, "dense: %zu rows are too many", m);
     if (!e.sums && n == 1 && p % 4 == 0 && aligned16(b) && aligned16(out) && aligned16(e.bias) && aligned16(e.gate) && aligned16(e.out2)) {
         size_t blocks = (m * (p / 4) + TPB - 1) / TPB;
@@ -336,6 +355,14 @@ int launch_ordered(const float* a, const float* b, float* out, size_t m, size_t 
         if (blocks > cap) blocks = cap;
         launch_pdl(gemm_outer_kernel, (unsigned)blocks, TPB, 0, stream, a, b, out, m, p / 4, e);
         DCG_LAUNCH_CHECK("gemm_outer_kernel");
+        return DCG_OK;
+    }
+    if (n >= (1u << 30) || p >= (1u << 30)) {
+        size_t blocks = (m * p + TPB - 1) / TPB;
+        const size_t cap = (size_t)sm_count() * 16;
+        if (blocks > cap) blocks = cap;
+        launch_pdl(gemm_long_axis_kernel<TA, TB>, (unsigned)blocks, TPB, 0, stream, a, b, out, m, n, p, e);
+        DCG_LAUNCH_CHECK("gemm_long_axis_kernel");
         return DCG_OK;
     }
     const double per_lane = (double)m * (double)p / (128.0 * sm_count());
@@ -391,7 +418,7 @@ int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t
 // gemm_tall_tn_kernel, nor for more rows than a block adds up (1024 where a column tile is 32 wide): returns 1 there.
 int matmul_tn_sums(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, float* sums, cudaStream_t stream)
 {
-    if ((p <= 8 && m >= 1024) || m > (1u << 20)) return 1;
+    if ((p <= 8 && m >= 1024) || m > (1u << 20) || p >= (1u << 30)) return 1;
     DCG_CHECK_ARG(a && b && out && sums && m > 0 && n > 0 && p > 0, "matmul_tn_sums: bad arguments");
     DenseEpilogue e{};
     if (!colsum_order(n, p, aligned16(b), kSumSlabs, e.sum) || (e.sum.order.slabs << e.sum.order.lane_shift) * 16 > kSumSmem) return 1;

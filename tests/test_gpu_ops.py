@@ -212,6 +212,27 @@ def test_dense_is_bit_exact(pkg, dev, orc, m, n, p):
     assert np.array_equal(dx.cpu().numpy(), orc.mtm_mul(dy, b))
 
 
+def test_dense_with_an_axis_of_two_to_the_thirty(pkg, dev):
+    L, P = pkg.lib, (1 << 30) + 5
+    if torch.cuda.mem_get_info()[0] < 20 * P:
+        pytest.skip("needs %d GB" % (20 * P >> 30))
+    a, bias = torch.tensor([0.75, -1.25], device=dev), None
+    b = torch.empty((2 * P,), device=dev).uniform_(-1, 1)
+    out = torch.empty((P,), device=dev)
+    at = torch.tensor([0, 1, 2, 12345, (1 << 29) + 1, P - 2, P - 1], device=dev)
+
+    def check(x, y):
+        ref = (x * 0.75) + (y * -1.25)
+        assert torch.equal(out[at], ref)
+
+    pkg._lib.check(L.dcg_matmul(a.data_ptr(), b.data_ptr(), bias, out.data_ptr(), 1, 2, P, _s()))
+    check(b[:P][at], b[P:][at])
+    pkg._lib.check(L.dcg_matmul_tn(a.data_ptr(), b.data_ptr(), out.data_ptr(), 1, 2, P, _s()))
+    check(b[:P][at], b[P:][at])
+    pkg._lib.check(L.dcg_matmul_nt(a.data_ptr(), b.data_ptr(), out.data_ptr(), 1, 2, P, _s()))
+    check(b[2 * at], b[2 * at + 1])
+
+
 # the form for a few reduction steps and its limits, the outer product from either storage, stores of whole words and of single
 # ones, unaligned operands and results
 @pytest.mark.parametrize("m,n,p,off", [(700, 1, 640, 0), (700, 2, 641, 0), (650, 15, 642, 0), (650, 16, 644, 0), (650, 17, 644, 0),
