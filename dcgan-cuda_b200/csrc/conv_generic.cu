@@ -676,8 +676,10 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
     }
 }
 
-bool ordered_ok(const dcg_conv_desc& d)
+// `cols` columns in tiles of `tile` where there are as many as to matter, `classes` parity classes: grid.y and grid.z.
+bool ordered_ok(const dcg_conv_desc& d, int cols, int tile, long long classes = 1)
 {
+    if (cols > 65535 * tile || classes > 65535) return false;
     // element offsets are 32-bit
     const long long x = (long long)d.n * d.h * d.w * d.c, y = (long long)d.n * d.ho * d.wo * d.o, k = (long long)d.kh * d.kw * d.c * d.o;
     return d.kh * d.kw <= kOrdMaxTaps && x < (1ll << 31) && y < (1ll << 31) && k < (1ll << 31);
@@ -840,7 +842,7 @@ int conv_fwd_generic(const dcg_conv_desc& d, const float* x, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.ho * d.wo * d.o;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d)) return launch_ordered_fwd(d, x, k, y, ep, stream);
+    if (ordered_ok(d, d.o, 64)) return launch_ordered_fwd(d, x, k, y, ep, stream);
     conv_fwd_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, k, y, d, ep, total);
     DCG_LAUNCH_CHECK("conv_fwd_generic_kernel");
@@ -852,7 +854,7 @@ int conv_dx_generic(const dcg_conv_desc& d, const float* dy, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.h * d.w * d.c;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d)) return launch_ordered_dx(d, dy, k, dx, ep, stream);
+    if (ordered_ok(d, d.c, 32, (long long)d.stride_h * d.stride_w)) return launch_ordered_dx(d, dy, k, dx, ep, stream);
     conv_dx_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         dy, k, dx, d, ep, total);
     DCG_LAUNCH_CHECK("conv_dx_generic_kernel");
@@ -864,7 +866,7 @@ int conv_dk_generic(const dcg_conv_desc& d, const float* x, const float* dy, flo
 {
     const size_t total = (size_t)d.kh * d.kw * d.c * d.o;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d)) return launch_ordered_dk(d, x, dy, dk, stream);
+    if (ordered_ok(d, d.o, 64)) return launch_ordered_dk(d, x, dy, dk, stream);
     conv_dk_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, dy, dk, d, total);
     DCG_LAUNCH_CHECK("conv_dk_generic_kernel");

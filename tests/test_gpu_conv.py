@@ -173,6 +173,24 @@ def test_fp32_taps_outside_the_image_are_skipped(pkg, dev, orc, shape):
         assert np.array_equal(got.cpu().numpy(), ref, equal_nan=True), name
 
 
+# more column tiles and more parity classes than a grid has rows and layers of blocks
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1, 4200000, 1), (1, 1, 1, 2100000, 1, 2, 1), (1, 300, 300, 2, 1, 3, 300)])
+def test_fp32_extents_beyond_a_grid(pkg, dev, orc, shape):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    x, k = seeded((N, H, W, C), 243), seeded((K, K, C, O), 244)
+    dy = seeded((N, -(-H // s), -(-W // s), O), 245)
+    xd, kd, dyd = (torch.from_numpy(a).to(dev) for a in (x, k, dy))
+    y = F.conv2d_fwd(xd, kd, (s, s), precision=pkg.PREC_FP32)
+    dx = F.conv2d_dx(dyd, kd, (H, W), (s, s), precision=pkg.PREC_FP32)
+    dk = F.conv2d_dk(xd, dyd, (K, K), (s, s), precision=pkg.PREC_FP32)
+    _check(y, orc.conv2d(x, k, (s, s)), pkg.PREC_FP32, pkg, "fwd")
+    dx_ref = np.zeros((N, H, W, C), np.float32)   # one tap: the gradient of the pixels that were read
+    dx_ref[:, ::s, ::s] = orc.conv2d_input_grad(dy, k, 1, dy.shape[1:3])
+    _check(dx, dx_ref, pkg.PREC_FP32, pkg, "dx")
+    _check(dk, orc.conv2d_kernel_grad(dy, x, s, (0, 0))[:K, :K], pkg.PREC_FP32, pkg, "dk")
+
+
 @pytest.mark.parametrize("shape", [(40, 64, 64, 3, 5, 64, 2), (40, 60, 52, 3, 5, 64, 2), (37, 64, 64, 4, 5, 32, 2)])
 def test_three_channel_layers_with_persistent_ctas(pkg, dev, orc, shape):
     """More tiles than SMs: the forward of a <= 4-channel layer and the GEMM of its input gradient run as
