@@ -40,6 +40,16 @@ static int check_precision(int precision, const char* who)
     return DCG_OK;
 }
 
+// Channel counts that are no multiple of 32 go to the CUDA cores, which need no scratch, where there is too little of it for the
+// tensor path; the kernels of other counts ask for theirs.
+bool conv_scratch_optional(const dcg_conv_desc& d, int kind) { return (kind != kConvDx && d.o % 32 != 0) || (kind == kConvDk && d.c > 4 && d.c % 32 != 0); }
+
+static bool on_tensor_path(const dcg_conv_desc& d, int kind, bool x3, const void* ws, size_t ws_bytes)
+{
+    if (!conv_tc_supported(d, kind, x3)) return false;
+    return !conv_scratch_optional(d, kind) || conv_tc_workspace(d, kind, x3) <= (ws ? ws_bytes : 0);
+}
+
 }  // namespace dcg
 
 using namespace dcg;
@@ -61,7 +71,7 @@ extern "C" int dcg_conv2d_fwd(const dcg_conv_desc* desc, const float* x, const f
     DCG_CHECK_ARG(x && k && y, "dcg_conv2d_fwd: null tensor pointer");
     const EpilogueArgs e = make_epilogue(ep);
     const bool x3 = precision == DCG_PREC_3XTF32;
-    if (precision != DCG_PREC_FP32 && conv_tc_supported(*desc, kConvFwd, x3) && aligned16(x) && aligned16(k) &&
+    if (precision != DCG_PREC_FP32 && on_tensor_path(*desc, kConvFwd, x3, workspace, workspace_bytes) && aligned16(x) && aligned16(k) &&
         aligned16(y) && epilogue_aligned(e))
         return conv_tc_fwd(*desc, x, k, y, e, workspace, workspace_bytes, as_stream(stream), x3);
     return conv_fwd_generic(*desc, x, k, y, e, as_stream(stream));
@@ -77,7 +87,7 @@ extern "C" int dcg_conv2d_dx(const dcg_conv_desc* desc, const float* dy, const f
     DCG_CHECK_ARG(dy && k && dx, "dcg_conv2d_dx: null tensor pointer");
     const EpilogueArgs e = make_epilogue(ep);
     const bool x3 = precision == DCG_PREC_3XTF32;
-    if (precision != DCG_PREC_FP32 && conv_tc_supported(*desc, kConvDx, x3) && aligned16(dy) && aligned16(k) &&
+    if (precision != DCG_PREC_FP32 && on_tensor_path(*desc, kConvDx, x3, workspace, workspace_bytes) && aligned16(dy) && aligned16(k) &&
         aligned16(dx) && epilogue_aligned(e))
         return conv_tc_dx(*desc, dy, k, dx, e, workspace, workspace_bytes, as_stream(stream), x3);
     return conv_dx_generic(*desc, dy, k, dx, e, as_stream(stream));
@@ -92,7 +102,7 @@ extern "C" int dcg_conv2d_dk(const dcg_conv_desc* desc, const float* x, const fl
     if ((st = check_precision(precision, "dcg_conv2d_dk"))) return st;
     DCG_CHECK_ARG(x && dy && dk, "dcg_conv2d_dk: null tensor pointer");
     const bool x3 = precision == DCG_PREC_3XTF32;
-    if (precision != DCG_PREC_FP32 && conv_tc_supported(*desc, kConvDk, x3) && aligned16(x) && aligned16(dy) &&
+    if (precision != DCG_PREC_FP32 && on_tensor_path(*desc, kConvDk, x3, workspace, workspace_bytes) && aligned16(x) && aligned16(dy) &&
         aligned16(dk))
         return conv_tc_dk(*desc, x, dy, dk, workspace, workspace_bytes, as_stream(stream), x3);
     return conv_dk_generic(*desc, x, dy, dk, as_stream(stream));

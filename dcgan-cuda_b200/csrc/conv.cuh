@@ -28,6 +28,9 @@ int conv_tc_dx(const dcg_conv_desc& d, const float* dy, const float* k, float* d
 int conv_tc_dk(const dcg_conv_desc& d, const float* x, const float* dy, float* dk,
                void* ws, size_t ws_bytes, cudaStream_t stream, bool x3 = false);
 
+// Whether the operator runs, on the CUDA cores, with less scratch than dcg_conv_workspace_bytes asks for.
+bool conv_scratch_optional(const dcg_conv_desc& d, int kind);
+
 // Testing hooks of the tensor path.  wait_cycles: > 0 sets the limit of every barrier wait (SM clocks),
 // -1 restores the default, 0 leaves it; skip_stage: pipeline stage the producer leaves out (-1: none,
 // -2: leave as is).

@@ -46,8 +46,9 @@ enum dcg_act {
 };
 
 enum dcg_precision {
-    DCG_PREC_TF32 = 0,   /* tcgen05 kind::tf32, fp32 accumulate in TMEM; falls back to
-                            DCG_PREC_FP32 kernels for shapes the tensor path cannot take */
+    DCG_PREC_TF32 = 0,   /* tcgen05 kind::tf32, fp32 accumulate in TMEM: channel counts that are
+                            multiples of four (dk: of at least eight, or up to four input channels),
+                            16-byte aligned tensors, strides up to eight; DCG_PREC_FP32 kernels else */
     DCG_PREC_3XTF32 = 1, /* opt-in: operand = TF32 part + residual, three tensor-core products per
                             K step; <= 1e-5 * max|ref|, about three times the TF32 cost */
     DCG_PREC_FP32 = 2    /* CUDA-core fp32 with the reference CPU's summation order,
@@ -91,7 +92,9 @@ typedef struct dcg_epilogue {
 /* ---- convolutions -------------------------------------------------------- */
 
 /* Scratch bytes the three conv entry points need for `desc` at `precision`
- * (kind: 0 = fwd, 1 = dx, 2 = dk).  0 when none is needed. */
+ * (kind: 0 = fwd, 1 = dx, 2 = dk).  0 when none is needed.  With less, fwd and dk
+ * of channel counts that are no multiple of 32 run on the CUDA cores (fp32); any
+ * other call returns DCG_ERR_WORKSPACE. */
 size_t dcg_conv_workspace_bytes(const dcg_conv_desc* desc, int kind, int precision);
 
 /* y = conv2d(x, k) [+ epilogue].

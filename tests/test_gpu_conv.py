@@ -4,6 +4,7 @@ DCG_PREC_FP32 keeps the reference CPU's summation order with unfused multiply/ad
 reproduce the oracle bit for bit.  DCG_PREC_TF32 (tcgen05, fp32 accumulate) must stay within
 1e-2 * max|ref| per output tensor - the tolerance stated for the TF32 tensor-core path.
 """
+import ctypes
 import threading
 
 import numpy as np
@@ -457,6 +458,34 @@ def test_ragged_channel_counts_with_epilogue(pkg, dev, shape, prec_name):
     tol = TF32_TOL if prec_name == "tf32" else 3e-5
     for name, a, b in zip(("y", "z", "dx", "raw"), *got.values()):
         assert (a - b).abs().max().item() <= tol * b.abs().max().item(), name
+
+
+def test_ragged_channel_counts_without_scratch(pkg, dev):
+    """They ran on the CUDA cores before they took the tensor path, and still do where there is no scratch for that - as
+    operators and as nodes of a context with little scratch of its caller; counts that always needed scratch ask for it."""
+    F, L, N = pkg.functional, pkg.lib, pkg.nodes
+    x, k, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((1, (4, 32, 32, 36)), (2, (3, 3, 36, 40)), (3, (4, 32, 32, 40))))
+    y, dk = torch.zeros_like(dy), torch.zeros_like(k)
+    d = F.conv_desc(x.shape, k.shape, (1, 1))
+    assert all(L.dcg_conv_workspace_bytes(ctypes.byref(d), kind, pkg.PREC_TF32) > 256 for kind in (pkg._lib.KIND_FWD, pkg._lib.KIND_DK))
+    refs = F.conv2d_fwd(x, k, (1, 1), precision=pkg.PREC_FP32), F.conv2d_dk(x, dy, (3, 3), (1, 1), precision=pkg.PREC_FP32)
+    stream, scratch = torch.cuda.current_stream().cuda_stream, torch.empty((256,), dtype=torch.uint8, device=dev)
+    for ws, size in ((None, 0), (scratch.data_ptr(), 256)):
+        y.zero_(), dk.zero_()
+        pkg._lib.check(L.dcg_conv2d_fwd(ctypes.byref(d), x.data_ptr(), k.data_ptr(), y.data_ptr(), None, pkg.PREC_TF32, ws, size, stream))
+        pkg._lib.check(L.dcg_conv2d_dk(ctypes.byref(d), x.data_ptr(), dy.data_ptr(), dk.data_ptr(), pkg.PREC_TF32, ws, size, stream))
+        assert torch.equal(y, refs[0]) and torch.equal(dk, refs[1])
+    y.zero_(), dk.zero_()
+    ctx = ctypes.c_void_p()
+    pkg._lib.check(L.dcg_context_create(ctypes.byref(ctx), pkg.PREC_TF32, scratch.data_ptr(), 256, stream))
+    nodes = [N.op_conv2d(x, k, (1, 1), 2, 2, y, x.shape, k.shape), N.op_conv2d_kernel_grad(dy, x, (1, 1), dk, dy.shape, x.shape, (2, 2))]
+    pkg._lib.check(L.dcg_run_nodes(ctx, (pkg._lib.Node * 2)(*nodes), 2, 1))
+    torch.cuda.synchronize()
+    L.dcg_context_destroy(ctx)
+    assert torch.equal(y, refs[0]) and torch.equal(dk, refs[1])
+    d2 = F.conv_desc((2, 16, 16, 128), (5, 5, 128, 256))
+    x2, k2, y2 = torch.zeros((2, 16, 16, 128), device=dev), torch.zeros((5, 5, 128, 256), device=dev), torch.zeros((2, 8, 8, 256), device=dev)
+    assert L.dcg_conv2d_fwd(ctypes.byref(d2), x2.data_ptr(), k2.data_ptr(), y2.data_ptr(), None, pkg.PREC_TF32, None, 0, stream) == pkg._lib.ERR_WORKSPACE
 
 
 @pytest.mark.parametrize("threads", [1, 2])
