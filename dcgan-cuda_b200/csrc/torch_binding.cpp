@@ -27,7 +27,8 @@ struct Error {};   // a Python exception is set
     throw Error();
 }
 
-PyObject* g_check = nullptr;   // _lib.check: raises DcgError for a status
+PyObject* g_check = nullptr;      // _lib.check: raises DcgError for a status
+PyObject* g_epilogue = nullptr;   // _lib.Epilogue
 
 const at::Tensor& tensor(PyObject* o)
 {
@@ -169,6 +170,9 @@ struct EpilogueView {
     explicit EpilogueView(PyObject* o, int flags = PyBUF_SIMPLE)
     {
         if (o == Py_None) return;
+        const int is_one = PyObject_IsInstance(o, g_epilogue);
+        if (is_one < 0) throw Error();
+        if (!is_one) fail(PyExc_TypeError, "expected an Epilogue");
         if (PyObject_GetBuffer(o, &view, flags) != 0) throw Error();
         if ((size_t)view.len != sizeof(dcg_epilogue)) { PyBuffer_Release(&view); fail(PyExc_TypeError, "expected an Epilogue"); }
         ep = static_cast<const dcg_epilogue*>(view.buf);
@@ -313,11 +317,16 @@ PyObject* fill_epilogue(PyObject*, PyObject* const* a, Py_ssize_t n)
     });
 }
 
-PyObject* set_check(PyObject*, PyObject* f)
+// (check, Epilogue): what this module needs of _lib
+PyObject* set_up(PyObject*, PyObject* const* a, Py_ssize_t n)
 {
-    Py_INCREF(f);
-    Py_XSETREF(g_check, f);
-    Py_RETURN_NONE;
+    return guarded(n, 2, [&]() -> PyObject* {
+        Py_INCREF(a[0]);
+        Py_XSETREF(g_check, a[0]);
+        Py_INCREF(a[1]);
+        Py_XSETREF(g_epilogue, a[1]);
+        Py_RETURN_NONE;
+    });
 }
 
 template <typename F>
@@ -329,7 +338,7 @@ PyMethodDef g_methods[] = {
     {"conv2d_dk", fastcall(conv2d_dk), METH_FASTCALL, nullptr},
     {"colsum", fastcall(colsum), METH_FASTCALL, nullptr},
     {"fill_epilogue", fastcall(fill_epilogue), METH_FASTCALL, nullptr},
-    {"set_check", set_check, METH_O, nullptr},
+    {"set_up", fastcall(set_up), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 

@@ -11,7 +11,7 @@ import torch
 from . import _binding, _lib
 from ._lib import AdamTensor, ConvDesc, Epilogue, check, lib
 
-_binding.set_check(check)
+_binding.set_up(check, Epilogue)
 
 
 def same_pad(in_size, k_size, stride):

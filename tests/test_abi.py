@@ -64,3 +64,12 @@ def test_adam_lr_t_is_host_side(pkg):
     import numpy as np
     expect = np.float32(2e-4) * np.sqrt(np.float32(1) - np.float32(0.999)) / (np.float32(1) - np.float32(0.5))
     assert abs(lr1 - float(expect)) < 1e-10
+
+
+def test_epilogues_of_another_type_are_refused(pkg):
+    """The native call path reads an Epilogue's memory: something else of the same size is not one."""
+    size = ctypes.sizeof(pkg._lib.Epilogue)
+    for other in (bytearray(size), (ctypes.c_char * size)(), bytes(size)):
+        with pytest.raises(TypeError):
+            pkg.functional._binding.fill_epilogue(other, None, None, None, 0, 0.0, None, 0, 0.0)
+    assert isinstance(pkg.functional.make_epilogue(act=pkg.ACT_TANH), pkg._lib.Epilogue)
