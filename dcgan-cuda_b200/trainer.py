@@ -131,7 +131,9 @@ class Trainer:
         with torch.cuda.stream(self.stream):
             yield
         caller.wait_stream(self.stream)
-        self._joined = caller
+        # Streams of torch's own (the default one or the pool's, whose ids are odd) live as long as the process.  Any other may be
+        # gone before the next call, its handle perhaps another stream's: nothing is left behind on those.
+        self._joined = caller if caller.stream_id == 0 or caller.stream_id & 1 else None
 
     def _replay(self, what):
         """Enqueues a captured graph on the caller's stream itself, if that is the one the trainer was last called from:

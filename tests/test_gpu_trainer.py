@@ -1,5 +1,7 @@
 """The DCGAN training step (dcg_trainer, node lists + fusion) against the CPU restatement of
 dcgan/main.cu built from oracle operators, on identical parameters and inputs."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -186,6 +188,34 @@ def test_replay_on_the_callers_stream_equals_eager(pkg, dev, monkeypatch, stream
         runs[replay] = [t.cpu() for t in images + losses + [tr.tensor("d_params"), tr.tensor("g_params")]]
         tr.close()
     assert all(torch.equal(a, b) for a, b in zip(runs[True], runs[False]))
+
+
+def test_a_callers_stream_may_be_destroyed_between_calls(pkg, dev):
+    """On streams that torch does not own the trainer keeps to its own stream, so that it never has to go back to one."""
+    rt = torch.cuda.cudart()
+    finals = []
+    for external in (False, True):
+        tr = pkg.Trainer(batch=4, seed=7, precision=pkg.PREC_FP32)
+        tr.x.copy_(torch.from_numpy(seeded((4, 64, 64, 3), 1)))
+        tr.z.copy_(torch.from_numpy(seeded((4, 100), 2)))
+        torch.cuda.synchronize()
+        for _ in range(3):
+            handle = ctypes.c_size_t()
+            if external:
+                assert int(rt.cudaStreamCreate(ctypes.addressof(handle))) == 0
+            with torch.cuda.stream(torch.cuda.ExternalStream(handle.value) if external else torch.cuda.current_stream()):
+                for _ in range(4):
+                    tr.step()
+                    tr.generate()
+                torch.cuda.current_stream().synchronize()
+            if external:
+                assert tr._joined is None
+                assert int(rt.cudaStreamDestroy(handle.value)) == 0
+            tr.step()
+        torch.cuda.synchronize()
+        finals.append([tr.tensor(n).cpu() for n in ("d_params", "g_params", "g_out")])
+        tr.close()
+    assert all(torch.equal(a, b) for a, b in zip(*finals))
 
 
 def test_g_backward_in_two_parts(pkg, dev):
