@@ -88,6 +88,15 @@ ProfScope::ProfScope(dcg_context* c, const char* name, double flops) : ctx(c), a
     ctx->recs.push_back(r);
 }
 
+void ProfScope::drop()
+{
+    if (!active) return;
+    active = false;
+    cudaEventDestroy(ctx->recs.back().e0);
+    cudaEventDestroy(ctx->recs.back().e1);
+    ctx->recs.pop_back();
+}
+
 ProfScope::~ProfScope()
 {
     if (active) cudaEventRecord(ctx->recs.back().e1, ctx->stream);
@@ -734,6 +743,7 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
                                                                                             b.type == DCG_OP_RELU_LEAKY ? b.alpha_leaky : 0.f, b.out1, ctx->stream);
                 if (cs < 0) return cs;
                 if (cs == 0) { i += 2; continue; }
+                scope.drop();
             }
             // loss + its gradient on the same labels and logits
             if (a.type == DCG_OP_SIGMOID_CROSS_ENTROPY && b.type == DCG_OP_SIGMOID_CROSS_ENTROPY_GRAD && a.in1 == b.in1 &&
@@ -780,6 +790,7 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
                 const int st = dcg::matmul_tn_sums(a.in1, a.in2, a.out1, a.len1, a.len2, a.len3, b.out1, ctx->stream);
                 if (st < 0) return st;
                 if (st == 0) { i += 2; continue; }
+                scope.drop();
             }
         }
         AdamTriple first;

@@ -10,6 +10,7 @@ namespace dcg {
 struct ProfScope {
     ProfScope(dcg_context* ctx, const char* name, double flops);
     ~ProfScope();
+    void drop();   // what it was opened for did not run: files nothing
     ProfScope(const ProfScope&) = delete;
     ProfScope& operator=(const ProfScope&) = delete;
     dcg_context* ctx;

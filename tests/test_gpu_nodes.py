@@ -346,6 +346,21 @@ def test_bias_gradient_beside_the_weight_gradient_is_the_column_sum(pkg, dev, ou
     assert (True, 1) in counts and (True, 2) not in counts and max(n for _, n in counts) >= 2
 
 
+def test_profile_of_pairs_that_do_not_fuse(pkg, dev):
+    """A dense layer with a long reduction and a weight gradient of many rows run by themselves: one call each in the profile."""
+    L, N = pkg.lib, pkg.nodes
+    x, w, b, z, a = (torch.empty(s, device=dev).uniform_() for s in ((8, 2048), (2048, 10), (10,), (8, 10), (8, 10)))
+    h, d, gw, gb = (torch.empty(s, device=dev).uniform_() for s in ((5000, 16), (5000, 36), (16, 36), (36,)))
+    ctx = pkg.Context(pkg.PREC_TF32)
+    pkg._lib.check(L.dcg_context_profile_begin(ctx._h))
+    ctx.run([N.op_mat_mul_add(x, w, b, z, 8, 2048, 10), N.op_relu(z, a, 80),
+             N.op_tmat_mat_mul(h, d, gw, 16, 5000, 36), N.op_mat_sum_cols(d, gb, 5000, 36)], fuse=True)
+    rows, n = (pkg._lib.ProfileRow * 16)(), ctypes.c_int()
+    pkg._lib.check(L.dcg_context_profile_end(ctx._h, rows, 16, ctypes.byref(n)))
+    ctx.close()
+    assert {rows[i].name.decode(): rows[i].calls for i in range(n.value)} == {"mat_mul_add": 1, "relu": 1, "tmat_mat_mul": 1, "mat_sum_cols": 1}
+
+
 def test_reshape_is_an_alias_and_unknown_nodes_fail(pkg, dev):
     """Reshape lowers to no instruction at all (src/ops/reshape.cu:20-44): the consumer reads the
     producer's buffer, so it is bit-exact by construction.  Unknown node types are errors."""
