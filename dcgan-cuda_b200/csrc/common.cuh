@@ -10,6 +10,7 @@
 #include <cstdio>
 
 #include "dcgan_b200.h"
+#include "per_device.cuh"
 
 namespace dcg {
 
@@ -79,6 +80,17 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);   // errors surface in DCG_LAUNCH_CHECK
 }
 #endif
+
+// Lets `kernel` have `bytes` of dynamic shared memory.  The attribute belongs to a device, so each that launches the kernel sets
+// it, the first time.
+template <typename Kernel>
+inline cudaError_t allow_smem(OncePerDevice& once, Kernel kernel, size_t bytes)
+{
+    int device = -1;
+    const cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    return (cudaError_t)once(device, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
+}
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 

@@ -10,7 +10,6 @@
 // conv_ordered_dk_kernel are register-tiled GEMMs on operand tiles that cp.async gathers straight from the
 // NHWC / HWIO tensors; the conv_*_generic kernels further down (one thread per output, as
 // src/gpu/conv2d_naive.hh) remain for kernels with more than kOrdMaxTaps taps, whose tiles would not fit.
-#include <mutex>
 #include <type_traits>
 
 #include "common.cuh"
@@ -700,12 +699,8 @@ template <int TM, int TN, int TX, int TY, int STAGES, int U>
 int launch_ordered_fwd_taps(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep, cudaStream_t stream)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_ordered_fwd_kernel<TM, TN, TX, TY, STAGES, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
-    });
-    DCG_CUDA(attr_err);
+    static OncePerDevice once;
+    DCG_CUDA(allow_smem(once, conv_ordered_fwd_kernel<TM, TN, TX, TY, STAGES, U>, kOrdSmem));
     const int taps = d.kh * d.kw, qc = ord_channels(taps, d.c);
     const size_t smem = (size_t)STAGES * (BMT * ord_row_pitch(taps, qc) + qc * taps * ord_pitch(BNT)) * sizeof(float);
     const long long pixels = (long long)d.n * d.ho * d.wo;
@@ -731,12 +726,8 @@ template <int TM, int TN, int TX, int TY, int STAGES>
 int launch_ordered_dx_tile(const dcg_conv_desc& d, const float* dy, const float* k, float* dx, const EpilogueArgs& ep, cudaStream_t stream)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_ordered_dx_kernel<TM, TN, TX, TY, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
-    });
-    DCG_CUDA(attr_err);
+    static OncePerDevice once;
+    DCG_CUDA(allow_smem(once, conv_ordered_dx_kernel<TM, TN, TX, TY, STAGES>, kOrdSmem));
     const int mh = (d.h + d.stride_h - 1) / d.stride_h, mw = (d.w + d.stride_w - 1) / d.stride_w;   // of the largest class
     const int taps = ((d.kh + d.stride_h - 1) / d.stride_h) * ((d.kw + d.stride_w - 1) / d.stride_w);
     const int qc = ord_channels(taps, d.o);
@@ -781,12 +772,8 @@ int launch_ordered_dk_tile(const dcg_conv_desc& d, const float* x, const float* 
 {
     constexpr int BMT = TM * TY, BNT = TN * TX;
     const size_t smem = (size_t)GROUPS * STAGES * 32 * (ord_pitch(BMT) + ord_pitch(BNT)) * 4 + (GROUPS > 1 ? (size_t)GROUPS * BMT * BNT * 4 : 0);
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_ordered_dk_kernel<TM, TN, TX, TY, STAGES, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrdSmem);
-    });
-    DCG_CUDA(attr_err);
+    static OncePerDevice once;
+    DCG_CUDA(allow_smem(once, conv_ordered_dk_kernel<TM, TN, TX, TY, STAGES, GROUPS>, kOrdSmem));
     const int M = d.kh * d.kw * d.c;
     const dim3 grid((unsigned)((M + BMT - 1) / BMT), (unsigned)((d.o + BNT - 1) / BNT));
     launch_pdl(conv_ordered_dk_kernel<TM, TN, TX, TY, STAGES, GROUPS>, grid, TX * TY * GROUPS, smem, stream, x, dy, dk, d,

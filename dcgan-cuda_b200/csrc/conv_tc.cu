@@ -727,13 +727,8 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
         if (p.mt > 1) { form = 2 + p.mt / 4; kernel = more_taps[p.mt / 4][p.kind]; }
     }
     // each form is loaded when it is first needed, not all of them with the first convolution
-    static std::once_flag once[4][4];
-    static cudaError_t attr_err[4][4];
-    std::call_once(once[form][p.kind], [&] {
-        attr_err[form][p.kind] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    });
-    if (attr_err[form][p.kind] != cudaSuccess)
-        return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_tc_kernel): %s", cudaGetErrorString(attr_err[form][p.kind]));
+    static OncePerDevice once[4][4];
+    DCG_CUDA(allow_smem(once[form][p.kind], kernel, kMaxSmem));
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
     if (err != cudaSuccess) return fail(DCG_ERR_CUDA, "conv_tc_kernel launch: %s", cudaGetErrorString(err));
     count_launch();
@@ -831,13 +826,8 @@ struct Prepared {
 
 int launch_dxf(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t stream)
 {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_dxf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    });
-    if (attr_err != cudaSuccess)
-        return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_dxf_kernel): %s", cudaGetErrorString(attr_err));
+    static OncePerDevice once;
+    DCG_CUDA(allow_smem(once, conv_dxf_kernel, kMaxSmem));
     Params& p = pr.pl.p;
     p.out = out;
     p.ep = ep;
@@ -881,15 +871,8 @@ bool short_ok(const Plan& pl)
 
 int launch_short(Prepared& pr, bool narrow, float* out, const EpilogueArgs& ep, cudaStream_t stream)
 {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_fwd_short_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem / 2);
-        if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(conv_fwd_short_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem / 2);
-    });
-    if (attr_err != cudaSuccess)
-        return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_fwd_short_kernel): %s", cudaGetErrorString(attr_err));
+    static OncePerDevice once[2];
+    DCG_CUDA(allow_smem(once[narrow], narrow ? conv_fwd_short_kernel<true> : conv_fwd_short_kernel<false>, kMaxSmem / 2));
     Params& p = pr.pl.p;
     p.out = out;
     p.ep = ep;
@@ -971,16 +954,10 @@ bool plan_dx3(const dcg_conv_desc& d, Plan& pl, Dx3Args& g)
 
 int launch_dx3(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t stream)
 {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(conv_dx3_kernel<5, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-        if (attr_err == cudaSuccess)
-            attr_err = cudaFuncSetAttribute(conv_dx3_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    });
-    if (attr_err != cudaSuccess)
-        return fail(DCG_ERR_CUDA, "cudaFuncSetAttribute(conv_dx3_kernel): %s", cudaGetErrorString(attr_err));
     Params& p = pr.pl.p;
+    const bool five = p.KH == 5 && p.KW == 5;
+    static OncePerDevice once[2];
+    DCG_CUDA(allow_smem(once[five], five ? conv_dx3_kernel<5, 5> : conv_dx3_kernel<0, 0>, kMaxSmem));
     p.out = out;
     p.ep = ep;
     p.scratch = nullptr;
@@ -1000,7 +977,7 @@ int launch_dx3(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t st
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    const cudaError_t err = (p.KH == 5 && p.KW == 5)
+    const cudaError_t err = five
                                 ? cudaLaunchKernelEx(&cfg, conv_dx3_kernel<5, 5>, pr.ma, pr.mb, p, pr.dx3_args)
                                 : cudaLaunchKernelEx(&cfg, conv_dx3_kernel<0, 0>, pr.ma, pr.mb, p, pr.dx3_args);
     if (err != cudaSuccess) return fail(DCG_ERR_CUDA, "conv_dx3_kernel launch: %s", cudaGetErrorString(err));

@@ -6,7 +6,6 @@
 // the reference CPU loops (src/cpu/ops.hxx:56-105,375-390); two shape specialists go with it: few outputs / long
 // reduction (8192 -> 1), and tall output from a transposed operand (the head's weight gradient).
 #include <cstdint>
-#include <mutex>
 #include <type_traits>
 
 #include "colsum.cuh"
@@ -312,13 +311,8 @@ int launch_tile(const float* a, const float* b, float* out, size_t m, size_t n, 
 {
     constexpr int BM = TM * TY, BN = TN * TX;
     constexpr size_t smem = (size_t)STAGES * ((TA ? KC * (BM + 4) : BM * (KC + 4)) + (TB ? BN * (KC + 4) : KC * (BN + 4))) * sizeof(float);
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    });
-    DCG_CUDA(attr_err);
+    static OncePerDevice once;
+    DCG_CUDA(allow_smem(once, gemm_ordered_kernel<TA, TB, TM, TN, TX, TY, STAGES, KC>, smem));
     dim3 grid((unsigned)((p + BN - 1) / BN), (unsigned)((m + BM - 1) / BM));
     static_assert(smem >= kSumSmem && TX * TY <= 256, "the column sums run in the same blocks");
     if (e.sums) {   // a block each for the column tiles, up to 32: they are not to crowd the others on some of the SMs
