@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include <atomic>
+#include <type_traits>
 
 #include "colsum.cuh"
 #include "common.cuh"
@@ -211,21 +212,28 @@ colsum_partial_kernel(const float* __restrict__ a, float* __restrict__ partial,
 
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (group < groups) {
-        size_t r = r0 + ty;
-        for (; r < r1; r += 8 * (size_t)ty_count) {   // eight rows in flight per thread
+        // eight rows in flight per thread; the last ones of a slab with a test each (in every iteration the tests cost as much as the
+        // adds of a column by itself: 1000000 x 3 14.6 us, 12.5 without)
+        auto eight_rows = [&](size_t r, auto tested) {
             float4 v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const size_t ru = r + u * (size_t)ty_count;
                 v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (ru < r1) {
+                if (!decltype(tested)::value || ru < r1) {
                     if (VEC) v[u] = __ldg(reinterpret_cast<const float4*>(a + ru * cols) + group);
                     else v[u].x = __ldg(a + ru * cols + group);
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
-        }
+            for (int u = 0; u < 8; ++u) {
+                acc.x += v[u].x;
+                if (VEC) { acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
+            }
+        };
+        size_t r = r0 + ty;
+        for (; r + 7 * (size_t)ty_count < r1; r += 8 * (size_t)ty_count) eight_rows(r, std::false_type());
+        if (r < r1) eight_rows(r, std::true_type());
     }
     constexpr int W = VEC ? 4 : 1;
     float* mine = smem + ((size_t)ty * tx_count + tx) * W;
@@ -480,13 +488,14 @@ softmax_rows_kernel(const float* __restrict__ a, const float* __restrict__ y,
 
 // -(1/rows) sum_ij y_ij (logit_ij - logsumexp_i)
 constexpr int kXentRegs = 16;
+template <bool FEW>   // cols <= kXentRegs; kernels of their own: one with both loops ran rows of 2000 12% slower
 __device__ __forceinline__ float softmax_xent_block(const float* __restrict__ y, const float* __restrict__ logits, size_t rows,
                                                     size_t cols, float* red)
 {
     float acc = 0.f;
     for (size_t r = threadIdx.x; r < rows; r += blockDim.x) {
         const float* lr = logits + r * cols;
-        if (cols <= kXentRegs) {   // the whole row in flight at once (rows are not contiguous across threads)
+        if constexpr (FEW) {   // the whole row in flight at once (rows are not contiguous across threads)
             float l[kXentRegs], t[kXentRegs];
 #pragma unroll
             for (int c = 0; c < kXentRegs; ++c) {
@@ -515,19 +524,21 @@ __device__ __forceinline__ float softmax_xent_block(const float* __restrict__ y,
     return block_sum(acc, red);
 }
 
+template <bool FEW>
 __global__ void __launch_bounds__(512)
 softmax_xent_kernel(const float* __restrict__ y, const float* __restrict__ logits,
                     float* __restrict__ out, size_t rows, size_t cols)
 {
     pdl_enter();
     __shared__ float red[32];
-    const float acc = softmax_xent_block(y, logits, rows, cols, red);
+    const float acc = softmax_xent_block<FEW>(y, logits, rows, cols, red);
     if (threadIdx.x == 0) out[0] = -acc / (float)rows;
 }
 
 // Loss and its gradient in one launch: block 0 computes the loss, the others sixteen rows of the gradient each, so neither
 // waits for the other.  The expressions and the orders of the two kernels above, so the results are bit-identical.  Bound
 // by latency (a few dependent reads, exponentials and shuffles): 100 x 10 takes 3.8 us, 13.3 with all of it in one block.
+template <bool FEW>
 __global__ void __launch_bounds__(512)
 softmax_xent_both_kernel(const float* __restrict__ y, const float* __restrict__ logits, float* __restrict__ loss,
                          float* __restrict__ grad, size_t rows, size_t cols)
@@ -539,7 +550,7 @@ softmax_xent_both_kernel(const float* __restrict__ y, const float* __restrict__ 
         if (row < rows) softmax_row(logits, y, grad, row, rows, cols, 2, threadIdx.x & 31);
         return;
     }
-    const float acc = softmax_xent_block(y, logits, rows, cols, red);
+    const float acc = softmax_xent_block<FEW>(y, logits, rows, cols, red);
     if (threadIdx.x == 0) loss[0] = -acc / (float)rows;
 }
 
@@ -850,7 +861,7 @@ int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, flo
 int softmax_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t rows, size_t cols, cudaStream_t stream)
 {
     DCG_CHECK_ARG(y && logits && loss && grad && rows > 0 && cols > 0, "softmax_xent_with_grad: bad arguments");
-    launch_pdl(softmax_xent_both_kernel, (unsigned)(1 + (rows + 15) / 16), 512, 0, stream, y, logits, loss, grad, rows, cols);
+    launch_pdl(cols <= kXentRegs ? softmax_xent_both_kernel<true> : softmax_xent_both_kernel<false>, (unsigned)(1 + (rows + 15) / 16), 512, 0, stream, y, logits, loss, grad, rows, cols);
     DCG_LAUNCH_CHECK("softmax_xent_both_kernel");
     return DCG_OK;
 }
@@ -916,7 +927,7 @@ extern "C" int dcg_softmax_xent(const float* y, const float* logits, float* out,
                                 size_t cols, dcg_stream_t stream)
 {
     DCG_CHECK_ARG(y && logits && out && rows > 0 && cols > 0, "dcg_softmax_xent: bad arguments");
-    launch_pdl(softmax_xent_kernel, 1, 512, 0, as_stream(stream), y, logits, out, rows, cols);
+    launch_pdl(cols <= kXentRegs ? softmax_xent_kernel<true> : softmax_xent_kernel<false>, 1, 512, 0, as_stream(stream), y, logits, out, rows, cols);
     DCG_LAUNCH_CHECK("softmax_xent_kernel");
     return DCG_OK;
 }
