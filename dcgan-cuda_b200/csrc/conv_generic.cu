@@ -139,49 +139,40 @@ __device__ __forceinline__ float dk_sum(const float* __restrict__ x, const float
 }
 
 // The ordered kernels multiply taps outside the image as zeros where the reference skips them.  That adds +0 and leaves the same
-// bits unless the other factor is infinite or NaN, and then the result is not finite either: a thread with such a result computes
-// its outputs again with the sums above.
+// bits unless the other factor is infinite or NaN: then the result is NaN.  They note in g_nan_seen that there is one - for good,
+// so that launches of several streams need no order - and conv_nan_again_kernel behind them, which ends at once as long as there
+// has been none, computes NaN outputs again with the sums above.  (Sums in the ordered kernels themselves, called or inlined,
+// take registers from the main loops: training step at batch 8 6.11 -> 6.25 to 6.46 ms.  The launch between them is 0.3 to 0.9 us
+// of a layer by itself; in a list it also keeps the long blocks of the next kernel from starting early and piling up on the SMs
+// that are free first, 5.25 ms.)
+__device__ int g_nan_seen;
 template <int TM, int TN>
-__device__ __forceinline__ bool all_finite(const float (&v)[TM][TN])
+__device__ __forceinline__ bool any_nan(const float (&v)[TM][TN])
 {
-    bool ok = true;
+    bool nan = false;
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) ok = ok && isfinite(v[i][j]);
-    return ok;
+        for (int j = 0; j < TN; ++j) nan = nan || isnan(v[i][j]);
+    return nan;
 }
-// rows x cols outputs from (row0, col0) on, row_step and col_step apart.  Not inlined: nothing of it is live in the kernels' loops.
-__device__ __noinline__ void fwd_outputs_again(const float* x, const float* k, float* y, const dcg_conv_desc& d, const EpilogueArgs& ep,
-                                               long long row0, int row_step, int rows, int col0, int cols)
+
+enum OrderedKind { kOrdFwd, kOrdDx, kOrdDk };
+template <int KIND>
+__global__ void __launch_bounds__(kThreads)
+conv_nan_again_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, const dcg_conv_desc d, const EpilogueArgs ep,
+                      const size_t total)
 {
-    const long long pixels = (long long)d.n * d.ho * d.wo;
-    for (int i = 0; i < rows * cols; ++i) {
-        const long long p = row0 + (long long)(i / cols) * row_step;
-        const int ch = col0 + i % cols;
-        if (p >= pixels || ch >= d.o) continue;
-        const size_t idx = (size_t)p * d.o + ch;
-        y[idx] = epilogue_apply(ep, fwd_sum(x, k, d, p, ch), idx, ch);
-    }
-}
-// (rows are the pixels (ph + stride * i, pw + stride * j), mh x mw of them)
-__device__ __noinline__ void dx_outputs_again(const float* dy, const float* k, float* dx, const dcg_conv_desc& d, const EpilogueArgs& ep, int ph,
-                                              int pw, int mh, int mw, long long row0, int row_step, int rows, int col0, int col_step, int cols)
-{
-    const long long pixels = (long long)d.n * mh * mw;
-    for (int i = 0; i < rows * cols; ++i) {
-        const long long p = row0 + (long long)(i / cols) * row_step, t = p / mw;
-        const int ch = col0 + i % cols * col_step;
-        if (p >= pixels || ch >= d.c) continue;
-        const size_t pix = ((size_t)(t / mh) * d.h + (size_t)(t % mh) * d.stride_h + ph) * d.w + (size_t)(p % mw) * d.stride_w + pw;
-        dx[pix * d.c + ch] = epilogue_apply(ep, dx_sum(dy, k, d, pix, ch), pix * d.c + ch, ch);
-    }
-}
-__device__ __noinline__ void dk_outputs_again(const float* x, const float* dy, float* dk, const dcg_conv_desc& d, int row0, int rows, int col0, int cols)
-{
-    for (int i = 0; i < rows * cols; ++i) {
-        const int row = row0 + i / cols, o = col0 + i % cols;
-        if (row < d.kh * d.kw * d.c && o < d.o) dk[(size_t)row * d.o + o] = dk_sum(x, dy, d, row, o);
+    pdl_enter();
+    if (*reinterpret_cast<volatile int*>(&g_nan_seen) == 0) return;
+    const int cols = KIND == kOrdDx ? d.c : d.o;
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
+        if (!isnan(out[idx])) continue;
+        const size_t row = idx / cols;
+        const int col = (int)(idx % cols);
+        if (KIND == kOrdFwd) out[idx] = epilogue_apply(ep, fwd_sum(a, b, d, row, col), idx, col);
+        else if (KIND == kOrdDx) out[idx] = epilogue_apply(ep, dx_sum(a, b, d, row, col), idx, col);
+        else out[idx] = dk_sum(a, b, d, row, col);
     }
 }
 
@@ -191,7 +182,7 @@ __device__ __noinline__ void dk_outputs_again(const float* x, const float* dy, f
 // gathered sixteen bytes - four channels of one (row, tap) - at a time with cp.async and kept as it comes:
 // [row][channel quad][tap][4], row pitch 4 mod 8 words so that eight rows start in different bank quads.  The
 // weights of the forward are rows of output channels, [q][tap][channel].  Taps outside the image are zero-filled
-// (see all_finite).  Two to four stages of QC channels x all taps.
+// (see g_nan_seen).  Two to four stages of QC channels x all taps.
 // Bound by issue (the sum must stay unfused: two instructions per product; packed f32x2 arithmetic was measured
 // and is no faster, its operands have to be duplicated) and, where the outputs are few, by the latency of the
 // chain of dependent adds.  Measured, 5x5 / stride 2 layers: 18 TFLOP/s (a multiply and an add counted as two) of the
@@ -268,8 +259,7 @@ __host__ __device__ constexpr int ord_row_pitch(int taps, int qc) { return taps 
 template <int TM, int TN, int TX, int TY, int STAGES, int U>   // U divides the number of taps
 __global__ void __launch_bounds__(TX * TY)
 conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k, float* __restrict__ y,
-                        const __grid_constant__ dcg_conv_desc d, const __grid_constant__ EpilogueArgs ep, const int QC, const int vec_a,
-                        const int vec_b)
+                        const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec_a, const int vec_b)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY, LDB = ord_pitch(BNT);
     extern __shared__ __align__(16) float smem[];
@@ -357,7 +347,7 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
         __syncthreads();
         buf = buf + 1 == STAGES ? 0 : buf + 1;
     }
-    if (!all_finite(acc)) return fwd_outputs_again(x, k, y, d, ep, m0 + ty, TY, TM, n0 + tx * TN, TN);
+    if (any_nan(acc)) g_nan_seen = 1;
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const long long p = m0 + ty + i * TY;
@@ -378,7 +368,7 @@ conv_ordered_fwd_kernel(const float* __restrict__ x, const float* __restrict__ k
 template <int TM, int TN, int TX, int TY, int STAGES>
 __global__ void __launch_bounds__(TX * TY)
 conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k, float* __restrict__ dx,
-                       const __grid_constant__ dcg_conv_desc d, const __grid_constant__ EpilogueArgs ep, const int QC, const int vec)
+                       const dcg_conv_desc d, const EpilogueArgs ep, const int QC, const int vec)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY;
     extern __shared__ __align__(16) float smem[];
@@ -503,7 +493,7 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
             buf = buf + 1 == STAGES ? 0 : buf + 1;
         }
     }
-    if (!all_finite(tot)) return dx_outputs_again(dy, k, dx, d, ep, ph, pw, g.mh, g.mw, m0 + ty, TY, TM, n0 + tx, TX, TN);
+    if (any_nan(tot)) g_nan_seen = 1;
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const long long p = m0 + ty + i * TY;
@@ -531,7 +521,7 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
 template <int TM, int TN, int TX, int TY, int STAGES, int GROUPS>
 __global__ void __launch_bounds__(TX * TY * GROUPS)
 conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dk,
-                       const __grid_constant__ dcg_conv_desc d, const int vec_a, const int vec_b)
+                       const dcg_conv_desc d, const int vec_a, const int vec_b)
 {
     constexpr int BMT = TM * TY, BNT = TN * TX, THREADS = TX * TY, KP = 32, LDA = ord_pitch(BMT), LDB = ord_pitch(BNT);
     constexpr int STAGE = KP * (LDA + LDB);
@@ -662,7 +652,7 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
         }
     }
     if (group != 0) return;
-    if (!all_finite(tot)) return dk_outputs_again(x, dy, dk, d, m0 + ty * TM, TM, n0 + tx * TN, TN);
+    if (any_nan(tot)) g_nan_seen = 1;
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int row = m0 + ty * TM + i;
@@ -796,7 +786,7 @@ int launch_ordered_dk(const dcg_conv_desc& d, const float* x, const float* dy, f
 // ---- one thread per output: kernels with many taps ----------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
 conv_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ k, float* __restrict__ y,
-                        const __grid_constant__ dcg_conv_desc d, const EpilogueArgs ep, size_t total)
+                        const dcg_conv_desc d, const EpilogueArgs ep, size_t total)
 {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
@@ -806,7 +796,7 @@ conv_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ k
 
 __global__ void __launch_bounds__(kThreads)
 conv_dx_generic_kernel(const float* __restrict__ dy, const float* __restrict__ k, float* __restrict__ dx,
-                       const __grid_constant__ dcg_conv_desc d, const EpilogueArgs ep, size_t total)
+                       const dcg_conv_desc d, const EpilogueArgs ep, size_t total)
 {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
@@ -816,10 +806,24 @@ conv_dx_generic_kernel(const float* __restrict__ dy, const float* __restrict__ k
 
 __global__ void __launch_bounds__(kThreads)
 conv_dk_generic_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dk,
-                       const __grid_constant__ dcg_conv_desc d, size_t total)
+                       const dcg_conv_desc d, size_t total)
 {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < total) dk[idx] = dk_sum(x, dy, d, idx / d.o, (int)(idx % d.o));
+}
+
+// Behind an ordered launch of which some output has a tap outside the source.  An output that has replaced its gate stays as it is.
+template <int KIND>
+int nan_again(const float* a, const float* b, float* out, const dcg_conv_desc& d, const EpilogueArgs& ep, size_t total, cudaStream_t stream)
+{
+    const bool leaves = KIND == kOrdDx ? d.kh * d.kw * d.stride_h * d.stride_w > 1
+                                       : d.pad_top > 0 || d.pad_left > 0 || (d.ho - 1) * d.stride_h + d.kh > d.h || (d.wo - 1) * d.stride_w + d.kw > d.w;
+    if (!leaves || ep.gate == out) return DCG_OK;
+    size_t blocks = (total + kThreads - 1) / kThreads;
+    if (blocks > (size_t)sm_count()) blocks = sm_count();
+    launch_pdl(conv_nan_again_kernel<KIND>, (unsigned)blocks, kThreads, 0, stream, a, b, out, d, ep, total);
+    DCG_CUDA(cudaGetLastError());   // not counted: no operator's launch but a look behind one
+    return DCG_OK;
 }
 
 }  // namespace
@@ -829,7 +833,10 @@ int conv_fwd_generic(const dcg_conv_desc& d, const float* x, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.ho * d.wo * d.o;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d, d.o, 64)) return launch_ordered_fwd(d, x, k, y, ep, stream);
+    if (ordered_ok(d, d.o, 64)) {
+        const int st = launch_ordered_fwd(d, x, k, y, ep, stream);
+        return st ? st : nan_again<kOrdFwd>(x, k, y, d, ep, total, stream);
+    }
     conv_fwd_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, k, y, d, ep, total);
     DCG_LAUNCH_CHECK("conv_fwd_generic_kernel");
@@ -841,7 +848,10 @@ int conv_dx_generic(const dcg_conv_desc& d, const float* dy, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.h * d.w * d.c;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d, d.c, 32, (long long)d.stride_h * d.stride_w)) return launch_ordered_dx(d, dy, k, dx, ep, stream);
+    if (ordered_ok(d, d.c, 32, (long long)d.stride_h * d.stride_w)) {
+        const int st = launch_ordered_dx(d, dy, k, dx, ep, stream);
+        return st ? st : nan_again<kOrdDx>(dy, k, dx, d, ep, total, stream);
+    }
     conv_dx_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         dy, k, dx, d, ep, total);
     DCG_LAUNCH_CHECK("conv_dx_generic_kernel");
@@ -853,7 +863,10 @@ int conv_dk_generic(const dcg_conv_desc& d, const float* x, const float* dy, flo
 {
     const size_t total = (size_t)d.kh * d.kw * d.c * d.o;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d, d.o, 64)) return launch_ordered_dk(d, x, dy, dk, stream);
+    if (ordered_ok(d, d.o, 64)) {
+        const int st = launch_ordered_dk(d, x, dy, dk, stream);
+        return st ? st : nan_again<kOrdDk>(x, dy, dk, d, EpilogueArgs{}, total, stream);
+    }
     conv_dk_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, dy, dk, d, total);
     DCG_LAUNCH_CHECK("conv_dk_generic_kernel");

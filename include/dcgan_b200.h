@@ -480,7 +480,8 @@ int dcg_debug_conv_plan(const dcg_conv_desc* desc, int kind, int precision, int 
 uint64_t dcg_debug_fused_dx_launches(void);   /* launches of the class-fused input-gradient kernel so far */
 /* Library version and the architecture the kernels were built for ("sm_100a"). */
 const char* dcg_build_info(void);
-/* Kernels launched by this library since it was loaded (all contexts, all threads). */
+/* Kernels launched by this library since it was loaded (all contexts, all threads); the check for NaN behind an
+ * fp32 convolution is not counted. */
 uint64_t dcg_launches_total(void);
 
 #ifdef __cplusplus
