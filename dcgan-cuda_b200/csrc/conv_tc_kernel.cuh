@@ -536,8 +536,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp >= 2) {
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
-        // the warps of a lane quadrant (one per group) take the 32-column slabs in turn
-        for (int c0 = ((warp - 2) >> 2) * 32; c0 < p.bn; c0 += 32 * G) {
+        // the warps of a lane quadrant (one per group) take the 32-column slabs in turn (3xTF32: unrolled, for the sums of the
+        // slabs are registers only if nothing chooses among them at run time)
+#pragma unroll (X3 ? kX3Slabs : 1)
+        for (int sl = 0; sl < (X3 ? kX3Slabs : 256 / 32); ++sl) {
+            const int c0 = ((warp - 2) >> 2) * 32 + sl * 32 * G;
+            if (c0 >= p.bn) break;
             uint32_t r[32];
             const uint32_t tquad = tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
             const uint32_t taddr = tquad + (X3 ? (uint32_t)(((nq > 0 ? (nq - 1) / kX3Block : 0) & (x3_mains - 1)) * p.bn) : 0u);
@@ -555,18 +559,16 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (q < 16 || full) r[q] = __float_as_uint(__fadd_rn(__uint_as_float(r[q]), __uint_as_float(r2[q])));
             }
             if constexpr (X3) {   // add the accumulator of the small terms, then the blocks taken over before
-                uint32_t r2[32];
-                if (full) tmem_ld_32x32b_x32(tquad + (uint32_t)(x3_mains * p.bn), r2);
-                else tmem_ld_32x32b_x16(tquad + (uint32_t)(x3_mains * p.bn), r2);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int sl = 0; sl < kX3Slabs; ++sl)
-                    if (c0 / (32 * G) == sl) {
+                for (int half = 0; half < 2; ++half) {
+                    if (half == 1 && !full) break;
+                    uint32_t r2[32];   // (16 of them)
+                    tmem_ld_32x32b_x16(tquad + (uint32_t)(x3_mains * p.bn + 16 * half), r2);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                        for (int q = 0; q < 32; ++q)
-                            if (q < 16 || full)
-                                r[q] = __float_as_uint(__fadd_rn(__fadd_rn(x3_sum[sl][q], __uint_as_float(r[q])), __uint_as_float(r2[q])));
-                    }
+                    for (int q = 0; q < 16; ++q)
+                        r[16 * half + q] = __float_as_uint(__fadd_rn(__fadd_rn(x3_sum[sl][16 * half + q], __uint_as_float(r[16 * half + q])), __uint_as_float(r2[q])));
+                }
             }
             if (vec) {
                 if (multi) {
