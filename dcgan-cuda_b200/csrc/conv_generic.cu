@@ -144,7 +144,10 @@ __device__ __forceinline__ float dk_sum(const float* __restrict__ x, const float
 // has been none, computes NaN outputs again with the sums above.  (Sums in the ordered kernels themselves, called or inlined,
 // take registers from the main loops: training step at batch 8 6.11 -> 6.25 to 6.46 ms.  The launch between them is 0.3 to 0.9 us
 // of a layer by itself; in a list it also keeps the long blocks of the next kernel from starting early and piling up on the SMs
-// that are free first, 5.25 ms.)
+// that are free first, 5.25 ms.)  The kernels of small input and kernel gradients, for which a launch is long, do have such sums,
+// with 32-bit indexes and nothing unrolled; theirs cost nothing (9 x 9 x 5 images, 5 x 5: input gradient 4.5 us, 5.2 with a launch).
+__host__ __device__ constexpr bool dx_again_inside(int tm) { return tm == 1; }
+__host__ __device__ constexpr bool dk_again_inside(int tm, int tn) { return tm * tn <= 4; }
 __device__ int g_nan_seen;
 template <int TM, int TN>
 __device__ __forceinline__ bool any_nan(const float (&v)[TM][TN])
@@ -493,7 +496,32 @@ conv_ordered_dx_kernel(const float* __restrict__ dy, const float* __restrict__ k
             buf = buf + 1 == STAGES ? 0 : buf + 1;
         }
     }
-    if (any_nan(tot)) g_nan_seen = 1;
+    if constexpr (!dx_again_inside(TM)) {
+        if (any_nan(tot)) g_nan_seen = 1;
+    } else if (any_nan(tot)) {
+#pragma unroll 1
+        for (int i = 0; i < TM * TN; ++i) {
+            const int p = (int)m0 + ty + i / TN * TY, ch = n0 + tx + i % TN * TX;
+            if (p >= pixels || ch >= d.c) continue;
+            const int line = p / g.mw, n = line / g.mh, r0 = line % g.mh, c0 = p % g.mw;
+            float total = 0.f;
+#pragma unroll 1
+            for (int o = 0; o < d.o; ++o) {
+                float v = 0.f;
+#pragma unroll 1
+                for (int t = 0; t < T; ++t) {
+                    const int a = t / g.Tw, b = t % g.Tw, r = r0 + g.eh + a, c = c0 + g.ew + b;
+                    const int kt = (d.kh - 1 - r0h - d.stride_h * a) * d.kw + d.kw - 1 - r0w - d.stride_w * b;
+                    if (r >= 0 && r < d.ho && c >= 0 && c < d.wo)
+                        v = __fadd_rn(v, __fmul_rn(__ldg(dy + ((n * d.ho + r) * d.wo + c) * d.o + o), __ldg(k + (kt * d.c + ch) * d.o + o)));
+                }
+                total = __fadd_rn(total, v);
+            }
+            const size_t idx = ((size_t)((n * d.h + r0 * d.stride_h + ph) * d.w) + c0 * d.stride_w + pw) * d.c + ch;
+            dx[idx] = epilogue_apply(ep, total, idx, ch);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const long long p = m0 + ty + i * TY;
@@ -652,7 +680,30 @@ conv_ordered_dk_kernel(const float* __restrict__ x, const float* __restrict__ dy
         }
     }
     if (group != 0) return;
-    if (any_nan(tot)) g_nan_seen = 1;
+    if constexpr (!dk_again_inside(TM, TN)) {
+        if (any_nan(tot)) g_nan_seen = 1;
+    } else if (any_nan(tot)) {
+#pragma unroll 1
+        for (int i = 0; i < TM * TN; ++i) {
+            const int row = m0 + ty * TM + i / TN, o = n0 + tx * TN + i % TN;
+            if (row >= M || o >= d.o) continue;
+            const int t = row / d.c, q = row % d.c;
+            float total = 0.f;
+#pragma unroll 1
+            for (int n = 0; n < d.n; ++n) {
+                float v = 0.f;
+#pragma unroll 1
+                for (int p = 0; p < P; ++p) {
+                    const int h = p / d.wo * d.stride_h + t / d.kw - d.pad_top, w = p % d.wo * d.stride_w + t % d.kw - d.pad_left;
+                    if (h >= 0 && h < d.h && w >= 0 && w < d.w)
+                        v = __fadd_rn(v, __fmul_rn(__ldg(x + ((n * d.h + h) * d.w + w) * d.c + q), __ldg(dy + (n * P + p) * d.o + o)));
+                }
+                total = __fadd_rn(total, v);
+            }
+            dk[(size_t)row * d.o + o] = total;
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int row = m0 + ty * TM + i;
@@ -674,6 +725,20 @@ bool ordered_ok(const dcg_conv_desc& d, int cols, int tile, long long classes = 
     return d.kh * d.kw <= kOrdMaxTaps && x < (1ll << 31) && y < (1ll << 31) && k < (1ll << 31);
 }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// Behind an ordered launch of which some output has a tap outside the source.  An output that has replaced its gate stays as it is.
+template <int KIND>
+int nan_again(const float* a, const float* b, float* out, const dcg_conv_desc& d, const EpilogueArgs& ep, size_t total, cudaStream_t stream)
+{
+    const bool leaves = KIND == kOrdDx ? d.kh * d.kw * d.stride_h * d.stride_w > 1
+                                       : d.pad_top > 0 || d.pad_left > 0 || (d.ho - 1) * d.stride_h + d.kh > d.h || (d.wo - 1) * d.stride_w + d.kw > d.w;
+    if (!leaves || ep.gate == out) return DCG_OK;
+    size_t blocks = (total + kThreads - 1) / kThreads;
+    if (blocks > (size_t)sm_count()) blocks = sm_count();
+    launch_pdl(conv_nan_again_kernel<KIND>, (unsigned)blocks, kThreads, 0, stream, a, b, out, d, ep, total);
+    DCG_CUDA(cudaGetLastError());   // not counted: no operator's launch but a look behind one
+    return DCG_OK;
+}
 
 // Channels per stage: kOrdQuads words of `taps` each, no more than there are.
 int ord_channels(int taps, int contracted)
@@ -698,7 +763,7 @@ int launch_ordered_fwd_taps(const dcg_conv_desc& d, const float* x, const float*
     launch_pdl(conv_ordered_fwd_kernel<TM, TN, TX, TY, STAGES, U>, grid, TX * TY, smem, stream, x, k, y, d, ep, qc,
                d.c % 4 == 0 && aligned16(x) ? 1 : 0, d.o % 4 == 0 && aligned16(k) ? 1 : 0);
     DCG_LAUNCH_CHECK("conv_ordered_fwd_kernel");
-    return DCG_OK;
+    return nan_again<kOrdFwd>(x, k, y, d, ep, (size_t)pixels * d.o, stream);
 }
 
 template <int TM, int TN, int TX, int TY, int STAGES>
@@ -727,7 +792,7 @@ int launch_ordered_dx_tile(const dcg_conv_desc& d, const float* dy, const float*
     launch_pdl(conv_ordered_dx_kernel<TM, TN, TX, TY, STAGES>, grid, TX * TY, smem, stream, dy, k, dx, d, ep, qc,
                d.o % 4 == 0 && aligned16(dy) && aligned16(k) ? 1 : 0);
     DCG_LAUNCH_CHECK("conv_ordered_dx_kernel");
-    return DCG_OK;
+    return dx_again_inside(TM) ? DCG_OK : nan_again<kOrdDx>(dy, k, dx, d, ep, (size_t)d.n * d.h * d.w * d.c, stream);
 }
 
 // Tile choice by outputs per lane of the GPU (SMs x 128): the wider the thread tile the fewer instructions an output
@@ -769,7 +834,7 @@ int launch_ordered_dk_tile(const dcg_conv_desc& d, const float* x, const float* 
     launch_pdl(conv_ordered_dk_kernel<TM, TN, TX, TY, STAGES, GROUPS>, grid, TX * TY * GROUPS, smem, stream, x, dy, dk, d,
                d.c % 4 == 0 && aligned16(x) ? 1 : 0, d.o % 4 == 0 && aligned16(dy) ? 1 : 0);
     DCG_LAUNCH_CHECK("conv_ordered_dk_kernel");
-    return DCG_OK;
+    return dk_again_inside(TM, TN) ? DCG_OK : nan_again<kOrdDk>(x, dy, dk, d, EpilogueArgs{}, (size_t)M * d.o, stream);
 }
 
 int launch_ordered_dk(const dcg_conv_desc& d, const float* x, const float* dy, float* dk, cudaStream_t stream)
@@ -812,20 +877,6 @@ conv_dk_generic_kernel(const float* __restrict__ x, const float* __restrict__ dy
     if (idx < total) dk[idx] = dk_sum(x, dy, d, idx / d.o, (int)(idx % d.o));
 }
 
-// Behind an ordered launch of which some output has a tap outside the source.  An output that has replaced its gate stays as it is.
-template <int KIND>
-int nan_again(const float* a, const float* b, float* out, const dcg_conv_desc& d, const EpilogueArgs& ep, size_t total, cudaStream_t stream)
-{
-    const bool leaves = KIND == kOrdDx ? d.kh * d.kw * d.stride_h * d.stride_w > 1
-                                       : d.pad_top > 0 || d.pad_left > 0 || (d.ho - 1) * d.stride_h + d.kh > d.h || (d.wo - 1) * d.stride_w + d.kw > d.w;
-    if (!leaves || ep.gate == out) return DCG_OK;
-    size_t blocks = (total + kThreads - 1) / kThreads;
-    if (blocks > (size_t)sm_count()) blocks = sm_count();
-    launch_pdl(conv_nan_again_kernel<KIND>, (unsigned)blocks, kThreads, 0, stream, a, b, out, d, ep, total);
-    DCG_CUDA(cudaGetLastError());   // not counted: no operator's launch but a look behind one
-    return DCG_OK;
-}
-
 }  // namespace
 
 int conv_fwd_generic(const dcg_conv_desc& d, const float* x, const float* k, float* y,
@@ -833,10 +884,7 @@ int conv_fwd_generic(const dcg_conv_desc& d, const float* x, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.ho * d.wo * d.o;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d, d.o, 64)) {
-        const int st = launch_ordered_fwd(d, x, k, y, ep, stream);
-        return st ? st : nan_again<kOrdFwd>(x, k, y, d, ep, total, stream);
-    }
+    if (ordered_ok(d, d.o, 64)) return launch_ordered_fwd(d, x, k, y, ep, stream);
     conv_fwd_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, k, y, d, ep, total);
     DCG_LAUNCH_CHECK("conv_fwd_generic_kernel");
@@ -848,10 +896,7 @@ int conv_dx_generic(const dcg_conv_desc& d, const float* dy, const float* k, flo
 {
     const size_t total = (size_t)d.n * d.h * d.w * d.c;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d, d.c, 32, (long long)d.stride_h * d.stride_w)) {
-        const int st = launch_ordered_dx(d, dy, k, dx, ep, stream);
-        return st ? st : nan_again<kOrdDx>(dy, k, dx, d, ep, total, stream);
-    }
+    if (ordered_ok(d, d.c, 32, (long long)d.stride_h * d.stride_w)) return launch_ordered_dx(d, dy, k, dx, ep, stream);
     conv_dx_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         dy, k, dx, d, ep, total);
     DCG_LAUNCH_CHECK("conv_dx_generic_kernel");
@@ -863,10 +908,7 @@ int conv_dk_generic(const dcg_conv_desc& d, const float* x, const float* dy, flo
 {
     const size_t total = (size_t)d.kh * d.kw * d.c * d.o;
     if (total == 0) return DCG_OK;
-    if (ordered_ok(d, d.o, 64)) {
-        const int st = launch_ordered_dk(d, x, dy, dk, stream);
-        return st ? st : nan_again<kOrdDk>(x, dy, dk, d, EpilogueArgs{}, total, stream);
-    }
+    if (ordered_ok(d, d.o, 64)) return launch_ordered_dk(d, x, dy, dk, stream);
     conv_dk_generic_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
         x, dy, dk, d, total);
     DCG_LAUNCH_CHECK("conv_dk_generic_kernel");
