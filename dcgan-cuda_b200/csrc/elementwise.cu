@@ -488,14 +488,13 @@ softmax_rows_kernel(const float* __restrict__ a, const float* __restrict__ y,
 
 // -(1/rows) sum_ij y_ij (logit_ij - logsumexp_i)
 constexpr int kXentRegs = 16;
-template <bool FEW>   // cols <= kXentRegs; kernels of their own: one with both loops ran rows of 2000 12% slower
 __device__ __forceinline__ float softmax_xent_block(const float* __restrict__ y, const float* __restrict__ logits, size_t rows,
                                                     size_t cols, float* red)
 {
     float acc = 0.f;
     for (size_t r = threadIdx.x; r < rows; r += blockDim.x) {
         const float* lr = logits + r * cols;
-        if constexpr (FEW) {   // the whole row in flight at once (rows are not contiguous across threads)
+        if (cols <= kXentRegs) {   // the whole row in flight at once (rows are not contiguous across threads)
             float l[kXentRegs], t[kXentRegs];
 #pragma unroll
             for (int c = 0; c < kXentRegs; ++c) {
@@ -524,21 +523,19 @@ __device__ __forceinline__ float softmax_xent_block(const float* __restrict__ y,
     return block_sum(acc, red);
 }
 
-template <bool FEW>
 __global__ void __launch_bounds__(512)
 softmax_xent_kernel(const float* __restrict__ y, const float* __restrict__ logits,
                     float* __restrict__ out, size_t rows, size_t cols)
 {
     pdl_enter();
     __shared__ float red[32];
-    const float acc = softmax_xent_block<FEW>(y, logits, rows, cols, red);
+    const float acc = softmax_xent_block(y, logits, rows, cols, red);
     if (threadIdx.x == 0) out[0] = -acc / (float)rows;
 }
 
 // Loss and its gradient in one launch: block 0 computes the loss, the others sixteen rows of the gradient each, so neither
 // waits for the other.  The expressions and the orders of the two kernels above, so the results are bit-identical.  Bound
 // by latency (a few dependent reads, exponentials and shuffles): 100 x 10 takes 3.8 us, 13.3 with all of it in one block.
-template <bool FEW>
 __global__ void __launch_bounds__(512)
 softmax_xent_both_kernel(const float* __restrict__ y, const float* __restrict__ logits, float* __restrict__ loss,
                          float* __restrict__ grad, size_t rows, size_t cols)
@@ -550,7 +547,7 @@ softmax_xent_both_kernel(const float* __restrict__ y, const float* __restrict__ 
         if (row < rows) softmax_row(logits, y, grad, row, rows, cols, 2, threadIdx.x & 31);
         return;
     }
-    const float acc = softmax_xent_block<FEW>(y, logits, rows, cols, red);
+    const float acc = softmax_xent_block(y, logits, rows, cols, red);
     if (threadIdx.x == 0) loss[0] = -acc / (float)rows;
 }
 
@@ -861,7 +858,7 @@ int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, flo
 int softmax_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t rows, size_t cols, cudaStream_t stream)
 {
     DCG_CHECK_ARG(y && logits && loss && grad && rows > 0 && cols > 0, "softmax_xent_with_grad: bad arguments");
-    launch_pdl(cols <= kXentRegs ? softmax_xent_both_kernel<true> : softmax_xent_both_kernel<false>, (unsigned)(1 + (rows + 15) / 16), 512, 0, stream, y, logits, loss, grad, rows, cols);
+    launch_pdl(softmax_xent_both_kernel, (unsigned)(1 + (rows + 15) / 16), 512, 0, stream, y, logits, loss, grad, rows, cols);
     DCG_LAUNCH_CHECK("softmax_xent_both_kernel");
     return DCG_OK;
 }
@@ -927,7 +924,7 @@ extern "C" int dcg_softmax_xent(const float* y, const float* logits, float* out,
                                 size_t cols, dcg_stream_t stream)
 {
     DCG_CHECK_ARG(y && logits && out && rows > 0 && cols > 0, "dcg_softmax_xent: bad arguments");
-    launch_pdl(cols <= kXentRegs ? softmax_xent_kernel<true> : softmax_xent_kernel<false>, 1, 512, 0, as_stream(stream), y, logits, out, rows, cols);
+    launch_pdl(softmax_xent_kernel, 1, 512, 0, as_stream(stream), y, logits, out, rows, cols);
     DCG_LAUNCH_CHECK("softmax_xent_kernel");
     return DCG_OK;
 }
