@@ -537,7 +537,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         // the warps of a lane quadrant (one per group) take the 32-column slabs in turn (3xTF32: unrolled, for the sums of the
-        // slabs are registers only if nothing chooses among them at run time)
+        // slabs are registers only if nothing chooses among them at run time: as local memory they cost every launch 3 us, 8 -> 8
+        // input gradient 7.1 for 4.2 us)
 #pragma unroll (X3 ? kX3Slabs : 1)
         for (int sl = 0; sl < (X3 ? kX3Slabs : 256 / 32); ++sl) {
             const int c0 = ((warp - 2) >> 2) * 32 + sl * 32 * G;
