@@ -294,8 +294,24 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
     return best;
 }
 
+// The divisors of conv_tc_kernel's work decoding; `p` is complete.
+void set_divisors(Params& p, bool kernel_gradient)
+{
+    p.by_splits = FastDiv(p.splits);
+    p.by_n_tiles = FastDiv(p.n_tiles);
+    p.by_m_count = FastDiv(kernel_gradient ? p.m_tiles : p.tiles_w * p.tiles_h * p.tiles_n);
+    p.by_tiles_w = FastDiv(p.tiles_w);
+    p.by_tiles_h = FastDiv(p.tiles_h);
+    p.by_kchunks = FastDiv(p.kchunks);
+    p.by_kw = FastDiv(p.KW);
+    p.by_sh = FastDiv(p.sh);
+    p.by_sw = FastDiv(p.sw);
+    p.pt_mod = p.pt % p.sh;
+    p.pl_mod = p.pl % p.sw;
+}
+
 // False: the accumulators do not fit TMEM or the registers that take them over.
-bool finish_plan(Plan& pl)
+bool finish_plan(Plan& pl, bool kernel_gradient = false)
 {
     Params& p = pl.p;
     const int b_stage = p.bn * BK * 4;
@@ -333,6 +349,7 @@ bool finish_plan(Plan& pl)
     pl.smem = (size_t)stages * per_stage + (p.x3 ? (size_t)p.x3_bslots * b_stage : 0) + 1024 /*alignment slack*/ + 24 * stages + 64;
     p.skip_stage = -1;
     p.wait_cycles = kWaitCycles;
+    set_divisors(p, kernel_gradient);
     pl.partial_bytes = p.splits > 1 ? (size_t)pl.grid * BM * p.bn * sizeof(float) : 0;
     pl.ws_bytes = pl.partial_bytes;
     if (pl.xp_bytes || pl.k4_bytes) pl.ws_bytes = pl.k4_off() + align_up(pl.k4_bytes, 256);
@@ -643,7 +660,7 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
         p.splits = parts;
         p.ext_finish = parts > 1 ? 1 : 0;
         pl.grid = p.m_tiles * p.n_tiles * p.splits;
-        return finish_plan(pl);
+        return finish_plan(pl, true);
     }
     // M (128 accumulator rows) is the input-channel axis, so that dk rows are contiguous along the accumulator columns,
     // with the channels of four or two taps on top of one another where there are only 32 or 64 of them; or M is the
@@ -660,7 +677,7 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     p.mt = p.swap ? 1 : mt;
     if (pieces) { p.mt = 0; p.a_ch = p.swap ? d.o : d.c; p.b_ch = p.swap ? d.c : d.o; }
     use_tiling(pl, p.swap ? swapped : plain);
-    return finish_plan(pl);
+    return finish_plan(pl, true);
 }
 
 bool make_plan(const dcg_conv_desc& d, int kind, Plan& pl)

@@ -55,6 +55,21 @@ __device__ __forceinline__ unsigned long long global_ns()
 #define TC_DEBUG_BIT(bit) false
 #endif
 
+// Division of 0 <= n < 2^31 by a number that the host knows: a multiplication and a shift, where the integer division of a
+// run-time divisor is a subroutine of some seventy clocks.  m = floor(2^32 (2^s - d) / d) + 1 with s = ceil(log2 d) (Granlund
+// and Montgomery, "Division by invariant integers using multiplication").
+struct FastDiv {
+    uint32_t m, s, d;
+    FastDiv() = default;
+    __host__ explicit FastDiv(int divisor) : m(0), s(0), d((uint32_t)divisor)
+    {
+        while ((1u << s) < d) ++s;
+        m = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+    }
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s); }
+    __device__ __forceinline__ void divmod(int n, int& q, int& r) const { q = div(n); r = n - q * (int)d; }
+};
+
 struct Params {
     int N, H, W, C, KH, KW, O, Ho, Wo, sh, sw, pt, pl;
     int TW, TH, TN;               // pixel-tile extents (FWD/DX: the 128 rows; DK: the 32-pixel K step)
@@ -83,6 +98,9 @@ struct Params {
     float* out;                   // the output tensor
     float* scratch;               // splits > 1: partial tiles, [CTA][128 x bn], quad- or column-major
     EpilogueArgs ep;
+    // conv_tc_kernel: what a CTA divides by while nothing else runs on its SM (set_divisors)
+    FastDiv by_splits, by_n_tiles, by_m_count, by_tiles_w, by_tiles_h, by_kchunks, by_kw, by_sh, by_sw;
+    int pt_mod, pl_mod;           // pt % sh, pl % sw
 };
 
 // ---- PTX wrappers ----------------------------------------------------------------------------
@@ -265,6 +283,13 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t* r)
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld_32x32b_x4(uint32_t taddr, float4& v)
+{
+    uint32_t a, b, c, d;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(taddr) : "memory");
+    v = make_float4(__uint_as_float(a), __uint_as_float(b), __uint_as_float(c), __uint_as_float(d));
 }
 
 // 3xTF32: what the TF32 part of a value (its top 19 bits, which is what the tensor core reads) leaves over.

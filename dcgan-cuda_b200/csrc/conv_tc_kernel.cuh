@@ -92,23 +92,28 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
-    // ---- one-time setup (first: thread 0 and warp 1 are busy with it while everyone decodes) ---------
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < p.stages; ++s) {
-            mbar_init(full_bar + 8u * s, 1);
-            mbar_init(empty_bar + 8u * s, 1);
-            mbar_init(resid_bar + 8u * s, 128);
+    // ---- one-time setup -------------------------------------------------------------------------------
+    // With one CTA per SM nothing hides it: a CTA starts when its predecessor's has left.  So its steps are kept short - a lane
+    // per stage for the barriers, no division by run-time values - and everything that does not touch memory comes before the
+    // wait for the launch before (from a CTA's start to its first load it was 1.6 to 2.2 us: 64 -> 128 forward of 8 images 8.2 -> 7.3,
+    // of 64 images 16.2 -> 15.7 us).
+    if (warp == 0) {
+        if (lane < p.stages) {
+            mbar_init(full_bar + 8u * lane, 1);
+            mbar_init(empty_bar + 8u * lane, 1);
+            if (X3) mbar_init(resid_bar + 8u * lane, 128);
         }
-        mbar_init(tmem_full_bar, W);
-        if (X3) {
-            for (int i = 0; i < 2; ++i) {
-                mbar_init(promo_full_bar + 8u * i, 1);
-                mbar_init(promo_empty_bar + 8u * i, EPI);
-            }
+        if (X3 && lane < 2) {
+            mbar_init(promo_full_bar + 8u * lane, 1);
+            mbar_init(promo_empty_bar + 8u * lane, EPI);
+        }
+        if (lane == 0) {
+            mbar_init(tmem_full_bar, W);
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+        __syncwarp();
     }
     // 3xTF32 keeps the two small cross terms in an accumulator of their own: the tensor core rounds its
     // accumulator toward zero at every step, an error that grows with the number of steps and with the
@@ -130,54 +135,50 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // ---- decode this CTA's work item -------------------------------------------------------------
     // blockIdx.x = ((group * m_count + m) * n_tiles + n) * splits + split, where group is the parity
     // class (DX), the kernel tap (DK) or absent (FWD), and m a pixel tile (FWD/DX) or channel tile (DK).
-    int rem = blockIdx.x;
-    const int split = rem % p.splits; rem /= p.splits;
-    const int n_tile = rem % p.n_tiles; rem /= p.n_tiles;
-    int m_count;
-    if (MODE == MODE_DK) m_count = p.m_tiles;
-    else m_count = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int m_tile = rem % m_count;
-    const int group = rem / m_count;
+    int rem, split, n_tile, m_tile, group;
+    p.by_splits.divmod((int)blockIdx.x, rem, split);
+    p.by_n_tiles.divmod(rem, rem, n_tile);
+    p.by_m_count.divmod(rem, group, m_tile);
 
     // pixel-tile origin (FWD/DX)
     int j0 = 0, i0 = 0, n0 = 0;
     if (MODE != MODE_DK) {
-        j0 = (m_tile % p.tiles_w) * p.TW;
-        i0 = ((m_tile / p.tiles_w) % p.tiles_h) * p.TH;
-        n0 = (m_tile / (p.tiles_w * p.tiles_h)) * p.TN;
+        p.by_tiles_w.divmod(m_tile, n0, j0);
+        p.by_tiles_h.divmod(n0, n0, i0);
+        j0 *= p.TW; i0 *= p.TH; n0 *= p.TN;
     }
     // DX: parity class and its taps; DK: the kernel tap
     int ph = 0, pw = 0, rh = 0, rw = 0, eh = 0, ew = 0, taps_h = 1, taps_w = 1, tap_di = 0, tap_dj = 0;
     if (MODE == MODE_DX) {
         // classes in the order of their first taps, so those with the most taps (9, 6, 6, 4 of 5 x 5 / stride 2) start first and
         // a short one is what fills the last wave
-        rh = group / p.sw; rw = group % p.sw;
-        ph = (rh - p.pt % p.sh + p.sh) % p.sh; pw = (rw - p.pl % p.sw + p.sw) % p.sw;
-        eh = (ph + p.pt) / p.sh; ew = (pw + p.pl) / p.sw;
-        taps_h = rh < p.KH ? (p.KH - rh + p.sh - 1) / p.sh : 0;
-        taps_w = rw < p.KW ? (p.KW - rw + p.sw - 1) / p.sw : 0;
-    } else if (MODE == MODE_DK) {
-        if (p.narrow) { tap_di = 0; tap_dj = 0; }   // columns: 32 window slots per kernel row, all taps in one tile or two
-        else { tap_di = group * MT / p.KW; tap_dj = group * MT % p.KW; }   // (the first one)
+        p.by_sw.divmod(group, rh, rw);
+        ph = rh - p.pt_mod; if (ph < 0) ph += p.sh;
+        pw = rw - p.pl_mod; if (pw < 0) pw += p.sw;
+        eh = p.by_sh.div(ph + p.pt); ew = p.by_sw.div(pw + p.pl);
+        taps_h = rh < p.KH ? p.by_sh.div(p.KH - rh + p.sh - 1) : 0;
+        taps_w = rw < p.KW ? p.by_sw.div(p.KW - rw + p.sw - 1) : 0;
+    } else if (MODE == MODE_DK && !p.narrow) {   // (narrow: columns are 32 window slots per kernel row, all taps in one tile or two)
+        p.by_kw.divmod(group * MT, tap_di, tap_dj);   // (the first one)
     }
-    // K-stage range of this split
+    // K-stage range of this split: floor(stages * split / splits) on
     int total_stages;
     if (MODE == MODE_FWD) total_stages = p.narrow ? p.KH : p.KH * p.KW * p.kchunks;
     else if (MODE == MODE_DX) total_stages = taps_h * taps_w * p.kchunks;
     else total_stages = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int q0 = (int)((long long)total_stages * split / p.splits);
-    const int q1 = (int)((long long)total_stages * (split + 1) / p.splits);
-    const int nq = q1 - q0;
+    int each, over;
+    p.by_splits.divmod(total_stages, each, over);
+    const int q0 = each * split + p.by_splits.div(over * split);
+    const int nq = each * (split + 1) + p.by_splits.div(over * (split + 1)) - q0;
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d = *tmem_slot_ptr;
-    // Programmatic dependent launch: everything above (barriers, TMEM, descriptor prefetch) may run
-    // while the previous kernel of the stream is still draining; from here on its results are needed.
-    // The next kernel's CTAs may in turn be set up as soon as every CTA of this grid has got here.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // Programmatic dependent launch: everything up to pdl_enter() (barriers, TMEM, descriptor prefetch, the roles' own
+    // preparations) may run while the previous kernel of the stream is still draining; the producer and the epilogue
+    // warps call it before they touch memory.  The MMA warps only read what the producer has loaded.
+    // The next kernel's CTAs may in turn be set up as soon as every CTA of this grid has got there.
     if (threadIdx.x == 64) TC_TRACE(3073);
     TC_CTA_TRACE(1);
 #ifdef DCG_TC_TRACING
@@ -229,12 +230,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // counters of stage q0: FWD (chunk, tap, di, dj); DX (chunk, -, th, tw); DK (-, tile_n, tile_h, tile_w)
             int chunk = 0, tap = 0, di = 0, dj = 0;
             if (MODE == MODE_FWD && !p.narrow) {
-                tap = q0 / p.kchunks; chunk = q0 % p.kchunks; di = tap / p.KW; dj = tap % p.KW;
+                p.by_kchunks.divmod(q0, tap, chunk);
+                p.by_kw.divmod(tap, di, dj);
             } else if (MODE == MODE_DX) {
-                const int t = q0 / p.kchunks;
-                chunk = q0 % p.kchunks; di = t / taps_w; dj = t % taps_w;
+                p.by_kchunks.divmod(q0, di, chunk);
+                dj = di;
+                for (di = 0; dj >= taps_w && taps_w > 0; ++di) dj -= taps_w;
             } else if (MODE == MODE_DK) {
-                dj = q0 % p.tiles_w; di = (q0 / p.tiles_w) % p.tiles_h; tap = q0 / (p.tiles_w * p.tiles_h);
+                p.by_tiles_w.divmod(q0, tap, dj);
+                p.by_tiles_h.divmod(tap, tap, di);
             }
             const int wrap_dj = (MODE == MODE_FWD) ? p.KW : taps_w;
             auto advance = [&] {
@@ -249,11 +253,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int oh1 = 0, ow1 = 0, oh2 = 0, ow2 = 0, oh3 = 0, ow3 = 0;
             if (MT > 1) {
                 const int last = p.KH * p.KW - 1, t1 = min(group * MT + 1, last), t2 = min(group * MT + 2, last), t3 = min(group * MT + 3, last);
-                oh1 = t1 / p.KW - tap_di; ow1 = t1 % p.KW - tap_dj;
-                oh2 = t2 / p.KW - tap_di; ow2 = t2 % p.KW - tap_dj;
-                oh3 = t3 / p.KW - tap_di; ow3 = t3 % p.KW - tap_dj;
+                p.by_kw.divmod(t1, oh1, ow1); oh1 -= tap_di; ow1 -= tap_dj;
+                p.by_kw.divmod(t2, oh2, ow2); oh2 -= tap_di; ow2 -= tap_dj;
+                p.by_kw.divmod(t3, oh3, ow3); oh3 -= tap_di; ow3 -= tap_dj;
             }
             if (walker == 1) advance();
+            pdl_enter();
             for (int it = walker; it < nq; it += W) {
                 if (!mbar_wait_warp(empty_bar + 8u * s, phase ^ 1u, 0, it, wait_limit)) break;
                 const uint32_t fb = full_bar + 8u * s;
@@ -398,8 +403,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     }
     __syncwarp();
+    // how the epilogue threads walk the (row, quad) items of an unpartitioned tile: the first, and the step of EPI items
+    int item_r = 0, item_q = 0, step_r = 0, step_q = 0;
     if (warp >= 2) {
         // ===== epilogue, part 1 (warps 2..5; TMEM lane quadrant = warp % 4; thread = accumulator row) =====
+        const int qpr = p.bn >> 2;
+        item_r = (int)(threadIdx.x - 64) / qpr; item_q = (int)(threadIdx.x - 64) - item_r * qpr;
+        step_r = EPI / qpr; step_q = EPI - step_r * qpr;
+        pdl_enter();
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         // where does this accumulator row go?  (worked out while the main loop is still running)
@@ -527,9 +538,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const bool multi = S > 1;
     const bool finish_here = !p.ext_finish;   // else: partials only, a second kernel adds them
     const int qpr = p.bn >> 2;                // vector path: 16-byte column quads per row,
-    const int QPO = (qpr + S - 1) / S;        //   quads per share
+    const int QPO = p.by_splits.div(qpr + S - 1);   //   quads per share
     const int QS = BM + 1;                    // shared-memory quad pitch in 16-byte units (odd: lanes = quads hit distinct banks)
-    const int CL = (p.bn + S - 1) / S;        // scalar path: columns per share
+    const int CL = p.by_splits.div(p.bn + S - 1);   // scalar path: columns per share
+    // Vector path: a partition's own share stays in its TMEM, where the second phase reads it again (with two partitions half of
+    // what went through L2: 128 -> 256 forward of 64 images 16.9 -> 16.1 us, with the shorter set-up).  3xTF32 has part of it in
+    // registers of other threads.
+    const bool keep_own = vec && multi && finish_here && !X3;
+    const int own_q0 = part * QPO, own_q = keep_own ? QPO : 0;
     float* my_scratch = p.scratch + (size_t)blockIdx.x * BM * p.bn;
     const float* tile_scratch = p.scratch + (size_t)(blockIdx.x - part) * BM * p.bn;
     if (threadIdx.x == 64) TC_TRACE(3000);
@@ -576,7 +592,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     float4* d4 = reinterpret_cast<float4*>(my_scratch) + (size_t)(c0 >> 2) * BM + row;
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
-                        if (q < 4 || full)
+                        if ((q < 4 || full) && (unsigned)((c0 >> 2) + q - own_q0) >= (unsigned)own_q)
                             __stcg(d4 + q * BM, make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
                                                             __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3])));
                 } else {
@@ -617,13 +633,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int Qm = min(QPO, qpr - part * QPO);
             const bool by_row = multi || p.planes;               // thread = row (else: lanes walk the quads of a row)
             // by_row: the G threads of a row (tid_e, tid_e + 128, ...) take the quads in turn
-            const int my_row = tid_e & (BM - 1), my_half = tid_e >> 7;
+            const int my_row = (warp & 3) * 32 + lane, my_half = tid_e >> 7;   // (the rows of this warp's TMEM lanes)
             const int row_quads = multi ? Qm : qpr;              // by_row: quads of this row's share
             const int per_thread = by_row ? (row_quads > my_half ? (row_quads - my_half + G - 1) / G : 0)
                                           : (BM * qpr + EPI - 1) / EPI;   // single: 128 * qpr items over all threads
             const int quad0 = ch0 >> 2;                          // planes: global index of this tile's first quad
-            const int step_r = EPI / qpr, step_q = EPI % qpr;    // single: how (row, quad) moves when the item index grows by EPI
-            int rr = tid_e / qpr, q = tid_e % qpr;
+            int rr = item_r, q = item_q;
             const long long my_ro = s_rowoff[my_row];
             const float4* red4 = reinterpret_cast<const float4*>(red);
             const float4* ts4 = reinterpret_cast<const float4*>(tile_scratch);
@@ -643,10 +658,29 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                              : my_ro + cq[u];
                         src[u] = (multi ? ts4 + (size_t)qd * BM : red4 + qd * QS) + my_row;
                     }
+                    if (!X3 && multi) {   // this partition's own products first, the others' behind them in partition order
+                        const uint32_t at = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[u] = multi ? __ldcg(src[u]) : *src[u];
+                        for (int u = 0; u < 4; ++u) tmem_ld_32x32b_x4(at + (uint32_t)cq[u], acc[u]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (W == 2 && nq > 1) {   // the odd stages' accumulator
+                            float4 odd[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) tmem_ld_32x32b_x4(at + (uint32_t)(p.bn + cq[u]), odd[u]);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                acc[u].x = __fadd_rn(acc[u].x, odd[u].x); acc[u].y = __fadd_rn(acc[u].y, odd[u].y);
+                                acc[u].z = __fadd_rn(acc[u].z, odd[u].z); acc[u].w = __fadd_rn(acc[u].w, odd[u].w);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) acc[u] = multi ? __ldcg(src[u]) : *src[u];
+                    }
 #pragma unroll 2
-                    for (int sidx = 1; sidx < S; ++sidx) {   // two partitions' loads in flight; the adds keep partition order
+                    for (int i = 1; i < S; ++i) {   // two partitions' loads in flight
+                        const int sidx = X3 || i > part ? i : i - 1;
                         float4 v[4];
 #pragma unroll
                         for (int u = 0; u < 4; ++u) v[u] = __ldcg(src[u] + (size_t)sidx * BM * qpr);
