@@ -496,7 +496,7 @@ namespace {
 // On the tensor path a wide dense layer (the generator's 100 -> 8192 projection) is a 1x1 convolution over
 // a 1x1 image: x [m,1,1,n], k [1,1,n,p], bias in the epilogue; K that is not a multiple of 32 is zero-filled by
 // TMA.  With act_out the activation node that follows is part of the same launch (nd->out1 still receives the
-// pre-activation).  Returns 1 if the shape or the precision keeps the node off the tensor path.
+// pre-activation, unless it is flagged dead).  Returns 1 if the shape or the precision keeps the node off the tensor path.
 int run_dense_on_tensor_path(dcg_context* ctx, const dcg_node* nd, int act, float alpha, float* act_out)
 {
     const size_t m = nd->len1, n = nd->len2, pp = nd->len3;
@@ -520,7 +520,7 @@ int run_dense_on_tensor_path(dcg_context* ctx, const dcg_node* nd, int act, floa
     if (act_out) {
         ep.act = act;
         ep.alpha = alpha;
-        ep.pre_act = nd->out1;
+        if (!(nd->flags & DCG_NODE_OUT_DEAD)) ep.pre_act = nd->out1;
         out = act_out;
     }
     ProfScope scope(act_out ? ctx : nullptr, "mat_mul_add", 0.0);   // the fused form does not pass through dcg_run_node
@@ -633,7 +633,7 @@ int matmul_act(const float* a, const float* b, const float* bias, float* out, si
                float* act_out, cudaStream_t stream);
 int matmul_tn_sums(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, float* sums, cudaStream_t stream);
 int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const float* gate,
-                    float* gated_out, int gate_act, float gate_alpha, cudaStream_t stream);
+                    float* gated_out, int gate_act, float gate_alpha, bool out_dead, cudaStream_t stream);
 }  // namespace dcg
 
 namespace {
@@ -773,7 +773,8 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
                 disjoint({b.out1, b.len1}, {{a.in1, a.len1 * a.len2}, {a.in2, a.len2 * a.len3}, {a.out1, b.len1}})) {
                 ProfScope scope(ctx, "mat_tmat_mul_gated", 0.0);
                 const int st = dcg::matmul_nt_gated(a.in1, a.in2, a.out1, a.len1, a.len2, a.len3, b.in1, b.out1, gact,
-                                                    b.type == DCG_OP_LEAKY_RELU_GRAD ? b.cons1 : 0.f, ctx->stream);
+                                                    b.type == DCG_OP_LEAKY_RELU_GRAD ? b.cons1 : 0.f,
+                                                    (a.flags & DCG_NODE_OUT_DEAD) != 0, ctx->stream);
                 if (st) return st;
                 i += 2;
                 continue;

@@ -49,6 +49,7 @@ struct DenseEpilogue {
     float* sums;     // TA only: column sums of B, as dcg_colsum adds them, by the first `sum_rows` rows of blocks
     ColsumTile sum;
     int sum_rows;
+    bool out_dead;   // `out` need not be written (gemm_outer_kernel leaves it out)
 };
 
 // out[m,p] = A[m,n] B[n,p]: TM x TN outputs per thread, TX x TY threads per block, STAGES stages of KC reduction steps
@@ -210,7 +211,7 @@ gemm_outer_kernel(const float* __restrict__ a, const float* __restrict__ b, floa
             const float4 w = __ldg(reinterpret_cast<const float4*>(e.bias) + c4);
             v[0] = __fadd_rn(v[0], w.x); v[1] = __fadd_rn(v[1], w.y); v[2] = __fadd_rn(v[2], w.z); v[3] = __fadd_rn(v[3], w.w);
         }
-        reinterpret_cast<float4*>(out)[i] = make_float4(v[0], v[1], v[2], v[3]);
+        if (!e.out_dead) reinterpret_cast<float4*>(out)[i] = make_float4(v[0], v[1], v[2], v[3]);
         if (e.out2) {
             if (e.gate) {
                 const float4 g = __ldg(reinterpret_cast<const float4*>(e.gate) + i);
@@ -398,12 +399,15 @@ int matmul_act(const float* a, const float* b, const float* bias, float* out, si
     return matmul_nn(a, b, out, m, n, p, DenseEpilogue{bias, nullptr, act_out, act, alpha}, stream);
 }
 
-// dcg_matmul_nt followed by dcg_act_grad(gate, out) -> gated_out as one launch (node fusion of the backend).
+// dcg_matmul_nt followed by dcg_act_grad(gate, out) -> gated_out as one launch (node fusion of the backend).  `out_dead`: nobody
+// reads `out`.
 int matmul_nt_gated(const float* a, const float* b, float* out, size_t m, size_t n, size_t p, const float* gate,
-                    float* gated_out, int gate_act, float gate_alpha, cudaStream_t stream)
+                    float* gated_out, int gate_act, float gate_alpha, bool out_dead, cudaStream_t stream)
 {
     DCG_CHECK_ARG(a && b && out && gate && gated_out && m > 0 && n > 0 && p > 0, "matmul_nt_gated: bad arguments");
-    return launch_ordered<false, true>(a, b, out, m, n, p, DenseEpilogue{nullptr, gate, gated_out, gate_act, gate_alpha}, stream);
+    DenseEpilogue e{nullptr, gate, gated_out, gate_act, gate_alpha};
+    e.out_dead = out_dead;
+    return launch_ordered<false, true>(a, b, out, m, n, p, e, stream);
 }
 
 // dcg_matmul_tn and the column sums of its right operand as one launch (node fusion of the backend): the weight and the bias

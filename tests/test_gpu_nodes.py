@@ -158,6 +158,29 @@ def test_dead_intermediates_are_skipped_only_when_flagged(pkg, dev):
     ctx.close()
 
 
+def test_dead_dense_intermediates(pkg, dev):
+    """A flagged pre-activation of a wide dense layer, and a flagged product under an activation gradient, are not written;
+    what reads them comes out as without the flag."""
+    N = pkg.nodes
+    m, n, p = 32, 100, 1024
+    x, w, bias = (_t(seeded(s, 916 + i) * np.float32(0.1), dev) for i, s in enumerate([(m, n), (n, p), (p,)]))
+    col, row = _t(seeded((m, 1), 914), dev), _t(seeded((p, 1), 915), dev)
+    outs = []
+    for dead in (0, pkg._lib.NODE_OUT_DEAD):
+        z, a, prod, gated = (torch.full((m, p), -7.0, device=dev) for _ in range(4))
+        nodes = [N.op_mat_mul_add(x, w, bias, z, m, n, p), N.op_relu_leaky(z, a, m * p, 0.2),
+                 N.op_mat_tmat_mul(col, row, prod, m, 1, p), N.op_leaky_relu_grad(a, prod, gated, 0.2, m * p)]
+        nodes[0].flags = nodes[2].flags = dead
+        ctx = pkg.Context(pkg.PREC_TF32)
+        ctx.run(nodes, fuse=True)
+        torch.cuda.synchronize()
+        assert ctx.launch_count() == 2
+        assert bool((z == -7.0).all()) == bool((prod == -7.0).all()) == bool(dead)
+        outs.append((a.cpu().numpy(), gated.cpu().numpy()))
+        ctx.close()
+    assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
+
+
 def test_adam_triples_fuse_into_one_launch(pkg, dev, orc):
     """AdamOptimizer::minimize lowers each variable to moment_update, moment_update(sq), adam_update
     (src/api/adam-optimizer.cu:24-59); a run of such triples becomes one multi-tensor launch."""
