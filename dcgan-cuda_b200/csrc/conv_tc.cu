@@ -624,6 +624,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     pl.smem = (size_t)units * kCfUnit + fixed;
     p.skip_stage = -1;
     p.wait_cycles = kWaitCycles;
+    set_divisors(p, false);
     pl.partial_bytes = 0;
     pl.ws_bytes = 0;
     return true;
@@ -962,6 +963,7 @@ bool plan_dx3(const dcg_conv_desc& d, Plan& pl, Dx3Args& g)
     g.lo = lo;
     g.tiles_per_img = (d.h + 2 * R - 1) / (2 * R);
     g.tiles = d.n * g.tiles_per_img;
+    g.by_tiles_per_img = FastDiv(g.tiles_per_img);
     pl.grid = g.tiles < sm_count() ? g.tiles : sm_count();
     pl.smem = 1024 + (size_t)p.kchunks * 128 * BK * 4 + (size_t)kDx3Stages * A_STAGE_BYTES +
               (size_t)d.kh * d.kw * kDx3Rows * 32 * 16 + 16 * kDx3Stages + 64;

@@ -144,15 +144,18 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int ncls = t.ncls, nwin = t.nwin;
     const uint32_t b_bytes = (uint32_t)p.bn * BK * 4;
 
-    if (threadIdx.x == 0) {
-        for (int u = 0; u < kCfBars; ++u) {
-            mbar_init(full_bar + 8u * u, 1);
-            mbar_init(empty_bar + 8u * u, 1);
+    if (warp == 0) {   // a lane per barrier
+        if (lane < kCfBars) {
+            mbar_init(full_bar + 8u * lane, 1);
+            mbar_init(empty_bar + 8u * lane, 1);
         }
-        for (int c = 0; c < 4; ++c) mbar_init(cls_bar + 8u * c, 1);
+        if (lane < 4) mbar_init(cls_bar + 8u * lane, 1);
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+        __syncwarp();
     }
     int tmem_cols = 32;
     while (tmem_cols < ncls * p.bn) tmem_cols <<= 1;
@@ -161,10 +164,11 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // blockIdx.x = pixel tile * n_tiles + channel tile
-    const int n_tile = blockIdx.x % p.n_tiles, m_tile = blockIdx.x / p.n_tiles;
-    const int j0 = (m_tile % p.tiles_w) * p.TW;
-    const int i0 = ((m_tile / p.tiles_w) % p.tiles_h) * p.TH;
-    const int n0 = (m_tile / (p.tiles_w * p.tiles_h)) * p.TN;
+    int n_tile, m_tile, j0, i0, n0;
+    p.by_n_tiles.divmod((int)blockIdx.x, m_tile, n_tile);
+    p.by_tiles_w.divmod(m_tile, n0, j0);
+    p.by_tiles_h.divmod(n0, n0, i0);
+    j0 *= p.TW; i0 *= p.TH; n0 *= p.TN;
     const int ch0 = n_tile * p.bn;
     const int ncols_valid = min(p.bn, p.C - ch0);
 
@@ -172,8 +176,6 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d = *tmem_slot_ptr;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == 0 || warp == 2 + kCfEpi / 32) {
         // ===== TMA producers: for every table entry, for every channel chunk: the window, then its weight tiles =====
@@ -188,6 +190,7 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             used |= ((1u << (end - first)) - 1u) << first;
         };
         bool alive = true;
+        pdl_enter();
         for (int w = 0; w < nwin && alive; ++w) {
             const CfWin& wn = t.win[w];
             const int aj = j0 + wn.sx, ai = i0 + wn.sy, np = wn.n, nu = wn.units;
@@ -300,6 +303,7 @@ conv_dxf_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const float* patch1 = reinterpret_cast<const float*>(patch);
         // 16-byte stores need whole column quads in every row; else element by element
         const bool vec = (p.C & 3) == 0 && (ncols_valid & 3) == 0;
+        pdl_enter();
         for (int ci = 0; ci < ncls; ++ci) {
             const int cls = t.order[ci];
             const int ph = cls / p.sw, pw = cls % p.sw;
