@@ -250,8 +250,9 @@ int decode_conv(const dcg_node* nd, ConvCall& cc)
 
 int run_conv(dcg_context* ctx, const ConvCall& cc, const dcg_epilogue* ep)
 {
-    const size_t need = dcg_conv_workspace_bytes(&cc.d, cc.kind, ctx->precision);
-    const bool fixed = ctx->ws && !ctx->owns_ws;   // the caller's scratch: it may be too small for what can do without
+    const bool fixed = ctx->ws && !ctx->owns_ws;   // the caller's scratch: it may be too small for what can do without, or with less
+    const size_t need = fixed && ctx->precision != DCG_PREC_FP32 ? conv_tc_workspace_least(cc.d, cc.kind, ctx->precision == DCG_PREC_3XTF32)
+                                                                 : dcg_conv_workspace_bytes(&cc.d, cc.kind, ctx->precision);
     int st = fixed && conv_scratch_optional(cc.d, cc.kind) ? DCG_OK : ensure_workspace(ctx, need);
     if (st) return st;
     char name[96];

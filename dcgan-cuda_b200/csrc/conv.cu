@@ -47,7 +47,7 @@ bool conv_scratch_optional(const dcg_conv_desc& d, int kind) { return (kind != k
 static bool on_tensor_path(const dcg_conv_desc& d, int kind, bool x3, const void* ws, size_t ws_bytes)
 {
     if (!conv_tc_supported(d, kind, x3)) return false;
-    return !conv_scratch_optional(d, kind) || conv_tc_workspace(d, kind, x3) <= (ws ? ws_bytes : 0);
+    return !conv_scratch_optional(d, kind) || conv_tc_workspace_least(d, kind, x3) <= (ws ? ws_bytes : 0);
 }
 
 }  // namespace dcg

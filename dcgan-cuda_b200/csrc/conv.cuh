@@ -21,6 +21,8 @@ int conv_dk_generic(const dcg_conv_desc& d, const float* x, const float* dy, flo
 // tensor path takes the shape; *_workspace its scratch need in bytes.
 bool conv_tc_supported(const dcg_conv_desc& d, int kind, bool x3 = false);
 size_t conv_tc_workspace(const dcg_conv_desc& d, int kind, bool x3 = false);
+// ... and the least a call can do with (a kernel gradient has a form that takes less scratch).
+size_t conv_tc_workspace_least(const dcg_conv_desc& d, int kind, bool x3);
 int conv_tc_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y,
                 const EpilogueArgs& ep, void* ws, size_t ws_bytes, cudaStream_t stream, bool x3 = false);
 int conv_tc_dx(const dcg_conv_desc& d, const float* dy, const float* k, float* dx,

@@ -266,11 +266,17 @@ constexpr int kMaxSharedWidth = 160;
 // Channel counts between the powers of two get one tile instead of two (96 -> 160 forward of 13 images of 51 x 75: 35 for 59).
 // `m_count`: tiles along the other axis, times classes or taps; `store_cost`: clocks per column of an unpartitioned epilogue;
 // `loads`: TMA loads per stage, of which two are in the figures above; `b_pieces`: B comes in loads of 32 columns.
+// `partials_bytes` (kernel gradients): partial tiles that a second launch adds may take so much scratch.  A tile then has as many
+// partitions as fill the SMs, not the eight CTAs of a cluster: the launch costs about 4 us, which long reductions over few tiles
+// earn many times over (1 x 1, 8 -> 16 channels, 20 images of 64 x 64: 46 us in one cluster of eight, 10.4 in 148 partitions;
+// 3 x 3, 96 -> 160, 13 images of 75 x 51: 49 and 30; 64 -> 128 of 64 images, 3xTF32: 53 and 42).
 struct Tiling {
     int bn, n_tiles, splits, grid;
+    bool second_launch;
     double cost;
 };
-Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost, int loads = 2, bool b_pieces = false)
+Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost, int loads = 2, bool b_pieces = false,
+                     size_t partials_bytes = 0)
 {
     static const int forced = env_int("DCG_TC_BN");
     const int sms = sm_count();
@@ -289,7 +295,18 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
         const double loop = 1200.0 + (max_stages + t.splits - 1) / t.splits * (stage + 20.0 * (loads - 2 + (b_pieces ? (t.bn + 31) / 32 - 1 : 0)));
         const double epilogue = t.bn * (t.splits > 1 ? 55.0 : (double)store_cost);
         t.cost = t.bn <= kMaxSharedWidth && !t_plan_x3 ? waves * loop + epilogue : waves * (loop + epilogue);
+        t.second_launch = false;
         if (best.grid == 0 || t.cost < best.cost) best = t;
+        // the same tiles with a second launch
+        const int tiles = m_count * t.n_tiles;
+        t.splits = std::min(sms / tiles, min_stages / 4);
+        t.grid = tiles * t.splits;
+        const size_t bytes = (size_t)t.grid * BM * t.bn * sizeof(float);
+        if (t.splits <= 1 || t.grid <= best.grid || bytes > partials_bytes) continue;
+        t.second_launch = true;
+        t.cost = 1200.0 + (max_stages + t.splits - 1) / t.splits * (stage + 20.0 * (loads - 2 + (b_pieces ? (t.bn + 31) / 32 - 1 : 0))) + t.bn * 18.0 +
+                 6500.0 + bytes / 2500.0;
+        if (t.cost < best.cost) best = t;
     }
     return best;
 }
@@ -406,6 +423,7 @@ void base_params(Params& p, const dcg_conv_desc& d)
 void use_tiling(Plan& pl, const Tiling& t)
 {
     pl.p.bn = t.bn; pl.p.n_tiles = t.n_tiles; pl.p.splits = t.splits;
+    pl.p.ext_finish = t.second_launch;
     pl.grid = t.grid;
 }
 
@@ -630,7 +648,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     return true;
 }
 
-bool plan_dk(const dcg_conv_desc& d, Plan& pl)
+bool plan_dk(const dcg_conv_desc& d, Plan& pl, size_t ws_bytes)
 {
     const bool narrow = narrow_ok(d, 4e5);
     if (!narrow && (!pieces_ok(d, d.c) || !pieces_ok(d, d.o) || d.stride_h > 8 || d.stride_w > 8)) return false;
@@ -671,8 +689,8 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     const int rows_c = (d.c + BM - 1) / BM, rows_o = (d.o + BM - 1) / BM;
     static const int roles = env_int("DCG_TC_ROLES");
     auto row_pieces = [&](int ch) { return pieces ? (ch < BM ? (ch + 31) / 32 : BM / 32) - 1 : 0; };
-    const Tiling plain = choose_tiling((taps + mt - 1) / mt * rows_c, d.o, 32, stages, stages, 20, 1 + mt + row_pieces(d.c), pieces);
-    const Tiling swapped = choose_tiling(taps * rows_o, d.c, 32, stages, stages, 30, 2 + row_pieces(d.o), pieces);
+    const Tiling plain = choose_tiling((taps + mt - 1) / mt * rows_c, d.o, 32, stages, stages, 20, 1 + mt + row_pieces(d.c), pieces, ws_bytes);
+    const Tiling swapped = choose_tiling(taps * rows_o, d.c, 32, stages, stages, 30, 2 + row_pieces(d.o), pieces, ws_bytes);
     p.swap = roles ? roles == 2 : swapped.cost < plain.cost;
     p.m_tiles = p.swap ? rows_o : rows_c;
     p.mt = p.swap ? 1 : mt;
@@ -681,12 +699,13 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl)
     return finish_plan(pl, true);
 }
 
-bool make_plan(const dcg_conv_desc& d, int kind, Plan& pl)
+// `ws_bytes`: scratch that there is, as far as a plan may do with less.
+bool make_plan(const dcg_conv_desc& d, int kind, Plan& pl, size_t ws_bytes = (size_t)-1)
 {
     switch (kind) {
     case kConvFwd: return plan_fwd(d, pl);
     case kConvDx: return plan_dx(d, pl);
-    case kConvDk: return plan_dk(d, pl);
+    case kConvDk: return plan_dk(d, pl, ws_bytes);
     default: return false;
     }
 }
@@ -771,7 +790,12 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, c
     (void)channels;
     const int st = launch_grid<MODE>(ma, mb, p, pl.grid, pl.smem, stream);
     if (st) return st;
-    if (p.ext_finish) {
+    if (p.ext_finish && !p.narrow) {
+        const dim3 fgrid((unsigned)(pl.grid / p.splits), (unsigned)(BM / kFinishRows * (p.bn / kFinishCols)));
+        launch_pdl(p.swap ? dk_finish_kernel<true> : dk_finish_kernel<false>, fgrid, 256, 0, stream, p.scratch, out, p.splits, p.bn, p.n_tiles,
+                   p.m_tiles, p.mt > 1 ? p.mt : 1, p.KH * p.KW, p.C, p.O);
+        DCG_LAUNCH_CHECK("dk_finish_kernel");
+    } else if (p.ext_finish) {
         const dim3 fgrid((unsigned)(p.bn * p.n_tiles), (unsigned)((p.O + 31) / 32));
         launch_pdl(dk_narrow_finish_kernel, fgrid, 256, 0, stream, p.scratch, out, p.splits, p.bn, p.n_tiles, p.KH, p.KW, p.C, p.O);
         DCG_LAUNCH_CHECK("dk_narrow_finish_kernel");
@@ -1135,7 +1159,7 @@ int build_dx(const dcg_conv_desc& d, const float* dy, const float* k, void* ws, 
 int build_dk(const dcg_conv_desc& d, const float* x, const float* dy, void* ws, size_t ws_bytes, Prepared& pr)
 {
     Plan& pl = pr.pl;
-    if (!plan_dk(d, pl)) return fail(DCG_ERR_UNSUPPORTED, "conv dk: shape not supported by the tensor path");
+    if (!plan_dk(d, pl, ws ? ws_bytes : 0)) return fail(DCG_ERR_UNSUPPORTED, "conv dk: shape not supported by the tensor path");
     const Params& p = pl.p;
     CUtensorMap mx, mdy;
     int st;
@@ -1206,7 +1230,7 @@ struct QueryKey {
 };
 struct QueryAnswer {
     bool supported;
-    size_t ws_bytes;
+    size_t ws_bytes, ws_least;   // what the best plan takes, and what the call can do with
 };
 std::mutex g_query_mutex;
 std::unordered_map<QueryKey, QueryAnswer, BytesHash<QueryKey>, BytesEqual<QueryKey>> g_query;
@@ -1224,8 +1248,10 @@ QueryAnswer query(const dcg_conv_desc& d, int kind, bool x3)
     }
     PlanX3 scope(x3);
     Plan pl;
-    QueryAnswer a{make_plan(d, kind, pl), 0};
-    if (a.supported) a.ws_bytes = pl.ws_bytes;
+    QueryAnswer a{make_plan(d, kind, pl), 0, 0};
+    if (a.supported) a.ws_bytes = a.ws_least = pl.ws_bytes;
+    Plan least;
+    if (a.supported && kind == kConvDk && make_plan(d, kind, least, 0)) a.ws_least = least.ws_bytes;
     std::lock_guard<std::mutex> lock(g_query_mutex);
     if (g_query.size() >= 4096) g_query.clear();
     g_query[key] = a;
@@ -1237,6 +1263,7 @@ QueryAnswer query(const dcg_conv_desc& d, int kind, bool x3)
 bool conv_tc_supported(const dcg_conv_desc& d, int kind, bool x3) { return query(d, kind, x3).supported; }
 
 size_t conv_tc_workspace(const dcg_conv_desc& d, int kind, bool x3) { return query(d, kind, x3).ws_bytes; }
+size_t conv_tc_workspace_least(const dcg_conv_desc& d, int kind, bool x3) { return query(d, kind, x3).ws_least; }
 
 int conv_tc_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y, const EpilogueArgs& ep,
                 void* ws, size_t ws_bytes, cudaStream_t stream, bool x3)

@@ -191,5 +191,55 @@ col2im_kernel(const float4* __restrict__ ycol, float* __restrict__ out, int N, i
     }
 }
 
+// Adds the partial tiles of a kernel gradient whose K partitions are no cluster: a block per 32 rows x 8 columns of a tile, whose
+// eight warps take the partitions in turn, so that few tiles of many partitions are still read by the whole chip (a block per 32
+// columns that walks the partitions one after the other took 45 us for a 1 x 1 kernel in 148 of them); then the warps' sums in
+// order.  SWAP false: the rows of a tile are input channels (of `mt` taps on top of one another), its columns output channels,
+// the partials lie quad by quad (lane = row); true: the rows are output channels, along which dk is contiguous as the partials are.
+constexpr int kFinishRows = 32, kFinishCols = 8;
+template <bool SWAP>
+__global__ void __launch_bounds__(256)
+dk_finish_kernel(const float* __restrict__ partial, float* __restrict__ dk, int splits, int bn, int n_tiles, int m_tiles, int mt, int taps, int C, int O)
+{
+    pdl_enter();
+    const int tile = blockIdx.x, n_tile = tile % n_tiles, m = tile / n_tiles, m_tile = m % m_tiles, group = m / m_tiles;
+    const int row0 = (blockIdx.y & (BM / kFinishRows - 1)) * kFinishRows, col0 = blockIdx.y / (BM / kFinishRows) * kFinishCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t step = (size_t)BM * bn;   // floats of a partial tile
+    const float* src = partial + (size_t)tile * splits * step;
+    __shared__ float sums[8][kFinishRows][kFinishCols + 1];
+    float acc[kFinishCols];
+#pragma unroll
+    for (int u = 0; u < kFinishCols; ++u) acc[u] = 0.f;
+#pragma unroll 4
+    for (int s = warp; s < splits; s += 8) {
+        const float* at = src + s * step;
+        if constexpr (SWAP) {
+#pragma unroll
+            for (int u = 0; u < kFinishCols; ++u) acc[u] += __ldcg(at + (size_t)(col0 + u) * BM + row0 + lane);
+        } else {
+            const float4* at4 = reinterpret_cast<const float4*>(at) + (size_t)(col0 >> 2) * BM + row0 + lane;
+            const float4 v = __ldcg(at4), w = __ldcg(at4 + BM);
+            acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+            acc[4] += w.x; acc[5] += w.y; acc[6] += w.z; acc[7] += w.w;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kFinishCols; ++u) sums[warp][lane][u] = acc[u];
+    __syncthreads();
+    const int row = SWAP ? threadIdx.x & 31 : threadIdx.x >> 3, col = SWAP ? threadIdx.x >> 5 : threadIdx.x & 7;
+    float r = sums[0][row][col];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) r += sums[w][row][col];
+    const int ch = n_tile * bn + col0 + col;   // channel along the columns
+    if constexpr (SWAP) {
+        const int o = m_tile * BM + row0 + row;
+        if (o < O && ch < C) dk[((size_t)group * C + ch) * O + o] = r;
+    } else {
+        const int rows_per_tap = BM / mt, t = (row0 + row) / rows_per_tap, c = m_tile * BM + row0 + row - t * rows_per_tap, tap = group * mt + t;
+        if (c < C && tap < taps && ch < O) dk[((size_t)tap * C + c) * O + ch] = r;
+    }
+}
+
 }  // namespace
 }  // namespace dcg

@@ -548,6 +548,36 @@ def test_k_partition_counts(pkg, dev, batch):
         assert torch.equal(u, v), name
 
 
+# kernel gradients of few tiles, whose partitions a second launch adds: one tap and nine, four taps to a tile, the channel
+# roles swapped, ragged channels, a last partition tile that is nearly empty
+@pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", [(4, 60, 60, 64, 1, 128, 1), (8, 40, 40, 32, 3, 64, 1), (6, 64, 64, 256, 1, 64, 1), (16, 50, 50, 40, 3, 44, 1),
+                                   (20, 64, 64, 8, 1, 16, 1), (13, 75, 51, 96, 3, 160, 1), (5, 61, 47, 132, 1, 260, 2)])
+def test_kernel_gradients_of_many_partitions(pkg, dev, shape, prec_name):
+    import ctypes
+    F, L = pkg.functional, pkg.lib
+    N, H, W, C, K, O, s = shape
+    prec = getattr(pkg, PRECS[prec_name])
+    x, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((57, (N, H, W, C)), (58, (N, -(-H // s), -(-W // s), O))))
+    pt, pl = (max((-(-e // s) - 1) * s + K - e, 0) for e in (H, W))
+    xp = torch.nn.functional.pad(x.double().permute(0, 3, 1, 2), (pl // 2, pl - pl // 2, pt // 2, pt - pt // 2))
+    ref = torch.nn.grad.conv2d_weight(xp, (O, C, K, K), dy.double().permute(0, 3, 1, 2), stride=s).permute(2, 3, 1, 0)
+    # operands of 11 bits: 2^-10 of each product at most, which average out; else the rounding of a fp32 sum
+    tol = TF32_TOL if prec_name == "tf32" else 1e-5
+    got = [F.conv2d_dk(x, dy, (K, K), (s, s), precision=prec) for _ in range(2)]
+    assert torch.equal(*got)
+    # with less scratch than asked for: fewer partitions
+    d = F.conv_desc(x.shape, (K, K, C, O), (s, s), None, None)
+    need = L.dcg_conv_workspace_bytes(ctypes.byref(d), pkg._lib.KIND_DK, prec)
+    small, less = torch.empty(need - 256, dtype=torch.uint8, device=dev), torch.zeros_like(got[0])
+    assert L.dcg_conv2d_dk(ctypes.byref(d), x.data_ptr(), dy.data_ptr(), less.data_ptr(), prec, small.data_ptr(), small.numel(),
+                           torch.cuda.current_stream().cuda_stream) == 0, L.dcg_last_error()
+    torch.cuda.synchronize()
+    assert L.dcg_device_status() == 0
+    for dk in (got[0], less):
+        assert (dk - ref).abs().max().item() <= tol * ref.abs().max().item()
+
+
 def test_deterministic(pkg, dev):
     """Two runs of every operator give identical bits (fixed-order split-K reduction)."""
     F = pkg.functional
