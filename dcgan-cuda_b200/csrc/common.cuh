@@ -138,6 +138,49 @@ __device__ __forceinline__ float act_grad_apply(float gate, float dout, int act,
     }
 }
 
+// The same for values that a thread holds together.  The choice is made once for all of them; within an unrolled loop it was a
+// chain of branches around the long forms for every value.
+template <int N, typename F>
+__device__ __forceinline__ void each_value(float4 (&v)[N], F f)
+{
+#pragma unroll
+    for (int u = 0; u < N; ++u) { v[u].x = f(v[u].x); v[u].y = f(v[u].y); v[u].z = f(v[u].z); v[u].w = f(v[u].w); }
+}
+template <int N, typename F>
+__device__ __forceinline__ void each_value(float (&v)[N], F f)
+{
+#pragma unroll
+    for (int u = 0; u < N; ++u) v[u] = f(v[u]);
+}
+template <int N, typename F>
+__device__ __forceinline__ void each_pair(float4 (&v)[N], const float4 (&w)[N], F f)
+{
+#pragma unroll
+    for (int u = 0; u < N; ++u) { v[u].x = f(v[u].x, w[u].x); v[u].y = f(v[u].y, w[u].y); v[u].z = f(v[u].z, w[u].z); v[u].w = f(v[u].w, w[u].w); }
+}
+template <int N, typename F>
+__device__ __forceinline__ void each_pair(float (&v)[N], const float (&w)[N], F f)
+{
+#pragma unroll
+    for (int u = 0; u < N; ++u) v[u] = f(v[u], w[u]);
+}
+template <typename V>
+__device__ __forceinline__ void act_apply_all(V& v, int act, float alpha)
+{
+    if (act == DCG_ACT_LEAKY) each_value(v, [&](float a) { return act_apply(a, DCG_ACT_LEAKY, alpha); });
+    else if (act == DCG_ACT_RELU) each_value(v, [&](float a) { return act_apply(a, DCG_ACT_RELU, alpha); });
+    else if (act == DCG_ACT_TANH) each_value(v, [&](float a) { return act_apply(a, DCG_ACT_TANH, alpha); });
+    else if (act == DCG_ACT_SIGMOID) each_value(v, [&](float a) { return act_apply(a, DCG_ACT_SIGMOID, alpha); });
+}
+template <typename V>
+__device__ __forceinline__ void act_grad_apply_all(V& v, const V& gate, int act, float alpha)
+{
+    if (act == DCG_ACT_LEAKY) each_pair(v, gate, [&](float a, float g) { return act_grad_apply(g, a, DCG_ACT_LEAKY, alpha); });
+    else if (act == DCG_ACT_RELU) each_pair(v, gate, [&](float a, float g) { return act_grad_apply(g, a, DCG_ACT_RELU, alpha); });
+    else if (act == DCG_ACT_TANH) each_pair(v, gate, [&](float a, float g) { return act_grad_apply(g, a, DCG_ACT_TANH, alpha); });
+    else if (act == DCG_ACT_SIGMOID) each_pair(v, gate, [&](float a, float g) { return act_grad_apply(g, a, DCG_ACT_SIGMOID, alpha); });
+}
+
 // Epilogue parameters as passed to kernels (a copy of dcg_epilogue with NULL
 // meaning "absent").
 struct EpilogueArgs {

@@ -40,6 +40,7 @@
 //                        CTA, their accumulators merged into wide MMAs
 //   conv_tc_short.cuh    conv_fwd_short_kernel: the short-K forward GEMMs of the 3-channel layers as
 //                        persistent CTAs with resident weights and a double-buffered accumulator
+//   conv_tc_rgb.cuh      conv_fwd_rgb_kernel: forward of a <= 4-channel layer straight from its image
 //   conv_tc_dx3.cuh      conv_dx3_kernel: input gradient of a 3-channel layer, GEMM + gather in one kernel
 //   conv_tc_narrow.cuh   repack, partition-finish and gather helpers of the 3-channel layers
 #include <cuda.h>
@@ -58,6 +59,7 @@
 #include "conv_tc_kernel.cuh"
 #include "conv_tc_dxf.cuh"
 #include "conv_tc_short.cuh"
+#include "conv_tc_rgb.cuh"
 #include "conv_tc_dx3.cuh"
 #include "conv_tc_narrow.cuh"
 
@@ -85,14 +87,13 @@ EncodeTiledFn encode_fn()
 }
 
 // dims/strides innermost first; strides[i] is the byte stride of dimension i+1.
-int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, bool mn_major,
+int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, CUtensorMapSwizzle swizzle,
                const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* estrides)
 {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(DCG_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void*>(base), dims,
-                          strides, box, estrides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                          strides, box, estrides, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         return fail(DCG_ERR_CUDA,
@@ -103,6 +104,12 @@ int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* d
                     rank > 3 ? box[3] : 0, rank > 4 ? box[4] : 0);
     }
     return DCG_OK;
+}
+
+int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, bool mn_major,
+               const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* estrides)
+{
+    return encode_map(map, base, rank, dims, mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, strides, box, estrides);
 }
 
 // Activation [N, Hh, Ww, Cc] as a 4-D map (c, w, h, n) with a (32, tw, th, tn)-element box and
@@ -699,11 +706,51 @@ bool plan_dk(const dcg_conv_desc& d, Plan& pl, size_t ws_bytes)
     return finish_plan(pl, true);
 }
 
+// The forward of a <= 4-channel layer from its image (conv_fwd_rgb_kernel): all output channels in one tile, everything it keeps
+// in shared memory.  It needs no scratch and is the quicker one at every size measured; the weights' rows have to be TMA rows.
+bool plan_rgb(const dcg_conv_desc& d, Plan& pl, RgbArgs& g)
+{
+    if (t_plan_x3 || d.c > 4 || d.o % 32 != 0 || d.o > 128 || d.kw > 8 || d.kh * (d.kw * d.c <= 16 ? 16 : 32) > kRgbMaxChunks * BK) return false;
+    Params& p = pl.p;
+    base_params(p, d);
+    pixel_tile(BM, d.wo, d.ho, p.TW, p.TH, p.TN);
+    p.tiles_w = (d.wo + p.TW - 1) / p.TW; p.tiles_h = (d.ho + p.TH - 1) / p.TH; p.tiles_n = (d.n + p.TN - 1) / p.TN;
+    p.bn = d.o;
+    p.stages = 2;
+    p.skip_stage = -1;
+    p.wait_cycles = kWaitCycles;
+    set_divisors(p, false);
+    g.kwc = d.kw * d.c;
+    const int places = g.kwc <= 16 ? 16 : 32;
+    g.chunks = (d.kh * places + BK - 1) / BK;
+    g.ksteps = d.kh * places / 8;
+    const long long rows = (long long)p.TN * ((p.TH - 1) * d.stride_h + d.kh), row_len = ((long long)(p.TW - 1) * d.stride_w + d.kw) * d.c;
+    if (rows * row_len * 4 > kMaxSmem) return false;
+    g.rows = (int)rows; g.row_len = (int)row_len;
+    // image rows of whole 16 bytes: a patch is one box of (row, rows, images)
+    const int box = (int)align_up(row_len + 3, 4);
+    g.tma = d.w * d.c % 4 == 0 && box <= 256 && (p.TH - 1) * d.stride_h + d.kh <= 256;
+    g.pitch = g.tma ? box : (g.row_len + 1) & ~1;
+    g.patch_tx = (unsigned)(rows * g.pitch * 4);
+    g.patch_bytes = (int)align_up((rows * g.pitch + places + 4) * 4, 128);   // (the last pixel's places end beyond its row)
+    g.tiles = p.tiles_w * p.tiles_h * p.tiles_n;
+    pl.grid = g.tiles < sm_count() ? g.tiles : sm_count();
+    for (g.patches = 4; g.patches >= 2; --g.patches) {
+        pl.smem = rgb_smem(g.chunks, p.bn, (size_t)g.patches * g.patch_bytes);
+        if (pl.smem <= (size_t)kMaxSmem) return true;
+    }
+    return false;
+}
+
 // `ws_bytes`: scratch that there is, as far as a plan may do with less.
 bool make_plan(const dcg_conv_desc& d, int kind, Plan& pl, size_t ws_bytes = (size_t)-1)
 {
+    RgbArgs rgb;
     switch (kind) {
-    case kConvFwd: return plan_fwd(d, pl);
+    case kConvFwd:
+        if (plan_rgb(d, pl, rgb)) return true;
+        pl = Plan{};
+        return plan_fwd(d, pl);
     case kConvDx: return plan_dx(d, pl);
     case kConvDk: return plan_dk(d, pl, ws_bytes);
     default: return false;
@@ -864,6 +911,8 @@ struct Prepared {
     CfTable cf;
     bool dx3 = false;   // input gradient of a <= 4-channel layer as one GEMM + gather kernel (conv_dx3_kernel)
     Dx3Args dx3_args;
+    bool rgb = false;   // forward of a <= 4-channel layer from its image (conv_fwd_rgb_kernel)
+    RgbArgs rgb_args;
 };
 
 int launch_dxf(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t stream)
@@ -1028,6 +1077,26 @@ int launch_dx3(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t st
     return DCG_OK;
 }
 
+// `maps`: of the output tensors and the gate (32 pixels x 32 channels; absent ones are not read).
+int launch_rgb(Prepared& pr, const CUtensorMap (&maps)[4], const float* x, float* out, const EpilogueArgs& ep, cudaStream_t stream)
+{
+    Params& p = pr.pl.p;
+    using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params, RgbArgs, const float*);
+    static const Kernel kernels[2][2] = {{conv_fwd_rgb_kernel<16, false>, conv_fwd_rgb_kernel<16, true>},
+                                         {conv_fwd_rgb_kernel<32, false>, conv_fwd_rgb_kernel<32, true>}};
+    const int wide = pr.rgb_args.kwc > 16, even = p.sw * p.C % 2 == 0;
+    static OncePerDevice once[2][2];
+    DCG_CUDA(allow_smem(once[wide][even], kernels[wide][even], kMaxSmem));
+    p.out = out;
+    p.ep = ep;
+    p.scratch = nullptr;
+    p.wait_cycles = g_wait_cycles.load();
+    launch_pdl(kernels[wide][even], (unsigned)pr.pl.grid, kRgbThreads, pr.pl.smem, stream, pr.mb, maps[0], maps[1], maps[2], maps[3], pr.ma, p, pr.rgb_args,
+               x);
+    DCG_LAUNCH_CHECK("conv_fwd_rgb_kernel");
+    return DCG_OK;
+}
+
 struct CacheKey {
     int dev, kind, x3;
     dcg_conv_desc d;
@@ -1068,6 +1137,22 @@ size_t g_cache_next = 0;
 int build_fwd(const dcg_conv_desc& d, const float* x, const float* k, void* ws, size_t ws_bytes, Prepared& pr)
 {
     Plan& pl = pr.pl;
+    pr.rgb = plan_rgb(d, pl, pr.rgb_args);
+    if (pr.rgb) {   // k [kh][kw * C + c][o] as (o%32, kw * C + c, kh, o/32), box (32, places, 32 / places, o/32), zero-filled beyond
+        const cuuint64_t kwc = (cuuint64_t)pr.rgb_args.kwc, places = kwc <= 16 ? 16 : 32;
+        const cuuint64_t dims[4] = {32, kwc, (cuuint64_t)d.kh, (cuuint64_t)(d.o / 32)};
+        const cuuint64_t strides[3] = {(cuuint64_t)d.o * 4, kwc * d.o * 4, 128};
+        const cuuint32_t box[4] = {32, (cuuint32_t)places, (cuuint32_t)(32 / places), (cuuint32_t)(d.o / 32)};
+        const cuuint32_t es[4] = {1, 1, 1, 1};
+        const int st = encode_map(&pr.mb, k, 4, dims, true, strides, box, es);
+        if (st || !pr.rgb_args.tma) return st;
+        const cuuint64_t line = (cuuint64_t)d.w * d.c;   // x as (w * c, h, n), plain rows
+        const cuuint64_t xdims[3] = {line, (cuuint64_t)d.h, (cuuint64_t)d.n};
+        const cuuint64_t xstrides[2] = {line * 4, line * d.h * 4};
+        const cuuint32_t xbox[3] = {(cuuint32_t)pr.rgb_args.pitch, (cuuint32_t)(pr.rgb_args.rows / pl.p.TN), (cuuint32_t)pl.p.TN};
+        return encode_map(&pr.ma, x, 3, xdims, CU_TENSOR_MAP_SWIZZLE_NONE, xstrides, xbox, es);
+    }
+    pl = Plan{};
     if (!plan_fwd(d, pl)) return fail(DCG_ERR_UNSUPPORTED, "conv fwd: shape not supported by the tensor path");
     const Params& p = pl.p;
     int st;
@@ -1272,6 +1357,15 @@ int conv_tc_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y
     Prepared pr;
     int st = prepared_call(kConvFwd, d, x, k, ws, ws_bytes, pr);
     if (st) return st;
+    if (pr.rgb) {
+        const Params& p = pr.pl.p;
+        const int tw = std::min(p.TW, 32), th = std::min(p.TH, 32 / tw), tn = 32 / (tw * th);   // 32 accumulator rows
+        CUtensorMap maps[4]{};
+        const float* tensors[4] = {y, ep.raw_out, ep.pre_act, ep.gate};
+        for (int i = 0; i < 4; ++i)
+            if (tensors[i] && (st = map_act_4d(&maps[i], tensors[i], d.n, d.ho, d.wo, d.o, tw, th, tn, 1, 1))) return st;
+        return launch_rgb(pr, maps, x, y, ep, stream);
+    }
     if (pr.pl.p.narrow) {
         float *xp, *k4;
         if ((st = narrow_prepare(d, pr.pl, x, k, ws, ws_bytes, stream, &xp, &k4))) return st;

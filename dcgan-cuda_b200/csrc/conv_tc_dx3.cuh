@@ -118,13 +118,10 @@ __device__ __forceinline__ void dx3_gather_pairs(const Params& p, const Dx3Args&
 #pragma unroll
                 for (int q = 0; q < 6; ++q) f[q] = __fadd_rn(f[q], q % 3 == 0 ? b0 : q % 3 == 1 ? b1 : b2);
             }
-            if (e.act != DCG_ACT_NONE) {
-#pragma unroll
-                for (int q = 0; q < 6; ++q) f[q] = act_apply(f[q], e.act, e.alpha);
-            }
+            act_apply_all(f, e.act, e.alpha);
             if (e.gate) {
-#pragma unroll
-                for (int q = 0; q < 6; ++q) f[q] = act_grad_apply(q & 1 ? gate[q >> 1].y : gate[q >> 1].x, f[q], e.gate_act, e.gate_alpha);
+                const float gv[6] = {gate[0].x, gate[0].y, gate[1].x, gate[1].y, gate[2].x, gate[2].y};
+                act_grad_apply_all(f, gv, e.gate_act, e.gate_alpha);
             }
             float2* o = reinterpret_cast<float2*>(p.out + pix * 3);
 #pragma unroll

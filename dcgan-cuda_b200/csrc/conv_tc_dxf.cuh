@@ -81,26 +81,8 @@ __device__ __forceinline__ void cf_chain_store4(const EpilogueArgs& e, float* ou
         for (int u = 0; u < 4; ++u)
             if (goff[u] >= 0) *reinterpret_cast<float4*>(e.pre_act + goff[u]) = acc[u];
     }
-    if (e.act != DCG_ACT_NONE) {
-        const int act = e.act;
-        const float alpha = e.alpha;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            acc[u].x = act_apply(acc[u].x, act, alpha); acc[u].y = act_apply(acc[u].y, act, alpha);
-            acc[u].z = act_apply(acc[u].z, act, alpha); acc[u].w = act_apply(acc[u].w, act, alpha);
-        }
-    }
-    if (e.gate) {
-        const int gact = e.gate_act;
-        const float galpha = e.gate_alpha;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            acc[u].x = act_grad_apply(gate[u].x, acc[u].x, gact, galpha);
-            acc[u].y = act_grad_apply(gate[u].y, acc[u].y, gact, galpha);
-            acc[u].z = act_grad_apply(gate[u].z, acc[u].z, gact, galpha);
-            acc[u].w = act_grad_apply(gate[u].w, acc[u].w, gact, galpha);
-        }
-    }
+    act_apply_all(acc, e.act, e.alpha);
+    if (e.gate) act_grad_apply_all(acc, gate, e.gate_act, e.gate_alpha);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
         if (goff[u] >= 0) *reinterpret_cast<float4*>(out + goff[u]) = acc[u];

@@ -724,30 +724,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         for (int u = 0; u < 4; ++u)
                             if (goff[u] >= 0) *reinterpret_cast<float4*>(e.pre_act + goff[u]) = acc[u];
                     }
-                    if (e.act != DCG_ACT_NONE) {
-                        const int act = e.act;
-                        const float alpha = e.alpha;
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            acc[u].x = act_apply(acc[u].x, act, alpha); acc[u].y = act_apply(acc[u].y, act, alpha);
-                            acc[u].z = act_apply(acc[u].z, act, alpha); acc[u].w = act_apply(acc[u].w, act, alpha);
-                        }
-                    }
+                    act_apply_all(acc, e.act, e.alpha);
                     if (e.gate) {
                         float4 gg[4];
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
                             gg[u] = goff[u] >= 0 ? __ldg(reinterpret_cast<const float4*>(e.gate + goff[u]))
                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-                        const int gact = e.gate_act;
-                        const float galpha = e.gate_alpha;
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            acc[u].x = act_grad_apply(gg[u].x, acc[u].x, gact, galpha);
-                            acc[u].y = act_grad_apply(gg[u].y, acc[u].y, gact, galpha);
-                            acc[u].z = act_grad_apply(gg[u].z, acc[u].z, gact, galpha);
-                            acc[u].w = act_grad_apply(gg[u].w, acc[u].w, gact, galpha);
-                        }
+                        act_grad_apply_all(acc, gg, e.gate_act, e.gate_alpha);
                     }
                 }
 #pragma unroll

@@ -578,6 +578,34 @@ def test_kernel_gradients_of_many_partitions(pkg, dev, shape, prec_name):
         assert (dk - ref).abs().max().item() <= tol * ref.abs().max().item()
 
 
+# <= 4 input channels straight from the image: patches by TMA and by 4-byte copies (rows that are no 16 bytes), 16 and 32 places
+# per kernel row, even and odd pixel distances, tiles of several images, one and many tiles per CTA, one to four column slabs
+@pytest.mark.parametrize("shape", [(1, 64, 64, 3, 5, 64, 2), (130, 64, 64, 3, 5, 64, 2), (3, 63, 61, 3, 5, 32, 2), (4, 20, 20, 1, 5, 32, 2),
+                                   (6, 40, 30, 3, 3, 96, 1), (2, 50, 64, 2, 4, 128, 2), (3, 17, 19, 3, 7, 64, 1), (40, 9, 7, 3, 3, 32, 1),
+                                   (2, 40, 200, 3, 5, 64, 1), (1, 5, 5, 3, 5, 64, 2), (9, 30, 28, 4, 8, 32, 2), (2, 64, 64, 3, 1, 64, 1)])
+def test_forward_of_rgb_layers(pkg, dev, shape):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    ho, wo = -(-H // s), -(-W // s)
+    x, k, bias, gate = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
+                        ((61, (N, H, W, C)), (62, (K, K, C, O)), (63, (O,)), (64, (N, ho, wo, O))))
+    ref = F.conv2d_fwd(x, k, (s, s), precision=pkg.PREC_FP32)
+    tol = TF32_TOL * ref.abs().max().item()
+    assert (F.conv2d_fwd(x, k, (s, s)) - ref).abs().max().item() <= tol
+    # the whole chain: every tensor it writes, a gate beside the bias, and nothing beyond the ragged border
+    for gated in (None, gate):
+        raw, pre, out = (torch.full((N + 1, ho, wo, O), 7.0, device=dev) for _ in range(3))
+        ep = F.make_epilogue(bias=bias, act=pkg.ACT_LEAKY, alpha=0.2, pre_act=pre[:N], raw_out=raw[:N], gate=gated, gate_act=pkg.ACT_RELU if gated is not None else pkg.ACT_NONE)
+        F.conv2d_fwd(x, k, (s, s), epilogue=ep, out=out[:N])
+        torch.cuda.synchronize()
+        assert pkg.lib.dcg_device_status() == 0
+        assert (raw[:N] - ref).abs().max().item() <= tol
+        assert torch.equal(pre[:N], raw[:N] + bias)
+        y = torch.where(pre[:N] < 0, pre[:N] * 0.2, pre[:N])
+        assert torch.equal(out[:N], y if gated is None else torch.where(gate > 0, y, torch.zeros_like(y)))
+        assert all(bool((t[N] == 7.0).all()) for t in (raw, pre, out))
+
+
 def test_deterministic(pkg, dev):
     """Two runs of every operator give identical bits (fixed-order split-K reduction)."""
     F = pkg.functional
