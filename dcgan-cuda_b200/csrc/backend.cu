@@ -629,6 +629,8 @@ extern "C" int dcg_run_node(dcg_context* ctx, const dcg_node* nd)
 
 namespace dcg {
 int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t n, cudaStream_t stream);
+int sigmoid_xent_two_with_grad(const float* const y[2], const float* const logits[2], float* const loss[2], float* const grad[2], const size_t n[2],
+                               float* sum, cudaStream_t stream);
 int softmax_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t rows, size_t cols, cudaStream_t stream);
 int matmul_act(const float* a, const float* b, const float* bias, float* out, size_t m, size_t n, size_t p, int act, float alpha,
                float* act_out, cudaStream_t stream);
@@ -706,6 +708,30 @@ extern "C" int dcg_run_nodes(dcg_context* ctx, const dcg_node* nodes, int count,
 }
 
 namespace {
+// A sigmoid cross-entropy and its gradient on the same labels and logits, as one launch may run them.
+bool is_sigmoid_xent_pair(const dcg_node& a, const dcg_node& b)
+{
+    return a.type == DCG_OP_SIGMOID_CROSS_ENTROPY && b.type == DCG_OP_SIGMOID_CROSS_ENTROPY_GRAD && a.in1 == b.in1 && a.in2 == b.in2 &&
+           a.len1 == b.len1 && a.len1 <= 65536 && disjoint({a.out1, 1}, {{a.in1, a.len1}, {a.in2, a.len1}, {b.out1, b.len1}}) &&
+           same_or_disjoint({b.out1, b.len1}, {a.in1, a.len1}) && same_or_disjoint({b.out1, b.len1}, {a.in2, a.len1});
+}
+// Two of them and the sum of their losses, n[0] to n[4], none of which writes what another one's launch still reads.
+bool is_two_sigmoid_xents(const dcg_node* n)
+{
+    if (!is_sigmoid_xent_pair(n[0], n[1]) || !is_sigmoid_xent_pair(n[2], n[3])) return false;
+    const dcg_node& s = n[4];
+    if (s.type != DCG_OP_ADD || s.len1 != 1 || s.in1 != n[0].out1 || s.in2 != n[2].out1) return false;
+    for (int i = 1; i < 5; ++i)
+        if (n[i].flags & DCG_NODE_SIDE) return false;
+    for (int i = 0; i < 2; ++i) {
+        const dcg_node &mine = n[2 * i], &other = n[2 - 2 * i];
+        const Operand loss{mine.out1, 1}, grad{n[2 * i + 1].out1, mine.len1}, sum{s.out1, 1};
+        const Operand y{other.in1, other.len1}, x{other.in2, other.len1}, loss2{other.out1, 1}, grad2{n[3 - 2 * i].out1, other.len1};
+        if (!disjoint(loss, {y, x, loss2, grad2}) || !disjoint(grad, {y, x, grad2}) || !disjoint(sum, {y, x, loss2, grad2})) return false;
+    }
+    return true;
+}
+
 int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
 {
     int i = 0;
@@ -747,10 +773,18 @@ int run_nodes_impl(dcg_context* ctx, const dcg_node* nodes, int count, int fuse)
                 scope.drop();
             }
             // loss + its gradient on the same labels and logits
-            if (a.type == DCG_OP_SIGMOID_CROSS_ENTROPY && b.type == DCG_OP_SIGMOID_CROSS_ENTROPY_GRAD && a.in1 == b.in1 &&
-                a.in2 == b.in2 && a.len1 == b.len1 && a.len1 <= 65536 &&
-                disjoint({a.out1, 1}, {{a.in1, a.len1}, {a.in2, a.len1}, {b.out1, b.len1}}) &&
-                same_or_disjoint({b.out1, b.len1}, {a.in1, a.len1}) && same_or_disjoint({b.out1, b.len1}, {a.in2, a.len1})) {
+            if (i + 4 < count && is_two_sigmoid_xents(nodes + i)) {
+                ProfScope scope(ctx, "sigmoid_xent_two_with_grad", 0.0);
+                const dcg_node* n = nodes + i;
+                const float *y[2] = {n[0].in1, n[2].in1}, *x[2] = {n[0].in2, n[2].in2};
+                float *loss[2] = {n[0].out1, n[2].out1}, *grad[2] = {n[1].out1, n[3].out1};
+                const size_t len[2] = {n[0].len1, n[2].len1};
+                const int st = dcg::sigmoid_xent_two_with_grad(y, x, loss, grad, len, n[4].out1, ctx->stream);
+                if (st) return st;
+                i += 5;
+                continue;
+            }
+            if (is_sigmoid_xent_pair(a, b)) {
                 ProfScope scope(ctx, "sigmoid_xent_with_grad", 0.0);
                 const int st = dcg::sigmoid_xent_with_grad(a.in1, a.in2, a.out1, b.out1, a.len1, ctx->stream);
                 if (st) return st;

@@ -398,20 +398,40 @@ sigmoid_xent_grad_kernel(const float* __restrict__ y, const float* __restrict__ 
 
 // Loss and its gradient in one launch (the two nodes are neighbours in a training list): the same
 // expressions as the two kernels above, element for element, so the results are bit-identical.
+struct XentPair {
+    const float *y, *x;
+    float *loss, *grad;
+    size_t n;
+};
+__device__ __forceinline__ float sigmoid_xent_pair(const XentPair& p, float* red)   // the loss, in thread 0
+{
+    float s = 0.f;
+    for (size_t i = threadIdx.x; i < p.n; i += blockDim.x) {
+        const float xi = __ldg(p.x + i), yi = __ldg(p.y + i);
+        s += xi >= 0.f ? xi - xi * yi + logf(1.f + expf(-xi)) : -xi * yi + logf(1.f + expf(xi));
+        p.grad[i] = (act_apply(xi, DCG_ACT_SIGMOID, 0.f) - yi) / (float)p.n;
+    }
+    s = block_sum(s, red) / (float)p.n;
+    if (threadIdx.x == 0) p.loss[0] = s;
+    return s;
+}
 __global__ void __launch_bounds__(512)
-sigmoid_xent_both_kernel(const float* __restrict__ y, const float* __restrict__ x, float* __restrict__ loss,
-                         float* __restrict__ grad, size_t n)
+sigmoid_xent_both_kernel(const XentPair p)
 {
     pdl_enter();
     __shared__ float red[32];
-    float s = 0.f;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const float xi = __ldg(x + i), yi = __ldg(y + i);
-        s += xi >= 0.f ? xi - xi * yi + logf(1.f + expf(-xi)) : -xi * yi + logf(1.f + expf(xi));
-        grad[i] = (act_apply(xi, DCG_ACT_SIGMOID, 0.f) - yi) / (float)n;
-    }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) loss[0] = s / (float)n;
+    sigmoid_xent_pair(p, red);
+}
+
+// Two losses with their gradients and the sum of the losses, as a discriminator has them: one launch for three (from
+// the logits to the head's input gradient 6.9 -> 4.6 us of a step of 8 images, in which nothing else runs).
+__global__ void __launch_bounds__(512)
+sigmoid_xent_two_kernel(const XentPair p, const XentPair q, float* __restrict__ sum)
+{
+    pdl_enter();
+    __shared__ float red[2][32];
+    const float a = sigmoid_xent_pair(p, red[0]), b = sigmoid_xent_pair(q, red[1]);
+    if (threadIdx.x == 0) sum[0] = __fadd_rn(a, b);
 }
 
 __global__ void __launch_bounds__(512)
@@ -850,8 +870,19 @@ namespace dcg {
 int sigmoid_xent_with_grad(const float* y, const float* logits, float* loss, float* grad, size_t n, cudaStream_t stream)
 {
     DCG_CHECK_ARG(y && logits && loss && grad && n > 0, "sigmoid_xent_with_grad: bad arguments");
-    launch_pdl(sigmoid_xent_both_kernel, 1, 512, 0, stream, y, logits, loss, grad, n);
+    launch_pdl(sigmoid_xent_both_kernel, 1, 512, 0, stream, XentPair{y, logits, loss, grad, n});
     DCG_LAUNCH_CHECK("sigmoid_xent_both_kernel");
+    return DCG_OK;
+}
+// Two of these and dcg_add of the losses.  Neither writes what the other one reads.
+int sigmoid_xent_two_with_grad(const float* const y[2], const float* const logits[2], float* const loss[2], float* const grad[2], const size_t n[2],
+                               float* sum, cudaStream_t stream)
+{
+    for (int i = 0; i < 2; ++i)
+        DCG_CHECK_ARG(y[i] && logits[i] && loss[i] && grad[i] && sum && n[i] > 0, "sigmoid_xent_two_with_grad: bad arguments");
+    launch_pdl(sigmoid_xent_two_kernel, 1, 512, 0, stream, XentPair{y[0], logits[0], loss[0], grad[0], n[0]},
+               XentPair{y[1], logits[1], loss[1], grad[1], n[1]}, sum);
+    DCG_LAUNCH_CHECK("sigmoid_xent_two_kernel");
     return DCG_OK;
 }
 // dcg_softmax_xent and dcg_softmax_xent_grad as one launch.

@@ -158,6 +158,34 @@ def test_dead_intermediates_are_skipped_only_when_flagged(pkg, dev):
     ctx.close()
 
 
+@pytest.mark.parametrize("n", [1, 64, 700])
+def test_two_losses_and_their_sum_are_one_launch(pkg, dev, n):
+    """A discriminator's two losses with their gradients and the sum: bit for bit what the five nodes give; where one of them
+    writes what another still reads, launches of their own."""
+    N = pkg.nodes
+    y = [torch.full((n,), v, device=dev) for v in (0.0, 1.0)]
+    results = []
+    for case in ("nodes", "fused", "gradient over the other logits"):
+        x = [_t(seeded((n,), 970 + i) * np.float32(4), dev) for i in range(2)]
+        loss, total = [torch.zeros(1, device=dev) for _ in range(2)], torch.zeros(1, device=dev)
+        grad = [x[1] if case.startswith("gradient") else torch.empty(n, device=dev), torch.empty(n, device=dev)]
+        nodes = [N.op_sigmoid_cross_entropy(y[0], x[0], loss[0], n), N.op_sigmoid_cross_entropy_grad(y[0], x[0], grad[0], n),
+                 N.op_sigmoid_cross_entropy(y[1], x[1], loss[1], n), N.op_sigmoid_cross_entropy_grad(y[1], x[1], grad[1], n),
+                 N.op_add(loss[0], loss[1], total, 1)]
+        ctx = pkg.Context(pkg.PREC_TF32)
+        ctx.run(nodes, fuse=case != "nodes")
+        torch.cuda.synchronize()
+        assert ctx.launch_count() == {"nodes": 5, "fused": 1}.get(case, 3)
+        results.append([t.cpu().numpy() for t in loss + grad + [total]])
+        ctx.close()
+    for a, b in zip(results[0], results[1]):
+        assert np.array_equal(a, b)
+    # the second pair reads the first one's gradient as its logits there
+    g = results[2][2]
+    assert np.array_equal(g, results[0][2])
+    np.testing.assert_allclose(results[2][1], np.mean(np.maximum(g, 0) - g + np.log1p(np.exp(-np.abs(g)))), rtol=1e-5)
+
+
 def test_dead_dense_intermediates(pkg, dev):
     """A flagged pre-activation of a wide dense layer, and a flagged product under an activation gradient, are not written;
     what reads them comes out as without the flag."""
