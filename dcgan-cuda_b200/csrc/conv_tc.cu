@@ -349,7 +349,7 @@ bool finish_plan(Plan& pl, bool kernel_gradient = false)
     }
     // two CTAs per SM when the grid has more CTAs than SMs, else one deep pipeline
     const bool half = pl.grid > sm_count() && p.bn <= kMaxSharedWidth && !p.x3;
-    p.kind = p.x3 ? kX3 : half ? kShared : p.bn <= 64 || p.mt > 1 ? kDual : p.splits == 1 ? kAlone : kShared;
+    p.kind = p.x3 ? (p.bn <= kX3Width<kX3> ? kX3 : kX3Wide) : half ? kShared : p.bn <= 64 || p.mt > 1 ? kDual : p.splits == 1 ? kAlone : kShared;
     if (p.x3 && p.bn > kX3MaxWidth) return false;
     if (tmem_columns(p.kind, p.bn, p.x3_slots) > (half ? 256 : 512)) return false;
     const int budget = half ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
@@ -773,7 +773,7 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    static const int groups[] = {kGroups<kShared>, kGroups<kX3>, kGroups<kAlone>, kGroups<kDual>};
+    static const int groups[kKinds] = {kGroups<kShared>, kGroups<kX3>, kGroups<kAlone>, kGroups<kDual>, kGroups<kX3Wide>};
     cfg.blockDim = dim3((unsigned)(64 + 128 * groups[p.kind]));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -795,15 +795,20 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
     cfg.attrs = attr;
     cfg.numAttrs = na;
     using Kernel = void (*)(CUtensorMap, CUtensorMap, Params);
+    // (only the kernel gradient of an RGB layer is wider than 128 columns in 3xTF32)
     static const Kernel kernels[] = {conv_tc_kernel<MODE, kShared>, conv_tc_kernel<MODE, kX3>, conv_tc_kernel<MODE, kAlone>,
                                      conv_tc_kernel<MODE, kDual>};
     int form = 0;
-    Kernel kernel = kernels[p.kind];
+    Kernel kernel = p.kind == kX3Wide ? nullptr : kernels[p.kind];
     if constexpr (MODE != MODE_DX) {
         static const Kernel pieces[] = {conv_tc_kernel<MODE, kShared, 0>, conv_tc_kernel<MODE, kX3, 0>, conv_tc_kernel<MODE, kAlone, 0>,
                                         conv_tc_kernel<MODE, kDual, 0>};
-        if (p.mt == 0) { form = 1; kernel = pieces[p.kind]; }
+        if (p.mt == 0 && p.kind != kX3Wide) { form = 1; kernel = pieces[p.kind]; }
     }
+    if constexpr (MODE == MODE_DK) {
+        if (p.kind == kX3Wide) { form = p.mt == 0; kernel = p.mt == 0 ? conv_tc_kernel<MODE_DK, kX3Wide, 0> : conv_tc_kernel<MODE_DK, kX3Wide>; }
+    }
+    if (!kernel) return fail(DCG_ERR_UNSUPPORTED, "conv_tc_kernel: no kernel of %d columns for this operator", p.bn);
     if constexpr (MODE == MODE_DK) {
         static const Kernel more_taps[2][4] = {
             {conv_tc_kernel<MODE_DK, kShared, 2>, conv_tc_kernel<MODE_DK, kX3, 2>, nullptr, conv_tc_kernel<MODE_DK, kDual, 2>},
@@ -811,7 +816,7 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
         if (p.mt > 1) { form = 2 + p.mt / 4; kernel = more_taps[p.mt / 4][p.kind]; }
     }
     // each form is loaded when it is first needed, not all of them with the first convolution
-    static OncePerDevice once[4][4];
+    static OncePerDevice once[4][kKinds];
     DCG_CUDA(allow_smem(once[form][p.kind], kernel, kMaxSmem));
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
     if (err != cudaSuccess) return fail(DCG_ERR_CUDA, "conv_tc_kernel launch: %s", cudaGetErrorString(err));

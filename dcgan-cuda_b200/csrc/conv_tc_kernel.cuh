@@ -11,36 +11,41 @@ namespace {
 // TF32.  Measured, 128 -> 256 channels at batch 64: forward 91 -> 49 us, input gradient 124 -> 61, kernel gradient
 // 80 -> 57; relative error against float64 4e-7 at every layer (3.6e-7 to 4.7e-6 before).
 constexpr int kX3Block = 4;   // K stages per block: sixteen truncating steps in a row
-constexpr int kX3Slabs = 2;    // 32-column slabs per epilogue warp, every third slab: at most 192 columns (kX3MaxWidth)
 
 // Kinds of launch.
 //   kShared   the plain one; two CTAs per SM where the grid is large enough
-//   kX3       3xTF32
+//   kX3       3xTF32, up to 128 columns
+//   kX3Wide   3xTF32, up to 192 columns (the kernel gradient of an RGB layer)
 //   kAlone    one CTA per SM and no K partitions: more threads for the epilogue (64 -> 128 forward of 64 images 16.6 -> 15.5
 //             us; with partitions the cluster barrier of the larger CTA costs more, +0.6 to 1 us)
 //   kDual     one CTA per SM and at most 64 columns: the MMAs of a stage are too short to cover the hand-over to the next, so
 //             two warps issue them in turn, each into an accumulator of its own, and two warps load (64 -> 128 kernel
 //             gradient of 64 images 22.9 -> 20.4 us; from 128 columns on there was nothing to gain)
-enum Kind { kShared, kX3, kAlone, kDual };
-// Groups of four epilogue warps, one warp per TMEM lane quadrant each.  3xTF32 has three: taking a stage apart is bound by
-// latency, and with two groups it paced the loop.
-template <int KIND> constexpr int kGroups = KIND == kX3 ? 3 : KIND == kAlone ? 4 : 2;
-
-constexpr int kX3MaxWidth = 32 * kGroups<kX3> * kX3Slabs;
+enum Kind { kShared, kX3, kAlone, kDual, kX3Wide, kKinds };
+__host__ __device__ constexpr bool is_x3(int kind) { return kind == kX3 || kind == kX3Wide; }
+// Groups of four epilogue warps, one warp per TMEM lane quadrant each.  3xTF32: taking a stage apart (2500 clocks, most of them
+// waits for shared memory, which the MMAs' operands keep busy) and taking over the sums (1300 every fourth stage) pace the
+// loop, so there are as many groups as registers allow: with four, a warp sums one 32-column slab of the tile, with three,
+// two.  (Against three throughout: step of 64 images 3095 -> 3058 us, 64 -> 3 input gradient of 64 images 41.3 -> 38.3.)
+template <int KIND> constexpr int kGroups = KIND == kX3Wide ? 3 : KIND == kX3 || KIND == kAlone ? 4 : 2;
+template <int KIND> constexpr int kX3Slabs = KIND == kX3Wide ? 2 : 1;   // slabs per epilogue warp, every kGroups-th one
+template <int KIND> constexpr int kX3Width = 32 * kGroups<KIND> * kX3Slabs<KIND>;
+constexpr int kX3MaxWidth = kX3Width<kX3Wide>;
 // 3xTF32: accumulators of the large terms.
 __host__ __device__ constexpr int x3_accumulators(int bn) { return bn <= 128 ? 2 : 1; }
 // TMEM columns of a CTA: at most 512, or 256 where two share an SM.
 __host__ __device__ constexpr int tmem_columns(int kind, int bn, int x3_slots)
 {
-    return kind == kX3 ? (x3_accumulators(bn) + 1) * bn + 64 * x3_slots : kind == kDual ? 2 * bn : bn;
+    return is_x3(kind) ? (x3_accumulators(bn) + 1) * bn + 64 * x3_slots : kind == kDual ? 2 * bn : bn;
 }
 
 // Adds the accumulator's slabs of this warp to `sum`.
-__device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs][32], uint32_t tmem_quad, int group, int bn)
+template <int KIND>
+__device__ __forceinline__ void x3_take_over(float (&sum)[kX3Slabs<KIND>][32], uint32_t tmem_quad, int group, int bn)
 {
 #pragma unroll
-    for (int sl = 0; sl < kX3Slabs; ++sl) {
-        const int c0 = group * 32 + sl * 32 * kGroups<kX3>;
+    for (int sl = 0; sl < kX3Slabs<KIND>; ++sl) {
+        const int c0 = group * 32 + sl * 32 * kGroups<KIND>;
         if (c0 < bn) {
             uint32_t r[32];
             const bool full = bn - c0 >= 32;
@@ -63,7 +68,7 @@ __global__ void __launch_bounds__(64 + 128 * kGroups<KIND>, KIND == kShared ? 2 
 conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ Params p)
 {
-    constexpr bool X3 = KIND == kX3, PIECES = TAPS == 0;
+    constexpr bool X3 = is_x3(KIND), PIECES = TAPS == 0;
     constexpr int MT = PIECES ? 1 : TAPS;
     // Warps that take the stages in turn, as producers and as MMA issuers.  With two of them the ring has an even number of
     // stages: a stage is then always the same warp's, which makes the parity of its barriers unambiguous.
@@ -204,10 +209,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     float* red = reinterpret_cast<float*>(smem_raw + (a_base - smem_u32(smem_raw)));
     long long* s_rowoff = reinterpret_cast<long long*>(red + kRedFloats(p.bn));
 
-    float x3_sum[X3 ? kX3Slabs : 1][32];   // 3xTF32: the blocks of stages taken over so far
+    constexpr int SLABS = kX3Slabs<KIND>;
+    float x3_sum[SLABS][32];   // 3xTF32: the blocks of stages taken over so far
     if constexpr (X3) {
 #pragma unroll
-        for (int sl = 0; sl < kX3Slabs; ++sl)
+        for (int sl = 0; sl < SLABS; ++sl)
 #pragma unroll
             for (int q = 0; q < 32; ++q) x3_sum[sl][q] = 0.f;
     }
@@ -449,7 +455,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // the stage's TMEM columns.  B: element-wise on the raw bytes of the stage, so the swizzled layout carries
             // over unchanged.
             // Everything but the stores to TMEM is done before the slot is free, so that little stands between the MMAs that
-            // free it and those that read it next.
+            // free it and those that read it next; B first, while the registers of A's values can hold eight of its words in flight.
             const int group = (warp - 2) >> 2, tid_r = (threadIdx.x - 64) & 127;
             int turn = 0;
             const int b_q = b_stage_bytes / 16;   // 16-byte words of a B tile
@@ -467,6 +473,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int it = 0; it < nq; ++it) {
                 if (turn == group) {
                     if (!__all_sync(0xffffffffu, mbar_wait(full_bar + 8u * s, phase, 4, it, wait_limit))) break;
+                    if (!mma_done(p.x3_bslots, it)) break;
+                    const float4* bsrc = reinterpret_cast<const float4*>(smem_raw + (b_base + (uint32_t)s * b_stage_bytes - smem_u32(smem_raw)));
+                    float4* bdst = reinterpret_cast<float4*>(smem_raw + (bs_base + (uint32_t)(it & x3_bslot_mask) * b_stage_bytes - smem_u32(smem_raw)));
+#pragma unroll 8
+                    for (int i = tid_r; i < b_q; i += 128) bdst[i] = tf32_residual(bsrc[i]);
                     const uint8_t* asrc = smem_raw + (a_base + (uint32_t)s * A_STAGE_BYTES - smem_u32(smem_raw));
                     float v[32];
                     if (MODE != MODE_DK) {   // K-major: the row's 128 bytes, 16-byte chunk j at j ^ (row & 7)
@@ -480,11 +491,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         for (int k = 0; k < 32; ++k)
                             v[k] = *reinterpret_cast<const float*>(asrc + quad * 4096 + k * 128 + (((lane >> 3) ^ (k & 3)) << 5) + (lane & 7) * 4);
                     }
-                    if (!mma_done(p.x3_bslots, it)) break;
-                    const float4* bsrc = reinterpret_cast<const float4*>(smem_raw + (b_base + (uint32_t)s * b_stage_bytes - smem_u32(smem_raw)));
-                    float4* bdst = reinterpret_cast<float4*>(smem_raw + (bs_base + (uint32_t)(it & x3_bslot_mask) * b_stage_bytes - smem_u32(smem_raw)));
-#pragma unroll 4
-                    for (int i = tid_r; i < b_q; i += 128) bdst[i] = tf32_residual(bsrc[i]);
                     if (!mma_done(p.x3_slots, it)) break;
                     const uint32_t ahi = tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)(x3_a0 + 64 * (it & x3_slot_mask));
                     tmem_st_32x32b_x32(ahi, v);
@@ -506,7 +512,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     got = __all_sync(0xffffffffu, got);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (!got) break;
-                    x3_take_over(x3_sum, tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.bn), group, p.bn);
+                    x3_take_over<KIND>(x3_sum, tmem_d + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * p.bn), group, p.bn);
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(promo_empty_bar + 8u * buf) : "memory");
                     ++taken;
@@ -555,8 +561,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // the warps of a lane quadrant (one per group) take the 32-column slabs in turn (3xTF32: unrolled, for the sums of the
         // slabs are registers only if nothing chooses among them at run time: as local memory they cost every launch 3 us, 8 -> 8
         // input gradient 7.1 for 4.2 us)
-#pragma unroll (X3 ? kX3Slabs : 1)
-        for (int sl = 0; sl < (X3 ? kX3Slabs : 256 / 32); ++sl) {
+#pragma unroll (X3 ? SLABS : 1)
+        for (int sl = 0; sl < (X3 ? SLABS : 256 / 32); ++sl) {
             const int c0 = ((warp - 2) >> 2) * 32 + sl * 32 * G;
             if (c0 >= p.bn) break;
             uint32_t r[32];
