@@ -428,7 +428,9 @@ void build_discriminator_backward(dcg_trainer* t, std::vector<dcg_node>& L, cons
         L.push_back(n_binary(DCG_OP_LEAKY_RELU_GRAD, t->da[ps][i].p, t->dda[i + 1].p, t->ddz[i].p, rows * kDChan[i + 1], 0.2f));
         if (grads) {
             L.push_back(grad_node(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->ddz[i].p, nullptr, grads[2 * i + 1].p, rows, kDChan[i + 1])));
-            L.push_back(grad_node(n_conv2d_kernel_grad(t->ddz[i].p, in, grads[2 * i].p, B, h, kDChan[i], kDChan[i + 1])));
+            // (the last of them where nothing follows on the main stream: beside the one before it, not behind it)
+            const dcg_node dk = n_conv2d_kernel_grad(t->ddz[i].p, in, grads[2 * i].p, B, h, kDChan[i], kDChan[i + 1]);
+            L.push_back(i == 0 && !to_image ? dk : grad_node(dk));
         }
         // the input gradient is only ever read by the activation gradient that follows it
         if (i > 0)
@@ -493,16 +495,20 @@ void build_lists(dcg_trainer* t)
         const size_t rows = (size_t)B * hw * hw;
         const float* in = i == 0 ? t->g0a.p : t->ga[i - 1].p;
         G.push_back(side(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->dgz[i].p, nullptr, t->g_grad[2 * i + 1].p, rows, kGChan[i + 1])));
-        G.push_back(side(n_conv2d_transpose_kernel_grad(t->dgz[i].p, in, t->g_grad[2 * i].p, B, h, kGChan[i], kGChan[i + 1])));
+        const dcg_node dk = n_conv2d_transpose_kernel_grad(t->dgz[i].p, in, t->g_grad[2 * i].p, B, h, kGChan[i], kGChan[i + 1]);
+        if (i > 0) G.push_back(side(dk));
         float* dprev_a = i == 0 ? t->dg0a.p : t->dga[i - 1].p;
         G.push_back(dead(n_conv2d_transpose_input_grad(t->dgz[i].p, t->g_param[2 * i].p, dprev_a, B, h, kGChan[i], kGChan[i + 1])));
         float* dprev_z = i == 0 ? t->dg0z.p : t->dgz[i - 1].p;
         // (gated by the activation, as in the discriminator)
         const size_t nprev = i == 0 ? (size_t)B * 8192 : (size_t)B * h * h * kGChan[i];
         G.push_back(n_binary(gact_grad, in, dprev_a, dprev_z, nprev, 0.2f));
+        if (i == 0) {   // the last kernel gradient on the main stream, which has nothing more to do, not behind the one before it
+            G.push_back(side(n_mat3(DCG_OP_TMAT_MAT_MUL, t->z.p, t->dg0z.p, t->g_grad[8].p, kZ, B, 8192)));
+            G.push_back(side(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->dg0z.p, nullptr, t->g_grad[9].p, B, 8192)));
+            G.push_back(dk);
+        }
     }
-    G.push_back(side(n_mat3(DCG_OP_TMAT_MAT_MUL, t->z.p, t->dg0z.p, t->g_grad[8].p, kZ, B, 8192)));
-    G.push_back(side(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->dg0z.p, nullptr, t->g_grad[9].p, B, 8192)));
 }
 
 int run_list(dcg_trainer* t, const std::vector<dcg_node>& all, dcg_trainer::ListGraph& g, size_t begin = 0,
