@@ -38,6 +38,7 @@
 //   conv_tc_kernel.cuh   conv_tc_kernel<MODE, KIND>, the general kernel described above
 //   conv_tc_dxf.cuh      conv_dxf_kernel: input gradient with all parity classes of a pixel tile in one
 //                        CTA, their accumulators merged into wide MMAs
+//   conv_tc_walk.cuh     conv_tc_walk_kernel: forward and input gradient of layers with more tiles than SMs
 //   conv_tc_short.cuh    conv_fwd_short_kernel: the short-K forward GEMMs of the 3-channel layers as
 //                        persistent CTAs with resident weights and a double-buffered accumulator
 //   conv_tc_rgb.cuh      conv_fwd_rgb_kernel: forward of a <= 4-channel layer straight from its image
@@ -58,6 +59,7 @@
 #include "conv_tc_common.cuh"
 #include "conv_tc_kernel.cuh"
 #include "conv_tc_dxf.cuh"
+#include "conv_tc_walk.cuh"
 #include "conv_tc_short.cuh"
 #include "conv_tc_rgb.cuh"
 #include "conv_tc_dx3.cuh"
@@ -279,12 +281,14 @@ constexpr int kMaxSharedWidth = 160;
 // 3 x 3, 96 -> 160, 13 images of 75 x 51: 49 and 30; 64 -> 128 of 64 images, 3xTF32: 53 and 42).
 struct Tiling {
     int bn, n_tiles, splits, grid;
-    bool second_launch;
+    bool second_launch, walk;
     double cost;
 };
 Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max_stages, int store_cost, int loads = 2, bool b_pieces = false,
-                     size_t partials_bytes = 0)
+                     size_t partials_bytes = 0, bool may_walk = false)
 {
+    static const int no_walk = env_int("DCG_TC_NO_WALK");
+    if (no_walk || t_plan_x3) may_walk = false;
     static const int forced = env_int("DCG_TC_BN");
     const int sms = sm_count();
     const int widest = t_plan_x3 ? 128 : 256;   // 3xTF32: accumulators, residuals and A operands share TMEM
@@ -303,6 +307,8 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
         const double epilogue = t.bn * (t.splits > 1 ? 55.0 : (double)store_cost);
         t.cost = t.bn <= kMaxSharedWidth && !t_plan_x3 ? waves * loop + epilogue : waves * (loop + epilogue);
         t.second_launch = false;
+        t.walk = may_walk && t.splits == 1 && t.grid > sms;
+        if (t.walk) t.cost = 1200.0 + waves * (double)max_stages * stage + epilogue;
         if (best.grid == 0 || t.cost < best.cost) best = t;
         // the same tiles with a second launch
         const int tiles = m_count * t.n_tiles;
@@ -311,6 +317,7 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
         const size_t bytes = (size_t)t.grid * BM * t.bn * sizeof(float);
         if (t.splits <= 1 || t.grid <= best.grid || bytes > partials_bytes) continue;
         t.second_launch = true;
+        t.walk = false;
         t.cost = 1200.0 + (max_stages + t.splits - 1) / t.splits * (stage + 20.0 * (loads - 2 + (b_pieces ? (t.bn + 31) / 32 - 1 : 0))) + t.bn * 18.0 +
                  6500.0 + bytes / 2500.0;
         if (t.cost < best.cost) best = t;
@@ -352,6 +359,15 @@ bool finish_plan(Plan& pl, bool kernel_gradient = false)
     p.kind = p.x3 ? (p.bn <= kX3Width<kX3> ? kX3 : kX3Wide) : half ? kShared : p.bn <= 64 || p.mt > 1 ? kDual : p.splits == 1 ? kAlone : kShared;
     if (p.x3 && p.bn > kX3MaxWidth) return false;
     if (tmem_columns(p.kind, p.bn, p.x3_slots) > (half ? 256 : 512)) return false;
+    if (p.walk) {
+        p.stages = 8;
+        while (walk_smem(p.stages, p.bn) > (size_t)kMaxSmem) --p.stages;
+        pl.smem = walk_smem(p.stages, p.bn);
+        p.skip_stage = -1;
+        p.wait_cycles = kWaitCycles;
+        set_divisors(p, kernel_gradient);
+        return true;   // no scratch
+    }
     const int budget = half ? (kMaxSmem / 2 - 2048) : (kMaxSmem - 2048);
     int stages = (budget - (p.x3 ? p.x3_bslots * b_stage : 0)) / per_stage;
     if (stages > 8) stages = 8;
@@ -431,6 +447,7 @@ void use_tiling(Plan& pl, const Tiling& t)
 {
     pl.p.bn = t.bn; pl.p.n_tiles = t.n_tiles; pl.p.splits = t.splits;
     pl.p.ext_finish = t.second_launch;
+    pl.p.walk = t.walk;
     pl.grid = t.grid;
 }
 
@@ -463,7 +480,7 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
         p.splits = choose_splits(m_count * p.n_tiles, stages);
         pl.grid = m_count * p.n_tiles * p.splits;
     } else {
-        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35, 2, pieces));
+        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35, 2, pieces, 0, !pieces));
     }
     return finish_plan(pl);
 }
@@ -504,7 +521,7 @@ bool plan_dx(const dcg_conv_desc& d, Plan& pl)
     const int min_taps = (d.kh / d.stride_h) * (d.kw / d.stride_w);
     const int max_taps = ((d.kh + d.stride_h - 1) / d.stride_h) * ((d.kw + d.stride_w - 1) / d.stride_w);
     use_tiling(pl, choose_tiling(classes * p.tiles_w * p.tiles_h * p.tiles_n, d.c, 16, (min_taps < 1 ? 1 : min_taps) * p.kchunks,
-                                 max_taps * p.kchunks, 20));
+                                 max_taps * p.kchunks, 20, 2, false, 0, true));
     return finish_plan(pl);
 }
 
@@ -825,6 +842,16 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
 }
 
 template <int MODE>
+int launch_walk(const CUtensorMap& ma, const CUtensorMap& mb, const Plan& pl, cudaStream_t stream)
+{
+    static OncePerDevice once;
+    DCG_CUDA(allow_smem(once, conv_tc_walk_kernel<MODE>, kMaxSmem));
+    launch_pdl(conv_tc_walk_kernel<MODE>, (unsigned)std::min(pl.grid, sm_count()), kWalkThreads, pl.smem, stream, ma, mb, pl.p, pl.grid);
+    DCG_LAUNCH_CHECK("conv_tc_walk_kernel");
+    return DCG_OK;
+}
+
+template <int MODE>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, const EpilogueArgs& ep,
            int channels, void* ws, size_t ws_bytes, cudaStream_t stream)
 {
@@ -840,6 +867,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, Plan& pl, float* out, c
         p.scratch = static_cast<float*>(ws);
     }
     (void)channels;
+    if constexpr (MODE != MODE_DK)
+        if (p.walk) return launch_walk<MODE>(ma, mb, pl, stream);
     const int st = launch_grid<MODE>(ma, mb, p, pl.grid, pl.smem, stream);
     if (st) return st;
     if (p.ext_finish && !p.narrow) {
@@ -1439,7 +1468,7 @@ bool conv_tc_plan(const dcg_conv_desc& d, int kind, bool x3, int plan[6])
     Plan pl;
     if (!make_plan(d, kind, pl)) return false;
     const Params& p = pl.p;
-    const int values[6] = {p.bn, p.n_tiles, p.splits, p.stages, tmem_columns(p.kind, p.bn, p.x3_slots), (int)pl.smem};
+    const int values[6] = {p.bn, p.n_tiles, p.splits, p.stages, p.walk ? 2 * p.bn : tmem_columns(p.kind, p.bn, p.x3_slots), (int)pl.smem};
     for (int i = 0; i < 6; ++i) plan[i] = values[i];
     return true;
 }

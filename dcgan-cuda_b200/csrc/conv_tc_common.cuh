@@ -86,6 +86,7 @@ struct Params {
     int a_ch, b_ch;               // mt == 0: channels along M (DK) and N of the MN-major operands
     int swap;                     // DK: M axis is o (A from dy, B from x)
     int narrow;                   // FWD/DK with <= 4 input channels: x is read through the window map
+    int walk;                     // more tiles than SMs, walked by persistent CTAs (conv_tc_walk_kernel)
     int ext_finish;               // the K partitions only write partials; a second kernel adds them (narrow DK)
     int planes;                   // FWD: 16-byte column quad q of output pixel r goes to out[(q * pixels + r) * 4]
     int o_store;                  // FWD: output columns >= o_store are padding and never stored (0: store all O)

@@ -606,6 +606,31 @@ def test_forward_of_rgb_layers(pkg, dev, shape):
         assert all(bool((t[N] == 7.0).all()) for t in (raw, pre, out))
 
 
+# more tiles than SMs, walked by persistent CTAs: one to three tiles each and a last round that is nearly empty, widths of 16 to 192
+# columns, the last column tile partly beyond the channels, parity classes, channels that are no multiple of four, one stage a tile
+@pytest.mark.parametrize("shape", [(24, 48, 48, 32, 1, 192, 1), (13, 75, 51, 96, 3, 160, 1), (32, 40, 40, 64, 3, 96, 1), (37, 60, 60, 20, 5, 64, 2),
+                                   (40, 33, 35, 6, 3, 32, 1), (150, 12, 11, 32, 3, 288, 1), (20, 64, 64, 8, 1, 32, 1)])
+def test_more_tiles_than_sms(pkg, dev, shape):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    ho, wo = -(-H // s), -(-W // s)
+    x, k, dy, bias, gate = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
+                            ((65, (N, H, W, C)), (66, (K, K, C, O)), (67, (N, ho, wo, O)), (68, (O,)), (69, (N, H, W, C))))
+    pre = [torch.empty((N, ho, wo, O), device=dev) for _ in range(2)]
+    results = []
+    pkg.lib.dcg_debug_set_dx_mode(0)
+    try:
+        for i, prec in enumerate((pkg.PREC_TF32, pkg.PREC_FP32)):
+            results.append([F.conv2d_fwd(x, k, (s, s), epilogue=F.make_epilogue(bias=bias, act=pkg.ACT_LEAKY, pre_act=pre[i]), precision=prec), pre[i],
+                            F.conv2d_dx(dy, k, (H, W), (s, s), epilogue=F.make_epilogue(gate=gate, gate_act=pkg.ACT_RELU), precision=prec)])
+    finally:
+        pkg.lib.dcg_debug_set_dx_mode(-1)
+    torch.cuda.synchronize()
+    assert pkg.lib.dcg_device_status() == 0
+    for name, a, b in zip(("fwd", "pre-activation", "dx"), *results):
+        assert (a - b).abs().max().item() <= TF32_TOL * b.abs().max().item(), name
+
+
 def test_deterministic(pkg, dev):
     """Two runs of every operator give identical bits (fixed-order split-K reduction)."""
     F = pkg.functional
