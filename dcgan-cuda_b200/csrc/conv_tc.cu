@@ -308,7 +308,7 @@ Tiling choose_tiling(int m_count, int n_ch, int granule, int min_stages, int max
         t.cost = t.bn <= kMaxSharedWidth && !t_plan_x3 ? waves * loop + epilogue : waves * (loop + epilogue);
         t.second_launch = false;
         t.walk = may_walk && t.splits == 1 && t.grid > sms;
-        if (t.walk) t.cost = 1200.0 + waves * (double)max_stages * stage + epilogue;
+        if (t.walk) t.cost = 1200.0 + waves * (double)max_stages * (stage + (b_pieces ? 20.0 * ((t.bn + 31) / 32 - 1) : 0.0)) + epilogue;
         if (best.grid == 0 || t.cost < best.cost) best = t;
         // the same tiles with a second launch
         const int tiles = m_count * t.n_tiles;
@@ -480,7 +480,7 @@ bool plan_fwd(const dcg_conv_desc& d, Plan& pl, bool fit = true)
         p.splits = choose_splits(m_count * p.n_tiles, stages);
         pl.grid = m_count * p.n_tiles * p.splits;
     } else {
-        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35, 2, pieces, 0, !pieces));
+        use_tiling(pl, choose_tiling(m_count, d.o, 32, stages, stages, 35, 2, pieces, 0, true));
     }
     return finish_plan(pl);
 }
@@ -844,9 +844,12 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
 template <int MODE>
 int launch_walk(const CUtensorMap& ma, const CUtensorMap& mb, const Plan& pl, cudaStream_t stream)
 {
-    static OncePerDevice once;
-    DCG_CUDA(allow_smem(once, conv_tc_walk_kernel<MODE>, kMaxSmem));
-    launch_pdl(conv_tc_walk_kernel<MODE>, (unsigned)std::min(pl.grid, sm_count()), kWalkThreads, pl.smem, stream, ma, mb, pl.p, pl.grid);
+    using Kernel = void (*)(CUtensorMap, CUtensorMap, Params, int);
+    static const Kernel kernels[2] = {conv_tc_walk_kernel<MODE>, conv_tc_walk_kernel<MODE, MODE == MODE_FWD>};
+    static OncePerDevice once[2];
+    const int pieces = pl.p.mt == 0;
+    DCG_CUDA(allow_smem(once[pieces], kernels[pieces], kMaxSmem));
+    launch_pdl(kernels[pieces], (unsigned)std::min(pl.grid, sm_count()), kWalkThreads, pl.smem, stream, ma, mb, pl.p, pl.grid);
     DCG_LAUNCH_CHECK("conv_tc_walk_kernel");
     return DCG_OK;
 }

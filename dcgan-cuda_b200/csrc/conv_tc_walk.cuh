@@ -21,7 +21,8 @@ __host__ __device__ constexpr size_t walk_smem(int stages, int bn)
     return 1024 + (size_t)stages * (A_STAGE_BYTES + bn * BK * 4) + kWalkEpi / 32 * kWalkPatch + 16 * stages + 64;
 }
 
-template <int MODE>
+// PIECES (forward): ragged channel counts, B in loads of 32 columns, of which those that exist.
+template <int MODE, bool PIECES = false>
 __global__ void __launch_bounds__(kWalkThreads, 1)
 conv_tc_walk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ Params p, const int tiles)
@@ -98,13 +99,14 @@ conv_tc_walk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 0 || warp == 2 + kWalkEpi / 32) {
         // ===== TMA producers: both walk all stages, one loads the even and one the odd ones =====
         const int mine = warp == 0 ? 0 : 1;
-        const uint32_t tx_bytes = (uint32_t)(p.TW * p.TH * p.TN * BK * 4) + b_stage;
+        const uint32_t a_bytes = (uint32_t)(p.TW * p.TH * p.TN * BK * 4);
         int s = 0, it = 0;
         uint32_t phase = 0;
         bool alive = true;
         pdl_enter();
         for (int tile = blockIdx.x; tile < tiles && alive; tile += gridDim.x) {
             const Tile t = decode(tile);
+            const int pieces = PIECES ? min(p.bn >> 5, (p.b_ch - t.n_tile * p.bn + 31) >> 5) : 0;
             int chunk = 0, tap = 0, di = 0, dj = 0;
             for (int q = 0; q < t.nq; ++q, ++it) {
                 if ((it & 1) == mine) {
@@ -112,10 +114,15 @@ conv_tc_walk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if (it != p.skip_stage && elect_one()) {
                         const uint32_t fb = full_bar + 8u * s;
                         const uint32_t a_dst = a_base + (uint32_t)s * A_STAGE_BYTES, b_dst = b_base + (uint32_t)s * b_stage;
-                        mbar_expect_tx(fb, tx_bytes);
+                        mbar_expect_tx(fb, a_bytes + (PIECES ? (uint32_t)pieces * kPieceBytes : b_stage));
                         if (MODE == MODE_FWD) {
                             tma_load_4d(a_dst, &map_a, fb, chunk * BK, p.sw * t.j0 + dj - p.pl, p.sh * t.i0 + di - p.pt, t.n0);
-                            tma_load_4d(b_dst, &map_b, fb, 0, chunk * BK, tap, t.n_tile * (p.bn / 32));
+                            if constexpr (PIECES) {
+                                for (int i = 0; i < pieces; ++i)
+                                    tma_load_4d(b_dst + i * kPieceBytes, &map_b, fb, t.n_tile * p.bn + 32 * i, chunk * BK, tap, 0);
+                            } else {
+                                tma_load_4d(b_dst, &map_b, fb, 0, chunk * BK, tap, t.n_tile * (p.bn / 32));
+                            }
                         } else {   // (di, dj) count the taps of this parity class: kernel tap (rh + sh*di, rw + sw*dj)
                             tma_load_4d(a_dst, &map_a, fb, chunk * BK, t.j0 + t.ew - dj, t.i0 + t.eh - di, t.n0);
                             tma_load_4d(b_dst, &map_b, fb, chunk * BK, t.n_tile * p.bn, t.rw + p.sw * dj, t.rh + p.sh * di);
