@@ -496,7 +496,8 @@ void build_lists(dcg_trainer* t)
         const float* in = i == 0 ? t->g0a.p : t->ga[i - 1].p;
         G.push_back(side(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->dgz[i].p, nullptr, t->g_grad[2 * i + 1].p, rows, kGChan[i + 1])));
         const dcg_node dk = n_conv2d_transpose_kernel_grad(t->dgz[i].p, in, t->g_grad[2 * i].p, B, h, kGChan[i], kGChan[i + 1]);
-        if (i > 0) G.push_back(side(dk));
+        const bool last = i == 0 && t->batched_d;
+        if (!last) G.push_back(side(dk));
         float* dprev_a = i == 0 ? t->dg0a.p : t->dga[i - 1].p;
         G.push_back(dead(n_conv2d_transpose_input_grad(t->dgz[i].p, t->g_param[2 * i].p, dprev_a, B, h, kGChan[i], kGChan[i + 1])));
         float* dprev_z = i == 0 ? t->dg0z.p : t->dgz[i - 1].p;
@@ -506,7 +507,7 @@ void build_lists(dcg_trainer* t)
         if (i == 0) {   // the last kernel gradient on the main stream, which has nothing more to do, not behind the one before it
             G.push_back(side(n_mat3(DCG_OP_TMAT_MAT_MUL, t->z.p, t->dg0z.p, t->g_grad[8].p, kZ, B, 8192)));
             G.push_back(side(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->dg0z.p, nullptr, t->g_grad[9].p, B, 8192)));
-            G.push_back(dk);
+            if (last) G.push_back(dk);
         }
     }
 }
