@@ -24,10 +24,11 @@
 // activation-gradient gate) into HBM; in the 3xTF32 variant they also build the residual tiles of
 // every stage.  A ring of smem stages (A 16 KB + B BN*128 B, 128-byte swizzle; 7 deep with one
 // CTA per SM) is handed over with mbarriers: TMA complete_tx -> MMA, tcgen05.commit -> TMA.
-// The K partitions of one tile form a thread-block cluster: each writes its fp32 partial tile to
-// scratch (L2-resident), the cluster meets at a hardware barrier, and every CTA then adds the
-// partials of its share of the tile in partition order (deterministic) and finishes it, fused
-// epilogue included - one launch per convolution, no reduction kernel.
+// The K partitions of one tile form a thread-block cluster: each writes the other partitions' shares of its
+// fp32 partial tile to scratch (L2-resident), the cluster meets at a hardware barrier, and every CTA then
+// adds the others' partials to its own share, in partition order (deterministic), and finishes it, fused
+// epilogue included - one launch per convolution.  Kernel gradients of few tiles take more partitions than a
+// cluster holds and a second launch that adds them (dk_finish_kernel).
 //
 // Every wait is bounded: a barrier that does not complete within ~1 s makes the waiting role
 // record an error code in a device status word and leave; TMEM is always released.

@@ -531,11 +531,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     // ===== the K partitions of a tile meet =====
     // The S partitions of one tile form a thread-block cluster, which guarantees that they run at the
-    // same time and gives them a hardware barrier.  Each partition writes its partial accumulator
-    // to scratch (it stays in L2), the cluster meets, and partition j then finishes a 1/S share of
-    // the tile: it adds the S partials in partition order - so the result does not depend on timing -
-    // applies the fused chain and writes the final tensor.  (Handing the partials over through
-    // distributed shared memory instead was measured at under 10 bytes per clock and SM.)
+    // same time and gives them a hardware barrier.  Each partition writes the others' shares of its partial
+    // accumulator to scratch (it stays in L2), the cluster meets, and partition j then finishes a 1/S share of
+    // the tile: it adds the others' partials to its own in partition order - so the result does not depend
+    // on timing - applies the fused chain and writes the final tensor.  (Through distributed shared memory, by
+    // stores or by bulk copies that the receiver's barrier counts, it takes as long or longer.)
     // Partials are stored quad-major, [CTA][16-byte column quad][row]: lanes are consecutive rows, so
     // both the partial stores and the loads of the second phase move 512 contiguous bytes per warp.
     // Without partitions the same layout in shared memory (quad pitch QS) is the transposition buffer
