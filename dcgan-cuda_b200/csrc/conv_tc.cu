@@ -47,7 +47,9 @@
 //   conv_tc_narrow.cuh   repack, partition-finish and gather helpers of the 3-channel layers
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -537,6 +539,27 @@ int dxf_mode()
     return m >= 0 ? m : from_env;
 }
 
+// Whether the parity classes are quicker as tiles of their own, walked by persistent CTAs, than all of them together in `tiles`
+// tiles of `bn` columns.  In clocks: a (class, tap) pair of a 32-channel chunk takes 233 of them at 64 columns and 297 at 128 in
+// the class-fused kernel, a stage of the other one 300 at 128 columns and 512 at 256; a column of a class costs an epilogue 20,
+// of which half of the shorter of loop and epilogue is hidden.  The class-fused tiles are four times as large, in boxes of powers
+// of two and of at most 128 columns, which leaves much of them empty where the image, the channels or the last wave do not fit: 3 x 3 /
+// stride 2, 192 -> 64, 30 images of 33 x 47 27.0 us fused, 13.6 apart; 192 -> 192, 32 images of 96 x 96 165 and 111.
+// Where they fit, fused is quicker (5 x 5 / stride 2, 64 -> 128 of 64 images 16.4 and 22.2, 256 -> 512 of 512 images 74 and 90).
+bool classes_apart_quicker(const dcg_conv_desc& d, int tiles, int bn, int ncls)
+{
+    Plan apart;
+    if (!plan_dx(d, apart) || !apart.p.walk) return false;
+    const Params& p = apart.p;
+    const double sms = sm_count(), pairs = (double)d.kh * d.kw * ((d.o + BK - 1) / BK);
+    auto both = [](double loop, double epilogue) { return std::max(loop, epilogue) + 0.5 * std::min(loop, epilogue); };
+    const double fused = std::ceil(tiles / sms) * both(pairs * (bn <= 64 ? 233.0 : 169.0 + bn), 20.0 * ncls * bn);
+    const double stage = p.bn > 128 ? 300.0 + (p.bn - 128) * (212.0 / 128) : 300.0;
+    const double mine = both((double)p.tiles_w * p.tiles_h * p.tiles_n * p.n_tiles * pairs / sms * stage, std::ceil(apart.grid / sms) * 20.0 * p.bn) +
+                        0.5 * stage * pairs / ncls;   // (the classes differ in length)
+    return mine < 0.9 * fused;
+}
+
 // The class-fused input gradient (conv_dxf_kernel): windows of dy, the (class, tap) pairs that read each, and
 // the order of both.
 bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
@@ -663,6 +686,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     int units = (kMaxSmem - fixed) / kCfUnit;
     if (units > kCfMaxUnits) units = kCfMaxUnits;
     if (units < 3 * max_units) return false;   // three stages in flight
+    if (mode == 1 && classes_apart_quicker(d, tiles, bn, ncls)) return false;
     p.stages = units;
     pl.smem = (size_t)units * kCfUnit + fixed;
     p.skip_stage = -1;

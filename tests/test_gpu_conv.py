@@ -609,7 +609,7 @@ def test_forward_of_rgb_layers(pkg, dev, shape):
 # more tiles than SMs, walked by persistent CTAs: one to three tiles each and a last round that is nearly empty, widths of 16 to 192
 # columns, the last column tile partly beyond the channels, parity classes, channels that are no multiple of four, one stage a tile
 @pytest.mark.parametrize("shape", [(24, 48, 48, 32, 1, 192, 1), (13, 75, 51, 96, 3, 160, 1), (32, 40, 40, 64, 3, 96, 1), (37, 60, 60, 20, 5, 64, 2),
-                                   (40, 33, 35, 6, 3, 32, 1), (150, 12, 11, 32, 3, 288, 1), (20, 64, 64, 8, 1, 32, 1)])
+                                   (40, 33, 35, 6, 3, 32, 1), (150, 12, 11, 32, 3, 288, 1), (20, 64, 64, 8, 1, 32, 1), (16, 50, 50, 40, 3, 44, 1)])
 def test_more_tiles_than_sms(pkg, dev, shape):
     F = pkg.functional
     N, H, W, C, K, O, s = shape
@@ -629,6 +629,20 @@ def test_more_tiles_than_sms(pkg, dev, shape):
     assert pkg.lib.dcg_device_status() == 0
     for name, a, b in zip(("fwd", "pre-activation", "dx"), *results):
         assert (a - b).abs().max().item() <= TF32_TOL * b.abs().max().item(), name
+
+
+# parity classes together where their tiles fit the layer, as tiles of their own where they would be half empty
+@pytest.mark.parametrize("shape,fused", [((64, 32, 32, 64, 5, 128, 2), True), ((30, 33, 47, 192, 3, 64, 2), False), ((9, 96, 96, 192, 3, 64, 2), False)])
+def test_parity_classes_together_or_apart(pkg, dev, shape, fused):
+    F = pkg.functional
+    N, H, W, C, K, O, s = shape
+    k, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((71, (K, K, C, O)), (72, (N, -(-H // s), -(-W // s), O))))
+    before = pkg.lib.dcg_debug_fused_dx_launches()
+    got, ref = (F.conv2d_dx(dy, k, (H, W), (s, s), precision=p) for p in (pkg.PREC_TF32, pkg.PREC_FP32))
+    torch.cuda.synchronize()
+    assert pkg.lib.dcg_device_status() == 0
+    assert pkg.lib.dcg_debug_fused_dx_launches() - before == int(fused)
+    assert (got - ref).abs().max().item() <= TF32_TOL * ref.abs().max().item()
 
 
 def test_deterministic(pkg, dev):
