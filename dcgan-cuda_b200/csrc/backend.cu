@@ -9,8 +9,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <initializer_list>
-#include <mutex>
-#include <set>
 #include <string>
 #include <utility>
 #include <vector>
@@ -32,8 +30,7 @@ struct dcg_context {
     cudaStream_t stream = nullptr;
     int precision = DCG_PREC_TF32;
     void* ws = nullptr;
-    size_t ws_bytes = 0;          // usable by the operators; an owned allocation has the ticket words behind it
-    unsigned* tickets = nullptr;  // kColsumTicketBytes of zeroed ticket words of the column sums (owned scratch only)
+    size_t ws_bytes = 0;
     bool owns_ws = false;
     // Bumped whenever something a captured CUDA graph bakes in changes: a scratch buffer (main or
     // side) moved, or the precision (which selects kernels and plans) was switched.
@@ -46,7 +43,6 @@ struct dcg_context {
     cudaStream_t side[2] = {nullptr, nullptr};
     void* side_ws[2] = {nullptr, nullptr};
     size_t side_ws_bytes[2] = {0, 0};
-    unsigned* side_tickets[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
     bool side_busy[2] = {false, false}, side_failed = false;
     uint64_t launches_base = 0;
@@ -58,23 +54,6 @@ namespace dcg {
 
 bool context_is_profiling(const dcg_context* ctx) { return ctx && ctx->profiling; }
 uint64_t context_generation(const dcg_context* ctx) { return ctx ? ctx->generation : 0; }
-
-namespace {
-std::mutex g_registry_mutex;
-std::set<dcg_context*> g_registry;
-}  // namespace
-
-void contexts_reset_tickets()
-{
-    std::lock_guard<std::mutex> lock(g_registry_mutex);
-    cudaDeviceSynchronize();
-    for (dcg_context* c : g_registry) {
-        if (c->tickets) cudaMemset(c->tickets, 0, kColsumTicketBytes);
-        for (int i = 0; i < 2; ++i)
-            if (c->side_tickets[i]) cudaMemset(c->side_tickets[i], 0, kColsumTicketBytes);
-    }
-    cudaGetLastError();
-}
 
 // Times everything enqueued on the context's stream during its lifetime when profiling is on.
 ProfScope::ProfScope(dcg_context* c, const char* name, double flops) : ctx(c), active(c && c->profiling)
@@ -129,20 +108,15 @@ int ensure_workspace(dcg_context* ctx, size_t bytes)
     if (ctx->ws) DCG_CUDA(cudaFree(ctx->ws));
     ctx->ws = nullptr;
     ctx->ws_bytes = 0;
-    ctx->tickets = nullptr;
     ++ctx->generation;   // graphs captured with the old address are stale
     const size_t want = align_up(bytes + bytes / 4, (size_t)1 << 20);
-    DCG_CUDA(cudaMalloc(&ctx->ws, want + kColsumTicketBytes));
-    // the ticket words of the column sums sit behind the usable part and start out zero
-    ctx->tickets = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(ctx->ws) + want);
-    DCG_CUDA(cudaMemset(ctx->tickets, 0, kColsumTicketBytes));
+    DCG_CUDA(cudaMalloc(&ctx->ws, want));
     ctx->ws_bytes = want;
     ctx->owns_ws = true;
     return DCG_OK;
 }
 
-// Column sum on the context's scratch.  Owned scratch carries its own zeroed ticket words; a
-// caller-provided buffer goes through the public entry point, which clears them per call.
+// Column sum on the context's scratch.  A caller-provided buffer goes through the public entry point and its demands.
 int context_colsum(dcg_context* ctx, const float* a, float* out, size_t rows, size_t cols)
 {
     DCG_CHECK_ARG(a && out && rows > 0 && cols > 0 && cols <= 0x7fffffffu, "column sum node: bad operands");
@@ -155,7 +129,7 @@ int context_colsum(dcg_context* ctx, const float* a, float* out, size_t rows, si
     const size_t need = colsum_partial_bytes_max(rows, cols);
     int st = ensure_workspace(ctx, need > 0 ? need : 1);
     if (st) return st;
-    return colsum_launch(a, out, rows, cols, ctx->ws, ctx->ws_bytes, ctx->tickets, ctx->stream);
+    return colsum_launch(a, out, rows, cols, ctx->ws, ctx->ws_bytes, ctx->stream);
 }
 
 struct ConvCall {
@@ -453,10 +427,6 @@ extern "C" int dcg_context_create(dcg_context** out, int precision, void* worksp
     ctx->ws_bytes = workspace_bytes;
     ctx->owns_ws = false;
     ctx->launches_base = launches_total();
-    {
-        std::lock_guard<std::mutex> lock(g_registry_mutex);
-        g_registry.insert(ctx);
-    }
     *out = ctx;
     return DCG_OK;
 }
@@ -464,10 +434,6 @@ extern "C" int dcg_context_create(dcg_context** out, int precision, void* worksp
 extern "C" void dcg_context_destroy(dcg_context* ctx)
 {
     if (!ctx) return;
-    {
-        std::lock_guard<std::mutex> lock(g_registry_mutex);
-        g_registry.erase(ctx);
-    }
     if (ctx->owns_ws && ctx->ws) cudaFree(ctx->ws);
     for (int i = 0; i < 2; ++i) {
         if (ctx->side_ws[i]) cudaFree(ctx->side_ws[i]);
@@ -670,7 +636,6 @@ int run_side_node(dcg_context* ctx, const dcg_node* nd)
     std::swap(ctx->stream, ctx->side[i]);
     std::swap(ctx->ws, ctx->side_ws[i]);
     std::swap(ctx->ws_bytes, ctx->side_ws_bytes[i]);
-    std::swap(ctx->tickets, ctx->side_tickets[i]);
     const bool owns = ctx->owns_ws;
     ctx->owns_ws = true;
     const int st = dcg_run_node(ctx, nd);
@@ -678,7 +643,6 @@ int run_side_node(dcg_context* ctx, const dcg_node* nd)
     std::swap(ctx->stream, ctx->side[i]);
     std::swap(ctx->ws, ctx->side_ws[i]);
     std::swap(ctx->ws_bytes, ctx->side_ws_bytes[i]);
-    std::swap(ctx->tickets, ctx->side_tickets[i]);
     ctx->side_busy[i] = true;
     return st;
 }

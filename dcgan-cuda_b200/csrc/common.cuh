@@ -94,16 +94,10 @@ inline cudaError_t allow_smem(OncePerDevice& once, Kernel kernel, size_t bytes)
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// ---- column sums: internal launch with caller-owned ticket words (elementwise.cu) ---------------
-// kColsumTicketBytes of ZEROED device memory that only stream-ordered launches share; the kernel
-// leaves them zero.  colsum_partial_bytes_max: scratch for the partial sums alone (0: none needed).
-constexpr size_t kColsumTicketBytes = 4096;
-int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* workspace, size_t workspace_bytes,
-                  unsigned* tickets, cudaStream_t stream);
+// ---- column sums: internal launch (elementwise.cu) -----------------------------------------------
+// colsum_partial_bytes_max: scratch for the partial sums alone (0: none needed).
+int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 size_t colsum_partial_bytes_max(size_t rows, size_t cols);
-// Clears the ticket words of every live context (after a kernel reported an error, a launch may
-// have left some of them counted up).  Synchronises the device.
-void contexts_reset_tickets();
 // Status word of the fused data-parallel update (dp_adam.cu): DCG_OK, or DCG_ERR_DEVICE after a wait for
 // a peer ran out.  Reads and clears; the caller has synchronised the device.
 int dp_status_check();

@@ -1522,7 +1522,6 @@ int conv_tc_device_status(int* detail /* [4] */)
     if (h[0] != 0) {
         const int zero[4] = {0, 0, 0, 0};
         DCG_CUDA(cudaMemcpyToSymbol(g_tc_status, zero, sizeof(zero)));
-        contexts_reset_tickets();   // a launch that gave up may have left column-sum tickets counted up
         return fail(DCG_ERR_DEVICE, "tensor-path kernel gave up waiting: code %d block %d role %d stage %d",
                     h[0], h[1], h[2], h[3]);
     }

@@ -125,81 +125,18 @@ update_kernel(const float* __restrict__ dv, float* __restrict__ out,
 }
 
 // ---- column sums (bias gradient) ---------------------------------------------
-// Block (tx over column groups, ty over rows) reduces a slab of rows into
-// partial[slab][cols].  VEC: a column group is one float4.  The slabs of one column tile are
-// then added by whichever of its blocks finishes last (a ticket per column tile tells it so):
-// lane l adds slabs l, l+L, ... and the lane sums are added in lane order, so the result depends
-// on the launch shape only, never on which block came last.  `tickets` == nullptr leaves the
-// slabs to colsum_final_kernel.
-// The ticket words belong to whoever owns the scratch of the launch (they sit behind the partial
-// sums in the caller's buffer, or at the tail of a context's scratch allocation), so two launches
-// only ever share tickets if they share scratch - which already requires them to be stream-ordered.
-// They must be zero when a launch starts; every adder resets the ticket it consumed.
-constexpr int kTicketTiles = 16, kSlabGroup = 16, kMaxSlabs = 1008;
-constexpr int kTicketsPerTile = 1 + kMaxSlabs / kSlabGroup;         // group-level ticket + one per slab group
-constexpr size_t kTicketBytes = (size_t)kTicketTiles * kTicketsPerTile * sizeof(unsigned);
-static_assert(kTicketBytes == dcg::kColsumTicketBytes, "ticket area size is part of the scratch contract");
-
-// One block adds `nrows` rows of src ([nrows][cols]) for its column tile into dst: thread = (column
-// group, lane); lane l adds rows l, l+L, ... through four independent accumulators (four loads in
-// flight), combined in a fixed order; the lane sums are then added in lane order.  The result
-// depends on the launch shape only.
-template <bool VEC>
-__device__ __forceinline__ void colsum_add_rows(const float* __restrict__ src, unsigned nrows, float* __restrict__ dst,
-                                                unsigned cols, int tx_count, unsigned groups, float* smem)
-{
-    constexpr int W = VEC ? 4 : 1;
-    const int lanes = blockDim.x / tx_count;     // >= 8
-    const int g = threadIdx.x % tx_count, l = threadIdx.x / tx_count;
-    const unsigned grp = blockIdx.x * tx_count + g;
-    float4 t[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) t[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (grp < groups) {
-        unsigned k = l;
-        for (; k + 3 * lanes < nrows; k += 4 * lanes) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float* p = src + (size_t)(k + u * lanes) * cols + (size_t)grp * W;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (VEC) v = __ldcg(reinterpret_cast<const float4*>(p));
-                else v.x = __ldcg(p);
-                t[u].x += v.x; t[u].y += v.y; t[u].z += v.z; t[u].w += v.w;
-            }
-        }
-        for (int u = 0; k < nrows; k += lanes, ++u) {   // at most three rows left per lane
-            const float* p = src + (size_t)k * cols + (size_t)grp * W;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (VEC) v = __ldcg(reinterpret_cast<const float4*>(p));
-            else v.x = __ldcg(p);
-            t[u & 3].x += v.x; t[u & 3].y += v.y; t[u & 3].z += v.z; t[u & 3].w += v.w;
-        }
-    }
-    float4 s4;
-    s4.x = (t[0].x + t[1].x) + (t[2].x + t[3].x); s4.y = (t[0].y + t[1].y) + (t[2].y + t[3].y);
-    s4.z = (t[0].z + t[1].z) + (t[2].z + t[3].z); s4.w = (t[0].w + t[1].w) + (t[2].w + t[3].w);
-    __syncthreads();                             // smem is reused: [lane][group][W]
-    float* slot = smem + ((size_t)l * tx_count + g) * W;
-    slot[0] = s4.x;
-    if (VEC) { slot[1] = s4.y; slot[2] = s4.z; slot[3] = s4.w; }
-    __syncthreads();
-    if (l == 0 && grp < groups) {
-#pragma unroll
-        for (int q = 0; q < W; ++q) {
-            float r = smem[(size_t)g * W + q];
-            for (int j = 1; j < lanes; ++j) r += smem[((size_t)j * tx_count + g) * W + q];
-            dst[(size_t)grp * W + q] = r;
-        }
-    }
-}
+// Block (tx over column groups, ty over rows) reduces a slab of rows into partial[slab][cols].  VEC: a column group is one
+// float4.  A second launch adds the slabs, set up under the first one: sixteen slabs at a time, then those sums
+// (colsum_meet_kernel), or over eight lanes where the column tiles are many (colsum_final_kernel).  The result depends on the
+// launch shape only.
+constexpr int kMeetTiles = 16, kSlabGroup = 16, kMaxSlabs = 1008;
 
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
 colsum_partial_kernel(const float* __restrict__ a, float* __restrict__ partial,
-                      size_t rows, unsigned cols, unsigned rows_per_slab, int tx_count,
-                      float* __restrict__ out, unsigned* __restrict__ tickets)
+                      size_t rows, unsigned cols, unsigned rows_per_slab, int tx_count)
 {
-    pdl_enter();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ float smem[];  // [ty_count][tx_count * (VEC ? 4 : 1)]
     const int ty_count = blockDim.x / tx_count;
     const int tx = threadIdx.x % tx_count;
@@ -235,6 +172,9 @@ colsum_partial_kernel(const float* __restrict__ a, float* __restrict__ partial,
         for (; r + 7 * (size_t)ty_count < r1; r += 8 * (size_t)ty_count) eight_rows(r, std::false_type());
         if (r < r1) eight_rows(r, std::true_type());
     }
+    // the next kernel is let in only now: its blocks would hold registers that other streams' kernels can use meanwhile
+    // (a training step of 256 images 0.5 % quicker than with the second launch let in at the start)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int W = VEC ? 4 : 1;
     float* mine = smem + ((size_t)ty * tx_count + tx) * W;
     mine[0] = acc.x;
@@ -253,58 +193,64 @@ colsum_partial_kernel(const float* __restrict__ a, float* __restrict__ partial,
 #pragma unroll
         for (int q = 0; q < W; ++q) dst[q] = mine[q];
     }
-    if (tickets == nullptr) return;
-    // ---- two levels of "whoever finishes last adds": 16 slabs -> one group row, all group rows -> out ----
-    // tickets of this column tile: [0] the group level, [1 + g] slab group g.  Each adder resets its
-    // ticket, so a set is ready for the next launch that uses it.
-    unsigned* my_tickets = tickets + (size_t)blockIdx.x * kTicketsPerTile;
-    const unsigned slabs = gridDim.y, n_groups = (slabs + kSlabGroup - 1) / kSlabGroup;
-    const unsigned g_idx = blockIdx.y / kSlabGroup;
-    const unsigned g_first = g_idx * kSlabGroup;
-    const unsigned g_count = slabs - g_first < (unsigned)kSlabGroup ? slabs - g_first : (unsigned)kSlabGroup;
-    float* level2 = partial + (size_t)slabs * cols;      // [n_groups][cols], behind the slab rows
-    __shared__ unsigned s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(my_tickets + 1 + g_idx, 1u);
-        s_last = (t == g_count - 1) ? 1u : 0u;
-        if (s_last) my_tickets[1 + g_idx] = 0u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    colsum_add_rows<VEC>(partial + (size_t)g_first * cols, g_count, n_groups > 1 ? level2 + (size_t)g_idx * cols : out,
-                         cols, tx_count, groups, smem);
-    if (n_groups == 1) return;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(my_tickets, 1u);
-        s_last = (t == n_groups - 1) ? 1u : 0u;
-        if (s_last) my_tickets[0] = 0u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    colsum_add_rows<VEC>(level2, n_groups, out, cols, tx_count, groups, smem);
 }
 
-// Clears the ticket words of a caller's buffer.  A kernel, for a memset between two launches keeps the second one from being set
-// up under the first (a layer of 13 images of 75 x 51, 96 -> 160 channels, called op by op 122.5 -> 119.5 us).
-static_assert(kTicketBytes % sizeof(unsigned) == 0, "cleared by words");
-__global__ void __launch_bounds__(256)
-clear_tickets_kernel(unsigned* __restrict__ tickets)
+// Adds the slabs of kMeetCols columns: a thread per group of sixteen slabs and column, all its loads in flight, then a thread per
+// lane and column, then one per column.  A column tile of the first kernel had L lanes (threads over rows): lane l adds slabs
+// l, l + L, ... of a group and the lanes are added in lane order; the groups' sums in the same way, a lane with four sums that
+// take turns.  Bound by its launch and a trip to L2.  Blocks of the first kernel that find out by tickets who comes last, and add
+// then, take five trips after the loads and a launch in front that clears the tickets: 4340 x 156 8.7 us, 3.9 now, 65536 x 64
+// 10.0 and 5.0, 49725 x 160 10.9 and 6.8, 262144 x 64 12.3 and 8.4.
+constexpr int kMeetCols = 4, kMeetGroups = kMaxSlabs / kSlabGroup, kMeetThreads = 256;
+static_assert(kMaxSlabs % kSlabGroup == 0 && kMeetCols * kMeetGroups <= kMeetThreads, "a thread per group of slabs and column");
+__global__ void __launch_bounds__(kMeetThreads)
+colsum_meet_kernel(const float* __restrict__ partial, float* __restrict__ out, unsigned slabs, unsigned cols, unsigned lanes)
 {
     pdl_enter();
-    for (unsigned i = threadIdx.x; i < kTicketBytes / sizeof(unsigned); i += 256) tickets[i] = 0u;
+    __shared__ float sums[kMeetGroups][kMeetCols], lane_sums[kMeetGroups][kMeetCols];
+    const unsigned tx = threadIdx.x % kMeetCols, ty = threadIdx.x / kMeetCols, c = blockIdx.x * kMeetCols + tx;
+    const unsigned n_groups = (slabs + kSlabGroup - 1) / kSlabGroup;
+    if (ty < n_groups && c < cols) {
+        float v[kSlabGroup];
+#pragma unroll
+        for (unsigned u = 0; u < kSlabGroup; ++u) {
+            const unsigned k = ty * kSlabGroup + u;
+            v[u] = k < slabs ? __ldcg(partial + (size_t)k * cols + c) : 0.f;
+        }
+        if (lanes == kSlabGroup / 2) {
+#pragma unroll
+            for (unsigned u = 0; u < kSlabGroup / 2; ++u) { v[u] += v[u + kSlabGroup / 2]; v[u + kSlabGroup / 2] = 0.f; }
+        }
+        float r = v[0];
+#pragma unroll
+        for (unsigned u = 1; u < kSlabGroup; ++u) r += v[u];
+        if (n_groups == 1) out[c] = r;
+        sums[ty][tx] = r;
+    }
+    if (n_groups == 1) return;
+    __syncthreads();
+    const unsigned n_lanes = min(lanes, n_groups);
+    if (ty < n_lanes) {
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (unsigned i = 0; i < kMeetGroups / 8 + 1; ++i)
+            if (ty + i * lanes < n_groups) t[i & 3] += sums[ty + i * lanes][tx];
+        lane_sums[ty][tx] = (t[0] + t[1]) + (t[2] + t[3]);
+    }
+    __syncthreads();
+    if (ty == 0 && c < cols) {
+        float r = lane_sums[0][tx];
+#pragma unroll 8
+        for (unsigned j = 1; j < n_lanes; ++j) r += lane_sums[j][tx];
+        out[c] = r;
+    }
 }
 
 // The same sums for a few hundred rows, a column tile per block: at most kSmallSlabs slabs of at most four rows per lane, side
 // by side with all loads in flight at once.  The plan of colsum_partial_kernel sets the order of the additions and this kernel only
-// spreads them over threads, so the result is the same bit for bit; what is saved is the hand-over of partial sums between blocks
-// and the memset of the ticket words.
-constexpr unsigned kSmallSlabs = 8;
+// spreads them over threads, so the result is the same bit for bit; what is saved is the hand-over of partial sums between blocks.
+constexpr unsigned kSmallSlabs = kSlabGroup, kSmallPlaces = 2048;   // (sixteen slabs of 128 lanes, eight of 256: up to
+    // there the one launch is the quicker, 400 x 160 2.8 us against 3.1, 512 x 512 2.9 and 3.2; 900 x 64 even, 3.2 and 3.0)
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
 colsum_small_kernel(const float* __restrict__ a, float* __restrict__ out, unsigned rows, unsigned cols, const dcg::ColsumOrder order, int tile_shift)
@@ -750,7 +696,7 @@ ColsumPlan colsum_plan(size_t rows, size_t cols, bool ptr_aligned)
     if (p.rows_per_slab < 1) p.rows_per_slab = 1;
     p.slabs = (unsigned)((rows + p.rows_per_slab - 1) / p.rows_per_slab);
     if (p.slabs < 1) p.slabs = 1;
-    p.small = p.slabs <= kSmallSlabs && p.rows_per_slab <= 4u * (unsigned)ty;
+    p.small = p.slabs <= kSmallSlabs && p.slabs * (unsigned)ty <= kSmallPlaces && p.rows_per_slab <= 4u * (unsigned)ty;
     return p;
 }
 
@@ -758,7 +704,7 @@ ColsumPlan colsum_plan(size_t rows, size_t cols, bool ptr_aligned)
 size_t colsum_partial_bytes(const ColsumPlan& p, size_t cols)
 {
     if (p.slabs <= 1 || p.small) return 0;
-    // slab rows plus one row per group of kSlabGroup slabs (the second level of the in-kernel sum)
+    // slab rows, and one row per group of kSlabGroup slabs (kept in shared memory since; see kColsumScratchTail)
     return (size_t)(p.slabs + (p.slabs + kSlabGroup - 1) / kSlabGroup) * cols * sizeof(float);
 }
 }  // namespace
@@ -769,21 +715,19 @@ bool colsum_order(size_t rows, size_t cols, bool aligned, unsigned max_slabs, Co
     const ColsumPlan p = colsum_plan(rows, cols, aligned);
     const int lanes = kThreads / p.tx_count;
     if (p.slabs > max_slabs || p.rows_per_slab > 4u * (unsigned)lanes) return false;
-    if (p.slabs > kSlabGroup * kSlabGroup) return false;   // (colsum_add_rows keeps four sums per lane from here on)
-    const bool tickets = p.grid_x <= (unsigned)kTicketTiles;   // otherwise colsum_final_kernel adds all slabs, over eight lanes
+    if (p.slabs > kSlabGroup * kSlabGroup) return false;   // (colsum_meet_kernel keeps four sums per lane from here on)
+    const bool meet = p.grid_x <= (unsigned)kMeetTiles;   // otherwise colsum_final_kernel adds all slabs, over eight lanes
     int lane_shift = 0;
     while (1 << lane_shift < lanes) ++lane_shift;
-    t.order = ColsumOrder{p.rows_per_slab, p.slabs, tickets ? (unsigned)kSlabGroup : p.slabs, lane_shift, tickets ? lanes : 8};
+    t.order = ColsumOrder{p.rows_per_slab, p.slabs, meet ? (unsigned)kSlabGroup : p.slabs, lane_shift, meet ? lanes : 8};
     t.vec = p.vec;
     t.groups = p.groups;
     t.widest = 8 - lane_shift;   // the plan's own tile
     return true;
 }
 
-// The launch behind dcg_colsum.  `tickets`: kColsumTicketBytes of zeroed device memory owned by the
-// caller of this launch (see above), or nullptr to finish with a second kernel instead.
-int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* workspace, size_t workspace_bytes,
-                  unsigned* tickets, cudaStream_t stream)
+// The launches behind dcg_colsum.
+int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* workspace, size_t workspace_bytes, cudaStream_t stream)
 {
     const ColsumPlan p = colsum_plan(rows, cols, aligned16(a) && aligned16(workspace));
     const size_t need = colsum_partial_bytes(p, cols);
@@ -806,15 +750,18 @@ int colsum_launch(const float* a, float* out, size_t rows, size_t cols, void* wo
     }
     const dim3 grid(p.grid_x, p.slabs);
     const size_t smem = (size_t)kThreads * (p.vec ? 4 : 1) * sizeof(float);
-    if (p.slabs <= 1 || p.grid_x > (unsigned)kTicketTiles) tickets = nullptr;   // nothing to add / too many column tiles
     if (p.vec)
         launch_pdl(colsum_partial_kernel<true>, grid, kThreads, smem, stream,
-            a, partial, rows, (unsigned)cols, p.rows_per_slab, p.tx_count, out, tickets);
+            a, partial, rows, (unsigned)cols, p.rows_per_slab, p.tx_count);
     else
         launch_pdl(colsum_partial_kernel<false>, grid, kThreads, smem, stream,
-            a, partial, rows, (unsigned)cols, p.rows_per_slab, p.tx_count, out, tickets);
+            a, partial, rows, (unsigned)cols, p.rows_per_slab, p.tx_count);
     DCG_LAUNCH_CHECK("colsum_partial_kernel");
-    if (p.slabs > 1 && !tickets) {
+    if (p.slabs > 1 && p.grid_x <= (unsigned)kMeetTiles) {
+        launch_pdl(colsum_meet_kernel, (unsigned)((cols + kMeetCols - 1) / kMeetCols), kMeetThreads, 0, stream,
+            partial, out, p.slabs, (unsigned)cols, (unsigned)(kThreads / p.tx_count));
+        DCG_LAUNCH_CHECK("colsum_meet_kernel");
+    } else if (p.slabs > 1) {
         launch_pdl(colsum_final_kernel, (unsigned)((cols + 31) / 32), 256, 0, stream,
             partial, out, p.slabs, (unsigned)cols);
         DCG_LAUNCH_CHECK("colsum_final_kernel");
@@ -831,11 +778,14 @@ size_t colsum_partial_bytes_max(size_t rows, size_t cols)
 }
 }  // namespace dcg
 
+// What callers are asked for beyond the partial sums: nothing uses it, but the limit of dcg_colsum_noalloc and the sizes that
+// callers have laid out follow from it.
+constexpr size_t kColsumScratchTail = 4096;
 extern "C" size_t dcg_colsum_workspace_bytes(size_t rows, size_t cols)
 {
     const size_t partial = dcg::colsum_partial_bytes_max(rows, cols);
     if (partial == 0) return 0;
-    return align_up(partial, 256) + kTicketBytes;   // partial sums, then the ticket words
+    return align_up(partial, 256) + kColsumScratchTail;
 }
 
 extern "C" int dcg_colsum(const float* a, float* out, size_t rows, size_t cols, void* workspace,
@@ -844,18 +794,12 @@ extern "C" int dcg_colsum(const float* a, float* out, size_t rows, size_t cols, 
     DCG_CHECK_ARG(a && out, "dcg_colsum: null pointer");
     DCG_CHECK_ARG(cols > 0 && cols <= 0x7fffffffu && rows > 0, "dcg_colsum: bad shape %zu x %zu", rows, cols);
     const size_t need = dcg_colsum_workspace_bytes(rows, cols);
-    unsigned* tickets = nullptr;
     if (need > 0) {
         if (!workspace || workspace_bytes < need)
             return fail(DCG_ERR_WORKSPACE, "dcg_colsum: workspace %zu < %zu bytes", workspace_bytes, need);
         DCG_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 3u) == 0, "dcg_colsum: workspace is not 4-byte aligned");
-        // the caller's buffer may hold anything: clear the ticket words behind the partial sums on the
-        // same stream (never an allocation)
-        tickets = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(workspace) + need - kTicketBytes);
-        launch_pdl(clear_tickets_kernel, 1, 256, 0, as_stream(stream), tickets);
-        DCG_LAUNCH_CHECK("clear_tickets_kernel");
     }
-    return dcg::colsum_launch(a, out, rows, cols, workspace, need ? need - kTicketBytes : 0, tickets, as_stream(stream));
+    return dcg::colsum_launch(a, out, rows, cols, workspace, need, as_stream(stream));
 }
 
 extern "C" int dcg_rowsum(const float* a, float* out, size_t rows, size_t cols, dcg_stream_t stream)
