@@ -369,19 +369,27 @@ dcg_node side(dcg_node n)
     return n;
 }
 
+// What gates the gradient of a leaky relu.  The activation has the sign of the pre-activation, which then need not be written
+// (the lists flag it dead), with one exception: 0.2 times -1 or -2 times 2^-149 is -0.  The fp32 path promises the reference's
+// bits, so there the pre-activation is written and gates.  (A relu's activation is positive exactly where its input is.)
+bool gates_by_pre_activation(const dcg_trainer* t) { return t->cfg.precision == DCG_PREC_FP32; }
+
 // Generator forward: dcgan/main.cu:89-120 and :288 (tanh on the last layer's pre-activation).
 void build_generator(dcg_trainer* t, std::vector<dcg_node>& L)
 {
     const int B = t->cfg.batch;
     const int act = t->cfg.g_leaky ? DCG_OP_RELU_LEAKY : DCG_OP_RELU;
-    L.push_back(dead(n_mat_mul_add(t->z.p, t->g_param[8].p, t->g_param[9].p, t->g0z.p, B, kZ, 8192)));
+    const bool gates = t->cfg.g_leaky && gates_by_pre_activation(t);
+    auto pre = [&](dcg_node n) { return gates ? n : dead(n); };
+    L.push_back(pre(n_mat_mul_add(t->z.p, t->g_param[8].p, t->g_param[9].p, t->g0z.p, B, kZ, 8192)));
     L.push_back(n_unary(act, t->g0z.p, t->g0a.p, (size_t)B * 8192, 0.2f));
     const float* in = t->g0a.p;   // reshape to [B,4,4,512] is an alias (src/ops/reshape.cu:20-44)
     for (int i = 0; i < kLayers; ++i) {
         const int h = 4 << i, hw = 2 * h;
         const size_t rows = (size_t)B * hw * hw;
         L.push_back(dead(n_conv2d_transpose(in, t->g_param[2 * i].p, t->gc[i].p, B, h, kGChan[i], kGChan[i + 1])));
-        L.push_back(dead(n_rows_cols(DCG_OP_MAT_RVECT_ADD, t->gc[i].p, t->g_param[2 * i + 1].p, t->gz[i].p, rows, kGChan[i + 1])));
+        const dcg_node z = n_rows_cols(DCG_OP_MAT_RVECT_ADD, t->gc[i].p, t->g_param[2 * i + 1].p, t->gz[i].p, rows, kGChan[i + 1]);
+        L.push_back(i < kLayers - 1 ? pre(z) : dead(z));   // (tanh takes its output)
         if (i < kLayers - 1) {
             L.push_back(n_unary(act, t->gz[i].p, t->ga[i].p, rows * kGChan[i + 1], 0.2f));
             in = t->ga[i].p;
@@ -399,7 +407,8 @@ void build_discriminator(dcg_trainer* t, std::vector<dcg_node>& L, const float* 
         const int h = 64 >> i, ho = h / 2;
         const size_t rows = (size_t)B * ho * ho;
         L.push_back(dead(n_conv2d(in, t->d_param[2 * i].p, t->dc[ps][i].p, B, h, kDChan[i], kDChan[i + 1])));
-        L.push_back(dead(n_rows_cols(DCG_OP_MAT_RVECT_ADD, t->dc[ps][i].p, t->d_param[2 * i + 1].p, t->dz[ps][i].p, rows, kDChan[i + 1])));
+        const dcg_node z = n_rows_cols(DCG_OP_MAT_RVECT_ADD, t->dc[ps][i].p, t->d_param[2 * i + 1].p, t->dz[ps][i].p, rows, kDChan[i + 1]);
+        L.push_back(gates_by_pre_activation(t) ? z : dead(z));
         L.push_back(n_unary(DCG_OP_RELU_LEAKY, t->dz[ps][i].p, t->da[ps][i].p, rows * kDChan[i + 1], 0.2f));
         in = t->da[ps][i].p;
     }
@@ -423,9 +432,9 @@ void build_discriminator_backward(dcg_trainer* t, std::vector<dcg_node>& L, cons
         const int h = 64 >> i, ho = h / 2;
         const size_t rows = (size_t)B * ho * ho;
         const float* in = i == 0 ? img : t->da[ps][i - 1].p;
-        // dda[i+1] is produced by the layer above; its leaky gradient is this layer's dz.  The gate is the activation: it has the
-        // sign of the pre-activation, so that this need not be written (build_generator, build_discriminator flag it dead)
-        L.push_back(n_binary(DCG_OP_LEAKY_RELU_GRAD, t->da[ps][i].p, t->dda[i + 1].p, t->ddz[i].p, rows * kDChan[i + 1], 0.2f));
+        // dda[i+1] is produced by the layer above; its leaky gradient is this layer's dz
+        const float* gate = gates_by_pre_activation(t) ? t->dz[ps][i].p : t->da[ps][i].p;
+        L.push_back(n_binary(DCG_OP_LEAKY_RELU_GRAD, gate, t->dda[i + 1].p, t->ddz[i].p, rows * kDChan[i + 1], 0.2f));
         if (grads) {
             L.push_back(grad_node(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->ddz[i].p, nullptr, grads[2 * i + 1].p, rows, kDChan[i + 1])));
             // (the last of them where nothing follows on the main stream: beside the one before it, not behind it)
@@ -501,9 +510,9 @@ void build_lists(dcg_trainer* t)
         float* dprev_a = i == 0 ? t->dg0a.p : t->dga[i - 1].p;
         G.push_back(dead(n_conv2d_transpose_input_grad(t->dgz[i].p, t->g_param[2 * i].p, dprev_a, B, h, kGChan[i], kGChan[i + 1])));
         float* dprev_z = i == 0 ? t->dg0z.p : t->dgz[i - 1].p;
-        // (gated by the activation, as in the discriminator)
         const size_t nprev = i == 0 ? (size_t)B * 8192 : (size_t)B * h * h * kGChan[i];
-        G.push_back(n_binary(gact_grad, in, dprev_a, dprev_z, nprev, 0.2f));
+        const float* zprev = i == 0 ? t->g0z.p : t->gz[i - 1].p;
+        G.push_back(n_binary(gact_grad, t->cfg.g_leaky && gates_by_pre_activation(t) ? zprev : in, dprev_a, dprev_z, nprev, 0.2f));
         if (i == 0) {   // the last kernel gradient on the main stream, which has nothing more to do, not behind the one before it
             G.push_back(side(n_mat3(DCG_OP_TMAT_MAT_MUL, t->z.p, t->dg0z.p, t->g_grad[8].p, kZ, B, 8192)));
             G.push_back(side(n_rows_cols(DCG_OP_MAT_SUM_COLS, t->dg0z.p, nullptr, t->g_grad[9].p, B, 8192)));

@@ -80,6 +80,39 @@ def test_gradients_match_cpu_model(pkg, dev, orc, prec_name, tol, fuse):
     tr.close()
 
 
+@pytest.mark.parametrize("fuse", [False, True])
+@pytest.mark.parametrize("net", ["d", "g"])
+def test_smallest_negative_pre_activations_close_the_gate(pkg, dev, orc, net, fuse):
+    """Pre-activations of -1 and -2 times 2^-149, whose leaky activation is -0: the fp32 path gates their gradients as the
+    CPU model does, in the discriminator's first layer and in a leaky generator's dense layer."""
+    B = 2
+    rng = np.random.default_rng(11)
+    st = M.init_state(rng, B)
+    layer = 0 if net == "d" else 4   # its pre-activations are its bias
+    st[net][2 * layer][...] = 0
+    st[net][2 * layer + 1] = (np.float32(-2.0 ** -149) * (1 + np.arange(st[net][2 * layer + 1].size) % 2)).astype(np.float32)
+    assert (st[net][2 * layer + 1] < 0).all()
+    x = rng.uniform(-1, 1, (B, 64, 64, 3)).astype(np.float32)
+    z = rng.uniform(-1, 1, (B, 100)).astype(np.float32)
+    tr = pkg.Trainer(batch=B, precision=pkg.PREC_FP32, fuse=fuse, g_leaky=True)
+    _load_state(tr, st)
+    tr.x.copy_(torch.from_numpy(x))
+    tr.z.copy_(torch.from_numpy(z))
+    if net == "d":
+        _, gf, gr = M.run(M.d_gradients(orc, st, x, z, True))
+        tr.d_backward()
+        pairs = [("d_grad1", gf[1]), ("d_gradb1", gr[1])]
+    else:
+        _, gg = M.run(M.g_gradients(orc, st, z, True))
+        tr.g_backward()
+        pairs = [("g_grad9", gg[9])]
+    torch.cuda.synchronize()
+    # (through an open gate five times as much; the bound is that of test_gradients_match_cpu_model)
+    for name, ref in pairs:
+        assert np.abs(ref).max() > 0 and _maxrel(tr.tensor(name).cpu().numpy(), ref.reshape(-1)) <= 2e-5, name
+    tr.close()
+
+
 def test_iteration_matches_cpu_model(pkg, dev, orc):
     """Two whole iterations (D update + 2 G updates each) on the fp32 path: parameters after the
     Adam updates follow the CPU model (Adam itself is bit-exact; the gradients carry reduction-order
