@@ -377,6 +377,15 @@ bool finish_plan(Plan& pl, bool kernel_gradient = false)
     static const int forced_stages = env_int("DCG_TC_STAGES");
     if (forced_stages > 0 && forced_stages < stages) stages = forced_stages;
     if (stages < 2) stages = 2;
+    // 3xTF32: the groups of warps tell the rounds of the ring apart with as many stages as groups or two more, and kX3Wide, which
+    // looks once more, with one more, too.  So four stages for five at 112 and 128 columns, which is also quicker (a step of 64
+    // images 3037 -> 2962 us, 128 -> 256 forward of 64 images 41.7 -> 39.6; five stages and that look 3071 to 3111, six with fewer residuals of B
+    // 3343), and still four at 160 (kernel gradient of an RGB layer of 64 images 26.1 -> 26.2 us; three stages 29.4).
+    if (p.x3) {
+        const int groups = epilogue_groups(p.kind);
+        if (stages < groups) return false;
+        if (stages == groups + 1 && p.kind != kX3Wide) --stages;
+    }
     if (p.kind == kDual) stages &= ~1;
     // the epilogue parks the 128 x bn tile (padded rows) and 128 row offsets in the (by then idle) stage ring
     while ((size_t)stages * per_stage < (size_t)kRedFloats(p.bn) * 4 + BM * 8) stages += p.kind == kDual ? 2 : 1;
@@ -815,8 +824,7 @@ int launch_grid(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, i
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    static const int groups[kKinds] = {kGroups<kShared>, kGroups<kX3>, kGroups<kAlone>, kGroups<kDual>, kGroups<kX3Wide>};
-    cfg.blockDim = dim3((unsigned)(64 + 128 * groups[p.kind]));
+    cfg.blockDim = dim3((unsigned)(64 + 128 * epilogue_groups(p.kind)));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -1501,6 +1509,29 @@ bool conv_tc_plan(const dcg_conv_desc& d, int kind, bool x3, int plan[6])
     return true;
 }
 
+bool conv_tc_form(const dcg_conv_desc& d, int kind, bool x3, int form[4])
+{
+    PlanX3 scope(x3);
+    Prepared pr;
+    Plan& pl = pr.pl;
+    int kernel = DCG_FORM_TILES;
+    if (kind == kConvFwd && plan_rgb(d, pl, pr.rgb_args)) kernel = DCG_FORM_RGB;
+    else if (kind == kConvDx && plan_dx3(d, pl, pr.dx3_args)) kernel = DCG_FORM_RGB_GRAD;
+    else if (kind == kConvDx && plan_dxf(d, pl = Plan{}, pr.cf)) kernel = DCG_FORM_CLASSES;
+    else {
+        pl = Plan{};
+        if (!make_plan(d, kind, pl)) return false;
+        if (pl.p.walk) kernel = DCG_FORM_WALK;
+        else if ((pl.p.narrow || pl.ycol_bytes) && kind != kConvDk && short_ok(pl)) kernel = DCG_FORM_SHORT;
+    }
+    const Params& p = pl.p;
+    form[0] = kernel;
+    form[1] = p.ext_finish;
+    form[2] = kernel == DCG_FORM_TILES ? epilogue_groups(p.kind) : 0;
+    form[3] = kernel == DCG_FORM_TILES && p.x3 ? p.x3_slots : 0;
+    return true;
+}
+
 void conv_tc_set_dx_mode(int mode) { g_dxf_mode.store(mode < 0 || mode > 2 ? -1 : mode); }
 unsigned long long conv_tc_fused_dx_launches() { return g_dxf_launches.load(); }
 
@@ -1545,6 +1576,14 @@ extern "C" int dcg_debug_conv_plan(const dcg_conv_desc* desc, int kind, int prec
     const int st = dcg::conv_check_desc(desc, "dcg_debug_conv_plan");
     if (st) return st;
     if (precision == DCG_PREC_FP32 || !plan || !dcg::conv_tc_plan(*desc, kind, precision == DCG_PREC_3XTF32, plan)) return DCG_ERR_UNSUPPORTED;
+    return DCG_OK;
+}
+
+extern "C" int dcg_debug_conv_form(const dcg_conv_desc* desc, int kind, int precision, int form[4])
+{
+    const int st = dcg::conv_check_desc(desc, "dcg_debug_conv_form");
+    if (st) return st;
+    if (precision == DCG_PREC_FP32 || !form || !dcg::conv_tc_form(*desc, kind, precision == DCG_PREC_3XTF32, form)) return DCG_ERR_UNSUPPORTED;
     return DCG_OK;
 }
 

@@ -28,6 +28,11 @@ __host__ __device__ constexpr bool is_x3(int kind) { return kind == kX3 || kind 
 // loop, so there are as many groups as registers allow: with four, a warp sums one 32-column slab of the tile, with three,
 // two.  (Against three throughout: step of 64 images 3095 -> 3058 us, 64 -> 3 input gradient of 64 images 41.3 -> 38.3.)
 template <int KIND> constexpr int kGroups = KIND == kX3Wide ? 3 : KIND == kX3 || KIND == kAlone ? 4 : 2;
+inline int epilogue_groups(int kind)
+{
+    static const int groups[kKinds] = {kGroups<kShared>, kGroups<kX3>, kGroups<kAlone>, kGroups<kDual>, kGroups<kX3Wide>};
+    return groups[kind];
+}
 template <int KIND> constexpr int kX3Slabs = KIND == kX3Wide ? 2 : 1;   // slabs per epilogue warp, every kGroups-th one
 template <int KIND> constexpr int kX3Width = 32 * kGroups<KIND> * kX3Slabs<KIND>;
 constexpr int kX3MaxWidth = kX3Width<kX3Wide>;
@@ -472,6 +477,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             };
             for (int it = 0; it < nq; ++it) {
                 if (turn == group) {
+                    // A wait by parity passes at once on the phase before the last, so a group has to know that the load one round of
+                    // the ring earlier has landed.  With as many stages as groups that was its own stage, with two more it is one
+                    // whose MMAs it has seen done; with one more it looks at the stage's release first (finish_plan)
+                    if (KIND == kX3Wide && !mma_done(p.stages, it)) break;
                     if (!__all_sync(0xffffffffu, mbar_wait(full_bar + 8u * s, phase, 4, it, wait_limit))) break;
                     if (!mma_done(p.x3_bslots, it)) break;
                     const float4* bsrc = reinterpret_cast<const float4*>(smem_raw + (b_base + (uint32_t)s * b_stage_bytes - smem_u32(smem_raw)));

@@ -472,11 +472,23 @@ const char* dcg_last_error(void);
  *  dcg_debug_fused_dx_launches  how often the fused kernel has been launched (tests check which kernel ran);
  *  dcg_debug_conv_plan       how the general tensor-path kernel would run `desc` (kind and precision as for
  *                            dcg_conv_workspace_bytes): tile width, column tiles, K partitions, stages, TMEM columns, bytes
- *                            of shared memory; DCG_ERR_UNSUPPORTED where it does not take the shape.  Needs no GPU. */
+ *                            of shared memory; DCG_ERR_UNSUPPORTED where it does not take the shape.  Needs no GPU;
+ *  dcg_debug_conv_form       which kernel takes it: dcg_conv_form, 1 where a second launch adds the K partitions, then
+ *                            for DCG_FORM_TILES the groups of epilogue warps and (3xTF32) the stages whose residuals are
+ *                            kept.  As above. */
+enum dcg_conv_form {
+    DCG_FORM_TILES = 0,     /* one CTA per tile and K partition */
+    DCG_FORM_WALK = 1,      /* persistent CTAs that walk the tiles */
+    DCG_FORM_RGB = 2,       /* forward of <= 4 channels from its image */
+    DCG_FORM_CLASSES = 3,   /* input gradient, parity classes of a tile in one CTA */
+    DCG_FORM_RGB_GRAD = 4,  /* input gradient of <= 4 channels, products and gather in one kernel */
+    DCG_FORM_SHORT = 5      /* few reduction steps, resident weights */
+};
 void dcg_debug_set_wait_limit(long long sm_clocks);
 void dcg_debug_skip_stage(int stage);
 void dcg_debug_set_dx_mode(int mode);
 int dcg_debug_conv_plan(const dcg_conv_desc* desc, int kind, int precision, int plan[6]);
+int dcg_debug_conv_form(const dcg_conv_desc* desc, int kind, int precision, int form[4]);
 uint64_t dcg_debug_fused_dx_launches(void);   /* launches of the class-fused input-gradient kernel so far */
 /* Library version and the architecture the kernels were built for ("sm_100a"). */
 const char* dcg_build_info(void);

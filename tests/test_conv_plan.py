@@ -31,3 +31,57 @@ def test_tall_kernels_of_rgb_layers_in_3xtf32(pkg):
     for k in range(1, 9):
         plans = [p for call, p in _plans(pkg, [(4, 40, 36, 3, k, 64, 2)], pkg.PREC_3XTF32) if call[-1] == pkg._lib.KIND_DK]
         assert len(plans) == 1 and plans[0][:2] == ([32 * k, 1] if k <= 6 else [128, 2])
+
+
+def _ambiguous_waits(stages, groups, slots, looks, steps=120):
+    """Waits of the groups of warps that take 3xTF32 stages apart that a parity does not decide: the barrier may still be in the
+    phase before the one waited for (the wait passes at once, on the one before that), or may be beyond it (it never passes).  What
+    a group knows is what it has waited for: loads that have landed (its own stages, and all whose MMAs are done), MMAs that are
+    done (they end in order).  What it holds up is the MMAs from its next stage on."""
+    found = []
+    for g in range(groups):
+        landed, done, turn = set(), -1, g   # turn: its next stage
+        for it in range(steps):
+            def full(i):       # the load of stage i, between those of i - stages and i + stages
+                nonlocal done
+                if (i >= stages and i - stages not in landed and i - stages > done) or turn > i:
+                    found.append((g, i))
+                landed.add(i)
+                done = max(done, i - stages)   # whoever loaded it waited for the stage's release
+
+            def released(i):   # the MMAs of stage i
+                nonlocal done
+                if i < 0:
+                    return
+                if i - stages > done or turn > i + stages:
+                    found.append((g, i))
+                done = max(done, i)
+
+            if it % groups == g:
+                if looks:
+                    released(it - stages)
+                full(it)
+                released(it - (4 if stages >= 4 else 2))
+                released(it - slots)
+                turn = it + groups
+            if it % 4 == 1 and it > 4:   # the sums of a block of four stages are taken over
+                done = max(done, it - 2)
+    return found
+
+
+def test_3xtf32_waits_are_unambiguous(pkg):
+    """Every plan's ring, groups of warps and kept residuals.  Rings of one stage more than groups have such waits unless a group
+    looks at the release of its stage first, as the three groups of the wide tiles do."""
+    assert _ambiguous_waits(5, 4, 2, False) and _ambiguous_waits(4, 3, 2, False)
+    form, seen = (ctypes.c_int * 4)(), set()
+    shapes = [(n, 40, 36, c, k, o, s) for n in (1, 8, 64) for c in (3, 8, 16, 32, 64, 80, 100, 128, 256) for k in range(1, 9)
+              for o in (8, 32, 48, 64, 96, 100, 112, 128, 160, 192, 256) for s in (1, 2)]
+    for call, (width, _, _, stages, _, _) in _plans(pkg, shapes, pkg.PREC_3XTF32):
+        n, h, w, c, k, o, s, kind = call
+        desc = pkg.functional.conv_desc((n, h, w, c), (k, k, c, o), (s, s))
+        assert pkg.lib.dcg_debug_conv_form(ctypes.byref(desc), kind, pkg.PREC_3XTF32, form) == 0
+        if form[0] == 0:
+            seen.add((stages, form[2], form[3]))
+    assert {groups for _, groups, _ in seen} == {3, 4}
+    for plan in seen:
+        assert not _ambiguous_waits(*plan, plan[1] == 3), plan
