@@ -1160,6 +1160,7 @@ int launch_rgb(Prepared& pr, const CUtensorMap (&maps)[4], const float* x, float
     p.out = out;
     p.ep = ep;
     p.scratch = nullptr;
+    p.skip_stage = g_test_skip_stage.load();
     p.wait_cycles = g_wait_cycles.load();
     launch_pdl(kernels[wide][even], (unsigned)pr.pl.grid, kRgbThreads, pr.pl.smem, stream, pr.mb, maps[0], maps[1], maps[2], maps[3], pr.ma, p, pr.rgb_args,
                x);

@@ -107,12 +107,13 @@ conv_fwd_rgb_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_cons
     if (warp < kRgbBuilders / 32) {
         // ===== builders =====
         const int rows_per_img = (p.TH - 1) * p.sh + p.KH, line = p.W * p.C;
+        bool alive = true;   // (a warp that gave up loads nothing more: nobody would wait for it before the CTA leaves)
         auto copy = [&](int tile, int buf) {   // by TMA, or a warp per row of the patch; a group even where there is no such tile, for groups are counted
             int j0, i0, n0;
             origin(tile, j0, i0, n0);
             const int first = (j0 * p.sw - p.pl) * p.C;
             if (g.tma) {
-                if (warp == 0 && tile < g.tiles && elect_one()) {
+                if (warp == 0 && alive && tile < g.tiles && elect_one()) {
                     mbar_expect_tx(patch_bar + 8u * buf, g.patch_tx);
                     tma_load_3d(patch_base + (uint32_t)(buf * g.patch_bytes), &map_x, patch_bar + 8u * buf, first & ~3, i0 * p.sh - p.pt, n0);
                 }
@@ -142,7 +143,6 @@ conv_fwd_rgb_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_cons
         for (int b = 0; b < g.patches - 1; ++b, ahead += step) copy(ahead, b);
         int buf_in = g.patches - 1, buf_out = 0;
         uint32_t phase_out = 0;
-        bool alive = true;
         int n = 0;
         for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++n) {
             const int buf = n & 1;
@@ -186,7 +186,7 @@ conv_fwd_rgb_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_cons
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> tensor core reads
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + 8u * buf) : "memory");
+            if (lane == 0 && n != p.skip_stage) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + 8u * buf) : "memory");
         }
     } else if (warp == kMmaWarp) {
         // ===== the weights, then the products: A K-major, B MN-major (chunks of 32 columns 4096 B apart, 4-row groups 512 B apart) =====
@@ -241,7 +241,7 @@ conv_fwd_rgb_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_cons
                     tma_load_4d(stage + kRgbStage, &map_gate, gate_bar + 8u * w, sl * 32, j, i, img);
                 }
             };
-            if (e.gate && first < nslabs) load_gate(first);
+            if (ok && e.gate && first < nslabs) load_gate(first);
             ok = ok && mbar_wait_warp(acc_full + 8u * buf, (uint32_t)(n >> 1) & 1u, 2, n, wait_limit);   // (waits in vain once at most)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int sl = first; sl < nslabs; sl += 2) {
@@ -298,7 +298,7 @@ conv_fwd_rgb_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_cons
                         act_grad_apply_all(four, gate, e.gate_act, e.gate_alpha);
                         v[4 * q] = four[0]; v[4 * q + 1] = four[1]; v[4 * q + 2] = four[2]; v[4 * q + 3] = four[3];
                     }
-                    if (sl + 2 < nslabs) load_gate(sl + 2);
+                    if (ok && sl + 2 < nslabs) load_gate(sl + 2);
                 }
                 put(&map_out);
             }

@@ -463,9 +463,11 @@ const char* dcg_last_error(void);
 /* Testing hooks of the tensor-path convolution kernels (no counterpart in the reference; process-wide,
  * they affect launches enqueued after the call):
  *  dcg_debug_set_wait_limit  limit of every bounded barrier wait in SM clocks (<= 0 restores ~1 s);
- *  dcg_debug_skip_stage      the TMA producer leaves pipeline stage `stage` of every tile out (< 0: never), so
- *                            that a consumer's wait runs into the limit: the kernel then records the failure,
- *                            still terminates, and dcg_device_status() returns DCG_ERR_DEVICE;
+ *  dcg_debug_skip_stage      the TMA producer leaves pipeline stage `stage` of every tile out (DCG_FORM_WALK: of every CTA;
+ *                            DCG_FORM_RGB: a CTA's operand tile of that number is not handed over; the forms without
+ *                            such a hook run as ever; < 0: never), so that a consumer's wait runs into the limit: the
+ *                            kernel then records the failure, still terminates, and dcg_device_status() returns
+ *                            DCG_ERR_DEVICE;
  *  dcg_debug_set_dx_mode     which input-gradient kernel the tensor path plans: 0 = one tile per parity class,
  *                            1 = the parity classes of a tile fused in one CTA where one CTA per tile fills the
  *                            GPU (default), 2 = fused wherever the shape allows, < 0 = back to the default;

@@ -769,3 +769,41 @@ def test_bounded_wait_runs_out_and_the_context_survives(pkg, dev):
     y32 = F.conv2d_fwd(xd, kd, precision=pkg.PREC_FP32)   # bit-equal to the oracle (test_conv_fwd_dx_dk)
     torch.cuda.synchronize()
     assert (y - y32).abs().max().item() <= TF32_TOL * y32.abs().max().item()
+
+
+# one stage of the pipeline never comes: kernel (dcg_conv_form), operator, precision, shape (n, h, w, c, k, o, s), the stage
+GIVE_UP = [(2, "fwd", "tf32", (64, 64, 64, 3, 5, 64, 2), 1)]
+
+
+@pytest.mark.parametrize("form,op,prec_name,shape,stage", GIVE_UP)
+def test_a_wait_that_runs_out_in_each_kernel(pkg, dev, form, op, prec_name, shape, stage):
+    """As above, without K partitions: every wait ends, the status tells, a call right after is clean - with a gate, whose values
+    an RGB forward fetches while it waits."""
+    import ctypes
+    F, L = pkg.functional, pkg.lib
+    n, h, w, c, k, o, s = shape
+    prec, kind = getattr(pkg, PRECS[prec_name]), {"fwd": pkg._lib.KIND_FWD, "dx": pkg._lib.KIND_DX}[op]
+    d, plan, got = F.conv_desc((n, h, w, c), (k, k, c, o), (s, s)), (ctypes.c_int * 6)(), (ctypes.c_int * 4)()
+    assert L.dcg_debug_conv_form(ctypes.byref(d), kind, prec, got) == 0 and got[0] == form
+    assert L.dcg_debug_conv_plan(ctypes.byref(d), kind, prec, plan) == 0 and plan[2] == 1
+    x, kk, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((81, (n, h, w, c)), (82, (k, k, c, o)), (83, (n, -(-h // s), -(-w // s), o))))
+    gate = dy if op == "fwd" else x
+    ep = F.make_epilogue(gate=gate, gate_act=pkg.ACT_RELU)
+
+    def call(p):
+        return F.conv2d_fwd(x, kk, (s, s), epilogue=ep, precision=p) if op == "fwd" else F.conv2d_dx(dy, kk, (h, w), (s, s), epilogue=ep, precision=p)
+
+    assert L.dcg_device_status() == 0
+    try:
+        L.dcg_debug_set_wait_limit(2_000_000)   # ~1 ms of SM clocks
+        L.dcg_debug_skip_stage(stage)
+        call(prec)
+        torch.cuda.synchronize()
+    finally:
+        L.dcg_debug_skip_stage(-1)
+        L.dcg_debug_set_wait_limit(0)
+    assert L.dcg_device_status() == pkg._lib.ERR_DEVICE
+    got, ref = call(prec), call(pkg.PREC_FP32)
+    torch.cuda.synchronize()
+    assert L.dcg_device_status() == 0
+    assert (got - ref).abs().max().item() <= TF32_TOL * ref.abs().max().item()
