@@ -1162,6 +1162,9 @@ int launch_rgb(Prepared& pr, const CUtensorMap (&maps)[4], const float* x, float
     p.scratch = nullptr;
     p.skip_stage = g_test_skip_stage.load();
     p.wait_cycles = g_wait_cycles.load();
+    // the results of the chain leave as bulk copies in no order: of results for the same tensor only the last one
+    if (p.ep.pre_act == out) p.ep.pre_act = nullptr;
+    if (p.ep.raw_out == out || (p.ep.raw_out && p.ep.raw_out == p.ep.pre_act)) p.ep.raw_out = nullptr;
     launch_pdl(kernels[wide][even], (unsigned)pr.pl.grid, kRgbThreads, pr.pl.smem, stream, pr.mb, maps[0], maps[1], maps[2], maps[3], pr.ma, p, pr.rgb_args,
                x);
     DCG_LAUNCH_CHECK("conv_fwd_rgb_kernel");

@@ -606,6 +606,29 @@ def test_forward_of_rgb_layers(pkg, dev, shape):
         assert all(bool((t[N] == 7.0).all()) for t in (raw, pre, out))
 
 
+def test_rgb_forward_into_one_tensor(pkg, dev):
+    """Results of the chain that go to the same tensor: the last one stays, as it does in every other kernel."""
+    F = pkg.functional
+    x, k, bias = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((65, (40, 64, 64, 3)), (66, (5, 5, 3, 64)), (67, (64,))))
+
+    def call(**chain):
+        return F.conv2d_fwd(x, k, (2, 2), epilogue=F.make_epilogue(bias=bias, act=pkg.ACT_TANH, **chain), out=out)
+
+    out = torch.empty((40, 32, 32, 64), device=dev)
+    raw, pre = torch.empty_like(out), torch.empty_like(out)
+    y = call(raw_out=raw, pre_act=pre).clone()
+    assert pkg.lib.dcg_device_status() == 0 and torch.equal(pre, raw + bias)
+    for _ in range(5):
+        for first, second in ((out, out), (pre, out), (out, pre), (pre, pre)):   # raw and pre-activation
+            pre.zero_()
+            call(raw_out=first, pre_act=second)
+            assert torch.equal(out, y)
+            if second is pre:
+                assert torch.equal(pre, raw + bias)
+            elif first is pre:
+                assert torch.equal(pre, raw)
+
+
 # more tiles than SMs, walked by persistent CTAs: one to three tiles each and a last round that is nearly empty, widths of 16 to 192
 # columns, the last column tile partly beyond the channels, parity classes, channels that are no multiple of four, one stage a tile
 @pytest.mark.parametrize("shape", [(24, 48, 48, 32, 1, 192, 1), (13, 75, 51, 96, 3, 160, 1), (32, 40, 40, 64, 3, 96, 1), (37, 60, 60, 20, 5, 64, 2),
