@@ -91,12 +91,15 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
+std::atomic<unsigned long long> g_maps_encoded{0};
+
 // dims/strides innermost first; strides[i] is the byte stride of dimension i+1.
 int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, CUtensorMapSwizzle swizzle,
                const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* estrides)
 {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(DCG_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    g_maps_encoded.fetch_add(1, std::memory_order_relaxed);
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void*>(base), dims,
                           strides, box, estrides, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -974,15 +977,24 @@ int map_window(CUtensorMap* map, const float* xp, const dcg_conv_desc& d, const 
 // or the reference's Graph::run issues the same convolutions on the same buffers over and over, so
 // the result is kept per (device, operator, shape, operand addresses, scratch address, precision)
 // in a small table; a hit leaves only the launch.
+// What an RGB forward writes and its gate: output, raw result, pre-activation, gate.  They are no part of the key.
+struct RgbMaps {
+    const void* of[4];   // the tensor that a map is of (null: none yet)
+    CUtensorMap map[4];
+};
 struct Prepared {
     Plan pl;
     CUtensorMap ma, mb;
     bool dxf = false;   // input gradient with the parity classes fused (conv_dxf_kernel); cf is its table
-    CfTable cf;
+    union {
+        CfTable cf;
+        RgbMaps rgb_maps;   // rgb
+    };
     bool dx3 = false;   // input gradient of a <= 4-channel layer as one GEMM + gather kernel (conv_dx3_kernel)
     Dx3Args dx3_args;
     bool rgb = false;   // forward of a <= 4-channel layer from its image (conv_fwd_rgb_kernel)
     RgbArgs rgb_args;
+    Prepared() { std::memset(&rgb_maps, 0, sizeof(rgb_maps)); }
 };
 
 int launch_dxf(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t stream)
@@ -1147,8 +1159,7 @@ int launch_dx3(Prepared& pr, float* out, const EpilogueArgs& ep, cudaStream_t st
     return DCG_OK;
 }
 
-// `maps`: of the output tensors and the gate (32 pixels x 32 channels; absent ones are not read).
-int launch_rgb(Prepared& pr, const CUtensorMap (&maps)[4], const float* x, float* out, const EpilogueArgs& ep, cudaStream_t stream)
+int launch_rgb(Prepared& pr, const float* x, float* out, const EpilogueArgs& ep, cudaStream_t stream)
 {
     Params& p = pr.pl.p;
     using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, Params, RgbArgs, const float*);
@@ -1165,8 +1176,8 @@ int launch_rgb(Prepared& pr, const CUtensorMap (&maps)[4], const float* x, float
     // the results of the chain leave as bulk copies in no order: of results for the same tensor only the last one
     if (p.ep.pre_act == out) p.ep.pre_act = nullptr;
     if (p.ep.raw_out == out || (p.ep.raw_out && p.ep.raw_out == p.ep.pre_act)) p.ep.raw_out = nullptr;
-    launch_pdl(kernels[wide][even], (unsigned)pr.pl.grid, kRgbThreads, pr.pl.smem, stream, pr.mb, maps[0], maps[1], maps[2], maps[3], pr.ma, p, pr.rgb_args,
-               x);
+    launch_pdl(kernels[wide][even], (unsigned)pr.pl.grid, kRgbThreads, pr.pl.smem, stream, pr.mb, pr.rgb_maps.map[0], pr.rgb_maps.map[1], pr.rgb_maps.map[2],
+               pr.rgb_maps.map[3], pr.ma, p, pr.rgb_args, x);
     DCG_LAUNCH_CHECK("conv_fwd_rgb_kernel");
     return DCG_OK;
 }
@@ -1349,9 +1360,8 @@ int build_dk(const dcg_conv_desc& d, const float* x, const float* dy, void* ws, 
 }
 
 // Looks the call up, building and filing it on a miss.  The entry is copied out under the lock.
-int prepared_call(int kind, const dcg_conv_desc& d, const void* a, const void* b, void* ws, size_t ws_bytes, Prepared& out)
+int prepared_call(int kind, const dcg_conv_desc& d, const void* a, const void* b, void* ws, size_t ws_bytes, Prepared& out, CacheKey& key)
 {
-    CacheKey key;
     std::memset(&key, 0, sizeof(key));
     if (cudaGetDevice(&key.dev) != cudaSuccess) key.dev = -1;
     key.kind = kind; key.x3 = t_plan_x3 | (dxf_mode() << 1);   // the plan depends on both
@@ -1379,6 +1389,28 @@ int prepared_call(int kind, const dcg_conv_desc& d, const void* a, const void* b
         g_cache[g_cache_next] = CacheEntry{key, out};
         g_cache_next = (g_cache_next + 1) % kCacheEntries;
     }
+    return DCG_OK;
+}
+
+// Brings the output-side maps of an RGB forward in line with this call's tensors (boxes of 32 pixels x 32 channels, the rows of an
+// epilogue warp) and files those that were not there.
+int rgb_maps(const dcg_conv_desc& d, const CacheKey& key, const void* const (&tensors)[4], Prepared& pr)
+{
+    const Params& p = pr.pl.p;
+    const int tw = std::min(p.TW, 32), th = std::min(p.TH, 32 / tw), tn = 32 / (tw * th);
+    RgbMaps& m = pr.rgb_maps;
+    bool fresh = false;
+    for (int i = 0; i < 4; ++i) {
+        if (!tensors[i] || tensors[i] == m.of[i]) continue;   // (absent ones are not read)
+        const int st = map_act_4d(&m.map[i], static_cast<const float*>(tensors[i]), d.n, d.ho, d.wo, d.o, tw, th, tn, 1, 1);
+        if (st) return st;
+        m.of[i] = tensors[i];
+        fresh = true;
+    }
+    if (!fresh) return DCG_OK;
+    std::lock_guard<std::mutex> lock(g_cache_mutex);
+    const auto it = g_cache_at.find(key);
+    if (it != g_cache_at.end()) g_cache[it->second].prep.rgb_maps = m;
     return DCG_OK;
 }
 
@@ -1429,16 +1461,13 @@ int conv_tc_fwd(const dcg_conv_desc& d, const float* x, const float* k, float* y
 {
     PlanX3 scope(x3);
     Prepared pr;
-    int st = prepared_call(kConvFwd, d, x, k, ws, ws_bytes, pr);
+    CacheKey key;
+    int st = prepared_call(kConvFwd, d, x, k, ws, ws_bytes, pr, key);
     if (st) return st;
     if (pr.rgb) {
-        const Params& p = pr.pl.p;
-        const int tw = std::min(p.TW, 32), th = std::min(p.TH, 32 / tw), tn = 32 / (tw * th);   // 32 accumulator rows
-        CUtensorMap maps[4]{};
-        const float* tensors[4] = {y, ep.raw_out, ep.pre_act, ep.gate};
-        for (int i = 0; i < 4; ++i)
-            if (tensors[i] && (st = map_act_4d(&maps[i], tensors[i], d.n, d.ho, d.wo, d.o, tw, th, tn, 1, 1))) return st;
-        return launch_rgb(pr, maps, x, y, ep, stream);
+        const void* const tensors[4] = {y, ep.raw_out, ep.pre_act, ep.gate};
+        if ((st = rgb_maps(d, key, tensors, pr))) return st;
+        return launch_rgb(pr, x, y, ep, stream);
     }
     if (pr.pl.p.narrow) {
         float *xp, *k4;
@@ -1453,7 +1482,8 @@ int conv_tc_dx(const dcg_conv_desc& d, const float* dy, const float* k, float* d
 {
     PlanX3 scope(x3);
     Prepared pr;
-    int st = prepared_call(kConvDx, d, dy, k, ws, ws_bytes, pr);
+    CacheKey key;
+    int st = prepared_call(kConvDx, d, dy, k, ws, ws_bytes, pr, key);
     if (st) return st;
     Plan& pl = pr.pl;
     if (pr.dx3) return launch_dx3(pr, dx, ep, stream);
@@ -1492,7 +1522,8 @@ int conv_tc_dk(const dcg_conv_desc& d, const float* x, const float* dy, float* d
 {
     PlanX3 scope(x3);
     Prepared pr;
-    int st = prepared_call(kConvDk, d, x, dy, ws, ws_bytes, pr);
+    CacheKey key;
+    int st = prepared_call(kConvDk, d, x, dy, ws, ws_bytes, pr, key);
     if (st) return st;
     if (pr.pl.p.narrow) {
         float* xp;
@@ -1538,6 +1569,7 @@ bool conv_tc_form(const dcg_conv_desc& d, int kind, bool x3, int form[4])
 
 void conv_tc_set_dx_mode(int mode) { g_dxf_mode.store(mode < 0 || mode > 2 ? -1 : mode); }
 unsigned long long conv_tc_fused_dx_launches() { return g_dxf_launches.load(); }
+unsigned long long conv_tc_maps_encoded() { return g_maps_encoded.load(); }
 
 // wait_cycles: > 0 sets the limit, -1 restores the default, 0 leaves it; skip_stage: -2 leaves it.
 void conv_tc_set_hooks(long long wait_cycles, int skip_stage)
@@ -1591,6 +1623,7 @@ extern "C" int dcg_debug_conv_form(const dcg_conv_desc* desc, int kind, int prec
     return DCG_OK;
 }
 
+extern "C" uint64_t dcg_debug_maps_encoded(void) { return dcg::conv_tc_maps_encoded(); }
 extern "C" uint64_t dcg_debug_fused_dx_launches(void) { return dcg::conv_tc_fused_dx_launches(); }
 
 #ifdef DCG_TC_TRACING

@@ -606,6 +606,30 @@ def test_forward_of_rgb_layers(pkg, dev, shape):
         assert all(bool((t[N] == 7.0).all()) for t in (raw, pre, out))
 
 
+def test_repeated_calls_encode_no_tensor_maps(pkg, dev):
+    """Of a call on the same tensors none; of an RGB forward with another output that one's, and the results follow the tensors."""
+    F, encoded = pkg.functional, pkg.lib.dcg_debug_maps_encoded
+    for shape in ((8, 64, 64, 3, 5, 64, 2), (80, 32, 32, 32, 5, 64, 2)):   # (neither takes scratch, which has a new address each time)
+        N, H, W, C, K, O, s = shape
+        x, k, gate = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((68, (N, H, W, C)), (69, (K, K, C, O)), (70, (N, H // s, W // s, O))))
+        raw, pre, out, other = (torch.empty_like(gate) for _ in range(4))
+        ep = F.make_epilogue(act=pkg.ACT_LEAKY, raw_out=raw, pre_act=pre, gate=gate, gate_act=pkg.ACT_RELU)
+        F.conv2d_fwd(x, k, (s, s), epilogue=ep, out=out)
+        first = [t.clone() for t in (raw, pre, out)]
+        before = encoded()
+        for t in (raw, pre, out):
+            t.zero_()
+        F.conv2d_fwd(x, k, (s, s), epilogue=ep, out=out)
+        assert encoded() == before
+        assert all(torch.equal(a, b) for a, b in zip(first, (raw, pre, out)))
+        out.zero_()
+        F.conv2d_fwd(x, k, (s, s), epilogue=ep, out=other)
+        F.conv2d_fwd(x, k, (s, s), out=raw)
+        assert encoded() - before == (2 if C == 3 else 0)
+        assert torch.equal(other, first[2]) and not out.any() and torch.equal(raw, first[0])
+    assert pkg.lib.dcg_device_status() == 0
+
+
 def test_rgb_forward_into_one_tensor(pkg, dev):
     """Results of the chain that go to the same tensor: the last one stays, as it does in every other kernel."""
     F = pkg.functional
