@@ -150,6 +150,7 @@ SIGNATURES = {
     "dcg_debug_set_dx_mode": (None, [c_int]),
     "dcg_debug_conv_plan": (c_int, [ctypes.POINTER(ConvDesc), c_int, c_int, ctypes.POINTER(c_int)]),
     "dcg_debug_conv_form": (c_int, [ctypes.POINTER(ConvDesc), c_int, c_int, ctypes.POINTER(c_int)]),
+    "dcg_debug_dx_plans": (ctypes.c_uint64, []),
     "dcg_debug_maps_encoded": (ctypes.c_uint64, []),
     "dcg_debug_fused_dx_launches": (ctypes.c_uint64, []),
     "dcg_build_info": (ctypes.c_char_p, []),

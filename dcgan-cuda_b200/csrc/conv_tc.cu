@@ -509,8 +509,10 @@ dcg_conv_desc dx_gemm_desc(const dcg_conv_desc& d, int Jp)
     return g;
 }
 
+std::atomic<unsigned long long> g_dx_plans{0};
 bool plan_dx(const dcg_conv_desc& d, Plan& pl)
 {
+    g_dx_plans.fetch_add(1, std::memory_order_relaxed);
     if (d.c <= 4 && d.o % 32 == 0 && d.stride_h <= d.kh && d.stride_w <= d.kw) {
         const int Jp = (d.kh * d.kw * 4 + 31) / 32 * 32;   // four columns per tap
         pl.Jp = Jp;
@@ -551,6 +553,38 @@ int dxf_mode()
     return m >= 0 ? m : from_env;
 }
 
+// Keys are compared and hashed as bytes: they are zeroed before they are filled in.
+template <typename Key>
+struct BytesEqual {
+    bool operator()(const Key& u, const Key& v) const { return std::memcmp(&u, &v, sizeof(Key)) == 0; }
+};
+template <typename Key>
+struct BytesHash {
+    size_t operator()(const Key& k) const
+    {
+        static_assert(sizeof(Key) % 4 == 0, "hashed by 32-bit words");
+        uint32_t w[sizeof(Key) / 4];
+        std::memcpy(w, &k, sizeof(Key));
+        uint64_t h = 0xcbf29ce484222325ull;
+        for (uint32_t v : w) h = (h ^ v) * 0x100000001b3ull;
+        return (size_t)(h ^ (h >> 29));
+    }
+};
+
+// A call without its tensors: what is known from the shape alone is kept per such key.
+struct QueryKey {
+    int dev, kind, x3;
+    dcg_conv_desc d;
+};
+QueryKey query_key(const dcg_conv_desc& d, int kind, bool x3)
+{
+    QueryKey key;
+    std::memset(&key, 0, sizeof(key));
+    if (cudaGetDevice(&key.dev) != cudaSuccess) { cudaGetLastError(); key.dev = -1; }
+    key.kind = kind; key.x3 = x3; key.d = d;
+    return key;
+}
+
 // Whether the parity classes are quicker as tiles of their own, walked by persistent CTAs, than all of them together in `tiles`
 // tiles of `bn` columns.  In clocks: a (class, tap) pair of a 32-channel chunk takes 233 of them at 64 columns and 297 at 128 in
 // the class-fused kernel, a stage of the other one 300 at 128 columns and 512 at 256; a column of a class costs an epilogue 20,
@@ -558,7 +592,7 @@ int dxf_mode()
 // of two and of at most 128 columns, which leaves much of them empty where the image, the channels or the last wave do not fit: 3 x 3 /
 // stride 2, 192 -> 64, 30 images of 33 x 47 27.0 us fused, 13.6 apart; 192 -> 192, 32 images of 96 x 96 165 and 111.
 // Where they fit, fused is quicker (5 x 5 / stride 2, 64 -> 128 of 64 images 16.4 and 22.2, 256 -> 512 of 512 images 74 and 90).
-bool classes_apart_quicker(const dcg_conv_desc& d, int tiles, int bn, int ncls)
+bool classes_apart_modelled(const dcg_conv_desc& d, int tiles, int bn, int ncls)
 {
     Plan apart;
     if (!plan_dx(d, apart) || !apart.p.walk) return false;
@@ -570,6 +604,24 @@ bool classes_apart_quicker(const dcg_conv_desc& d, int tiles, int bn, int ncls)
     const double mine = both((double)p.tiles_w * p.tiles_h * p.tiles_n * p.n_tiles * pairs / sms * stage, std::ceil(apart.grid / sms) * 20.0 * p.bn) +
                         0.5 * stage * pairs / ncls;   // (the classes differ in length)
     return mine < 0.9 * fused;
+}
+
+// The same, kept: a call on new addresses is planned again, and this is a second plan (host time of an input gradient with new
+// addresses every time: 64 images of 32 x 32, 64 -> 128 9.1 -> 5.8 us; 20 of 33 x 47, 192 -> 64, classes apart 11.9 -> 7.5).
+bool classes_apart_quicker(const dcg_conv_desc& d, int tiles, int bn, int ncls)
+{
+    static std::mutex mutex;
+    static std::unordered_map<QueryKey, bool, BytesHash<QueryKey>, BytesEqual<QueryKey>> known;
+    const QueryKey key = query_key(d, kConvDx, false);
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        const auto it = known.find(key);
+        if (it != known.end()) return it->second;
+    }
+    const bool quicker = classes_apart_modelled(d, tiles, bn, ncls);
+    std::lock_guard<std::mutex> lock(mutex);
+    if (known.size() >= 4096) known.clear();
+    return known[key] = quicker;
 }
 
 // The class-fused input gradient (conv_dxf_kernel): windows of dy, the (class, tap) pairs that read each, and
@@ -599,6 +651,7 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     const int tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.n_tiles;
     // one CTA per tile, no K partitions: only where the tiles alone fill (most of) the GPU
     if (mode != 2 && tiles * 4 < sm_count() * 3) return false;
+    if (mode == 1 && classes_apart_quicker(d, tiles, bn, ncls)) return false;
     // every (class, tap) pair with the window it reads
     struct Pair { int sy, sx, cls, kh, kw; };
     std::vector<Pair> pairs;
@@ -698,7 +751,6 @@ bool plan_dxf(const dcg_conv_desc& d, Plan& pl, CfTable& t)
     int units = (kMaxSmem - fixed) / kCfUnit;
     if (units > kCfMaxUnits) units = kCfMaxUnits;
     if (units < 3 * max_units) return false;   // three stages in flight
-    if (mode == 1 && classes_apart_quicker(d, tiles, bn, ncls)) return false;
     p.stages = units;
     pl.smem = (size_t)units * kCfUnit + fixed;
     p.skip_stage = -1;
@@ -1194,24 +1246,6 @@ struct CacheEntry {
     Prepared prep;
 };
 
-// Keys are compared and hashed as bytes: they are zeroed before they are filled in.
-template <typename Key>
-struct BytesEqual {
-    bool operator()(const Key& u, const Key& v) const { return std::memcmp(&u, &v, sizeof(Key)) == 0; }
-};
-template <typename Key>
-struct BytesHash {
-    size_t operator()(const Key& k) const
-    {
-        static_assert(sizeof(Key) % 4 == 0, "hashed by 32-bit words");
-        uint32_t w[sizeof(Key) / 4];
-        std::memcpy(w, &k, sizeof(Key));
-        uint64_t h = 0xcbf29ce484222325ull;
-        for (uint32_t v : w) h = (h ^ v) * 0x100000001b3ull;
-        return (size_t)(h ^ (h >> 29));
-    }
-};
-
 constexpr size_t kCacheEntries = 512;
 std::mutex g_cache_mutex;
 std::vector<CacheEntry> g_cache;
@@ -1415,10 +1449,6 @@ int rgb_maps(const dcg_conv_desc& d, const CacheKey& key, const void* const (&te
 }
 
 // ---- what the entry points ask before a call: does the tensor path take the shape, and how much scratch does it need ----
-struct QueryKey {
-    int dev, kind, x3;
-    dcg_conv_desc d;
-};
 struct QueryAnswer {
     bool supported;
     size_t ws_bytes, ws_least;   // what the best plan takes, and what the call can do with
@@ -1428,10 +1458,7 @@ std::unordered_map<QueryKey, QueryAnswer, BytesHash<QueryKey>, BytesEqual<QueryK
 
 QueryAnswer query(const dcg_conv_desc& d, int kind, bool x3)
 {
-    QueryKey key;
-    std::memset(&key, 0, sizeof(key));
-    if (cudaGetDevice(&key.dev) != cudaSuccess) { cudaGetLastError(); key.dev = -1; }
-    key.kind = kind; key.x3 = x3; key.d = d;
+    const QueryKey key = query_key(d, kind, x3);
     {
         std::lock_guard<std::mutex> lock(g_query_mutex);
         const auto it = g_query.find(key);
@@ -1569,6 +1596,7 @@ bool conv_tc_form(const dcg_conv_desc& d, int kind, bool x3, int form[4])
 
 void conv_tc_set_dx_mode(int mode) { g_dxf_mode.store(mode < 0 || mode > 2 ? -1 : mode); }
 unsigned long long conv_tc_fused_dx_launches() { return g_dxf_launches.load(); }
+unsigned long long conv_tc_dx_plans() { return g_dx_plans.load(); }
 unsigned long long conv_tc_maps_encoded() { return g_maps_encoded.load(); }
 
 // wait_cycles: > 0 sets the limit, -1 restores the default, 0 leaves it; skip_stage: -2 leaves it.
@@ -1623,6 +1651,7 @@ extern "C" int dcg_debug_conv_form(const dcg_conv_desc* desc, int kind, int prec
     return DCG_OK;
 }
 
+extern "C" uint64_t dcg_debug_dx_plans(void) { return dcg::conv_tc_dx_plans(); }
 extern "C" uint64_t dcg_debug_maps_encoded(void) { return dcg::conv_tc_maps_encoded(); }
 extern "C" uint64_t dcg_debug_fused_dx_launches(void) { return dcg::conv_tc_fused_dx_launches(); }
 

@@ -491,6 +491,7 @@ void dcg_debug_skip_stage(int stage);
 void dcg_debug_set_dx_mode(int mode);
 int dcg_debug_conv_plan(const dcg_conv_desc* desc, int kind, int precision, int plan[6]);
 int dcg_debug_conv_form(const dcg_conv_desc* desc, int kind, int precision, int form[4]);
+uint64_t dcg_debug_dx_plans(void);            /* plans of an input gradient by the general kernel so far */
 uint64_t dcg_debug_maps_encoded(void);        /* tensor maps encoded on the host so far (a repeated call needs none) */
 uint64_t dcg_debug_fused_dx_launches(void);   /* launches of the class-fused input-gradient kernel so far */
 /* Library version and the architecture the kernels were built for ("sm_100a"). */

@@ -85,3 +85,18 @@ def test_3xtf32_waits_are_unambiguous(pkg):
     assert {groups for _, groups, _ in seen} == {3, 4}
     for plan in seen:
         assert not _ambiguous_waits(*plan, plan[1] == 3), plan
+
+
+def test_class_fused_input_gradients_are_planned_once(pkg):
+    """Where the parity classes stay together the general kernel is planned for the comparison only, once a shape and not with
+    every call on other tensors; where they do not, once a call is what it takes."""
+    form = (ctypes.c_int * 4)()
+    for shape, kernel, each in (((64, 32, 32, 64, 5, 128, 2), 3, 0), ((30, 33, 47, 192, 3, 64, 2), 1, 1)):
+        n, h, w, c, k, o, s = shape
+        desc = pkg.functional.conv_desc((n, h, w, c), (k, k, c, o), (s, s))
+        counts = []
+        for _ in range(3):
+            before = pkg.lib.dcg_debug_dx_plans()
+            assert pkg.lib.dcg_debug_conv_form(ctypes.byref(desc), pkg._lib.KIND_DX, pkg.PREC_TF32, form) == 0 and form[0] == kernel
+            counts.append(pkg.lib.dcg_debug_dx_plans() - before)
+        assert counts[1:] == [each] * 2
