@@ -1564,9 +1564,18 @@ bool conv_tc_plan(const dcg_conv_desc& d, int kind, bool x3, int plan[6])
 {
     PlanX3 scope(x3);
     Plan pl;
-    if (!make_plan(d, kind, pl)) return false;
+    RgbArgs rgb;
+    const bool is_rgb = kind == kConvFwd && plan_rgb(d, pl, rgb);
+    if (!is_rgb) {
+        pl = Plan{};
+        if (!make_plan(d, kind, pl)) return false;
+    }
     const Params& p = pl.p;
-    const int values[6] = {p.bn, p.n_tiles, p.splits, p.stages, p.walk ? 2 * p.bn : tmem_columns(p.kind, p.bn, p.x3_slots), (int)pl.smem};
+    // what the kernel allocates: two accumulators in a power of two of columns where it is persistent
+    int tmem = tmem_columns(p.kind, p.bn, p.x3_slots);
+    if (p.walk || is_rgb)
+        for (tmem = 32; tmem < 2 * p.bn;) tmem <<= 1;
+    const int values[6] = {p.bn, p.n_tiles, p.splits, p.stages, tmem, (int)pl.smem};
     for (int i = 0; i < 6; ++i) plan[i] = values[i];
     return true;
 }

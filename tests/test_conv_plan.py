@@ -100,3 +100,15 @@ def test_class_fused_input_gradients_are_planned_once(pkg):
             assert pkg.lib.dcg_debug_conv_form(ctypes.byref(desc), pkg._lib.KIND_DX, pkg.PREC_TF32, form) == 0 and form[0] == kernel
             counts.append(pkg.lib.dcg_debug_dx_plans() - before)
         assert counts[1:] == [each] * 2
+
+
+def test_persistent_kernels_report_both_accumulators(pkg):
+    """An RGB forward and a walked one: two accumulators, in the power of two of columns that is allocated."""
+    form = (ctypes.c_int * 4)()
+    for shape, kernel, columns in (((64, 64, 64, 3, 5, 64, 2), 2, 128), ((8, 64, 64, 3, 3, 96, 1), 2, 256), ((130, 64, 64, 3, 5, 128, 2), 2, 256),
+                                   ((16, 96, 96, 64, 1, 192, 1), 1, 256), ((37, 60, 60, 20, 5, 64, 2), 1, 128)):
+        plans = [p for call, p in _plans(pkg, [shape], pkg.PREC_TF32) if call[-1] == pkg._lib.KIND_FWD]
+        n, h, w, c, k, o, s = shape
+        desc = pkg.functional.conv_desc((n, h, w, c), (k, k, c, o), (s, s))
+        assert pkg.lib.dcg_debug_conv_form(ctypes.byref(desc), pkg._lib.KIND_FWD, pkg.PREC_TF32, form) == 0 and form[0] == kernel, shape
+        assert plans[0][0] == (96 if o == 192 else o) and plans[0][4] == columns, shape
