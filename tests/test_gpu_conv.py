@@ -548,16 +548,31 @@ def test_k_partition_counts(pkg, dev, batch):
         assert torch.equal(u, v), name
 
 
+def _form(pkg, shape, op, precision):
+    """What a call takes: dcg_conv_form, whether a second launch adds the K partitions, how many those are."""
+    import ctypes
+    N, H, W, C, K, O, s = shape
+    kh, kw = K if isinstance(K, tuple) else (K, K)
+    d, form, plan = pkg.functional.conv_desc((N, H, W, C), (kh, kw, C, O), (s, s)), (ctypes.c_int * 4)(), (ctypes.c_int * 6)()
+    kind = {"fwd": pkg._lib.KIND_FWD, "dx": pkg._lib.KIND_DX, "dk": pkg._lib.KIND_DK}[op]
+    if pkg.lib.dcg_debug_conv_form(ctypes.byref(d), kind, precision, form) or pkg.lib.dcg_debug_conv_plan(ctypes.byref(d), kind, precision, plan):
+        return None
+    return form[0], form[1], plan[2]
+
+
 # kernel gradients of few tiles, whose partitions a second launch adds: one tap and nine, four taps to a tile, the channel
 # roles swapped, ragged channels, a last partition tile that is nearly empty
 @pytest.mark.parametrize("prec_name", ["tf32", "3xtf32"])
 @pytest.mark.parametrize("shape", [(4, 60, 60, 64, 1, 128, 1), (8, 40, 40, 32, 3, 64, 1), (6, 64, 64, 256, 1, 64, 1), (16, 50, 50, 40, 3, 44, 1),
-                                   (20, 64, 64, 8, 1, 16, 1), (13, 75, 51, 96, 3, 160, 1), (5, 61, 47, 132, 1, 260, 2)])
+                                   (20, 64, 64, 8, 1, 16, 1), (13, 75, 51, 96, 3, 160, 1), (5, 61, 47, 132, 1, 260, 2), (9, 61, 47, 100, 1, 132, 2)])
 def test_kernel_gradients_of_many_partitions(pkg, dev, shape, prec_name):
     import ctypes
     F, L = pkg.functional, pkg.lib
     N, H, W, C, K, O, s = shape
     prec = getattr(pkg, PRECS[prec_name])
+    # (two of them stay with a cluster at one of the precisions)
+    if (C, prec_name) not in ((132, "tf32"), (96, "3xtf32")):
+        assert _form(pkg, shape, "dk", prec)[:2] == (0, 1) and _form(pkg, shape, "dk", prec)[2] > 8
     x, dy = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in ((57, (N, H, W, C)), (58, (N, -(-H // s), -(-W // s), O))))
     pt, pl = (max((-(-e // s) - 1) * s + K - e, 0) for e in (H, W))
     xp = torch.nn.functional.pad(x.double().permute(0, 3, 1, 2), (pl // 2, pl - pl // 2, pt // 2, pt - pt // 2))
@@ -582,13 +597,19 @@ def test_kernel_gradients_of_many_partitions(pkg, dev, shape, prec_name):
 # per kernel row, even and odd pixel distances, tiles of several images, one and many tiles per CTA, one to four column slabs
 @pytest.mark.parametrize("shape", [(1, 64, 64, 3, 5, 64, 2), (130, 64, 64, 3, 5, 64, 2), (3, 63, 61, 3, 5, 32, 2), (4, 20, 20, 1, 5, 32, 2),
                                    (6, 40, 30, 3, 3, 96, 1), (2, 50, 64, 2, 4, 128, 2), (3, 17, 19, 3, 7, 64, 1), (40, 9, 7, 3, 3, 32, 1),
-                                   (2, 40, 200, 3, 5, 64, 1), (1, 5, 5, 3, 5, 64, 2), (9, 30, 28, 4, 8, 32, 2), (2, 64, 64, 3, 1, 64, 1)])
+                                   (2, 40, 200, 3, 5, 64, 1), (1, 5, 5, 3, 5, 64, 2), (9, 30, 28, 4, 8, 32, 2), (2, 64, 64, 3, 1, 64, 1),
+                                   (3, 40, 38, 3, (3, 7), 64, 2), (5, 33, 40, 3, (4, 7), 32, 1), (2, 50, 64, 4, (2, 5), 128, 2), (9, 24, 20, 3, (3, 8), 96, 1),
+                                   (3, 21, 23, 3, (3, 6), 64, 1), (70, 40, 40, 3, (4, 7), 32, 2), (20, 64, 64, 4, 5, 64, 2)])
 def test_forward_of_rgb_layers(pkg, dev, shape):
     F = pkg.functional
     N, H, W, C, K, O, s = shape
+    kh, kw = K if isinstance(K, tuple) else (K, K)
+    # two whole operand tiles of every kernel row have to fit: 7 x 7 x 3, 8 x 8 x 4 and 5 x 5 x 4 keep the window form
+    kernel = {(7, 3): 0, (8, 4): 0, (5, 4): 5}.get((K, C), 2)
+    assert _form(pkg, shape, "fwd", pkg.PREC_TF32)[0] == kernel
     ho, wo = -(-H // s), -(-W // s)
     x, k, bias, gate = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
-                        ((61, (N, H, W, C)), (62, (K, K, C, O)), (63, (O,)), (64, (N, ho, wo, O))))
+                        ((61, (N, H, W, C)), (62, (kh, kw, C, O)), (63, (O,)), (64, (N, ho, wo, O))))
     ref = F.conv2d_fwd(x, k, (s, s), precision=pkg.PREC_FP32)
     tol = TF32_TOL * ref.abs().max().item()
     assert (F.conv2d_fwd(x, k, (s, s)) - ref).abs().max().item() <= tol
@@ -663,6 +684,10 @@ def test_more_tiles_than_sms(pkg, dev, shape):
     ho, wo = -(-H // s), -(-W // s)
     x, k, dy, bias, gate = (torch.from_numpy(seeded(t, i)).to(dev) for i, t in
                             ((65, (N, H, W, C)), (66, (K, K, C, O)), (67, (N, ho, wo, O)), (68, (O,)), (69, (N, H, W, C))))
+    pkg.lib.dcg_debug_set_dx_mode(0)
+    forms = [_form(pkg, shape, op, pkg.PREC_TF32) for op in ("fwd", "dx")]
+    pkg.lib.dcg_debug_set_dx_mode(-1)
+    assert forms == [(1, 0, 1) if C % 4 == 0 else None, (1, 0, 1)]   # (forwards of 6 channels are on the CUDA cores)
     pre = [torch.empty((N, ho, wo, O), device=dev) for _ in range(2)]
     results = []
     pkg.lib.dcg_debug_set_dx_mode(0)
@@ -819,7 +844,10 @@ def test_bounded_wait_runs_out_and_the_context_survives(pkg, dev):
 
 
 # one stage of the pipeline never comes: kernel (dcg_conv_form), operator, precision, shape (n, h, w, c, k, o, s), the stage
-GIVE_UP = [(2, "fwd", "tf32", (64, 64, 64, 3, 5, 64, 2), 1)]
+GIVE_UP = [(2, "fwd", "tf32", (64, 64, 64, 3, 5, 64, 2), 1), (1, "fwd", "tf32", (80, 32, 32, 32, 5, 64, 2), 3),
+           (1, "dx", "tf32", (37, 60, 60, 20, 1, 64, 1), 1), (0, "fwd", "tf32", (8, 48, 48, 64, 3, 128, 1), 3),
+           (0, "dx", "tf32", (8, 48, 48, 64, 3, 128, 1), 3), (0, "fwd", "3xtf32", (8, 48, 48, 64, 3, 128, 1), 3),
+           (0, "fwd", "3xtf32", (80, 32, 32, 32, 5, 64, 2), 9)]
 
 
 @pytest.mark.parametrize("form,op,prec_name,shape,stage", GIVE_UP)

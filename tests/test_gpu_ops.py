@@ -131,6 +131,44 @@ def test_colsum_order_of_additions(pkg, dev, cols):
         assert np.array_equal(got, _column_sums_in_order(a, sms)), (rows, cols)
 
 
+# more than sixteen groups of sixteen slabs, whose sums a lane adds with four sums that take turns: 8, 16 and 256 lanes, a last
+# slab and a last group that are short, rows that are no float4s
+@pytest.mark.parametrize("rows,cols", [(65536, 64), (49725, 160), (40000, 128), (300001, 10), (524288, 4), (262144, 64)])
+def test_colsum_order_of_many_slabs(pkg, dev, rows, cols):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    a = seeded((rows, cols), 517)
+    groups = cols // 4 if cols % 4 == 0 else cols
+    tx = 1
+    while tx < 32 and tx < groups:
+        tx *= 2
+    lanes, tiles = 256 // tx, -(-groups // tx)
+    per_slab = -(-rows // max(1, min(-(-4 * sms // tiles), 1008, -(-rows // (4 * lanes)))))
+
+    def tree(r):   # one slab
+        acc, h = np.zeros((lanes, cols), np.float32), lanes // 2
+        for i in range(0, len(r), lanes):
+            acc[:len(r[i:i + lanes])] += r[i:i + lanes]
+        while h:
+            acc[:h] += acc[h:2 * h]
+            h //= 2
+        return acc[0].copy()
+
+    def in_turns(r):   # lane l: rows l, l + lanes, ... in four sums; then the lanes in order
+        t = np.zeros((4, lanes, cols), np.float32)
+        for n, i in enumerate(range(0, len(r), lanes)):
+            t[n & 3, :len(r[i:i + lanes])] += r[i:i + lanes]
+        acc = (t[0] + t[1]) + (t[2] + t[3])
+        total = acc[0].copy()
+        for lane in acc[1:]:
+            total += lane
+        return total
+
+    slabs = np.stack([tree(a[r:r + per_slab]) for r in range(0, rows, per_slab)])
+    assert len(slabs) > 256 and tiles <= 16
+    ref = in_turns(np.stack([in_turns(slabs[g:g + 16]) for g in range(0, len(slabs), 16)]))
+    assert np.array_equal(pkg.functional.colsum(_t(a, dev)).cpu().numpy(), ref)
+
+
 def test_golden_small_ops(pkg, dev, golden):
     """The reference's unit-test tensors for bias add, activation gradients, losses, argmax."""
     L, g = pkg.lib, golden
