@@ -284,7 +284,11 @@ constexpr int kMaxSharedWidth = 160;
 // `partials_bytes` (kernel gradients): partial tiles that a second launch adds may take so much scratch.  A tile then has as many
 // partitions as fill the SMs, not the eight CTAs of a cluster: the launch costs about 4 us, which long reductions over few tiles
 // earn many times over (1 x 1, 8 -> 16 channels, 20 images of 64 x 64: 46 us in one cluster of eight, 10.4 in 148 partitions;
-// 3 x 3, 96 -> 160, 13 images of 75 x 51: 49 and 30; 64 -> 128 of 64 images, 3xTF32: 53 and 42).
+// 3 x 3, 96 -> 160, 13 images of 75 x 51: 49 and 30; 64 -> 128 of 64 images, 3xTF32: 53 and 42).  Its price in the model, 6500 clocks and
+// one per 2500 bytes, leaves the line where it pays: of ninety layers drawn at random (1 x 1 to 5 x 5, 8 to 256 channels, up to 40 GFLOP)
+// it is chosen for 22 in TF32, nineteen of them 7 % to 2.7 times quicker than the cluster and three 1, 3 and 10 % slower (1 x 1,
+// 32 -> 128, 39 images of 8 x 38: 8.7 and 9.7), and for 45 in 3xTF32, all of them 1.1 to 6.9 times quicker.  Of the 42 that keep the
+// cluster in TF32 half are quicker so (down to 0.77); eleven would gain 8 to 26 %.
 struct Tiling {
     int bn, n_tiles, splits, grid;
     bool second_launch, walk;
@@ -590,8 +594,10 @@ QueryKey query_key(const dcg_conv_desc& d, int kind, bool x3)
 // the class-fused kernel, a stage of the other one 300 at 128 columns and 512 at 256; a column of a class costs an epilogue 20,
 // of which half of the shorter of loop and epilogue is hidden.  The class-fused tiles are four times as large, in boxes of powers
 // of two and of at most 128 columns, which leaves much of them empty where the image, the channels or the last wave do not fit: 3 x 3 /
-// stride 2, 192 -> 64, 30 images of 33 x 47 27.0 us fused, 13.6 apart; 192 -> 192, 32 images of 96 x 96 165 and 111.
-// Where they fit, fused is quicker (5 x 5 / stride 2, 64 -> 128 of 64 images 16.4 and 22.2, 256 -> 512 of 512 images 74 and 90).
+// stride 2, 192 -> 64, 30 images of 33 x 47 26.7 us fused, 13.4 apart; 192 -> 192, 32 images of 96 x 96 165 and 109.
+// Where they fit, fused is quicker (5 x 5 / stride 2, 64 -> 128 of 64 images 15.6 and 21.0, 256 -> 512 of 512 images 69 and 81).
+// The factor of 0.9 keeps the line on the safe side: of seventy layers drawn at random with twenty for which both are possible,
+// apart is chosen for eighteen, all of them quicker so (0.39 to 0.98 of the fused time), and not for two that would take 0.84 and 0.87.
 bool classes_apart_modelled(const dcg_conv_desc& d, int tiles, int bn, int ncls)
 {
     Plan apart;

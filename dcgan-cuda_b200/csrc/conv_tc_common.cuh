@@ -77,7 +77,7 @@ struct Params {
     int m_tiles;                  // DK: 128-row tiles along the M channel axis
     int n_tiles;                  // BN-column tiles along the N channel axis
     int bn;                       // accumulator columns, multiple of 16, <= 256
-    int splits;                   // K partitions of a tile = CTAs per cluster (<= 8)
+    int splits;                   // K partitions of a tile: CTAs per cluster (<= 8), or, with ext_finish, up to as many as there are SMs
     int skip_stage;               // test hook: the producer leaves this pipeline stage out (-1: never)
     long long wait_cycles;        // SM clocks after which a barrier wait gives up
     int kchunks;                  // 32-wide chunks along the contracted channel axis (FWD: C, DX: O)
@@ -87,7 +87,7 @@ struct Params {
     int swap;                     // DK: M axis is o (A from dy, B from x)
     int narrow;                   // FWD/DK with <= 4 input channels: x is read through the window map
     int walk;                     // more tiles than SMs, walked by persistent CTAs (conv_tc_walk_kernel)
-    int ext_finish;               // the K partitions only write partials; a second kernel adds them (narrow DK)
+    int ext_finish;               // DK: the K partitions only write partials; a second kernel adds them
     int planes;                   // FWD: 16-byte column quad q of output pixel r goes to out[(q * pixels + r) * 4]
     int o_store;                  // FWD: output columns >= o_store are padding and never stored (0: store all O)
     int b_direct;                 // short-K GEMM: B is read from k itself, K-major (row = 4 * tap + channel, 32 o per row)

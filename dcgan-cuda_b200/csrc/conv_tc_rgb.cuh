@@ -12,6 +12,9 @@ namespace {
 // core: 16 (or 32) places per kernel row, of which KW * C are used; the weights come in the same order from where they are.
 // Persistent, one CTA per SM: the patches of the next tiles are copied, and the next rows built, while this tile's products and
 // its epilogue run (two operand tiles, two accumulators).
+// An operand tile holds all kernel rows, which limits the layers: rows of up to 16 values (KW * C) up to 5 x 5 with three channels or
+// 4 x 4 with four (with a stride and 96 or 128 outputs 5 x 5 x 3 only over small images), rows of more than 16 values only up to four of
+// them.  The others - 5 x 5 x 4, 6 x 6 x 3, 7 x 7 x 3 - keep the two launches.
 // What bounds it is the shared-memory pipe: a tile of 5 x 5 x 3 -> 64 is 800 clocks of building (8-byte reads of a lane, which a
 // lane stride of an even number of floats spreads over all banks, and one 16-byte store per four places) and 256 clocks to
 // stage the output, which TMA stores.  (Rows without places between them, element by element through a table: 2300 clocks; the

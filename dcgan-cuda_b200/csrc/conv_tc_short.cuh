@@ -5,8 +5,8 @@ namespace dcg {
 namespace {
 
 // ---- short-K forward GEMMs as persistent CTAs ---------------------------------------------------------
-// For the 3-channel layers that conv_fwd_rgb_kernel (large strides: the patch under a tile is too large) and
-// conv_dx3_kernel do not take.  Their two tensor-core launches have almost no K: the forward contracts five
+// For the <= 4-channel layers that conv_fwd_rgb_kernel (two operand tiles of all kernel rows and the patches have to fit
+// shared memory: 5 x 5 x 4, 7 x 7 x 3 and large strides do not) and conv_dx3_kernel do not take.  Their two tensor-core launches have almost no K: the forward contracts five
 // 32-float row windows per tile (A through the overlapping-window map, B = k4), the GEMM of the input
 // gradient two 32-channel chunks (a 1x1 convolution of dy against all taps, result in quad planes).
 // With one tile per CTA such a CTA spends its life on set-up, pipeline fill and epilogue (2-5 stages

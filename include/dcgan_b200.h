@@ -137,7 +137,8 @@ int dcg_act_grad(const float* gate, const float* dout, float* out, size_t n,
 
 /* out[c] = sum_r a[r, c]: the conv/dense bias gradient.
  * Replaces gpu::kernel_mat_sum_cols (src/gpu/sum.cu:111-151,238-243).
- * workspace: dcg_colsum_workspace_bytes(rows, cols) bytes (may be 0). */
+ * workspace: dcg_colsum_workspace_bytes(rows, cols) bytes (may be 0).  For shapes of many rows that is a little more
+ * than the partial sums take (a row per sixteen of them, and 4 KB), so that sizes laid out once stay valid. */
 size_t dcg_colsum_workspace_bytes(size_t rows, size_t cols);
 int dcg_colsum(const float* a, float* out, size_t rows, size_t cols,
                void* workspace, size_t workspace_bytes, dcg_stream_t stream);
